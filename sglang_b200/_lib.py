@@ -72,6 +72,14 @@ for _name, (_res, _args) in SIGNATURES.items():
     _fn.restype = _res
     _fn.argtypes = _args
 
+try:
+    from . import _host as host  # the native host path of the hot entry points (csrc/host.cpp)
+except ImportError as e:
+    raise ImportError(f"sglang_b200._host is missing or does not match this torch ({e}): build it with "
+                      "`python -m sglang_b200.build`") from e
+
+host.bind(LIB_PATH)
+
 
 def check(rc: int) -> None:
     """Turn a non-zero return code of the C ABI into the exception the reference op would raise."""

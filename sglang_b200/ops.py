@@ -11,7 +11,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from ._lib import check, lib
+from ._lib import check, host, lib
 
 FP8 = torch.float8_e4m3fn
 FP8_MAX = 448.0
@@ -82,6 +82,9 @@ def per_token_group_quant_fp8(
     x: torch.Tensor, group_size: int = 128, eps: float = 1e-10, column_major_scales: bool = False,
     scale_tma_aligned: bool = False,
 ) -> Tuple[torch.Tensor, torch.Tensor]:
+    out = host.quant(x, group_size, eps, column_major_scales, scale_tma_aligned)
+    if out is not None:
+        return out
     x_q = torch.empty_like(x, dtype=FP8)
     tokens = x.numel() // x.shape[-1]
     groups = x.shape[-1] // group_size
@@ -115,6 +118,9 @@ def silu_and_mul_quant_fp8(
 ) -> Tuple[torch.Tensor, torch.Tensor]:
     """[rows, 2d] -> (codes [rows, d], scales [rows, d/group]).  `num_rows` (device int32 scalar)
     limits the rows processed; the remaining rows of the outputs are left untouched."""
+    out = host.silu_mul_quant(x, group_size, eps, num_rows)
+    if out is not None:
+        return out
     _cuda_contig(x, "input")
     d = x.shape[-1] // 2
     rows = x.numel() // x.shape[-1]
@@ -249,6 +255,10 @@ def topk_sigmoid_out(topk_weights, topk_ids, gating, renormalize=False, correcti
 def moe_fused_gate(input: torch.Tensor, bias: torch.Tensor, num_expert_group: int, topk_group: int, topk: int,
                    num_fused_shared_experts: int = 0, routed_scaling_factor: float = 0.0,
                    apply_routed_scaling_factor_on_output: bool = False):
+    out = host.fused_gate(input, bias, num_expert_group, topk_group, topk, num_fused_shared_experts,
+                          routed_scaling_factor, bool(apply_routed_scaling_factor_on_output))
+    if out is not None:
+        return out
     _cuda_contig(input, "input")
     _cuda_contig(bias, "bias")
     if input.dim() != 2 or bias.numel() != input.shape[1] or bias.dtype != input.dtype:
@@ -362,6 +372,9 @@ def w8a8_block_fp8_matmul(
     """A [..., K] e4m3, B [N, K] e4m3, As [..., ceil(K/128)] f32 (any strides), Bs [ceil(N/128), ceil(K/128)] f32."""
     if list(block_size) != [128, 128]:
         raise RuntimeError("only block_size [128, 128] is supported")
+    C = host.matmul(A, B, As, Bs, output_dtype, bias)
+    if C is not None:
+        return C
     _cuda_contig(A, "A")
     _cuda_contig(B, "B")
     if A.dtype != FP8 or B.dtype != FP8:

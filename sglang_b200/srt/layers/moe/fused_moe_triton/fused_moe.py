@@ -88,11 +88,16 @@ def fused_experts_impl(
     else:
         out = torch.empty((num_tokens, w2.shape[1]), device=hidden_states.device, dtype=act_dtype)
 
+    # the plain form (16-bit activations, every id local, summed over the slots) is one native call per chunk
+    native = not (prequant or no_combine or apply_router_weight_on_input or has_filtered_ids)
     for begin in range(0, num_tokens, CHUNK_SIZE):
         end = min(begin + CHUNK_SIZE, num_tokens)
         x = hidden_states[begin:end]
         ids = topk_ids[begin:end].contiguous()
         wts = topk_weights[begin:end].contiguous()
+        if native and _ops.host.fused_experts(x, w1, w1_scale, w2, w2_scale, wts, ids, float(routed_scaling_factor),
+                                              out[begin:end]):
+            continue
         t = end - begin
         numel = t * topk
         if apply_router_weight_on_input:

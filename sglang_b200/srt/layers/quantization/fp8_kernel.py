@@ -49,6 +49,10 @@ def per_token_group_quant_fp8(
     assert x.is_contiguous(), "`x` is not contiguous"
     if dtype != fp8_dtype:
         raise NotImplementedError("only float8_e4m3fn output is on this path")
+    if not scale_ue8m0:
+        out = _ops.host.quant(x, group_size, eps, column_major_scales, scale_tma_aligned)
+        if out is not None:
+            return out
     x_q = torch.empty_like(x, device=x.device, dtype=dtype)
     x_s = create_per_token_group_quant_fp8_output_scale(
         x.shape, x.device, group_size, column_major_scales, scale_tma_aligned, scale_ue8m0

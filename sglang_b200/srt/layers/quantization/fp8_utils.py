@@ -24,6 +24,10 @@ def b200_w8a8_block_fp8_linear(
 ) -> torch.Tensor:
     """Same contract as `triton_w8a8_block_fp8_linear` (fp8_utils.py:306-326), plus the
     pre-quantised input form (`input_scale` given) of the flashinfer/deepgemm variants (:164-194)."""
+    if input_scale is None and block_size[0] == 128 and block_size[1] == 128:
+        output = _ops.host.linear(input, weight, weight_scale, bias)  # quantise and multiply in one native call
+        if output is not None:
+            return output
     input_2d = input.view(-1, input.shape[-1])
     output_shape = [*input.shape[:-1], weight.shape[0]]
     if input_scale is not None:
