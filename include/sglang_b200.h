@@ -187,6 +187,28 @@ int sglb200_moe_sum_reduce(const void* x, void* out, int dtype, int64_t tokens, 
                            float scale, void* stream);
 
 /*
+ * Whole layers in one call, every intermediate in one workspace (size from the query; 16-byte aligned).
+ *
+ * block_fp8_linear: C[M, N] = x[M, K] (bf16 / fp16) x W[N, K]^T, x quantised per 1 x 128 group, in x's type.
+ * Replaces: triton_w8a8_block_fp8_linear (python/sglang/srt/layers/quantization/fp8_utils.py:306-326).  K % 128 == 0;
+ *   otherwise as sglb200_fp8_blockwise_scaled_mm.
+ *
+ * fused_experts: out[t] = factor * sum_j topk_weights[t, j] * expert_{topk_ids[t, j]}(x[t]), an expert being
+ *   w2 x requantise(silu(gate) * up) with [gate; up] = w13 x.  w13 [E, 2I, H], w2 [E, Ho, I] e4m3 with 128 x 128 block
+ *   scales; slots with a negative id add nothing.
+ * Replaces: fused_experts_impl (python/sglang/srt/layers/moe/fused_moe_triton/fused_moe.py:369-667), block-FP8 branch.
+ */
+int64_t sglb200_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
+int sglb200_block_fp8_linear(const void* x, int dtype, const void* W, const float* w_s, void* C, const void* bias, int64_t M,
+                             int64_t N, int64_t K, void* workspace, int64_t workspace_bytes, void* stream);
+int64_t sglb200_fused_experts_workspace_bytes(int64_t tokens, int64_t topk, int num_experts, int64_t hidden,
+                                              int64_t intermediate, int64_t out_hidden, float factor);
+int sglb200_fused_experts(const void* x, int dtype, const void* w13, const float* w13_s, const void* w2, const float* w2_s,
+                          const float* topk_weights, const int32_t* topk_ids, void* out, int64_t tokens, int64_t topk,
+                          int num_experts, int64_t hidden, int64_t intermediate, int64_t out_hidden, float factor,
+                          void* workspace, int64_t workspace_bytes, void* stream);
+
+/*
  * The same sum over the slots k with topk_ids[t, k] >= 0 only ([tokens, topk] int32, ids local to this rank): under
  * expert parallelism the slots of experts that live on other ranks are never written and are skipped here instead
  * of being zero-filled and read.  The reference reaches the same result by writing zeros for filtered experts

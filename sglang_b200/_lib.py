@@ -36,6 +36,10 @@ SIGNATURES = {
     "sglb200_moe_align_block_size_noalloc": (_i32, [_vp, _i64, _i32, _i32, _vp, _vp, _vp, _i32, _vp]),
     "sglb200_moe_sum_reduce": (_i32, [_vp, _vp, _i32, _i64, _i64, _i64, _f32, _vp]),
     "sglb200_moe_sum_reduce_masked": (_i32, [_vp, _vp, _vp, _i32, _i64, _i64, _i64, _f32, _vp]),
+    "sglb200_block_fp8_linear_workspace_bytes": (_i64, [_i64, _i64, _i64]),
+    "sglb200_block_fp8_linear": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _i64, _vp]),
+    "sglb200_fused_experts_workspace_bytes": (_i64, [_i64, _i64, _i32, _i64, _i64, _i64, _f32]),
+    "sglb200_fused_experts": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _i64, _f32, _vp, _i64, _vp]),
     "sglb200_moe_align_drop_filtered": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp]),
     "sglb200_gather_sum_rows": (_i32, [_vp, _vp, _vp, _i32, _i64, _i32, _i64, _i64, _f32, _vp]),
     "sglb200_shuffle_mul_sum": (_i32, [_vp, _vp, _vp, _vp, _i32, _i64, _i32, _i64, _vp]),
@@ -71,6 +75,8 @@ for _name, (_res, _args) in SIGNATURES.items():
     _fn = getattr(lib, _name)  # AttributeError here = the .so is older than the header: rebuild
     _fn.restype = _res
     _fn.argtypes = _args
+
+import torch  # noqa: E402,F401  (its libraries have to be loaded before the module that links against them)
 
 try:
     from . import _host as host  # the native host path of the hot entry points (csrc/host.cpp)

@@ -31,6 +31,23 @@ int fail(int code, const char* fmt, ...);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// A launch that may be scheduled while the kernel before it in the stream is still running (programmatic stream
+// serialization): the kernel has to call griddepcontrol.wait before it touches anything that kernel reads or writes.
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

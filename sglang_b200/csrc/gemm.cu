@@ -44,9 +44,11 @@
 #include <cuda.h>
 
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "common.cuh"
+#include "gemm_common.cuh"
 #include "ptx_sm100.cuh"
 
 namespace sglb200 {
@@ -82,9 +84,6 @@ __device__ long long g_trace[3][kTraceUnits][kTraceStamps];  // [2] = the scout 
 #endif
 
 #define SGLB_WAIT(bar, parity) (p.wait_probes != ptx::kProbesNone && ptx::mbar_wait_quiet(bar, parity))
-#ifndef SGLB_FMA2
-#define SGLB_FMA2 1                        // promotion with packed float32 FMAs (two columns per instruction)
-#endif
 
 // Tile width BN: 192 columns with two TMEM accumulator buffers (the fewest bytes per FLOP from L2 and the fewest
 // tiles: best where there are waves of full tiles), or 128 columns with four buffers (more tiles for the same
@@ -179,18 +178,6 @@ struct SharedCtl {
 struct TileCoord {
   int m_tile, n_tile, expert;
 };
-
-// tile index -> (m_tile, n_tile): groups of `group_m` m-tiles sweep over n together, m fastest inside a group.
-// The activation rows of a group stay in L2 while the weight matrix streams past them once per group.
-__device__ __forceinline__ void tile_coord(int t, int tiles_m, int tiles_n, int group_m, int& m_tile, int& n_tile) {
-  const int per_group = group_m * tiles_n;
-  const int g = t / per_group;
-  const int first_m = g * group_m;
-  const int gsz = min(tiles_m - first_m, group_m);
-  const int r = t - g * per_group;
-  m_tile = first_m + r % gsz;
-  n_tile = r / gsz;
-}
 
 // A unit of work = one output tile x one K range.  Dense problems number their units: the tiles
 // [0, full_units) whole, then `splits` consecutive units per remaining tile.
@@ -640,14 +627,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
             for (int i = 0; i < kPiecesMax; ++i) {
               const float sc = piece_in_blk1[i] ? sc1 : sc0;
-#if SGLB_FMA2
               // two columns per instruction (packed float32 FMA: the same two IEEE operations): half the issue slots
 #pragma unroll
               for (int jj = 0; jj < 32; jj += 2) ptx::fma2(acc[32 * i + jj], acc[32 * i + jj + 1], r[i][jj], r[i][jj + 1], sc);
-#else
-#pragma unroll
-              for (int jj = 0; jj < 32; ++jj) acc[32 * i + jj] = fmaf(__uint_as_float(r[i][jj]), sc, acc[32 * i + jj]);
-#endif
             }
           }
           if (++buf == (uint32_t)kAccBufs) {
@@ -1006,9 +988,7 @@ struct MapKeyHash {
   }
 };
 
-// uint8 tensor [d2][d1][d0] (d0 contiguous) described with `rank` (2 or 3) dimensions,
-// box = 128 x box_rows (x 1), 128-byte swizzle, out-of-range elements read as zero.
-static int get_tensor_map(const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_rows, uint32_t rank,
+int get_tensor_map(const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_rows, uint32_t rank,
                           CUtensorMap* out) {
   static thread_local std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   const MapKey key{ptr, d0, d1, d2, box_rows, rank};
@@ -1060,7 +1040,7 @@ static int get_out_map(const void* ptr, uint64_t N, uint64_t rows, int out_fp16,
 // m-tiles per rasterization group: as many as keep the group's activation rows (128*K bytes per m-tile) within
 // a quarter of the L2 (measured: with half of it the streaming weight tiles start evicting the rows), in groups
 // of equal size, so that the weights are read from DRAM once per group and the activations once in all.
-static int choose_group_m(int64_t rows, int64_t K, int tile_rows = BM) {
+int choose_group_m(int64_t rows, int64_t K, int tile_rows) {
   const int64_t budget = 32ll << 20;
   int64_t gmax = budget / (tile_rows * K);
   if (gmax < 2) gmax = 2;
@@ -1074,11 +1054,7 @@ static int choose_group_m(int64_t rows, int64_t K, int tile_rows = BM) {
 // makes several waves, it wins: fewer tiles, fewer bytes per FLOP, and at large M the 128-wide tile runs at about
 // 0.85 of its rate.  Where one wave of 192-wide tiles leaves SMs idle and K is not split, the 128-wide tile's
 // extra tiles fill them.  Compared as waves x tile width, the 128-wide tile charged 150 instead of 128.
-#ifndef SGLB_FORCE_BN
-#define SGLB_FORCE_BN 0  // 128 or 192: one tile width for everything (measurements)
-#endif
 static int choose_bn(int64_t M, int64_t N, int64_t K) {
-  if (SGLB_FORCE_BN) return SGLB_FORCE_BN;
   const int sms = sm_count();
   const UnitPlan p192 = plan_units(M, N, K, 192, BM, sms);
   if (p192.scratch_blocks() > 0) return 192;
@@ -1090,7 +1066,6 @@ static int choose_bn(int64_t M, int64_t N, int64_t K) {
 // The expert-grouped form: rows per expert are not known on the host; with a handful of routed rows (decode) the
 // 128-wide tile spreads the few row blocks over more SMs, otherwise the 192-wide tile is ahead by 5-10 %.
 static int choose_bn_grouped(int64_t numel) {
-  if (SGLB_FORCE_BN) return SGLB_FORCE_BN;
   return numel <= 64 ? 128 : 192;
 }
 
@@ -1107,7 +1082,13 @@ static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
   return d;
 }
 
-static uint32_t g_wait_probes = ptx::kProbeLimit;  // sglb200_gemm_set_wait_probes
+// Few activation rows take the kernel with the weights on the M side (gemm_rows.cu): up to 64 rows its tiles follow the
+// rows there are, beyond that this kernel's 128-row tiles are at least half full.
+static bool use_rows(int64_t M) {
+  return M <= 64;
+}
+
+uint32_t g_gemm_wait_probes = ptx::kProbeLimit;
 
 template <class Cfg>
 static size_t gemm_smem_bytes() {
@@ -1153,7 +1134,7 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
   p.tiles_n = (int)((N + BN - 1) / BN);
   p.group_m = choose_group_m(M, K, kTileRows);
   p.out_fp16 = out_dtype;
-  p.wait_probes = g_wait_probes;
+  p.wait_probes = g_gemm_wait_probes;
   UnitPlan pl = dp.units;
   const int64_t tiles = ((M + kTileRows - 1) / kTileRows) * p.tiles_n;
   if (pl.scratch_blocks() > 0 &&
@@ -1225,10 +1206,10 @@ static int grouped_mm(const void* A, const float* a_s, const void* B, const floa
   p.M = max_rows, p.N = N, p.K = K;
   p.kb_total = (int)((K + BK - 1) / BK), p.nb_total = (int)((N + kScaleBlockN - 1) / kScaleBlockN);
   p.tiles_n = (int)((N + BN - 1) / BN);
-  p.group_m = choose_group_m(max_rows, K);
+  p.group_m = choose_group_m(max_rows, K, BM);
   p.as_stride_m = p.kb_total, p.as_stride_k = 1;
   p.numel = numel, p.scatter = scatter, p.out_fp16 = out_dtype;
-  p.wait_probes = g_wait_probes;
+  p.wait_probes = g_gemm_wait_probes;
   p.full_units = 0, p.splits = 1, p.kb_per_split = p.kb_total, p.partial = nullptr;  // grouped: one unit per tile
   p.sk_pieces = 2;
   CUtensorMap mc{};
@@ -1248,19 +1229,19 @@ using namespace sglb200;
 extern "C" int sglb200_gemm_status_clear(void) {
   const int zero = 0;
   SGLB_CUDA(cudaMemcpyToSymbol(g_gemm_status, &zero, sizeof(int)));
-  return SGLB200_OK;
+  return rows_gemm_status_clear();
 }
 
 extern "C" int sglb200_gemm_status(void) {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, g_gemm_status, sizeof(int)) != cudaSuccess) return -1;
-  return v;
+  return v != 0 ? v : rows_gemm_status();
 }
 
-extern "C" void sglb200_gemm_set_wait_probes(uint32_t probes) { g_wait_probes = probes == 0 ? ptx::kProbeLimit : probes; }
+extern "C" void sglb200_gemm_set_wait_probes(uint32_t probes) { g_gemm_wait_probes = probes == 0 ? ptx::kProbeLimit : probes; }
 
 extern "C" int64_t sglb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || use_rows(M)) return 0;
   return plan_dense(M, N, K).scratch_bytes();
 }
 
@@ -1268,6 +1249,13 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm(const void* A, const void* B, con
                                                void* C, const void* bias, int64_t M, int64_t N, int64_t K,
                                                int64_t as_stride_m, int64_t as_stride_k, int out_dtype,
                                                void* workspace, int64_t workspace_bytes, void* stream) {
+  return scaled_mm(A, B, a_s, b_s, C, bias, M, N, K, as_stride_m, as_stride_k, out_dtype, workspace, workspace_bytes, false,
+                   static_cast<cudaStream_t>(stream));
+}
+
+int sglb200::scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
+                       int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, void* workspace,
+                       int64_t workspace_bytes, bool after_quantizer, cudaStream_t st) {
   SGLB_REQUIRE(M >= 0 && N > 0 && K > 0, "fp8_blockwise_scaled_mm: bad shape M=%lld N=%lld K=%lld", (long long)M,
                (long long)N, (long long)K);
   SGLB_REQUIRE(K % 16 == 0, "fp8_blockwise_scaled_mm: K=%lld must be a multiple of 16", (long long)K);
@@ -1279,7 +1267,8 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm(const void* A, const void* B, con
   SGLB_REQUIRE(aligned16(A) && aligned16(B) && aligned16(C) && (bias == nullptr || aligned16(bias)),
                "fp8_blockwise_scaled_mm: A, B, C and bias must be 16-byte aligned");
   SGLB_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "fp8_blockwise_scaled_mm: dimension too large");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (use_rows(M))
+    return rows_dense_mm(A, B, a_s, b_s, C, bias, M, N, K, as_stride_m, as_stride_k, out_dtype, after_quantizer, st);
   const DensePlan dp = plan_dense(M, N, K);
   if (dp.bn == 128)
     return dense_mm<128>(dp, A, B, a_s, b_s, C, bias, M, N, K, as_stride_m, as_stride_k, out_dtype, workspace,
@@ -1377,7 +1366,7 @@ static int push_mm(const void* A, const void* B, const float* a_s, const float* 
   p.tiles_n = (int)((N + BN - 1) / BN);
   p.group_m = choose_group_m(M, K, kTileRows);
   p.out_fp16 = out_dtype;
-  p.wait_probes = g_wait_probes;
+  p.wait_probes = g_gemm_wait_probes;
   const int64_t tiles = ((M + kTileRows - 1) / kTileRows) * p.tiles_n;
   p.full_units = (int)tiles, p.splits = 1, p.kb_per_split = p.kb_total, p.partial = nullptr;  // one unit per tile
   p.sk_pieces = 2;

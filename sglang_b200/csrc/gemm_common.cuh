@@ -1,0 +1,52 @@
+// What the block-scaled GEMM kernels share: rasterization, TMA descriptors, the pipeline-wait setting.
+#pragma once
+#include <cuda.h>
+
+#include "common.cuh"
+
+namespace sglb200 {
+
+// tile index -> (m_tile, n_tile): groups of `group_m` m-tiles sweep over n together, m fastest inside a group.
+// The activation rows of a group stay in L2 while the weight matrix streams past them once per group.
+__device__ __forceinline__ void tile_coord(int t, int tiles_m, int tiles_n, int group_m, int& m_tile, int& n_tile) {
+  const int per_group = group_m * tiles_n;
+  const int g = t / per_group;
+  const int first_m = g * group_m;
+  const int gsz = min(tiles_m - first_m, group_m);
+  const int r = t - g * per_group;
+  m_tile = first_m + r % gsz;
+  n_tile = r / gsz;
+}
+
+// uint8 tensor [d2][d1][d0] (d0 contiguous) described with `rank` (2 or 3) dimensions, box = 128 x box_rows (x 1),
+// 128-byte swizzle, out-of-range elements read as zero.  Cached per argument tuple and thread.
+int get_tensor_map(const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_rows, uint32_t rank, CUtensorMap* out);
+
+// m-tiles per rasterization group for rows of K bytes (see gemm.cu).
+int choose_group_m(int64_t rows, int64_t K, int tile_rows);
+
+extern uint32_t g_gemm_wait_probes;  // probes after which a pipeline wait gives up (sglb200_gemm_set_wait_probes)
+
+// gemm.cu: the dense product (arguments as sglb200_fp8_blockwise_scaled_mm).  `after_quantizer`: the kernel before it in
+// the stream is this library's quantizer, launched by the same call, so that the weights may be fetched while that runs.
+int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M, int64_t N,
+              int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, void* workspace, int64_t workspace_bytes,
+              bool after_quantizer, cudaStream_t st);
+
+// gemm_rows.cu: the dense product for few activation rows, and the expert-grouped one on rows sorted with a padding of
+// 16 (`cumsum` = padded starts of the buckets, as the sort writes them; bucket 0 = filtered ids is skipped).
+// `gather_topk` > 0: A and a_s have a row per token, fetched by sorted slot / gather_topk; 0: a row per sorted row.
+// `nt` = activation rows per tile: 16, 32, 64 or 128.
+int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
+                  int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, bool after_quantizer,
+                  cudaStream_t st);
+int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const float* a_s, const void* B, const float* b_s, void* C,
+                    const int32_t* cumsum, const int32_t* sorted_ids, const float* row_weights, int64_t max_rows,
+                    int64_t numel, int num_experts, int64_t N, int64_t K, int gather_topk, int scatter, int out_dtype, int nt,
+                    bool pdl, cudaStream_t st);
+
+// gemm_rows.cu: status word of its kernels (0 ok, 1 a wait expired, -1 not readable), and its reset.
+int rows_gemm_status();
+int rows_gemm_status_clear();
+
+}  // namespace sglb200

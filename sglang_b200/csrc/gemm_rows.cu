@@ -1,0 +1,580 @@
+// Block-scaled FP8 GEMM for few activation rows per weight matrix (dense decode, experts with some rows each).
+//
+//   C[m,n] = out_t( sum_kb a_s[m,kb] * b_s[n/128,kb] * sum_{k in kb} A[m,k] * B[n,k] )      (as in gemm.cu)
+//
+// gemm.cu puts 128 activation rows on the lanes of the accumulator; with 1 to 64 rows most of what it stages, multiplies
+// and promotes is padding, and its tiles are wide, so a weight matrix makes few of them.  Here the operands trade
+// places: 128 WEIGHT rows are the M side of the tcgen05.mma, the activation rows are its N side, which comes in steps
+// of 16.  A tile of the accumulator is 128 weight rows (lanes) x up to NT activation rows (columns), and the work per
+// tile (staged bytes, MMA, promotion) follows the rows it has, rounded up to 16, chosen per tile at run time.
+//
+// What bounds it: HBM, as the weights are read once and everything else is small.  So the design is about bytes in
+// flight and about having none of the SMs wait: two CTAs per SM (NT <= 64) with about 100 KB of ring each, the
+// producer running ahead over tile boundaries, and K split over the CTAs of a thread-block cluster where a matrix has
+// fewer tiles than the GPU has CTA slots; the cluster adds its partial sums through distributed shared memory in
+// ascending K order, without a second kernel.  Launched after the quantizer with programmatic serialization, the
+// producer fetches its first weight tiles while the quantizer still runs.
+//
+// Roles (one CTA): warp 0 issues the TMA loads (all lanes: one box of 16 rows, or one gather of 4 rows, per lane and
+// slab), warp 1 issues the MMAs, warp 2 prepares the scales (a_s * b_s of eight slabs at a time, one product per
+// column, in shared memory), warps 4.. promote: TMEM -> registers, acc += partial * scale, then store.
+// Every mbarrier wait is bounded as in gemm.cu (status word, no trap).
+#include <cuda.h>
+
+#include "common.cuh"
+#include "gemm_rows.cuh"
+
+namespace sglb200 {
+
+template <int NT_, int kPromoWarps_, int kStages_, int kAccBufs_, int kCtasPerSm_>
+struct RowsCfg {
+  static constexpr int NT = NT_, kPromoWarps = kPromoWarps_, kStages = kStages_, kAccBufs = kAccBufs_,
+                       kCtasPerSm = kCtasPerSm_;
+  static constexpr int kThreads = 128 + kPromoWarps * 32;
+  static constexpr int kColGroups = kPromoWarps / 4;      // promotion warps per TMEM lane quadrant
+  static constexpr int kWarpCols = NT / kColGroups;       // columns one promotion warp owns
+  static constexpr int kCW = kWarpCols < 32 ? kWarpCols : 32;  // columns per tcgen05.ld
+  static constexpr int kChunks = kWarpCols / kCW;         // chunk i of group h: columns (h + i * kColGroups) * kCW ..
+  static constexpr uint32_t kStageBytes = kWBytes + NT * kRowsBK;
+  static constexpr int kTmemCols = kAccBufs * NT;
+  static_assert((kTmemCols & (kTmemCols - 1)) == 0 && kTmemCols >= 32 && kTmemCols * kCtasPerSm <= 512, "TMEM columns");
+  static_assert(NT % 16 == 0 && kStageBytes % 1024 == 0, "tile layout");
+};
+using Rows16 = RowsCfg<16, 4, 6, 8, 2>;
+using Rows32 = RowsCfg<32, 4, 5, 8, 2>;
+using Rows64 = RowsCfg<64, 4, 4, 4, 2>;
+using Rows128 = RowsCfg<128, 8, 6, 4, 1>;
+
+template <class Cfg>
+struct RowsCtl {
+  uint64_t full[Cfg::kStages], empty[Cfg::kStages];
+  uint64_t tmem_full[Cfg::kAccBufs], tmem_empty[Cfg::kAccBufs];
+  uint64_t sc_full[2], sc_empty[2];
+  uint32_t tmem_base;
+  int abort_flag;
+  int warp_sum[32];
+  alignas(16) float sc[2][kScBatch][Cfg::NT];  // a_s * b_s per slab and column
+  // (grouped: followed by tiles_before[experts + 1], the token tiles of the experts before e)
+};
+
+__device__ int g_rows_status = 0;  // 0 ok, 1 = a pipeline wait expired
+
+template <class Cfg, bool kGrouped>
+__global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
+    fp8_rows_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
+                         const RowsParams p) {
+  constexpr int NT = Cfg::NT, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs, kCW = Cfg::kCW, kChunks = Cfg::kChunks;
+  constexpr uint32_t kStageBytes = Cfg::kStageBytes;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  RowsCtl<Cfg>* ctl = reinterpret_cast<RowsCtl<Cfg>*>(tiles + kStages * kStageBytes);
+  int* tiles_before = reinterpret_cast<int*>(ctl + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  volatile int* abort_flag = &ctl->abort_flag;
+
+  ptx::launch_dependents();
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      ptx::mbar_init(ptx::smem_u32(&ctl->full[s]), 1);
+      ptx::mbar_init(ptx::smem_u32(&ctl->empty[s]), 1);
+    }
+    for (int b = 0; b < kAccBufs; ++b) {
+      ptx::mbar_init(ptx::smem_u32(&ctl->tmem_full[b]), 1);
+      ptx::mbar_init(ptx::smem_u32(&ctl->tmem_empty[b]), Cfg::kPromoWarps);
+    }
+    for (int d = 0; d < 2; ++d) {
+      ptx::mbar_init(ptx::smem_u32(&ctl->sc_full[d]), 32);
+      ptx::mbar_init(ptx::smem_u32(&ctl->sc_empty[d]), Cfg::kPromoWarps);
+    }
+    ctl->abort_flag = 0;
+    ptx::mbar_fence_init();
+    ptx::tma_prefetch_desc(&map_w);
+    ptx::tma_prefetch_desc(&map_a);
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(ptx::smem_u32(&ctl->tmem_base), Cfg::kTmemCols);
+    ptx::tmem_relinquish();
+  }
+  if constexpr (kGrouped) {
+    ptx::grid_dependency_wait();
+    rows_count_tiles<NT, Cfg::kThreads>(p, tiles_before, ctl->warp_sum);
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = ctl->tmem_base;
+  const int splits = p.splits;
+  const int rank = splits > 1 ? (int)(blockIdx.x % splits) : 0;
+  const int tile_first = splits > 1 ? (int)(blockIdx.x / splits) : (int)blockIdx.x;
+  const int tile_step = splits > 1 ? (int)(gridDim.x / splits) : (int)gridDim.x;
+  const int num_tiles = (kGrouped ? tiles_before[p.num_experts] : p.tiles_m) * p.tiles_n;
+  const int kb_begin = rank * p.kb_total / splits, kb_stop = (rank + 1) * p.kb_total / splits;
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer (all lanes) ------------------------------
+    const uint32_t bar_empty0 = ptx::smem_u32(&ctl->empty[0]), bar_full0 = ptx::smem_u32(&ctl->full[0]);
+    const uint32_t tiles0 = ptx::smem_u32(tiles);
+    // Slabs whose weights are already on their way: the first tile's, fetched before the activations can be.
+    int ahead = 0;
+    if (!kGrouped) {
+      if (p.early_weights && tile_first < num_tiles) {
+        const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, tile_first);
+        ahead = min(kStages, kb_stop - kb_begin);
+        if (lane == 0)
+          for (int s = 0; s < ahead; ++s) {
+            ptx::mbar_arrive_expect_tx(bar_full0 + s * 8, kWBytes + x.n_eff * kRowsBK);
+            ptx::tma_load_3d(tiles0 + s * kStageBytes, &map_w, bar_full0 + s * 8, (kb_begin + s) * kRowsBK, x.n_tile * kRowsBM, 0);
+          }
+        __syncwarp();
+      }
+      ptx::grid_dependency_wait();
+    }
+    uint32_t s = 0, ph = 0;
+    bool alive = true;
+    for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
+      const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+      const bool gather = kGrouped && p.gather_topk > 0;
+      int r[4] = {0, 0, 0, 0};
+      if (gather && lane * 4 < x.n_eff) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int id = p.sorted_ids[x.row0 + lane * 4 + j];
+          r[j] = id < p.numel ? id / p.gather_topk : 0;  // (padding fetches a valid row; its scale is zero)
+        }
+      }
+      const uint32_t bytes = kWBytes + x.n_eff * kRowsBK;
+      for (int kb = kb_begin; kb < kb_stop; ++kb) {
+        const uint32_t bar = bar_full0 + s * 8, dst = tiles0 + s * kStageBytes;
+        const int k0 = kb * kRowsBK;
+        if (ahead > 0) {
+          --ahead;
+        } else {
+          if (!ROWS_WAIT(bar_empty0 + s * 8, ph ^ 1u)) { *abort_flag = 1; alive = false; break; }
+          if (lane == 0) {
+            ptx::mbar_arrive_expect_tx(bar, bytes);
+            ptx::tma_load_3d(dst, &map_w, bar, k0, x.n_tile * kRowsBM, x.expert);
+          }
+          __syncwarp();
+        }
+        if (gather) {
+          if (lane * 4 < x.n_eff) ptx::tma_gather4(dst + kWBytes + lane * (4 * kRowsBK), &map_a, bar, k0, r[0], r[1], r[2], r[3]);
+        } else if (lane * 16 < x.n_eff) {
+          ptx::tma_load_2d(dst + kWBytes + lane * (16 * kRowsBK), &map_a, bar, k0, x.row0 + lane * 16);
+        }
+        if (++s == (uint32_t)kStages) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer ------------------------------
+    if (ptx::elect_one()) {
+      constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // see gemm.cu
+      const uint32_t desc_lo0 = ((ptx::smem_u32(tiles) & 0x3ffffu) >> 4) | (1u << 16);
+      const uint32_t bar_full0 = ptx::smem_u32(&ctl->full[0]), bar_empty0 = ptx::smem_u32(&ctl->empty[0]);
+      const uint32_t bar_tfull0 = ptx::smem_u32(&ctl->tmem_full[0]), bar_tempty0 = ptx::smem_u32(&ctl->tmem_empty[0]);
+      uint32_t s = 0, ph = 0, buf = 0, aph = 0;
+      bool alive = true;
+      for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
+        const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+        const uint32_t idesc = ptx::make_idesc_e4m3_f32(kRowsBM, x.n_eff);
+        for (int kb = kb_begin; kb < kb_stop; ++kb) {
+          if (!ROWS_WAIT(bar_tempty0 + buf * 8, aph ^ 1u) || !ROWS_WAIT(bar_full0 + s * 8, ph)) {
+            *abort_flag = 1;
+            alive = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t a_lo = desc_lo0 + s * (kStageBytes >> 4), b_lo = a_lo + (kWBytes >> 4);
+#pragma unroll
+          for (int k = 0; k < kRowsBK / 32; ++k)
+            ptx::mma_f8f6f4(tmem_base + buf * NT, ptx::pack_f32x2(a_lo + 2 * k, kDescHi), ptx::pack_f32x2(b_lo + 2 * k, kDescHi),
+                            idesc, k > 0 ? 1u : 0u);
+          ptx::mma_commit(bar_empty0 + s * 8);
+          ptx::mma_commit(bar_tfull0 + buf * 8);
+          if (++s == (uint32_t)kStages) {
+            s = 0;
+            ph ^= 1u;
+          }
+          if (++buf == (uint32_t)kAccBufs) {
+            buf = 0;
+            aph ^= 1u;
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    // ------------------------------ scales ------------------------------
+    // Lane l prepares columns l, l + 32, ..: eight slabs per step, all loads of a step in flight together and one
+    // step ahead of the promotion (two slots).
+    constexpr int kPer = (NT + 31) / 32;
+    const uint32_t bar_full0 = ptx::smem_u32(&ctl->sc_full[0]), bar_empty0 = ptx::smem_u32(&ctl->sc_empty[0]);
+    ptx::grid_dependency_wait();
+    uint32_t d = 0, dph = 0;
+    bool alive = true;
+    for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
+      const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+      const float* b_row = p.b_s + ((int64_t)x.expert * p.nb_total + x.n_tile) * p.kb_total;
+      const float* a_row[kPer];
+      bool on[kPer];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int j = lane + 32 * i;
+        on[i] = j < x.n_eff;
+        int64_t row = x.row0 + j;
+        if (kGrouped) {
+          if (on[i] && p.gather_topk > 0) {
+            const int id = p.sorted_ids[row];
+            on[i] = id < p.numel;
+            row = on[i] ? id / p.gather_topk : 0;
+          }
+        } else {
+          on[i] = row < p.M;
+        }
+        a_row[i] = p.a_s + row * p.as_stride_m;
+      }
+      for (int kb0 = kb_begin; kb0 < kb_stop; kb0 += kScBatch) {
+        float v[kPer][kScBatch];
+#pragma unroll
+        for (int b = 0; b < kScBatch; ++b) {
+          const float bs = kb0 + b < kb_stop ? __ldg(b_row + kb0 + b) : 0.f;
+#pragma unroll
+          for (int i = 0; i < kPer; ++i)
+            v[i][b] = on[i] && kb0 + b < kb_stop ? __ldg(a_row[i] + (int64_t)(kb0 + b) * p.as_stride_k) * bs : 0.f;
+        }
+        if (!ROWS_WAIT(bar_empty0 + d * 8, dph ^ 1u)) { *abort_flag = 1; alive = false; break; }
+#pragma unroll
+        for (int b = 0; b < kScBatch; ++b)
+#pragma unroll
+          for (int i = 0; i < kPer; ++i)
+            if (lane + 32 * i < NT) ctl->sc[d][b][lane + 32 * i] = v[i][b];
+        ptx::mbar_arrive(bar_full0 + d * 8);
+        d ^= 1u;
+        if (d == 0) dph ^= 1u;
+      }
+    }
+  } else if (warp >= 4) {
+    // ------------------------------ promotion + store ------------------------------
+    const int q = warp & 3, h = (warp - 4) >> 2;
+    constexpr int G = Cfg::kColGroups;
+    const uint32_t bar_tfull0 = ptx::smem_u32(&ctl->tmem_full[0]), bar_tempty0 = ptx::smem_u32(&ctl->tmem_empty[0]);
+    const uint32_t bar_sfull0 = ptx::smem_u32(&ctl->sc_full[0]), bar_sempty0 = ptx::smem_u32(&ctl->sc_empty[0]);
+    const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16) + h * kCW, sc0 = ptx::smem_u32(&ctl->sc[0][0][0]) + h * kCW * 4;
+    ptx::grid_dependency_wait();
+    uint32_t buf = 0, aph = 0, d = 0, dph = 0;
+    bool alive = true;
+    for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
+      const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+      const int n = x.n_tile * kRowsBM + q * 32 + lane;  // this thread's output column of C
+      int active = 0;                                    // chunks of this warp that hold columns of the tile
+#pragma unroll
+      for (int i = 0; i < kChunks; ++i) active += (h + i * G) * kCW < x.n_eff ? 1 : 0;
+      float acc[kChunks][kCW];
+#pragma unroll
+      for (int i = 0; i < kChunks; ++i)
+#pragma unroll
+        for (int j = 0; j < kCW; ++j) acc[i][j] = 0.f;
+      const int slabs = kb_stop - kb_begin;
+      for (int g = 0; g < slabs; ++g) {
+        const int b = g & (kScBatch - 1);
+        if ((b == 0 && !ROWS_WAIT(bar_sfull0 + d * 8, dph)) || !ROWS_WAIT(bar_tfull0 + buf * 8, aph)) {
+          *abort_flag = 1;
+          alive = false;
+          break;
+        }
+        ptx::tc_fence_after();
+        const uint32_t taddr = taddr0 + buf * NT, sc = sc0 + (d * kScBatch + b) * (NT * 4);
+        if (active == 0 && lane == 0) ptx::mbar_arrive(bar_tempty0 + buf * 8);
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i) {
+          if (i < active) {
+            uint32_t r[kCW];
+            if constexpr (kCW == 32) ptx::tmem_ld_32x32(taddr + i * (G * kCW), r);
+            else ptx::tmem_ld_32x16(taddr + i * (G * kCW), r);
+            ptx::tmem_ld_wait();
+            if (i == active - 1) {
+              ptx::tc_fence_before();
+              ptx::mbar_arrive_if(bar_tempty0 + buf * 8, lane == 0);
+            }
+#pragma unroll
+            for (int j = 0; j < kCW; j += 4) {
+              const float4 s4 = ptx::lds_f32x4(sc + (i * (G * kCW) + j) * 4);
+              ptx::fma2(acc[i][j], acc[i][j + 1], r[j], r[j + 1], s4.x, s4.y);
+              ptx::fma2(acc[i][j + 2], acc[i][j + 3], r[j + 2], r[j + 3], s4.z, s4.w);
+            }
+          }
+        }
+        if (b == kScBatch - 1 || g == slabs - 1) {
+          __syncwarp();
+          ptx::mbar_arrive_if(bar_sempty0 + d * 8, lane == 0);
+          d ^= 1u;
+          if (d == 0) dph ^= 1u;
+        }
+        if (++buf == (uint32_t)kAccBufs) {
+          buf = 0;
+          aph ^= 1u;
+        }
+      }
+      if (!alive) break;
+      if (splits > 1) {
+        // this CTA's partial sums, [column][weight row], over its ring: every slab has been consumed, and a cluster
+        // works on one tile only
+        float* part = reinterpret_cast<float*>(tiles) + q * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i)
+          if (i < active) {
+#pragma unroll
+            for (int j = 0; j < kCW; ++j) part[((h + i * G) * kCW + j) * kRowsBM] = acc[i][j];
+          }
+        continue;
+      }
+      // Two lanes (weight rows n, n + 1) exchange one value per pair of columns, so that each of them stores one
+      // 32-bit word: 64 bytes of one output row per 16 lanes.
+      const bool n_ok = n < p.N;  // (N is even: a pair is inside or outside as a whole)
+      float bias = 0.f;
+      if (!kGrouped && p.bias != nullptr && n_ok)
+        bias = p.out_fp16 ? __half2float(static_cast<const __half*>(p.bias)[n])
+                          : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n]);
+#pragma unroll
+      for (int i = 0; i < kChunks; ++i) {
+        if (i < active) {
+          const int col0 = (h + i * G) * kCW;
+          // destination row and routing weight of column col0 + lane; -1 = not stored
+          int dst = -1;
+          float w = 1.f;
+          if (lane < kCW && col0 + lane < x.n_eff) {
+            const int row = x.row0 + col0 + lane;
+            dst = row;
+            if (kGrouped) {
+              if (p.scatter) {
+                const int id = p.sorted_ids[row];
+                dst = id < p.numel ? id : -1;
+                if (p.row_weights != nullptr && dst >= 0) w = __ldg(p.row_weights + id);
+              }
+            } else if (row >= p.M) {
+              dst = -1;
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < kCW; j += 2) {
+            float v0 = acc[i][j] + bias, v1 = acc[i][j + 1] + bias;
+            if (kGrouped) {
+              v0 *= __shfl_sync(0xffffffffu, w, j);
+              v1 *= __shfl_sync(0xffffffffu, w, j + 1);
+            }
+            const bool odd = lane & 1;
+            const float other = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+            const float lo = odd ? other : v0, hi = odd ? v1 : other;
+            const int row = __shfl_sync(0xffffffffu, dst, j + (lane & 1));
+            uint32_t word;
+            if (p.out_fp16) {
+              const __half2 o = __floats2half2_rn(lo, hi);
+              word = *reinterpret_cast<const uint32_t*>(&o);
+            } else {
+              const __nv_bfloat162 o = __floats2bfloat162_rn(lo, hi);
+              word = *reinterpret_cast<const uint32_t*>(&o);
+            }
+            if (row >= 0 && n_ok)
+              *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + (n & ~1)) = word;
+          }
+        }
+      }
+    }
+  }
+
+  // ------------------------------ sum over the CTAs of a cluster ------------------------------
+  if (!kGrouped && splits > 1) {
+    __syncwarp();
+    ptx::cluster_sync();
+    const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, tile_first);
+    if (ctl->abort_flag == 0) {
+      // CTA `rank` adds columns rank, rank + splits, ..; a thread adds two neighbouring weight rows of a column
+      const int mine = (x.n_eff - rank + splits - 1) / splits;
+      const uint32_t part = ptx::smem_u32(tiles);
+      for (int i = tid; i < mine * (kRowsBM / 2); i += Cfg::kThreads) {
+        const int col = rank + (i / (kRowsBM / 2)) * splits, pair = i % (kRowsBM / 2);
+        const int n = x.n_tile * kRowsBM + pair * 2, row = x.row0 + col;
+        if (n >= p.N || row >= p.M) continue;
+        float2 v[kMaxSplits];
+#pragma unroll
+        for (int s = 0; s < kMaxSplits; ++s)  // all requested before the first is added
+          if (s < splits) v[s] = ptx::lds_cluster_f32x2(ptx::cluster_map(part + (col * kRowsBM + pair * 2) * 4, s));
+        float a = v[0].x, b = v[0].y;
+#pragma unroll
+        for (int s = 1; s < kMaxSplits; ++s)
+          if (s < splits) a += v[s].x, b += v[s].y;
+        uint32_t word;
+        if (p.out_fp16) {
+          if (p.bias != nullptr) {
+            const __half* bs = static_cast<const __half*>(p.bias) + n;
+            a += __half2float(bs[0]), b += __half2float(bs[1]);
+          }
+          const __half2 o = __floats2half2_rn(a, b);
+          word = *reinterpret_cast<const uint32_t*>(&o);
+        } else {
+          if (p.bias != nullptr) {
+            const __nv_bfloat16* bs = static_cast<const __nv_bfloat16*>(p.bias) + n;
+            a += __bfloat162float(bs[0]), b += __bfloat162float(bs[1]);
+          }
+          const __nv_bfloat162 o = __floats2bfloat162_rn(a, b);
+          word = *reinterpret_cast<const uint32_t*>(&o);
+        }
+        *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + n) = word;
+      }
+    }
+    ptx::cluster_sync();  // no CTA leaves while another reads its shared memory
+  }
+
+  // ------------------------------ teardown ------------------------------
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (ctl->abort_flag != 0 && tid == 0) {
+    atomicExch(&g_rows_status, 1);
+    // give TMA copies that may still be in flight time to land before the CTA's shared memory is released
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000ll) {
+    }
+  }
+  __syncthreads();
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem_base, Cfg::kTmemCols);
+  }
+}
+
+template <class Cfg, bool kGrouped>
+static size_t rows_smem_bytes(int num_experts) {
+  return (size_t)Cfg::kStages * Cfg::kStageBytes + sizeof(RowsCtl<Cfg>) + 1024 + (kGrouped ? sizeof(int) * (num_experts + 1) : 0);
+}
+
+// `pdl`: the launch may overlap the end of the kernel before it in the stream (the kernel waits by itself).
+template <class Cfg, bool kGrouped>
+static int launch_rows(const CUtensorMap& mw, const CUtensorMap& ma, const RowsParams& p, int64_t max_tiles, bool pdl,
+                       cudaStream_t st) {
+  auto kern = fp8_rows_gemm_kernel<Cfg, kGrouped>;
+  const size_t smem = rows_smem_bytes<Cfg, kGrouped>(p.num_experts);
+  static thread_local bool attr_set[64] = {false};  // the opt-in is per function and per device
+  int dev = 0;
+  SGLB_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+    SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)rows_smem_bytes<Cfg, kGrouped>(kMaxExperts)));
+    if (dev >= 0 && dev < 64) attr_set[dev] = true;
+  }
+  const int64_t slots = (int64_t)sm_count() * Cfg::kCtasPerSm;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.splits > 1 ? max_tiles * p.splits : (max_tiles < slots ? max_tiles : slots)), 1, 1);
+  cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  cfg.numAttrs = 0;
+  if (p.splits > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = (unsigned)p.splits;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  SGLB_CUDA(cudaLaunchKernelEx(&cfg, kern, mw, ma, p));
+  return SGLB200_OK;
+}
+
+// CTAs per cluster for a dense problem of `tiles` tiles and `kb` slabs: the split that finishes first, counted in
+// slabs of the busiest CTA slot (rounds of CTAs x slabs of a CTA), a CTA's start and end charged as three slabs and
+// the exchange of a cluster as two more.
+static int rows_splits(int64_t tiles, int kb, int64_t slots) {
+  int best = 1;
+  int64_t best_cost = -1;
+  for (int s = 1; s <= kMaxSplits && s <= kb; ++s) {
+    const int64_t rounds = (tiles * s + slots - 1) / slots;
+    const int64_t cost = s == 1 ? rounds * kb + 3 : rounds * ((kb + s - 1) / s + 5);
+    if (best_cost < 0 || cost < best_cost) best = s, best_cost = cost;
+  }
+  return best;
+}
+
+template <class Cfg>
+static int rows_dense_cfg(const void* A, const void* B, RowsParams& p, int64_t K, bool pdl, cudaStream_t st) {
+  CUtensorMap mw, ma;
+  int rc = get_tensor_map(B, (uint64_t)K, (uint64_t)p.N, 1, kRowsBM, 3, &mw);
+  if (rc) return rc;
+  rc = get_tensor_map(A, (uint64_t)K, (uint64_t)p.M, 1, 16, 2, &ma);
+  if (rc) return rc;
+  p.tiles_m = (int)((p.M + Cfg::NT - 1) / Cfg::NT);
+  p.group_m = choose_group_m(p.M, K, Cfg::NT);
+  const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
+  p.splits = rows_splits(tiles, p.kb_total, (int64_t)sm_count() * Cfg::kCtasPerSm);
+  return launch_rows<Cfg, false>(mw, ma, p, tiles, pdl, st);
+}
+
+int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
+                  int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, bool after_quantizer,
+                  cudaStream_t st) {
+  RowsParams p{};
+  p.a_s = a_s, p.b_s = b_s, p.C = C, p.bias = bias;
+  p.M = M, p.N = N, p.as_stride_m = as_stride_m, p.as_stride_k = as_stride_k;
+  p.kb_total = (int)((K + kRowsBK - 1) / kRowsBK), p.nb_total = (int)((N + 127) / 128), p.tiles_n = p.nb_total;
+  p.out_fp16 = out_dtype;
+  p.early_weights = after_quantizer ? 1 : 0;
+  p.wait_probes = g_gemm_wait_probes;
+  if (M <= 16) return rows_dense_cfg<Rows16>(A, B, p, K, after_quantizer, st);
+  if (M <= 32) return rows_dense_cfg<Rows32>(A, B, p, K, after_quantizer, st);
+  if (M <= 64) return rows_dense_cfg<Rows64>(A, B, p, K, after_quantizer, st);
+  return rows_dense_cfg<Rows128>(A, B, p, K, after_quantizer, st);
+}
+
+template <class Cfg>
+static int rows_grouped_cfg(const void* A, int64_t a_rows, const void* B, RowsParams& p, int64_t max_rows, int64_t K, bool pdl,
+                            cudaStream_t st) {
+  CUtensorMap mw, ma;
+  int rc = get_tensor_map(B, (uint64_t)K, (uint64_t)p.N, (uint64_t)p.num_experts, kRowsBM, 3, &mw);
+  if (rc) return rc;
+  rc = get_tensor_map(A, (uint64_t)K, (uint64_t)a_rows, 1, p.gather_topk > 0 ? 1 : 16, 2, &ma);
+  if (rc) return rc;
+  p.group_m = choose_group_m(max_rows, K, Cfg::NT);
+  p.splits = 1;
+  // every expert has at most one partial tile
+  int64_t tiles = max_rows / Cfg::NT + p.num_experts;
+  if (tiles > max_rows / 16) tiles = max_rows / 16;
+  return launch_rows<Cfg, true>(mw, ma, p, tiles * p.tiles_n, pdl, st);
+}
+
+int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const float* a_s, const void* B, const float* b_s, void* C,
+                    const int32_t* cumsum, const int32_t* sorted_ids, const float* row_weights, int64_t max_rows,
+                    int64_t numel, int num_experts, int64_t N, int64_t K, int gather_topk, int scatter, int out_dtype, int nt,
+                    bool pdl, cudaStream_t st) {
+  RowsParams p{};
+  p.a_s = a_s, p.b_s = b_s, p.C = C;
+  p.M = a_rows, p.N = N, p.as_stride_m = as_stride, p.as_stride_k = 1;
+  p.kb_total = (int)((K + kRowsBK - 1) / kRowsBK), p.nb_total = (int)((N + 127) / 128), p.tiles_n = p.nb_total;
+  p.out_fp16 = out_dtype, p.num_experts = num_experts, p.cumsum = cumsum, p.sorted_ids = sorted_ids, p.numel = numel;
+  p.gather_topk = gather_topk, p.scatter = scatter, p.row_weights = row_weights;
+  p.wait_probes = g_gemm_wait_probes;
+  switch (nt) {
+    case 16: return rows_grouped_cfg<Rows16>(A, a_rows, B, p, max_rows, K, pdl, st);
+    case 32: return rows_grouped_cfg<Rows32>(A, a_rows, B, p, max_rows, K, pdl, st);
+    case 64: return rows_grouped_cfg<Rows64>(A, a_rows, B, p, max_rows, K, pdl, st);
+    default: return rows_grouped_cfg<Rows128>(A, a_rows, B, p, max_rows, K, pdl, st);
+  }
+}
+
+int rows_gemm_status() {
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_rows_status, sizeof(int)) != cudaSuccess) return -1;
+  return v;
+}
+int rows_gemm_status_clear() {
+  const int zero = 0;
+  SGLB_CUDA(cudaMemcpyToSymbol(g_rows_status, &zero, sizeof(int)));
+  return SGLB200_OK;
+}
+
+}  // namespace sglb200

@@ -1,0 +1,106 @@
+// Shared parts of the kernels whose M side is the weights (gemm_rows.cu: one CTA per tile; gemm_pair.cu: CTA pairs):
+// launch parameters, the walk over tiles, the count of the experts' token tiles.
+#pragma once
+#include "common.cuh"
+#include "gemm_common.cuh"
+#include "ptx_sm100.cuh"
+
+namespace sglb200 {
+
+constexpr int kRowsBM = 128;                     // weight rows per tile
+constexpr int kRowsBK = 128;                     // K slab: one scale block
+constexpr uint32_t kWBytes = kRowsBM * kRowsBK;  // weight bytes per stage
+constexpr int kScBatch = 8;                      // slabs whose scales are prepared together
+constexpr int kMaxExperts = 1024;
+constexpr int kMaxSplits = 8;                    // CTAs of a cluster
+
+struct RowsParams {
+  const float* a_s;
+  const float* b_s;
+  void* C;
+  const void* bias;                // dense, optional
+  int64_t M, N;                    // dense: rows of A
+  int64_t as_stride_m, as_stride_k;
+  int kb_total, nb_total, tiles_n;
+  int tiles_m;                     // dense
+  int splits;                      // CTAs of a cluster, each with its part of K (1 = no cluster)
+  int early_weights;               // the weights may be read before the predecessor in the stream has finished
+  int out_fp16;
+  int group_m;                     // token tiles of a group sweep over the weight tiles together
+  // expert-grouped form
+  int num_experts;
+  const int32_t* cumsum;           // [experts + 2] padded starts of the buckets (bucket e + 1 = expert e), multiples of 16
+  const int32_t* sorted_ids;       // flat top-k slots in expert order, >= numel = padding
+  int64_t numel;
+  int gather_topk;                 // > 0: A has a row per token, fetched by slot / gather_topk; 0: A is in expert order
+  int scatter;                     // write row sorted_ids[r] instead of row r
+  const float* row_weights;        // scatter, optional
+  uint32_t wait_probes;
+};
+
+struct RowsTile {
+  int n_tile, row0, n_eff, expert;
+};
+
+template <int NT, bool kGrouped>
+__device__ __forceinline__ RowsTile rows_tile(const RowsParams& p, const int* tiles_before, int t) {
+  RowsTile x;
+  int m_tile;
+  if constexpr (kGrouped) {
+    int lo = 0, hi = p.num_experts;  // the expert with tiles_before[e] * tiles_n <= t < tiles_before[e + 1] * tiles_n
+    const int tt = t / p.tiles_n;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (tiles_before[mid] <= tt) lo = mid; else hi = mid;
+    }
+    x.expert = lo;
+    const int first = tiles_before[lo];
+    tile_coord(t - first * p.tiles_n, tiles_before[lo + 1] - first, p.tiles_n, p.group_m, m_tile, x.n_tile);
+    const int begin = p.cumsum[lo + 1], end = p.cumsum[lo + 2];
+    x.row0 = begin + m_tile * NT;
+    x.n_eff = min(NT, end - x.row0);
+  } else {
+    tile_coord(t, p.tiles_m, p.tiles_n, p.group_m, m_tile, x.n_tile);
+    x.expert = 0;
+    x.row0 = m_tile * NT;
+    x.n_eff = min(NT, ((int)p.M - x.row0 + 15) & ~15);
+  }
+  return x;
+}
+
+// Token tiles (of NT rows) of every expert and their exclusive scan into tiles_before[0 .. experts]: four experts per
+// thread, all NTHREADS threads of the block.  The scan is visible after the next __syncthreads.
+template <int NT, int NTHREADS>
+__device__ __forceinline__ void rows_count_tiles(const RowsParams& p, int* tiles_before, int* warp_sum) {
+  static_assert(NTHREADS * 4 >= kMaxExperts, "four experts per thread");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int cnt[4], mine = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int e = tid * 4 + k;
+    cnt[k] = e < p.num_experts ? (p.cumsum[e + 2] - p.cumsum[e + 1] + NT - 1) / NT : 0;
+    mine += cnt[k];
+  }
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  int before = incl - mine;
+  for (int w = 0; w < warp; ++w) before += warp_sum[w];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int e = tid * 4 + k;
+    if (e < p.num_experts) tiles_before[e] = before;
+    before += cnt[k];
+  }
+  if (tid == NTHREADS - 1) tiles_before[p.num_experts] = before;  // (experts beyond num_experts count 0)
+}
+
+#define ROWS_WAIT(bar, parity) \
+  (p.wait_probes != ptx::kProbesNone && (ptx::mbar_test(bar, parity) || ptx::mbar_wait_quiet(bar, parity)))
+
+}  // namespace sglb200

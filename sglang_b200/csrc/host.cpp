@@ -28,11 +28,10 @@ namespace {
   X(sglb200_silu_and_mul_quant_fp8)      \
   X(sglb200_gemm_workspace_bytes)        \
   X(sglb200_fp8_blockwise_scaled_mm)     \
-  X(sglb200_fp8_blockwise_grouped_mm)    \
-  X(sglb200_moe_align_workspace_bytes)   \
-  X(sglb200_moe_align_block_size)        \
-  X(sglb200_gather_rows_fp8)             \
-  X(sglb200_moe_sum_reduce)              \
+  X(sglb200_block_fp8_linear_workspace_bytes) \
+  X(sglb200_block_fp8_linear)            \
+  X(sglb200_fused_experts_workspace_bytes) \
+  X(sglb200_fused_experts)               \
   X(sglb200_topk_softmax)                \
   X(sglb200_moe_fused_gate)
 
@@ -98,16 +97,6 @@ Tensor make(at::IntArrayRef size, at::ScalarType dtype, c10::Device dev) {
 
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
-// Parts of one allocation, each on a 256-byte boundary.
-struct Carver {
-  int64_t bytes = 0;
-  int64_t take(int64_t n) {
-    const int64_t at = bytes;
-    bytes += (n + 255) & ~int64_t(255);
-    return at;
-  }
-};
-
 Tensor workspace(int64_t bytes, c10::Device dev) { return make({bytes > 0 ? bytes : 1}, at::kByte, dev); }
 
 PyObject* pair(Tensor a, Tensor b) {
@@ -119,7 +108,7 @@ PyObject* pair(Tensor a, Tensor b) {
   return r;
 }
 
-constexpr float kEps = 1e-10f, kFp8Max = 448.0f;
+constexpr float kFp8Max = 448.0f;
 
 // ---- quantizer ------------------------------------------------------------------------------------------------
 // quant(x, group_size, eps, column_major, tma_aligned) -> (codes, scales)
@@ -211,20 +200,12 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Py_RETURN_NONE;
   return guarded([&]() -> PyObject* {
     const int64_t M = x.numel() / K;
-    const int64_t scratch = abi.sglb200_gemm_workspace_bytes(M, N, K);
-    Carver c;
-    const int64_t at_q = c.take(M * K), at_s = c.take(M * (K / 128) * 4), at_p = c.take(scratch);
+    const int64_t bytes = abi.sglb200_block_fp8_linear_workspace_bytes(M, N, K);
     c10::DimVector shape(x.sizes().begin(), x.sizes().end());
     shape.back() = N;
-    Tensor out = make(shape, x.scalar_type(), x.device()), mem = workspace(c.bytes, x.device());
-    char* base = static_cast<char*>(mem.data_ptr());
-    void* st = stream_of(x);
-    float* xs = reinterpret_cast<float*>(base + at_s);
-    int rc = abi.sglb200_per_token_group_quant_fp8(x.data_ptr(), dt, base + at_q, xs, M, K, 128, kEps, -kFp8Max, kFp8Max, K / 128, 1, st);
-    if (rc) return raise_last(rc);
-    rc = abi.sglb200_fp8_blockwise_scaled_mm(base + at_q, w->data_ptr(), xs, static_cast<const float*>(ws->data_ptr()), out.data_ptr(),
-                                             bias ? bias->data_ptr() : nullptr, M, N, K, K / 128, 1, dt,
-                                             scratch ? base + at_p : nullptr, scratch, st);
+    Tensor out = make(shape, x.scalar_type(), x.device()), mem = workspace(bytes, x.device());
+    const int rc = abi.sglb200_block_fp8_linear(x.data_ptr(), dt, w->data_ptr(), static_cast<const float*>(ws->data_ptr()), out.data_ptr(),
+                                                bias ? bias->data_ptr() : nullptr, M, N, K, mem.data_ptr(), bytes, stream_of(x));
     if (rc) return raise_last(rc);
     return THPVariable_Wrap(std::move(out));
   });
@@ -332,39 +313,12 @@ PyObject* fused_experts(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       out->numel() != T * Ho)
     Py_RETURN_NONE;
   return guarded([&]() -> PyObject* {
-    constexpr int64_t block = 128;
-    const int64_t numel = T * k, hb = H / 128, ib = I / 128;
-    const int64_t cap = numel + (E + 1) * (block - 1);                                 // the sort's outputs
-    const int64_t rows = (numel + std::min(numel, E + 1) * (block - 1) + block - 1) / block * block;  // at most this many are used
-    const bool direct = k == 1 && factor == 1.0;  // one expert per token: the scatter epilogue writes the result itself
-    const int64_t sort_ws = abi.sglb200_moe_align_workspace_bytes(numel, (int)E + 1);
-    Carver c;
-    const int64_t o_q = c.take(T * H), o_s = c.take(T * hb * 4), o_sorted = c.take(cap * 4), o_eid = c.take((cap + block - 1) / block * 4),
-                  o_post = c.take(4), o_cum = c.take((E + 2) * 4), o_ws = c.take(sort_ws), o_a1 = c.take(rows * H),
-                  o_a1s = c.take(rows * hb * 4), o_ic1 = c.take(rows * N * 2), o_a2 = c.take(rows * I), o_a2s = c.take(rows * ib * 4),
-                  o_ic3 = direct ? 0 : c.take(numel * Ho * 2);
-    Tensor mem = workspace(c.bytes, x.device());
-    char* base = static_cast<char*>(mem.data_ptr());
-    void* st = stream_of(x);
-    auto f = [&](int64_t at) { return reinterpret_cast<float*>(base + at); };
-    auto i = [&](int64_t at) { return reinterpret_cast<int32_t*>(base + at); };
-    const int32_t* ids = static_cast<const int32_t*>(id->data_ptr());
-    int rc = abi.sglb200_per_token_group_quant_fp8(x.data_ptr(), dt, base + o_q, f(o_s), T, H, 128, kEps, -kFp8Max, kFp8Max, hb, 1, st);
-    if (!rc)
-      rc = abi.sglb200_moe_align_block_size(ids, numel, (int)E + 1, (int)block, i(o_sorted), i(o_eid), i(o_post), i(o_cum), 1,
-                                            sort_ws ? base + o_ws : nullptr, sort_ws, st);
-    if (!rc)
-      rc = abi.sglb200_gather_rows_fp8(base + o_q, f(o_s), base + o_a1, f(o_a1s), i(o_sorted), i(o_post), rows, numel, (int)k, H, hb, st);
-    if (!rc)
-      rc = abi.sglb200_fp8_blockwise_grouped_mm(base + o_a1, f(o_a1s), w1->data_ptr(), static_cast<const float*>(s1->data_ptr()),
-                                                base + o_ic1, i(o_sorted), i(o_eid), i(o_post), nullptr, rows, numel, (int)E, N, H, 0, dt, st);
-    if (!rc) rc = abi.sglb200_silu_and_mul_quant_fp8(base + o_ic1, dt, base + o_a2, f(o_a2s), rows, I, 128, kEps, i(o_post), st);
-    void* ic3 = direct ? out->data_ptr() : base + o_ic3;
-    if (!rc)
-      rc = abi.sglb200_fp8_blockwise_grouped_mm(base + o_a2, f(o_a2s), w2->data_ptr(), static_cast<const float*>(s2->data_ptr()), ic3,
-                                                i(o_sorted), i(o_eid), i(o_post), static_cast<const float*>(wt->data_ptr()), rows, numel,
-                                                (int)E, Ho, I, 1, dt, st);
-    if (!rc && !direct) rc = abi.sglb200_moe_sum_reduce(ic3, out->data_ptr(), dt, T, k, Ho, (float)factor, st);
+    const int64_t bytes = abi.sglb200_fused_experts_workspace_bytes(T, k, (int)E, H, I, Ho, (float)factor);
+    Tensor mem = workspace(bytes, x.device());
+    const int rc = abi.sglb200_fused_experts(
+        x.data_ptr(), dt, w1->data_ptr(), static_cast<const float*>(s1->data_ptr()), w2->data_ptr(), static_cast<const float*>(s2->data_ptr()),
+        static_cast<const float*>(wt->data_ptr()), static_cast<const int32_t*>(id->data_ptr()), out->data_ptr(), T, k, (int)E, H, I, Ho,
+        (float)factor, mem.data_ptr(), bytes, stream_of(x));
     if (rc) return raise_last(rc);
     Py_RETURN_TRUE;
   });

@@ -1,0 +1,167 @@
+// Whole layers as one call of the C ABI: the block-FP8 linear (quantise, multiply) and the routed experts of a MoE
+// layer (quantise, sort, multiply, activate + re-quantise, multiply, sum).  One workspace holds every intermediate;
+// the kernels follow one another with programmatic serialization where they can, so that the start of each overlaps
+// the end of the one before.
+#include <algorithm>
+
+#include "common.cuh"
+#include "gemm_common.cuh"
+
+namespace sglb200 {
+
+constexpr float kQuantEps = 1e-10f, kFp8Max = 448.0f;
+
+// Parts of one workspace, each on a 256-byte boundary.
+struct Carver {
+  int64_t bytes = 0;
+  int64_t take(int64_t n) {
+    const int64_t at = bytes;
+    bytes += (n + 255) & ~int64_t(255);
+    return at;
+  }
+};
+
+struct LinearParts {
+  int64_t q, s, gemm, gemm_bytes, total;
+};
+static LinearParts linear_parts(int64_t M, int64_t N, int64_t K) {
+  LinearParts x;
+  Carver c;
+  x.q = c.take(M * K);
+  x.s = c.take(M * (K / 128) * 4);
+  x.gemm_bytes = sglb200_gemm_workspace_bytes(M, N, K);
+  x.gemm = c.take(x.gemm_bytes);
+  x.total = c.bytes;
+  return x;
+}
+
+// How the routed experts run.  `tile` = activation rows per GEMM tile, `block` = padding of an expert's rows in the
+// sorted order.
+struct ExpertsPlan {
+  int tile, block;
+  int64_t cap, rows;  // entries of the sort's output; rows that can be in use
+  int64_t q, s, sorted, eid, post, cum, sort, sort_bytes, a1, a1s, ic1, a2, a2s, ic3, total;
+  bool direct;        // one expert per token and no factor: the second GEMM writes the result itself
+};
+
+constexpr int kRowsMaxExperts = 1024;  // experts of one call of the rows kernel
+
+static int experts_row_tile(int64_t numel, int64_t E) {
+  if (E > kRowsMaxExperts) return 0;
+  const int64_t avg = numel / std::min(numel, E);
+  if (avg <= 3) return 16;
+  if (avg <= 24) return 32;
+  if (avg <= 48) return 64;
+  return 0;
+}
+
+static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int64_t I, int64_t Ho, float factor) {
+  ExpertsPlan p{};
+  const int64_t numel = T * k;
+  p.tile = experts_row_tile(numel, E);
+  p.block = p.tile > 0 ? 16 : 128;
+  p.cap = numel + (E + 1) * (p.block - 1);
+  p.rows = (numel + std::min(numel, E + 1) * (p.block - 1) + p.block - 1) / p.block * p.block;
+  p.direct = k == 1 && factor == 1.0f;
+  p.sort_bytes = sglb200_moe_align_workspace_bytes(numel, (int)E + 1);
+  Carver c;
+  p.q = c.take(T * H), p.s = c.take(T * (H / 128) * 4);
+  p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4);
+  p.cum = c.take((E + 2) * 4), p.sort = c.take(p.sort_bytes);
+  if (p.tile == 0) p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
+  p.ic1 = c.take(p.rows * 2 * I * 2);
+  p.a2 = c.take(p.rows * I), p.a2s = c.take(p.rows * (I / 128) * 4);
+  if (!p.direct) p.ic3 = c.take(numel * Ho * 2);
+  p.total = c.bytes;
+  return p;
+}
+
+}  // namespace sglb200
+
+using namespace sglb200;
+
+extern "C" int64_t sglb200_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  return linear_parts(M, N, K).total;
+}
+
+extern "C" int sglb200_block_fp8_linear(const void* x, int dtype, const void* W, const float* w_s, void* C, const void* bias,
+                                        int64_t M, int64_t N, int64_t K, void* workspace, int64_t workspace_bytes,
+                                        void* stream) {
+  SGLB_REQUIRE(M >= 0 && N > 0 && K > 0 && K % 128 == 0, "block_fp8_linear: bad shape M=%lld N=%lld K=%lld (K a multiple of 128)",
+               (long long)M, (long long)N, (long long)K);
+  SGLB_REQUIRE(dtype == 0 || dtype == 1, "block_fp8_linear: dtype %d (0 bf16, 1 fp16)", dtype);
+  if (M == 0) return SGLB200_OK;
+  const LinearParts lp = linear_parts(M, N, K);
+  if (workspace == nullptr || !aligned16(workspace) || workspace_bytes < lp.total)
+    return fail(SGLB200_E_WORKSPACE, "block_fp8_linear: workspace of %lld bytes required, got %lld", (long long)lp.total,
+                (long long)workspace_bytes);
+  char* base = static_cast<char*>(workspace);
+  float* xs = reinterpret_cast<float*>(base + lp.s);
+  const int rc = sglb200_per_token_group_quant_fp8(x, dtype, base + lp.q, xs, M, K, 128, kQuantEps, -kFp8Max, kFp8Max, K / 128, 1,
+                                                   stream);
+  if (rc) return rc;
+  return scaled_mm(base + lp.q, W, xs, w_s, C, bias, M, N, K, K / 128, 1, dtype, base + lp.gemm, lp.gemm_bytes, true,
+                   static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int64_t sglb200_fused_experts_workspace_bytes(int64_t tokens, int64_t topk, int num_experts, int64_t hidden,
+                                                         int64_t intermediate, int64_t out_hidden, float factor) {
+  if (tokens <= 0 || topk <= 0 || num_experts <= 0 || hidden <= 0 || intermediate <= 0 || out_hidden <= 0) return 0;
+  return experts_plan(tokens, topk, num_experts, hidden, intermediate, out_hidden, factor).total;
+}
+
+extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, const float* w13_s, const void* w2,
+                                     const float* w2_s, const float* topk_weights, const int32_t* topk_ids, void* out,
+                                     int64_t tokens, int64_t topk, int num_experts, int64_t hidden, int64_t intermediate,
+                                     int64_t out_hidden, float factor, void* workspace, int64_t workspace_bytes,
+                                     void* stream) {
+  const int64_t T = tokens, k = topk, E = num_experts, H = hidden, I = intermediate, Ho = out_hidden, numel = T * k;
+  SGLB_REQUIRE(T >= 0 && k >= 1 && E >= 1 && H > 0 && H % 128 == 0 && I > 0 && I % 128 == 0 && Ho > 0 && Ho % 8 == 0,
+               "fused_experts: tokens=%lld topk=%lld experts=%lld hidden=%lld intermediate=%lld out=%lld", (long long)T,
+               (long long)k, (long long)E, (long long)H, (long long)I, (long long)Ho);
+  SGLB_REQUIRE(dtype == 0 || dtype == 1, "fused_experts: dtype %d (0 bf16, 1 fp16)", dtype);
+  if (T == 0) return SGLB200_OK;
+  SGLB_REQUIRE(x && w13 && w13_s && w2 && w2_s && topk_weights && topk_ids && out, "fused_experts: null pointer");
+  SGLB_REQUIRE(aligned16(w13) && aligned16(w2) && aligned16(out), "fused_experts: weights and out must be 16-byte aligned");
+  const ExpertsPlan p = experts_plan(T, k, E, H, I, Ho, factor);
+  if (workspace == nullptr || !aligned16(workspace) || workspace_bytes < p.total)
+    return fail(SGLB200_E_WORKSPACE, "fused_experts: workspace of %lld bytes required, got %lld", (long long)p.total,
+                (long long)workspace_bytes);
+  char* base = static_cast<char*>(workspace);
+  auto f = [&](int64_t at) { return reinterpret_cast<float*>(base + at); };
+  auto i = [&](int64_t at) { return reinterpret_cast<int32_t*>(base + at); };
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  void* ic3 = p.direct ? out : base + p.ic3;
+  const int64_t hb = H / 128, ib = I / 128;
+  int rc = sglb200_per_token_group_quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, stream);
+  if (rc) return rc;
+  rc = sglb200_moe_align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
+                                    p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, stream);
+  if (rc) return rc;
+  if (p.tile > 0) {
+    if (p.direct) SGLB_CUDA(cudaMemsetAsync(out, 0, T * Ho * 2, st));  // rows of negative ids are not written below
+    rc = rows_grouped_mm(base + p.q, T, hb, f(p.s), w13, w13_s, base + p.ic1, i(p.cum), i(p.sorted), nullptr, p.rows, numel, (int)E,
+                         2 * I, H, (int)k, 0, dtype, p.tile, true, st);
+    if (rc) return rc;
+    rc = sglb200_silu_and_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), stream);
+    if (rc) return rc;
+    rc = rows_grouped_mm(base + p.a2, p.rows, ib, f(p.a2s), w2, w2_s, ic3, i(p.cum), i(p.sorted), topk_weights, p.rows, numel,
+                         (int)E, Ho, I, 0, 1, dtype, p.tile, true, st);
+  } else {
+    rc = sglb200_gather_rows_fp8(base + p.q, f(p.s), base + p.a1, f(p.a1s), i(p.sorted), i(p.post), p.rows, numel, (int)k, H, hb,
+                                 stream);
+    if (rc) return rc;
+    rc = sglb200_fp8_blockwise_grouped_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.ic1, i(p.sorted), i(p.eid), i(p.post), nullptr,
+                                          p.rows, numel, (int)E, 2 * I, H, 0, dtype, stream);
+    if (rc) return rc;
+    rc = sglb200_silu_and_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), stream);
+    if (rc) return rc;
+    rc = sglb200_fp8_blockwise_grouped_mm(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights,
+                                          p.rows, numel, (int)E, Ho, I, 1, dtype, stream);
+  }
+  if (rc || p.direct) return rc;
+  // (the rows kernel leaves the slots of negative ids unwritten)
+  if (p.tile > 0) return sglb200_moe_sum_reduce_masked(ic3, topk_ids, out, dtype, T, k, Ho, factor, stream);
+  return sglb200_moe_sum_reduce(ic3, out, dtype, T, k, Ho, factor, stream);
+}

@@ -1,6 +1,7 @@
 // Memory-bound helpers of the MoE path for sm_100a: silu_and_mul, the top-k sum, and the row
 // gather into expert-sorted order.  All use 128-bit accesses and one pass over the data.
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 
 namespace sglb200 {
 
@@ -45,6 +46,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     moe_sum_reduce_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t total_chunks, int chunks_per_row,
                           int topk, float scale) {
+  ptx::launch_dependents();
+  ptx::grid_dependency_wait();
   const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (c >= total_chunks) return;
   const int64_t t = c / chunks_per_row;
@@ -81,6 +84,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     moe_sum_reduce_masked_kernel(const T* __restrict__ x, const int32_t* __restrict__ ids, T* __restrict__ out,
                                  int64_t total_chunks, int chunks_per_row, int topk, float scale) {
+  ptx::launch_dependents();
+  ptx::grid_dependency_wait();
   const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (c >= total_chunks) return;
   const int64_t t = c / chunks_per_row;
@@ -235,13 +240,12 @@ extern "C" int sglb200_moe_sum_reduce(const void* x, void* out, int dtype, int64
   SGLB_REQUIRE(blocks < (1ll << 31), "moe_sum_reduce: input too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == 0)
-    moe_sum_reduce_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), total, (int)(hidden / 8), (int)topk,
-        scale);
+    SGLB_CUDA(launch_pdl(moe_sum_reduce_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, st,
+                         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(out), total, (int)(hidden / 8),
+                         (int)topk, scale));
   else if (dtype == 1)
-    moe_sum_reduce_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(static_cast<const __half*>(x),
-                                                                    static_cast<__half*>(out), total,
-                                                                    (int)(hidden / 8), (int)topk, scale);
+    SGLB_CUDA(launch_pdl(moe_sum_reduce_kernel<__half>, (unsigned)blocks, 256, 0, st, static_cast<const __half*>(x),
+                         static_cast<__half*>(out), total, (int)(hidden / 8), (int)topk, scale));
   else
     return fail(SGLB200_E_UNSUPPORTED, "moe_sum_reduce: dtype code %d (0 bf16, 1 fp16)", dtype);
   SGLB_CUDA(cudaGetLastError());
@@ -330,12 +334,12 @@ extern "C" int sglb200_moe_sum_reduce_masked(const void* x, const int32_t* topk_
   SGLB_REQUIRE(blocks < (1ll << 31), "moe_sum_reduce_masked: input too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == 0)
-    moe_sum_reduce_masked_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(x), topk_ids, static_cast<__nv_bfloat16*>(out), total, (int)(hidden / 8),
-        (int)topk, scale);
+    SGLB_CUDA(launch_pdl(moe_sum_reduce_masked_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, st,
+                         static_cast<const __nv_bfloat16*>(x), topk_ids, static_cast<__nv_bfloat16*>(out), total,
+                         (int)(hidden / 8), (int)topk, scale));
   else if (dtype == 1)
-    moe_sum_reduce_masked_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(
-        static_cast<const __half*>(x), topk_ids, static_cast<__half*>(out), total, (int)(hidden / 8), (int)topk, scale);
+    SGLB_CUDA(launch_pdl(moe_sum_reduce_masked_kernel<__half>, (unsigned)blocks, 256, 0, st, static_cast<const __half*>(x),
+                         topk_ids, static_cast<__half*>(out), total, (int)(hidden / 8), (int)topk, scale));
   else
     return fail(SGLB200_E_UNSUPPORTED, "moe_sum_reduce_masked: dtype code %d (0 bf16, 1 fp16)", dtype);
   SGLB_CUDA(cudaGetLastError());

@@ -254,6 +254,12 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
 #pragma unroll
     for (int s = 0; s < kStreamStages; ++s) ptx::mbar_init(ptx::smem_u32(&bars[s]), 1);
     ptx::mbar_fence_init();
+  }
+  // In this order: what is launched on the trigger may then count on everything before this kernel being complete
+  // (the GEMM of a linear layer reads its weights at once).
+  ptx::grid_dependency_wait();
+  ptx::launch_dependents();
+  if (tid == 0) {
     for (int64_t i = 0; i < kStreamStages && i < my_tiles; ++i) issue(i);
   }
   __syncthreads();
@@ -355,6 +361,8 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
   __shared__ int s_abort;
   __shared__ int s_tiles_before[kMasked ? kMaskedMaxExperts + 1 : 1];  // tiles of the experts before e
   __shared__ int s_warp_sum[kStreamThreads / 32];
+  ptx::launch_dependents();
+  ptx::grid_dependency_wait();
   if (num_rows_dev != nullptr) {
     const int64_t lim = *num_rows_dev;
     rows = lim < rows ? lim : rows;
@@ -515,10 +523,9 @@ static int launch_quant_inst(const void* input, void* output_q, float* output_s,
   const int64_t tiles = (total_elems + kTileElems - 1) / kTileElems;
   const int64_t resident = (int64_t)sm_count() * (sizeof(T) == 4 ? 2 : 3);
   const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
-  kern<<<grid, kStreamThreads, smem, stream>>>(static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
+  SGLB_CUDA(launch_pdl(kern, grid, kStreamThreads, smem, stream, static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
                                                total_elems, groups_per_row, s_stride_token, s_stride_group, contiguous,
-                                               eps, qmin, qmax, g_stream_wait_probes);
-  SGLB_CUDA(cudaGetLastError());
+                                               eps, qmin, qmax, g_stream_wait_probes));
   return SGLB200_OK;
 }
 
@@ -560,10 +567,9 @@ static int launch_silu_mul_quant_kernel(const void* input, void* output_q, float
                                 : (rows * d + kTileElems - 1) / kTileElems;
   const int64_t resident = (int64_t)sm_count() * 3;
   const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
-  kern<<<grid, kStreamThreads, smem, stream>>>(static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
+  SGLB_CUDA(launch_pdl(kern, grid, kStreamThreads, smem, stream, static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
                                                rows, (int)d, num_rows_dev, eps, -448.0f, 448.0f, g_stream_wait_probes,
-                                               masked_m, num_experts, rows_per_expert);
-  SGLB_CUDA(cudaGetLastError());
+                                               masked_m, num_experts, rows_per_expert));
   return SGLB200_OK;
 }
 
