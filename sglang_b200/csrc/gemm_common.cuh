@@ -22,6 +22,10 @@ __device__ __forceinline__ void tile_coord(int t, int tiles_m, int tiles_n, int 
 // 128-byte swizzle, out-of-range elements read as zero.  Cached per argument tuple and thread.
 int get_tensor_map(const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t box_rows, uint32_t rank, CUtensorMap* out);
 
+// Output tensor [rows][N] of 2-byte elements, box = 64 columns x box_rows, 128-byte swizzle (matches the staging layout
+// written by the epilogues).  Cached likewise.
+int get_out_map(const void* ptr, uint64_t N, uint64_t rows, int out_fp16, uint32_t box_rows, CUtensorMap* out);
+
 // m-tiles per rasterization group for rows of K bytes (see gemm.cu).
 int choose_group_m(int64_t rows, int64_t K, int tile_rows);
 
@@ -36,7 +40,7 @@ int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, 
 // gemm_rows.cu: the dense product for few activation rows, and the expert-grouped one on rows sorted with a padding of
 // 16 (`cumsum` = padded starts of the buckets, as the sort writes them; bucket 0 = filtered ids is skipped).
 // `gather_topk` > 0: A and a_s have a row per token, fetched by sorted slot / gather_topk; 0: a row per sorted row.
-// `nt` = activation rows per tile: 16, 32, 64 or 128.
+// `nt` = activation rows per tile: 16, 32 or 64.
 int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
                   int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, bool after_quantizer,
                   cudaStream_t st);

@@ -43,7 +43,6 @@ struct RowsCfg {
 using Rows16 = RowsCfg<16, 4, 6, 8, 2>;
 using Rows32 = RowsCfg<32, 4, 5, 8, 2>;
 using Rows64 = RowsCfg<64, 4, 4, 4, 2>;
-using Rows128 = RowsCfg<128, 8, 6, 4, 1>;
 
 template <class Cfg>
 struct RowsCtl {
@@ -261,7 +260,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     constexpr int G = Cfg::kColGroups;
     const uint32_t bar_tfull0 = ptx::smem_u32(&ctl->tmem_full[0]), bar_tempty0 = ptx::smem_u32(&ctl->tmem_empty[0]);
     const uint32_t bar_sfull0 = ptx::smem_u32(&ctl->sc_full[0]), bar_sempty0 = ptx::smem_u32(&ctl->sc_empty[0]);
-    const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16) + h * kCW, sc0 = ptx::smem_u32(&ctl->sc[0][0][0]) + h * kCW * 4;
+    const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16) + h * kCW;
     ptx::grid_dependency_wait();
     uint32_t buf = 0, aph = 0, d = 0, dph = 0;
     bool alive = true;
@@ -285,7 +284,8 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
           break;
         }
         ptx::tc_fence_after();
-        const uint32_t taddr = taddr0 + buf * NT, sc = sc0 + (d * kScBatch + b) * (NT * 4);
+        const uint32_t taddr = taddr0 + buf * NT;
+        const float4* sc = reinterpret_cast<const float4*>(&ctl->sc[d][b][h * kCW]);
         if (active == 0 && lane == 0) ptx::mbar_arrive(bar_tempty0 + buf * 8);
 #pragma unroll
         for (int i = 0; i < kChunks; ++i) {
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
             }
 #pragma unroll
             for (int j = 0; j < kCW; j += 4) {
-              const float4 s4 = ptx::lds_f32x4(sc + (i * (G * kCW) + j) * 4);
+              const float4 s4 = sc[(i * (G * kCW) + j) / 4];
               ptx::fma2(acc[i][j], acc[i][j + 1], r[j], r[j + 1], s4.x, s4.y);
               ptx::fma2(acc[i][j + 2], acc[i][j + 3], r[j + 2], r[j + 3], s4.z, s4.w);
             }
@@ -527,8 +527,7 @@ int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b
   p.wait_probes = g_gemm_wait_probes;
   if (M <= 16) return rows_dense_cfg<Rows16>(A, B, p, K, after_quantizer, st);
   if (M <= 32) return rows_dense_cfg<Rows32>(A, B, p, K, after_quantizer, st);
-  if (M <= 64) return rows_dense_cfg<Rows64>(A, B, p, K, after_quantizer, st);
-  return rows_dense_cfg<Rows128>(A, B, p, K, after_quantizer, st);
+  return rows_dense_cfg<Rows64>(A, B, p, K, after_quantizer, st);
 }
 
 template <class Cfg>
@@ -562,7 +561,7 @@ int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const floa
     case 16: return rows_grouped_cfg<Rows16>(A, a_rows, B, p, max_rows, K, pdl, st);
     case 32: return rows_grouped_cfg<Rows32>(A, a_rows, B, p, max_rows, K, pdl, st);
     case 64: return rows_grouped_cfg<Rows64>(A, a_rows, B, p, max_rows, K, pdl, st);
-    default: return rows_grouped_cfg<Rows128>(A, a_rows, B, p, max_rows, K, pdl, st);
+    default: return fail(SGLB200_E_INVALID, "rows GEMM: %d rows per tile", nt);
   }
 }
 

@@ -1,5 +1,4 @@
-// Shared parts of the kernels whose M side is the weights (gemm_rows.cu: one CTA per tile; gemm_pair.cu: CTA pairs):
-// launch parameters, the walk over tiles, the count of the experts' token tiles.
+// Parts of gemm_rows.cu: launch parameters, the walk over tiles, the count of the experts' token tiles.
 #pragma once
 #include "common.cuh"
 #include "gemm_common.cuh"
