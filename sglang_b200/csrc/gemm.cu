@@ -215,37 +215,6 @@ __device__ __forceinline__ Unit decode_unit(const GemmParams& p, int u) {
   return x;
 }
 
-template <typename OutT, int kCols>
-__device__ __forceinline__ void store_row_chunk(OutT* dst, const float* v, const void* bias_v, int n0, int N) {
-  // up to kCols consecutive columns starting at n0 and ending before N, 8 per 16-byte store
-#pragma unroll
-  for (int j = 0; j < kCols / 8; ++j) {
-    const int n = n0 + j * 8;
-    if (n + 8 <= N) {
-      float x[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = v[j * 8 + i];
-      if (bias_v != nullptr) {
-        const uint4 braw = __ldg(reinterpret_cast<const uint4*>(static_cast<const OutT*>(bias_v) + n));
-        const OutT* b = reinterpret_cast<const OutT*>(&braw);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] += ElemTraits<OutT>::to_f32(b[i]);
-      }
-      uint4 raw;
-      OutT* o = reinterpret_cast<OutT*>(&raw);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = ElemTraits<OutT>::from_f32(x[i]);
-      *reinterpret_cast<uint4*>(dst + j * 8) = raw;
-    } else {
-      for (int i = 0; i < 8 && n + i < N; ++i) {
-        float x = v[j * 8 + i];
-        if (bias_v != nullptr) x += ElemTraits<OutT>::to_f32(static_cast<const OutT*>(bias_v)[n + i]);
-        dst[j * 8 + i] = ElemTraits<OutT>::from_f32(x);
-      }
-    }
-  }
-}
-
 template <bool kGrouped, int BN_>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     fp8_blockscale_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -750,24 +719,49 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         SGLB_STAMP(6);
         continue;
       }
-      int64_t out_row = row;
-      bool store_ok = row < rows;
-      if (kGrouped && p.scatter) {
-        const int32_t id = store_ok ? p.sorted_ids[row] : -1;
-        store_ok = id >= 0 && id < p.numel;
-        out_row = id;
-        if (store_ok && p.row_weights != nullptr) {
-          const float w = __ldg(p.row_weights + id);
+      // Grouped scatter: the rows go to the token-major slots that sorted_token_ids names.  Through this warp's part of the
+      // staging area (same layout), so that every store instruction writes 128 contiguous bytes of four rows; stored
+      // row by row from the accumulators, each lane wrote 16 bytes of its own row at a time, half a sector.
+      int dst = -1;
+      if (kGrouped && row < rows) {
+        const int32_t id = p.sorted_ids[row];
+        if (id >= 0 && id < p.numel) {
+          dst = id;
+          if (p.row_weights != nullptr) {
+            const float w = __ldg(p.row_weights + id);
 #pragma unroll
-          for (int j = 0; j < kEpiCols; ++j) acc[j] *= w;
+            for (int j = 0; j < kEpiCols; ++j) acc[j] *= w;
+          }
         }
       }
-      if (store_ok && n0 < n_end) {
-        if (p.out_fp16) {
-          store_row_chunk<__half, kEpiCols>(static_cast<__half*>(p.C) + out_row * p.N + n0, acc, p.bias, n0, n_end);
-        } else {
-          store_row_chunk<__nv_bfloat16, kEpiCols>(static_cast<__nv_bfloat16*>(p.C) + out_row * p.N + n0, acc, p.bias, n0,
-                                                   n_end);
+      const uint32_t stage0 = ptx::smem_u32(out_stage) + cgrp * (kEpiCols / 64) * kOutGroupBytes + q * 32 * 128;
+#pragma unroll
+      for (int g = 0; g < kEpiCols / 64; ++g) {
+        const uint32_t stage = stage0 + g * kOutGroupBytes;
+        __syncwarp();  // the part has been read
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          uint32_t word[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float v0 = acc[g * 64 + j * 8 + 2 * k], v1 = acc[g * 64 + j * 8 + 2 * k + 1];
+            if (p.out_fp16) {
+              const __half2 o = __floats2half2_rn(v0, v1);
+              word[k] = *reinterpret_cast<const uint32_t*>(&o);
+            } else {
+              const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
+              word[k] = *reinterpret_cast<const uint32_t*>(&o);
+            }
+          }
+          ptx::sts_128(stage + lane * 128 + ((j ^ (lane & 7)) << 4), make_uint4(word[0], word[1], word[2], word[3]));
+        }
+        __syncwarp();
+        const int piece = lane & 7, n = n0 + g * 64 + piece * 8;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r4 = k * 4 + (lane >> 3), to = __shfl_sync(0xffffffffu, dst, r4);
+          const uint4 v = ptx::lds_128(stage + r4 * 128 + ((piece ^ (r4 & 7)) << 4));
+          if (to >= 0 && n < n_end) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.C) + (int64_t)to * p.N + n) = v;
         }
       }
     }
