@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         continue;
       }
-      if (p.tma_out) {
+      if (!kGrouped || p.tma_out) {  // (dense tiles always leave this way)
         // Rows of C are contiguous: round to the output type, park the warp's 32 x 64 block in shared memory
         // (128-byte rows, 16-byte chunks XOR-swizzled by the row so that the 32 lanes of a store spread over
         // all banks); the storing thread (warp 2) hands the 128 x 64 blocks to the TMA engine, which clips them to
@@ -722,46 +722,48 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       // Grouped scatter: the rows go to the token-major slots that sorted_token_ids names.  Through this warp's part of the
       // staging area (same layout), so that every store instruction writes 128 contiguous bytes of four rows; stored
       // row by row from the accumulators, each lane wrote 16 bytes of its own row at a time, half a sector.
-      int dst = -1;
-      if (kGrouped && row < rows) {
-        const int32_t id = p.sorted_ids[row];
-        if (id >= 0 && id < p.numel) {
-          dst = id;
-          if (p.row_weights != nullptr) {
-            const float w = __ldg(p.row_weights + id);
+      if constexpr (kGrouped) {
+        int dst = -1;
+        if (row < rows) {
+          const int32_t id = p.sorted_ids[row];
+          if (id >= 0 && id < p.numel) {
+            dst = id;
+            if (p.row_weights != nullptr) {
+              const float w = __ldg(p.row_weights + id);
 #pragma unroll
-            for (int j = 0; j < kEpiCols; ++j) acc[j] *= w;
-          }
-        }
-      }
-      const uint32_t stage0 = ptx::smem_u32(out_stage) + cgrp * (kEpiCols / 64) * kOutGroupBytes + q * 32 * 128;
-#pragma unroll
-      for (int g = 0; g < kEpiCols / 64; ++g) {
-        const uint32_t stage = stage0 + g * kOutGroupBytes;
-        __syncwarp();  // the part has been read
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          uint32_t word[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float v0 = acc[g * 64 + j * 8 + 2 * k], v1 = acc[g * 64 + j * 8 + 2 * k + 1];
-            if (p.out_fp16) {
-              const __half2 o = __floats2half2_rn(v0, v1);
-              word[k] = *reinterpret_cast<const uint32_t*>(&o);
-            } else {
-              const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
-              word[k] = *reinterpret_cast<const uint32_t*>(&o);
+              for (int j = 0; j < kEpiCols; ++j) acc[j] *= w;
             }
           }
-          ptx::sts_128(stage + lane * 128 + ((j ^ (lane & 7)) << 4), make_uint4(word[0], word[1], word[2], word[3]));
         }
-        __syncwarp();
-        const int piece = lane & 7, n = n0 + g * 64 + piece * 8;
+        const uint32_t stage0 = ptx::smem_u32(out_stage) + cgrp * (kEpiCols / 64) * kOutGroupBytes + q * 32 * 128;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int r4 = k * 4 + (lane >> 3), to = __shfl_sync(0xffffffffu, dst, r4);
-          const uint4 v = ptx::lds_128(stage + r4 * 128 + ((piece ^ (r4 & 7)) << 4));
-          if (to >= 0 && n < n_end) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.C) + (int64_t)to * p.N + n) = v;
+        for (int g = 0; g < kEpiCols / 64; ++g) {
+          const uint32_t stage = stage0 + g * kOutGroupBytes;
+          __syncwarp();  // the part has been read
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            uint32_t word[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float v0 = acc[g * 64 + j * 8 + 2 * k], v1 = acc[g * 64 + j * 8 + 2 * k + 1];
+              if (p.out_fp16) {
+                const __half2 o = __floats2half2_rn(v0, v1);
+                word[k] = *reinterpret_cast<const uint32_t*>(&o);
+              } else {
+                const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
+                word[k] = *reinterpret_cast<const uint32_t*>(&o);
+              }
+            }
+            ptx::sts_128(stage + lane * 128 + ((j ^ (lane & 7)) << 4), make_uint4(word[0], word[1], word[2], word[3]));
+          }
+          __syncwarp();
+          const int piece = lane & 7, n = n0 + g * 64 + piece * 8;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int r4 = k * 4 + (lane >> 3), to = __shfl_sync(0xffffffffu, dst, r4);
+            const uint4 v = ptx::lds_128(stage + r4 * 128 + ((piece ^ (r4 & 7)) << 4));
+            if (to >= 0 && n < n_end) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.C) + (int64_t)to * p.N + n) = v;
+          }
         }
       }
     }
