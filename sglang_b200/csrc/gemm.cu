@@ -1245,13 +1245,15 @@ using namespace sglb200;
 extern "C" int sglb200_gemm_status_clear(void) {
   const int zero = 0;
   SGLB_CUDA(cudaMemcpyToSymbol(g_gemm_status, &zero, sizeof(int)));
-  return rows_gemm_status_clear();
+  const int rc = rows_gemm_status_clear();
+  return rc != SGLB200_OK ? rc : small_linear_status_clear();
 }
 
 extern "C" int sglb200_gemm_status(void) {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, g_gemm_status, sizeof(int)) != cudaSuccess) return -1;
-  return v != 0 ? v : rows_gemm_status();
+  if (v == 0) v = rows_gemm_status();
+  return v != 0 ? v : small_linear_status();
 }
 
 extern "C" void sglb200_gemm_set_wait_probes(uint32_t probes) { g_gemm_wait_probes = probes == 0 ? ptx::kProbeLimit : probes; }

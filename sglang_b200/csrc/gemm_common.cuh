@@ -31,6 +31,14 @@ int choose_group_m(int64_t rows, int64_t K, int tile_rows);
 
 extern uint32_t g_gemm_wait_probes;  // probes after which a pipeline wait gives up (sglb200_gemm_set_wait_probes)
 
+// quant.cu: the quantizers (arguments as the C ABI's).  `trigger`: the launch that follows may be scheduled early, as the
+// outputs are this call's own intermediates (see quant.cu).
+int quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s, int64_t num_tokens, int64_t hidden,
+              int group_size, float eps, float fp8_min, float fp8_max, int64_t s_stride_token, int64_t s_stride_group,
+              bool trigger, cudaStream_t st);
+int silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s, int64_t rows, int64_t d, int group_size,
+                       float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t st);
+
 // gemm.cu: the dense product (arguments as sglb200_fp8_blockwise_scaled_mm).  `after_quantizer`: the kernel before it in
 // the stream is this library's quantizer, launched by the same call, so that the weights may be fetched while that runs.
 int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M, int64_t N,
@@ -48,6 +56,13 @@ int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const floa
                     const int32_t* cumsum, const int32_t* sorted_ids, const float* row_weights, int64_t max_rows,
                     int64_t numel, int num_experts, int64_t N, int64_t K, int gather_topk, int scatter, int out_dtype, int nt,
                     bool pdl, cudaStream_t st);
+
+// gemm_small.cu: quantise + multiply in one launch; whether a problem is one for it.
+bool small_linear_fits(int64_t M, int64_t N, int64_t K);
+int small_linear(const void* x, int dtype, const void* B, const float* b_s, void* C, const void* bias, int64_t M, int64_t N,
+                 int64_t K, cudaStream_t st);
+int small_linear_status();
+int small_linear_status_clear();
 
 // gemm_rows.cu: status word of its kernels (0 ok, 1 a wait expired, -1 not readable), and its reset.
 int rows_gemm_status();

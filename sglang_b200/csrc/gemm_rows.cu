@@ -389,41 +389,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     __syncwarp();
     ptx::cluster_sync();
     const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, tile_first);
-    if (ctl->abort_flag == 0) {
-      // CTA `rank` adds columns rank, rank + splits, ..; a thread adds two neighbouring weight rows of a column
-      const int mine = (x.n_eff - rank + splits - 1) / splits;
-      const uint32_t part = ptx::smem_u32(tiles);
-      for (int i = tid; i < mine * (kRowsBM / 2); i += Cfg::kThreads) {
-        const int col = rank + (i / (kRowsBM / 2)) * splits, pair = i % (kRowsBM / 2);
-        const int n = x.n_tile * kRowsBM + pair * 2, row = x.row0 + col;
-        if (n >= p.N || row >= p.M) continue;
-        float2 v[kMaxSplits];
-#pragma unroll
-        for (int s = 0; s < kMaxSplits; ++s)  // all requested before the first is added
-          if (s < splits) v[s] = ptx::lds_cluster_f32x2(ptx::cluster_map(part + (col * kRowsBM + pair * 2) * 4, s));
-        float a = v[0].x, b = v[0].y;
-#pragma unroll
-        for (int s = 1; s < kMaxSplits; ++s)
-          if (s < splits) a += v[s].x, b += v[s].y;
-        uint32_t word;
-        if (p.out_fp16) {
-          if (p.bias != nullptr) {
-            const __half* bs = static_cast<const __half*>(p.bias) + n;
-            a += __half2float(bs[0]), b += __half2float(bs[1]);
-          }
-          const __half2 o = __floats2half2_rn(a, b);
-          word = *reinterpret_cast<const uint32_t*>(&o);
-        } else {
-          if (p.bias != nullptr) {
-            const __nv_bfloat16* bs = static_cast<const __nv_bfloat16*>(p.bias) + n;
-            a += __bfloat162float(bs[0]), b += __bfloat162float(bs[1]);
-          }
-          const __nv_bfloat162 o = __floats2bfloat162_rn(a, b);
-          word = *reinterpret_cast<const uint32_t*>(&o);
-        }
-        *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + n) = word;
-      }
-    }
+    if (ctl->abort_flag == 0) rows_cluster_sum<kMaxSplits>(p, x, rank, ptx::smem_u32(tiles), tid, Cfg::kThreads);
     ptx::cluster_sync();  // no CTA leaves while another reads its shared memory
   }
 

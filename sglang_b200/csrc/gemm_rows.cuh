@@ -1,4 +1,4 @@
-// Parts of gemm_rows.cu: launch parameters, the walk over tiles, the count of the experts' token tiles.
+// Shared by the kernels with the weights on the M side (gemm_rows.cu, gemm_small.cu): launch parameters, the walk over tiles, the count of the experts' token tiles.
 #pragma once
 #include "common.cuh"
 #include "gemm_common.cuh"
@@ -97,6 +97,46 @@ __device__ __forceinline__ void rows_count_tiles(const RowsParams& p, int* tiles
     before += cnt[k];
   }
   if (tid == NTHREADS - 1) tiles_before[p.num_experts] = before;  // (experts beyond num_experts count 0)
+}
+
+// The output of a tile whose K range was split over the CTAs of a cluster (at most kMost): sums their partial sums
+// ([column][weight row] of float32 at `part` in every CTA's shared memory) in ascending K order, adds the bias, rounds once.
+template <int kMost>
+__device__ __forceinline__ void rows_cluster_sum(const RowsParams& p, const RowsTile& x, int rank, uint32_t part, int tid,
+                                                 int threads) {
+  const int splits = p.splits;
+  // CTA `rank` adds columns rank, rank + splits, ..; a thread adds two neighbouring weight rows of a column
+  const int mine = (x.n_eff - rank + splits - 1) / splits;
+  for (int i = tid; i < mine * (kRowsBM / 2); i += threads) {
+    const int col = rank + (i / (kRowsBM / 2)) * splits, pair = i % (kRowsBM / 2);
+    const int n = x.n_tile * kRowsBM + pair * 2, row = x.row0 + col;
+    if (n >= p.N || row >= p.M) continue;
+    float2 v[kMost];
+#pragma unroll
+    for (int s = 0; s < kMost; ++s)  // all requested before the first is added
+      if (s < splits) v[s] = ptx::lds_cluster_f32x2(ptx::cluster_map(part + (col * kRowsBM + pair * 2) * 4, s));
+    float a = v[0].x, b = v[0].y;
+#pragma unroll
+    for (int s = 1; s < kMost; ++s)
+      if (s < splits) a += v[s].x, b += v[s].y;
+    uint32_t word;
+    if (p.out_fp16) {
+      if (p.bias != nullptr) {
+        const __half* bs = static_cast<const __half*>(p.bias) + n;
+        a += __half2float(bs[0]), b += __half2float(bs[1]);
+      }
+      const __half2 o = __floats2half2_rn(a, b);
+      word = *reinterpret_cast<const uint32_t*>(&o);
+    } else {
+      if (p.bias != nullptr) {
+        const __nv_bfloat16* bs = static_cast<const __nv_bfloat16*>(p.bias) + n;
+        a += __bfloat162float(bs[0]), b += __bfloat162float(bs[1]);
+      }
+      const __nv_bfloat162 o = __floats2bfloat162_rn(a, b);
+      word = *reinterpret_cast<const uint32_t*>(&o);
+    }
+    *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + n) = word;
+  }
 }
 
 #define ROWS_WAIT(bar, parity) \

@@ -203,9 +203,10 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int64_t bytes = abi.sglb200_block_fp8_linear_workspace_bytes(M, N, K);
     c10::DimVector shape(x.sizes().begin(), x.sizes().end());
     shape.back() = N;
-    Tensor out = make(shape, x.scalar_type(), x.device()), mem = workspace(bytes, x.device());
+    Tensor out = make(shape, x.scalar_type(), x.device()), mem;
+    if (bytes) mem = workspace(bytes, x.device());
     const int rc = abi.sglb200_block_fp8_linear(x.data_ptr(), dt, w->data_ptr(), static_cast<const float*>(ws->data_ptr()), out.data_ptr(),
-                                                bias ? bias->data_ptr() : nullptr, M, N, K, mem.data_ptr(), bytes, stream_of(x));
+                                                bias ? bias->data_ptr() : nullptr, M, N, K, bytes ? mem.data_ptr() : nullptr, bytes, stream_of(x));
     if (rc) return raise_last(rc);
     return THPVariable_Wrap(std::move(out));
   });

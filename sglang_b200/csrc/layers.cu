@@ -25,7 +25,8 @@ struct LinearParts {
   int64_t q, s, gemm, gemm_bytes, total;
 };
 static LinearParts linear_parts(int64_t M, int64_t N, int64_t K) {
-  LinearParts x;
+  LinearParts x{};
+  if (small_linear_fits(M, N, K)) return x;  // no intermediates
   Carver c;
   x.q = c.take(M * K);
   x.s = c.take(M * (K / 128) * 4);
@@ -92,14 +93,20 @@ extern "C" int sglb200_block_fp8_linear(const void* x, int dtype, const void* W,
                (long long)M, (long long)N, (long long)K);
   SGLB_REQUIRE(dtype == 0 || dtype == 1, "block_fp8_linear: dtype %d (0 bf16, 1 fp16)", dtype);
   if (M == 0) return SGLB200_OK;
+  if (small_linear_fits(M, N, K)) {
+    SGLB_REQUIRE(x && W && w_s && C, "block_fp8_linear: null pointer");
+    SGLB_REQUIRE(N % 8 == 0 && aligned16(x) && aligned16(W) && aligned16(C),
+                 "block_fp8_linear: N=%lld must be a multiple of 8, x, W and C 16-byte aligned", (long long)N);
+    return small_linear(x, dtype, W, w_s, C, bias, M, N, K, static_cast<cudaStream_t>(stream));
+  }
   const LinearParts lp = linear_parts(M, N, K);
   if (workspace == nullptr || !aligned16(workspace) || workspace_bytes < lp.total)
     return fail(SGLB200_E_WORKSPACE, "block_fp8_linear: workspace of %lld bytes required, got %lld", (long long)lp.total,
                 (long long)workspace_bytes);
   char* base = static_cast<char*>(workspace);
   float* xs = reinterpret_cast<float*>(base + lp.s);
-  const int rc = sglb200_per_token_group_quant_fp8(x, dtype, base + lp.q, xs, M, K, 128, kQuantEps, -kFp8Max, kFp8Max, K / 128, 1,
-                                                   stream);
+  const int rc = quant_fp8(x, dtype, base + lp.q, xs, M, K, 128, kQuantEps, -kFp8Max, kFp8Max, K / 128, 1, true,
+                           static_cast<cudaStream_t>(stream));
   if (rc) return rc;
   return scaled_mm(base + lp.q, W, xs, w_s, C, bias, M, N, K, K / 128, 1, dtype, base + lp.gemm, lp.gemm_bytes, true,
                    static_cast<cudaStream_t>(stream));
@@ -134,7 +141,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   void* ic3 = p.direct ? out : base + p.ic3;
   const int64_t hb = H / 128, ib = I / 128;
-  int rc = sglb200_per_token_group_quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, stream);
+  int rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
   if (rc) return rc;
   rc = sglb200_moe_align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
                                     p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, stream);
@@ -144,7 +151,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     rc = rows_grouped_mm(base + p.q, T, hb, f(p.s), w13, w13_s, base + p.ic1, i(p.cum), i(p.sorted), nullptr, p.rows, numel, (int)E,
                          2 * I, H, (int)k, 0, dtype, p.tile, true, st);
     if (rc) return rc;
-    rc = sglb200_silu_and_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), stream);
+    rc = silu_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), true, st);
     if (rc) return rc;
     rc = rows_grouped_mm(base + p.a2, p.rows, ib, f(p.a2s), w2, w2_s, ic3, i(p.cum), i(p.sorted), topk_weights, p.rows, numel,
                          (int)E, Ho, I, 0, 1, dtype, p.tile, true, st);
@@ -155,7 +162,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     rc = sglb200_fp8_blockwise_grouped_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.ic1, i(p.sorted), i(p.eid), i(p.post), nullptr,
                                           p.rows, numel, (int)E, 2 * I, H, 0, dtype, stream);
     if (rc) return rc;
-    rc = sglb200_silu_and_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), stream);
+    rc = silu_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), true, st);
     if (rc) return rc;
     rc = sglb200_fp8_blockwise_grouped_mm(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights,
                                           p.rows, numel, (int)E, Ho, I, 1, dtype, stream);

@@ -188,7 +188,6 @@ __global__ void __launch_bounds__(256)
                        float* __restrict__ dst_s, const int32_t* __restrict__ sorted_ids,
                        const int32_t* __restrict__ num_rows_dev, int64_t numel, int topk, int vecs_per_row,
                        int groups, int pieces_per_row) {
-  ptx::launch_dependents();
   ptx::grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const int64_t items = (int64_t)*num_rows_dev * pieces_per_row, step = (int64_t)gridDim.x * 8;

@@ -11,6 +11,7 @@
 //   amax  = max(|x|, eps)            scale = amax / fp8_max      (div.rn.f32)
 //   code  = cvt.rn.satfinite.e4m3( min(max(x / scale, fp8_min), fp8_max) )   (div.rn.f32)
 #include "common.cuh"
+#include "gemm_common.cuh"
 #include "ptx_sm100.cuh"
 #include "quant_math.cuh"
 
@@ -68,7 +69,7 @@ template <typename T, int LPG, bool kStdRange>
 __global__ void __launch_bounds__(kStreamThreads, 3)
     quant_stream_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q, float* __restrict__ out_s,
                         int64_t total_elems, int groups_per_row, int64_t s_stride_token, int64_t s_stride_group,
-                        bool s_contiguous, float eps, float qmin, float qmax, uint32_t probes) {
+                        bool s_contiguous, float eps, float qmin, float qmax, uint32_t probes, bool trigger) {
   constexpr int CE = Chunk<T>::kElems, NCH = Chunk<T>::kPerThread, GC = LPG * NCH;
   constexpr int G = LPG * kThreadElems;
   constexpr int kStreamStages = kStagesOf<T>;
@@ -98,9 +99,10 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
     ptx::mbar_fence_init();
   }
   // In this order: what is launched on the trigger may then count on everything before this kernel being complete
-  // (the GEMM of a linear layer reads its weights at once).
+  // (the GEMM of a linear layer reads its weights at once).  A kernel that writes e4m3 codes or block scales for the
+  // caller does not trigger: the codes could be the weights of the layer that follows.
   ptx::grid_dependency_wait();
-  ptx::launch_dependents();
+  if (trigger) ptx::launch_dependents();
   if (tid == 0) {
     for (int64_t i = 0; i < kStreamStages && i < my_tiles; ++i) issue(i);
   }
@@ -194,7 +196,7 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
     silu_mul_quant_stream_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q, float* __restrict__ out_s,
                                  int64_t rows, int d, const int32_t* __restrict__ num_rows_dev, float eps, float qmin,
                                  float qmax, uint32_t probes, const int32_t* __restrict__ masked_m, int num_experts,
-                                 int64_t rows_per_expert) {
+                                 int64_t rows_per_expert, bool trigger) {
   static_assert(sizeof(T) == 2, "16-bit inputs only");
   constexpr int CE = 8, NCH = 4, GC = LPG * NCH, G = LPG * kThreadElems;
   constexpr uint32_t kHalfBytes = kTileElems * 2;  // gate part of a stage; the up part follows it
@@ -203,7 +205,7 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
   __shared__ int s_abort;
   __shared__ int s_tiles_before[kMasked ? kMaskedMaxExperts + 1 : 1];  // tiles of the experts before e
   __shared__ int s_warp_sum[kStreamThreads / 32];
-  ptx::launch_dependents();
+  if (trigger) ptx::launch_dependents();
   ptx::grid_dependency_wait();
   if (num_rows_dev != nullptr) {
     const int64_t lim = *num_rows_dev;
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
 template <typename T, int LPG, bool kStd>
 static int launch_quant_inst(const void* input, void* output_q, float* output_s, int64_t total_elems,
                              int groups_per_row, int64_t s_stride_token, int64_t s_stride_group, bool contiguous,
-                             float eps, float qmin, float qmax, cudaStream_t stream) {
+                             float eps, float qmin, float qmax, bool trigger, cudaStream_t stream) {
   constexpr size_t smem = (size_t)kStagesOf<T> * kTileElems * sizeof(T);
   auto kern = quant_stream_kernel<T, LPG, kStd>;
   // opt in to the ring's dynamic shared memory (a per-function, per-device attribute; cheap to repeat)
@@ -367,14 +369,14 @@ static int launch_quant_inst(const void* input, void* output_q, float* output_s,
   const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
   SGLB_CUDA(launch_pdl(kern, grid, kStreamThreads, smem, stream, static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
                                                total_elems, groups_per_row, s_stride_token, s_stride_group, contiguous,
-                                               eps, qmin, qmax, g_stream_wait_probes));
+                                               eps, qmin, qmax, g_stream_wait_probes, trigger));
   return SGLB200_OK;
 }
 
 template <typename T>
 static int launch_quant(const void* input, void* output_q, float* output_s, int64_t num_tokens, int64_t hidden,
                         int group_size, float eps, float qmin, float qmax, int64_t s_stride_token,
-                        int64_t s_stride_group, cudaStream_t stream) {
+                        int64_t s_stride_group, bool trigger, cudaStream_t stream) {
   const int64_t total = num_tokens * hidden;
   const int groups_per_row = (int)(hidden / group_size);
   const bool contiguous = (s_stride_group == 1 && s_stride_token == groups_per_row);
@@ -382,10 +384,10 @@ static int launch_quant(const void* input, void* output_q, float* output_s, int6
   const bool std_range = (qmin == -448.0f && qmax == 448.0f);
 #define SGLB_LAUNCH_Q(LPG)                                                                                          \
   return std_range ? launch_quant_inst<T, LPG, true>(input, output_q, output_s, total, groups_per_row,              \
-                                                     s_stride_token, s_stride_group, contiguous, eps, qmin, qmax,   \
+                                                     s_stride_token, s_stride_group, contiguous, eps, qmin, qmax, trigger,   \
                                                      stream)                                                        \
                    : launch_quant_inst<T, LPG, false>(input, output_q, output_s, total, groups_per_row,             \
-                                                      s_stride_token, s_stride_group, contiguous, eps, qmin, qmax,  \
+                                                      s_stride_token, s_stride_group, contiguous, eps, qmin, qmax, trigger,  \
                                                       stream)
   switch (group_size) {
     case 32: SGLB_LAUNCH_Q(1);
@@ -400,7 +402,7 @@ static int launch_quant(const void* input, void* output_q, float* output_s, int6
 template <typename T, int LPG, bool kMasked>
 static int launch_silu_mul_quant_kernel(const void* input, void* output_q, float* output_s, int64_t rows, int64_t d,
                                         float eps, const int32_t* num_rows_dev, const int32_t* masked_m,
-                                        int num_experts, int64_t rows_per_expert, cudaStream_t stream) {
+                                        int num_experts, int64_t rows_per_expert, bool trigger, cudaStream_t stream) {
   constexpr size_t smem = (size_t)kSiluStages * 2 * kTileElems * sizeof(T);
   auto kern = silu_mul_quant_stream_kernel<T, LPG, kMasked>;
   SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -411,32 +413,32 @@ static int launch_silu_mul_quant_kernel(const void* input, void* output_q, float
   const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
   SGLB_CUDA(launch_pdl(kern, grid, kStreamThreads, smem, stream, static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
                                                rows, (int)d, num_rows_dev, eps, -448.0f, 448.0f, g_stream_wait_probes,
-                                               masked_m, num_experts, rows_per_expert));
+                                               masked_m, num_experts, rows_per_expert, trigger));
   return SGLB200_OK;
 }
 
 template <typename T, int LPG>
 static int launch_silu_mul_quant_inst(const void* input, void* output_q, float* output_s, int64_t rows, int64_t d,
-                                      float eps, const int32_t* num_rows_dev, cudaStream_t stream,
+                                      float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t stream,
                                       const int32_t* masked_m = nullptr, int num_experts = 0,
                                       int64_t rows_per_expert = 0) {
   if (masked_m != nullptr)
     return launch_silu_mul_quant_kernel<T, LPG, true>(input, output_q, output_s, rows, d, eps, nullptr, masked_m,
-                                                      num_experts, rows_per_expert, stream);
+                                                      num_experts, rows_per_expert, trigger, stream);
   return launch_silu_mul_quant_kernel<T, LPG, false>(input, output_q, output_s, rows, d, eps, num_rows_dev, nullptr, 0, 0,
-                                                     stream);
+                                                     trigger, stream);
 }
 
 template <typename T>
 static int launch_silu_mul_quant(const void* input, void* output_q, float* output_s, int64_t rows, int64_t d,
-                                 int group_size, float eps, const int32_t* num_rows_dev, cudaStream_t stream) {
+                                 int group_size, float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t stream) {
   if (rows * d == 0) return SGLB200_OK;
   SGLB_REQUIRE(d < (1ll << 30), "silu_mul_quant: d %lld too large", (long long)d);
   switch (group_size) {
-    case 32: return launch_silu_mul_quant_inst<T, 1>(input, output_q, output_s, rows, d, eps, num_rows_dev, stream);
-    case 64: return launch_silu_mul_quant_inst<T, 2>(input, output_q, output_s, rows, d, eps, num_rows_dev, stream);
-    case 128: return launch_silu_mul_quant_inst<T, 4>(input, output_q, output_s, rows, d, eps, num_rows_dev, stream);
-    case 256: return launch_silu_mul_quant_inst<T, 8>(input, output_q, output_s, rows, d, eps, num_rows_dev, stream);
+    case 32: return launch_silu_mul_quant_inst<T, 1>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
+    case 64: return launch_silu_mul_quant_inst<T, 2>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
+    case 128: return launch_silu_mul_quant_inst<T, 4>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
+    case 256: return launch_silu_mul_quant_inst<T, 8>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
     default: return fail(SGLB200_E_INVALID, "silu_mul_quant: group_size %d not in {32,64,128,256}", group_size);
   }
 }
@@ -447,7 +449,7 @@ static int launch_silu_mul_quant_masked(const void* input, void* output_q, float
                                         const int32_t* masked_m, cudaStream_t stream) {
   const int64_t rows = (int64_t)num_experts * rows_per_expert;
 #define SGLB_MASKED(LPG)                                                                                         \
-  return launch_silu_mul_quant_inst<T, LPG>(input, output_q, output_s, rows, d, eps, nullptr, stream, masked_m, \
+  return launch_silu_mul_quant_inst<T, LPG>(input, output_q, output_s, rows, d, eps, nullptr, false, stream, masked_m, \
                                             num_experts, rows_per_expert)
   switch (group_size) {
     case 32: SGLB_MASKED(1);
@@ -490,10 +492,10 @@ extern "C" int sglb200_silu_and_mul_masked_quant_fp8(const void* input, int dtyp
   }
 }
 
-extern "C" int sglb200_per_token_group_quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s,
+int sglb200::quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s,
                                                  int64_t num_tokens, int64_t hidden, int group_size, float eps,
                                                  float fp8_min, float fp8_max, int64_t s_stride_token,
-                                                 int64_t s_stride_group, void* stream) {
+                                                 int64_t s_stride_group, bool trigger, cudaStream_t st) {
   SGLB_REQUIRE(num_tokens >= 0 && hidden > 0, "quantizer: bad shape [%lld, %lld]", (long long)num_tokens,
                (long long)hidden);
   SGLB_REQUIRE(group_size > 0 && hidden % group_size == 0, "quantizer: hidden %lld not divisible by group_size %d",
@@ -502,41 +504,54 @@ extern "C" int sglb200_per_token_group_quant_fp8(const void* input, int in_dtype
   SGLB_REQUIRE(input && output_q && output_s, "quantizer: null pointer");
   SGLB_REQUIRE(aligned16(input) && (reinterpret_cast<uintptr_t>(output_q) & 7u) == 0,
                "quantizer: input must be 16-byte and output_q 8-byte aligned");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (in_dtype) {
     case 0:
       return launch_quant<__nv_bfloat16>(input, output_q, output_s, num_tokens, hidden, group_size, eps, fp8_min,
-                                         fp8_max, s_stride_token, s_stride_group, st);
+                                         fp8_max, s_stride_token, s_stride_group, trigger, st);
     case 1:
       return launch_quant<__half>(input, output_q, output_s, num_tokens, hidden, group_size, eps, fp8_min, fp8_max,
-                                  s_stride_token, s_stride_group, st);
+                                  s_stride_token, s_stride_group, trigger, st);
     case 2:
       return launch_quant<float>(input, output_q, output_s, num_tokens, hidden, group_size, eps, fp8_min, fp8_max,
-                                 s_stride_token, s_stride_group, st);
+                                 s_stride_token, s_stride_group, trigger, st);
     default:
       return fail(SGLB200_E_UNSUPPORTED, "quantizer: dtype code %d (0 bf16, 1 fp16, 2 fp32)", in_dtype);
   }
 }
 
-extern "C" int sglb200_silu_and_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s,
+extern "C" int sglb200_per_token_group_quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s,
+                                                 int64_t num_tokens, int64_t hidden, int group_size, float eps,
+                                                 float fp8_min, float fp8_max, int64_t s_stride_token,
+                                                 int64_t s_stride_group, void* stream) {
+  return quant_fp8(input, in_dtype, output_q, output_s, num_tokens, hidden, group_size, eps, fp8_min, fp8_max, s_stride_token,
+                   s_stride_group, false, static_cast<cudaStream_t>(stream));
+}
+
+int sglb200::silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s,
                                               int64_t rows, int64_t d, int group_size, float eps,
-                                              const int32_t* num_rows_dev, void* stream) {
+                                              const int32_t* num_rows_dev, bool trigger, cudaStream_t st) {
   SGLB_REQUIRE(rows >= 0 && d > 0 && group_size > 0 && d % group_size == 0,
                "silu_mul_quant: bad shape rows=%lld d=%lld group=%d", (long long)rows, (long long)d, group_size);
   if (rows == 0) return SGLB200_OK;
   SGLB_REQUIRE(input && output_q && output_s, "silu_mul_quant: null pointer");
   SGLB_REQUIRE(aligned16(input) && (reinterpret_cast<uintptr_t>(output_q) & 7u) == 0,
                "silu_mul_quant: input must be 16-byte and output_q 8-byte aligned");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (dtype) {
     case 0:
       return launch_silu_mul_quant<__nv_bfloat16>(input, output_q, output_s, rows, d, group_size, eps, num_rows_dev,
-                                                  st);
+                                                  trigger, st);
     case 1:
-      return launch_silu_mul_quant<__half>(input, output_q, output_s, rows, d, group_size, eps, num_rows_dev, st);
+      return launch_silu_mul_quant<__half>(input, output_q, output_s, rows, d, group_size, eps, num_rows_dev, trigger, st);
     default:
       return fail(SGLB200_E_UNSUPPORTED, "silu_mul_quant: dtype code %d (0 bf16, 1 fp16)", dtype);
   }
+}
+
+extern "C" int sglb200_silu_and_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s,
+                                              int64_t rows, int64_t d, int group_size, float eps,
+                                              const int32_t* num_rows_dev, void* stream) {
+  return silu_mul_quant_fp8(input, dtype, output_q, output_s, rows, d, group_size, eps, num_rows_dev, false,
+                            static_cast<cudaStream_t>(stream));
 }
 
 extern "C" void sglb200_stream_set_wait_probes(uint32_t probes) {

@@ -1,0 +1,70 @@
+"""GPU parity of whole layers (quantised linear, routed experts) at the sizes where their dispatch or tiles can go wrong:
+edges of the 16/32/64-row tiles and of the step to 128-row tiles, K ranges that do not divide evenly over a cluster, N
+that does not fill a tile, experts with no rows and with many."""
+import pytest
+import torch
+
+from oracle import block_fp8_oracle as O
+from tests.util import assert_close_fp, codes_to_fp8, make_act, make_weight, to_f32_np
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33, 64, 65, 130])
+@pytest.mark.parametrize("N,K", [(8, 256), (264, 1152), (640, 7168), (2112, 512)])
+@pytest.mark.parametrize("dtype,bias", [(torch.bfloat16, False), (torch.float16, True)])
+def test_linear_row_counts(M, N, K, dtype, bias):
+    from sglang_b200 import ops
+    from sglang_b200.srt.layers.quantization.fp8_utils import b200_w8a8_block_fp8_linear
+    x = make_act(M, K, M + N, dtype=dtype)
+    wq, ws = make_weight(N, K, N + K)
+    b = torch.randn(N, generator=torch.Generator().manual_seed(5)).to(dtype) if bias else None
+    xq, xs = O.per_token_group_quant_fp8(to_f32_np(x))
+    ref = O.w8a8_block_fp8_matmul(xq, wq, xs, ws, out_bf16=False).astype("float32")
+    if bias:
+        ref = ref + to_f32_np(b)
+    out = b200_w8a8_block_fp8_linear(x.cuda(), codes_to_fp8(wq), [128, 128], torch.from_numpy(ws).cuda(),
+                                     bias=None if b is None else b.cuda())
+    assert ops.gemm_status() == 0 and ops.stream_status() == 0
+    assert_close_fp(to_f32_np(out), ref)
+
+
+# (tokens, experts, topk): on average 1 to some hundred rows per expert, so that every tile height of the dispatch is taken;
+# the ids are skewed towards expert 0 and leave some experts without rows
+@pytest.mark.parametrize("T,E,topk", [(1, 8, 8), (5, 32, 2), (16, 8, 1), (40, 16, 4), (70, 6, 3), (160, 8, 2), (333, 4, 2)])
+def test_experts_row_counts(T, E, topk):
+    from sglang_b200 import ops
+    from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
+    H, I = 384, 256
+    g = torch.Generator().manual_seed(T + E)
+    x = make_act(T, H, T, outliers=False)
+    w13q, w13s = make_weight(2 * I, H, 1, std=0.05, experts=E)
+    w2q, w2s = make_weight(H, I, 2, std=0.05, experts=E)
+    logits = torch.randn(T, E, generator=g) - 0.5 * torch.arange(E)
+    w, ids = torch.topk(torch.softmax(logits, -1), topk, dim=-1)
+    ids = ids.to(torch.int32)
+    ref = O.fused_experts_block_fp8(to_f32_np(x), w13q, w13s, w2q, w2s, w.numpy(), ids.numpy(), 1.0)
+    out = fused_experts_impl(
+        x.cuda(), codes_to_fp8(w13q), codes_to_fp8(w2q), w.cuda(), ids.cuda(), use_fp8_w8a8=True,
+        w1_scale=torch.from_numpy(w13s).cuda(), w2_scale=torch.from_numpy(w2s).cuda(), block_shape=[128, 128])
+    assert ops.gemm_status() == 0 and ops.stream_status() == 0
+    assert_close_fp(to_f32_np(out), ref, rtol=2e-2, atol=2e-2)
+
+
+def test_experts_one_slot_with_filtered_ids():
+    """top-1 with ids of -1: the second product writes the result itself and the filtered rows are zero."""
+    from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
+    T, E, H, I = 37, 4, 256, 128
+    x = make_act(T, H, 3, outliers=False)
+    w13q, w13s = make_weight(2 * I, H, 1, std=0.05, experts=E)
+    w2q, w2s = make_weight(H, I, 2, std=0.05, experts=E)
+    ids = torch.randint(-1, E, (T, 1), generator=torch.Generator().manual_seed(7)).to(torch.int32)
+    w = torch.rand(T, 1, generator=torch.Generator().manual_seed(8))
+    out = fused_experts_impl(
+        x.cuda(), codes_to_fp8(w13q), codes_to_fp8(w2q), w.cuda(), ids.cuda(), use_fp8_w8a8=True,
+        w1_scale=torch.from_numpy(w13s).cuda(), w2_scale=torch.from_numpy(w2s).cuda(), block_shape=[128, 128])
+    got = to_f32_np(out)
+    on = (ids[:, 0] >= 0).numpy()
+    ref = O.fused_experts_block_fp8(to_f32_np(x)[on], w13q, w13s, w2q, w2s, w.numpy()[on], ids.numpy()[on], 1.0)
+    assert (got[~on] == 0).all()
+    assert_close_fp(got[on], ref, rtol=2e-2, atol=2e-2)
