@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "ptx_sm100.cuh"
 
 namespace sglb200 {
 
@@ -202,6 +203,9 @@ __global__ void __launch_bounds__(kAlignThreads)
   int* prefix = tot + B;                // [B+1]
   int* scratch = prefix + B + 1;        // [33]
   for (int i = threadIdx.x; i < kAlignWarps * B; i += kAlignThreads) wc[i] = 0;
+  // (in this order: a kernel started on the trigger may count on everything before this one being complete)
+  ptx::grid_dependency_wait();
+  ptx::launch_dependents();
   __syncthreads();
   count_chunk(ids, 0, numel, span, B, wc);
   __syncthreads();
@@ -601,10 +605,8 @@ extern "C" int sglb200_moe_align_block_size(const int32_t* topk_ids, int64_t num
   int span = 0;
   align_plan(numel, &chunks, &span);
   if (chunks == 1) {
-    moe_align_single_kernel<<<1, kAlignThreads, smem, st>>>(topk_ids, numel, span, B, block_size, sorted_token_ids, expert_ids,
-                                                            num_tokens_post_pad, cumsum_buffer,
-                                                            pad_sorted_token_ids != 0);
-    SGLB_CUDA(cudaGetLastError());
+    SGLB_CUDA(launch_pdl(moe_align_single_kernel, 1, kAlignThreads, smem, st, topk_ids, numel, span, B, block_size,
+                         sorted_token_ids, expert_ids, num_tokens_post_pad, cumsum_buffer, pad_sorted_token_ids != 0));
     return SGLB200_OK;
   }
   const int64_t need = sglb200_moe_align_workspace_bytes(numel, num_experts);
