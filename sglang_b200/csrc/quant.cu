@@ -1,11 +1,12 @@
 // 1 x G activation quantizer (float8_e4m3fn codes + float32 scales) and the fused
 // silu_and_mul + quantizer, for sm_100a.
 //
-// Both are streaming kernels on one skeleton: persistent CTAs walk tiles of 8192 elements that one thread
-// stages with bulk copies (cp.async.bulk) into a ring of shared-memory buffers completing on mbarriers, so
-// the bytes in flight per SM do not depend on registers or occupancy; every input byte is read from HBM
-// once; a thread owns 32 elements of one group per tile, the group maximum takes two shuffle rounds, and
-// every quad of lanes writes one full 32-byte sector of codes.
+// Both are bound by HBM, and have two forms.  Direct: a thread loads 16 elements of one group straight into registers
+// (one 256-bit load for 16-bit types), the group maximum takes log2(G / 16) shuffles, and the 16 codes leave in one
+// 128-bit store; no shared memory and no barrier, so no warp waits for another.  Ring (large inputs of the quantizer,
+// masked expert batches of the activation): persistent CTAs walk tiles of 8192 elements that one thread stages with bulk
+// copies (cp.async.bulk) into a ring of shared-memory buffers completing on mbarriers, so the bytes in flight per SM do
+// not depend on registers or occupancy; a thread owns 32 elements of one group per tile.
 //
 // Arithmetic contract (bit-exact with the reference CUDA kernel built without fast-math):
 //   amax  = max(|x|, eps)            scale = amax / fp8_max      (div.rn.f32)
@@ -17,7 +18,7 @@
 
 namespace sglb200 {
 
-// ---- streaming skeleton shared by the quantizer and the fused activation + quantizer ----------------
+// ---- ring: streaming skeleton shared by the quantizer and the masked activation + quantizer --------------
 //
 // A CTA walks tiles of kTileElems consecutive elements (tile t, t + gridDim.x, ...).  One thread stages
 // each tile with a 1-D bulk copy (cp.async.bulk) into a ring of kStreamStages shared-memory buffers that
@@ -160,8 +161,131 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
   }
 }
 
-// Fused silu_and_mul + quantizer on the same skeleton.  x is [rows, 2d] (gate | up); a tile is kTileElems
-// consecutive OUTPUT elements of the flat [rows, d] result, staged as one or more (gate, up) pairs of row
+// ---- direct forms: values straight to registers ---------------------------------------------------------
+
+constexpr int kQuantThreads = 256;
+constexpr int kLaneElems = 16;                            // elements of one group that a thread owns
+constexpr int kUnitElems = kQuantThreads * kLaneElems;    // 4096
+
+// A thread's 16 elements: `wide` (32-byte aligned) in 256-bit loads, else in 128-bit ones.
+template <int N>
+__device__ __forceinline__ void load_lane(uint4* r, const void* p, bool wide) {
+  const uint8_t* b = static_cast<const uint8_t*>(p);
+  if (wide) {
+#pragma unroll
+    for (int j = 0; j < N; j += 2)
+      asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(r[j].x), "=r"(r[j].y), "=r"(r[j].z), "=r"(r[j].w), "=r"(r[j + 1].x), "=r"(r[j + 1].y),
+                     "=r"(r[j + 1].z), "=r"(r[j + 1].w)
+                   : "l"(b + j * 16));
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(r[j].x), "=r"(r[j].y), "=r"(r[j].z), "=r"(r[j].w)
+                   : "l"(b + j * 16));
+  }
+}
+__device__ __forceinline__ void store_lane(uint8_t* p, const uint32_t* c, bool wide) {
+  if (wide) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(c[0], c[1], c[2], c[3]);
+  } else {
+    reinterpret_cast<uint2*>(p)[0] = make_uint2(c[0], c[1]);
+    reinterpret_cast<uint2*>(p)[1] = make_uint2(c[2], c[3]);
+  }
+}
+// Quotient of a group index; almost always both fit 32 bits, and a 64-bit division is a function call.
+__device__ __forceinline__ int64_t div_groups(int64_t g, int per_row) {
+  return g < (1ll << 32) ? (int64_t)((uint32_t)g / (uint32_t)per_row) : g / per_row;
+}
+
+struct ScaleLayout {
+  int groups_per_row;
+  int64_t stride_token, stride_group;
+  bool contiguous;  // [token][group], dense
+};
+
+// The quantizer, direct form.  A thread has U units of 16 elements in flight.
+// kTiled: for scales with adjacent tokens in adjacent words (the GEMM's layout).  The flat order writes them one word
+// per sector; here a warp takes one group column and its groups are 32 / LPG adjacent tokens in each unit, so that one
+// store instruction writes U * 32 / LPG adjacent scales - for groups of 128 exactly one sector - while the eight warps
+// of a CTA still read 2 KB runs of every row.
+template <typename T, int LPG, bool kStdRange, int U, bool kTiled>
+__global__ void __launch_bounds__(kQuantThreads)
+    quant_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q, float* __restrict__ out_s, int64_t tokens,
+                 ScaleLayout sl, float eps, float qmin, float qmax, bool wide_in, bool wide_out, bool trigger) {
+  constexpr int CE = Chunk<T>::kElems, NCH = kLaneElems / CE, G = LPG * kLaneElems;
+  constexpr int kWarpGroups = 32 / LPG;
+  static_assert(U <= LPG, "one lane of the group stores each unit's scale");
+  // In this order: what is launched on the trigger may then count on everything before this kernel being complete
+  // (the GEMM of a linear layer reads its weights at once).  A kernel that writes e4m3 codes or block scales for the
+  // caller does not trigger: the codes could be the weights of the layer that follows.
+  ptx::grid_dependency_wait();
+  if (trigger) ptx::launch_dependents();
+  const int l = threadIdx.x % LPG, slot = (threadIdx.x & 31) / LPG, warp = threadIdx.x >> 5;
+  int64_t ge[U];  // first element of the thread's group in each unit, -1 beyond the end
+  int64_t row0 = 0;
+  int col = 0;
+  if constexpr (kTiled) {
+    constexpr int kCols = kQuantThreads / 32;
+    const int ktiles = (sl.groups_per_row + kCols - 1) / kCols;
+    const int rt = (int)((unsigned)blockIdx.x / (unsigned)ktiles);
+    col = ((int)blockIdx.x - rt * ktiles) * kCols + warp;
+    row0 = (int64_t)rt * (U * kWarpGroups) + slot;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t row = row0 + u * kWarpGroups;
+      ge[u] = row < tokens && col < sl.groups_per_row ? (row * sl.groups_per_row + col) * G : -1;
+    }
+  } else {
+    const int64_t groups = tokens * sl.groups_per_row;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t g = ((int64_t)blockIdx.x * U + u) * (kUnitElems / G) + warp * kWarpGroups + slot;
+      ge[u] = g < groups ? g * G : -1;
+    }
+  }
+  uint4 raw[U][NCH];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+#pragma unroll
+    for (int j = 0; j < NCH; ++j) raw[u][j] = make_uint4(0, 0, 0, 0);
+    if (ge[u] >= 0) load_lane<NCH>(raw[u], x + ge[u] + l * kLaneElems, wide_in);
+  }
+  float my_scale = 0.f;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    float v[kLaneElems];
+#pragma unroll
+    for (int j = 0; j < NCH; ++j) unpack_chunk<T>(raw[u][j], v + j * CE);
+    uint32_t codes[NCH][CE / 4];
+    const float scale = quant_group<T, LPG, kStdRange, NCH>(raw[u], v, eps, qmin, qmax, codes);
+    if (l == u) my_scale = scale;
+    if (ge[u] >= 0) store_lane(out_q + ge[u] + l * kLaneElems, &codes[0][0], wide_out);
+  }
+  if (l < U) {  // lane u of a group stores the scale of unit u
+    int64_t e = ge[0];
+#pragma unroll
+    for (int u = 1; u < U; ++u)
+      if (l == u) e = ge[u];
+    if (e >= 0) {
+      if constexpr (kTiled) {
+        out_s[col * sl.stride_group + row0 + l * kWarpGroups] = my_scale;
+      } else {
+        const int64_t g = e / G;
+        if (sl.contiguous) {
+          out_s[g] = my_scale;
+        } else {
+          const int64_t t = div_groups(g, sl.groups_per_row);
+          out_s[t * sl.stride_token + (g - t * sl.groups_per_row) * sl.stride_group] = my_scale;
+        }
+      }
+    }
+  }
+}
+
+// Fused silu_and_mul + quantizer.  x is [rows, 2d] (gate | up).  In the ring a tile is kTileElems consecutive OUTPUT
+// elements of an expert's flat [rows, d] result, staged as one or more (gate, up) pairs of row
 // segments.  h = T(T(silu(gate)) * up): silu in float32 rounded to T, then one packed multiply (the product of
 // two 16-bit floats is exact in float32, so its single rounding equals rounding the float32 product), then
 // the quantizer arithmetic on h in registers.
@@ -184,91 +308,129 @@ struct Packed2<__half> {
   }
 };
 
-constexpr int kSiluStages = 2;  // 2 x (16 KB gate + 16 KB up) per CTA, three CTAs per SM (80 registers)
-
-constexpr int kMaskedMaxExperts = 1024;  // experts of one masked call (four per thread in the tile count scan)
-
-// kMasked: the input is [experts, rows_per_expert, 2d] and only the first masked_m[e] rows of expert e are valid
-// (the layout of python/sglang/srt/layers/moe/ep_moe/kernels.py:287-361).  The valid rows of every expert are cut
-// into tiles of their own, numbered one expert after the other; rows beyond masked_m[e] are neither read nor written.
-template <typename T, int LPG, bool kMasked>
-__global__ void __launch_bounds__(kStreamThreads, 3)
-    silu_mul_quant_stream_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q, float* __restrict__ out_s,
-                                 int64_t rows, int d, const int32_t* __restrict__ num_rows_dev, float eps, float qmin,
-                                 float qmax, uint32_t probes, const int32_t* __restrict__ masked_m, int num_experts,
-                                 int64_t rows_per_expert, bool trigger) {
-  static_assert(sizeof(T) == 2, "16-bit inputs only");
-  constexpr int CE = 8, NCH = 4, GC = LPG * NCH, G = LPG * kThreadElems;
-  constexpr uint32_t kHalfBytes = kTileElems * 2;  // gate part of a stage; the up part follows it
-  extern __shared__ __align__(128) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[kSiluStages];
-  __shared__ int s_abort;
-  __shared__ int s_tiles_before[kMasked ? kMaskedMaxExperts + 1 : 1];  // tiles of the experts before e
-  __shared__ int s_warp_sum[kStreamThreads / 32];
+// Direct form: as the quantizer, 16 gate and 16 up values a thread and unit.
+template <typename T, int LPG, int U>
+__global__ void __launch_bounds__(kQuantThreads)
+    silu_mul_quant_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q, float* __restrict__ out_s, int64_t rows,
+                          int d, const int32_t* __restrict__ num_rows_dev, float eps, bool wide_in, bool wide_out,
+                          bool trigger) {
+  constexpr int CE = Chunk<T>::kElems, NCH = kLaneElems / CE, G = LPG * kLaneElems;
   if (trigger) ptx::launch_dependents();
   ptx::grid_dependency_wait();
   if (num_rows_dev != nullptr) {
     const int64_t lim = *num_rows_dev;
     rows = lim < rows ? lim : rows;
   }
+  const int per_row = d / G, l = threadIdx.x % LPG;
+  const int64_t groups = rows * per_row;
+  const int64_t g0 = (int64_t)blockIdx.x * (U * (kUnitElems / G)) + threadIdx.x / LPG;
+  if (g0 - threadIdx.x / LPG >= groups) return;  // the grid is sized from the host-side bound on rows
+  uint4 graw[U][NCH], uraw[U][NCH];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+#pragma unroll
+    for (int j = 0; j < NCH; ++j) graw[u][j] = uraw[u][j] = make_uint4(0, 0, 0, 0);
+    const int64_t g = g0 + u * (kUnitElems / G);
+    if (g < groups) {
+      const T* gate = x + g * G + div_groups(g, per_row) * d + l * kLaneElems;
+      load_lane<NCH>(graw[u], gate, wide_in);
+      load_lane<NCH>(uraw[u], gate + d, wide_in);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    uint4 hraw[NCH];
+    float v[kLaneElems];
+#pragma unroll
+    for (int j = 0; j < NCH; ++j) {
+      float g[CE];
+      unpack_chunk<T>(graw[u][j], g);
+      const uint32_t up[4] = {uraw[u][j].x, uraw[u][j].y, uraw[u][j].z, uraw[u][j].w};
+      uint32_t h[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) h[k] = Packed2<T>::round_mul(silu_f32(g[2 * k]), silu_f32(g[2 * k + 1]), up[k]);
+      hraw[j] = make_uint4(h[0], h[1], h[2], h[3]);
+      unpack_chunk<T>(hraw[j], v + j * CE);
+    }
+    uint32_t codes[NCH][CE / 4];
+    const float scale = quant_group<T, LPG, true, NCH>(hraw, v, eps, -448.0f, 448.0f, codes);
+    const int64_t g = g0 + u * (kUnitElems / G);
+    if (g < groups) {
+      store_lane(out_q + g * G + l * kLaneElems, &codes[0][0], wide_out);
+      if (l == 0) out_s[g] = scale;
+    }
+  }
+}
+
+constexpr int kSiluStages = 2;  // 2 x (16 KB gate + 16 KB up) per CTA, three CTAs per SM (80 registers)
+
+constexpr int kMaskedMaxExperts = 1024;  // experts of one masked call (four per thread in the tile count scan)
+
+// Masked form: the input is [experts, rows_per_expert, 2d] and only the first masked_m[e] rows of expert e are valid
+// (the layout of python/sglang/srt/layers/moe/ep_moe/kernels.py:287-361).  The valid rows of every expert are cut
+// into tiles of their own, numbered one expert after the other; rows beyond masked_m[e] are neither read nor written.
+template <typename T, int LPG>
+__global__ void __launch_bounds__(kStreamThreads, 3)
+    silu_mul_quant_masked_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q, float* __restrict__ out_s,
+                                 int d, float eps, float qmin, float qmax, uint32_t probes,
+                                 const int32_t* __restrict__ masked_m, int num_experts, int64_t rows_per_expert) {
+  static_assert(sizeof(T) == 2, "16-bit inputs only");
+  constexpr int CE = 8, NCH = 4, GC = LPG * NCH, G = LPG * kThreadElems;
+  constexpr uint32_t kHalfBytes = kTileElems * 2;  // gate part of a stage; the up part follows it
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bars[kSiluStages];
+  __shared__ int s_abort;
+  __shared__ int s_tiles_before[kMaskedMaxExperts + 1];  // tiles of the experts before e
+  __shared__ int s_warp_sum[kStreamThreads / 32];
+  ptx::grid_dependency_wait();
   const uint32_t smem_base = ptx::smem_u32(smem_raw);
   const int tid = threadIdx.x;
-  int64_t total_elems = rows * d;
-  int64_t tiles = (total_elems + kTileElems - 1) / kTileElems;
   auto valid_rows = [&](int e) -> int64_t {
     const int64_t m = masked_m[e];
     return m < 0 ? 0 : (m > rows_per_expert ? rows_per_expert : m);
   };
-  if constexpr (kMasked) {
-    // exclusive scan of the experts' tile counts: four experts per thread, then the warps' sums
-    int cnt[4], mine = 0;
+  // exclusive scan of the experts' tile counts: four experts per thread, then the warps' sums
+  int cnt[4], mine = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int e = tid * 4 + k;
-      cnt[k] = e < num_experts ? (int)((valid_rows(e) * d + kTileElems - 1) / kTileElems) : 0;
-      mine += cnt[k];
-    }
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int up = __shfl_up_sync(0xffffffffu, incl, o);
-      if ((tid & 31) >= o) incl += up;
-    }
-    if ((tid & 31) == 31) s_warp_sum[tid >> 5] = incl;
-    __syncthreads();
-    int before = incl - mine;
-    for (int w = 0; w < (tid >> 5); ++w) before += s_warp_sum[w];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int e = tid * 4 + k;
-      if (e < num_experts) s_tiles_before[e] = before;
-      before += cnt[k];
-    }
-    if (tid == kStreamThreads - 1) s_tiles_before[num_experts] = before;  // (experts beyond num_experts count 0)
-    __syncthreads();
-    tiles = s_tiles_before[num_experts];
+  for (int k = 0; k < 4; ++k) {
+    const int e = tid * 4 + k;
+    cnt[k] = e < num_experts ? (int)((valid_rows(e) * d + kTileElems - 1) / kTileElems) : 0;
+    mine += cnt[k];
   }
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((tid & 31) >= o) incl += up;
+  }
+  if ((tid & 31) == 31) s_warp_sum[tid >> 5] = incl;
+  __syncthreads();
+  int before = incl - mine;
+  for (int w = 0; w < (tid >> 5); ++w) before += s_warp_sum[w];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int e = tid * 4 + k;
+    if (e < num_experts) s_tiles_before[e] = before;
+    before += cnt[k];
+  }
+  if (tid == kStreamThreads - 1) s_tiles_before[num_experts] = before;  // (experts beyond num_experts count 0)
+  __syncthreads();
+  const int64_t tiles = s_tiles_before[num_experts];
   if ((int64_t)blockIdx.x >= tiles) return;  // the grid is sized from the host-side bound on rows
   const int64_t my_tiles = (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
 
-  // tile i of this CTA: first element within its expert (or within the whole input), that range's element count, and
+  // tile i of this CTA: first element within its expert, that range's element count, and
   // the range's first row
   auto locate = [&](int64_t i, int64_t& e0, int64_t& lim, int64_t& row_base) {
     const int64_t gt = blockIdx.x + i * gridDim.x;
-    if constexpr (kMasked) {
-      int lo = 0, hi = num_experts;  // the expert with s_tiles_before[e] <= gt < s_tiles_before[e + 1]
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if ((int64_t)s_tiles_before[mid] <= gt) lo = mid; else hi = mid;
-      }
-      e0 = (gt - s_tiles_before[lo]) * (int64_t)kTileElems;
-      lim = valid_rows(lo) * d;
-      row_base = (int64_t)lo * rows_per_expert;
-    } else {
-      e0 = gt * (int64_t)kTileElems;
-      lim = total_elems;
-      row_base = 0;
+    int lo = 0, hi = num_experts;  // the expert with s_tiles_before[e] <= gt < s_tiles_before[e + 1]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if ((int64_t)s_tiles_before[mid] <= gt) lo = mid; else hi = mid;
     }
+    e0 = (gt - s_tiles_before[lo]) * (int64_t)kTileElems;
+    lim = valid_rows(lo) * d;
+    row_base = (int64_t)lo * rows_per_expert;
   };
 
   auto issue = [&](int64_t i) {  // thread 0 only
@@ -356,10 +518,12 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
   }
 }
 
+inline bool aligned_to(const void* p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; }
+
 template <typename T, int LPG, bool kStd>
-static int launch_quant_inst(const void* input, void* output_q, float* output_s, int64_t total_elems,
-                             int groups_per_row, int64_t s_stride_token, int64_t s_stride_group, bool contiguous,
-                             float eps, float qmin, float qmax, bool trigger, cudaStream_t stream) {
+static int launch_quant_ring(const void* input, void* output_q, float* output_s, int64_t total_elems,
+                             const ScaleLayout& sl, float eps, float qmin, float qmax, bool trigger,
+                             cudaStream_t stream) {
   constexpr size_t smem = (size_t)kStagesOf<T> * kTileElems * sizeof(T);
   auto kern = quant_stream_kernel<T, LPG, kStd>;
   // opt in to the ring's dynamic shared memory (a per-function, per-device attribute; cheap to repeat)
@@ -368,65 +532,91 @@ static int launch_quant_inst(const void* input, void* output_q, float* output_s,
   const int64_t resident = (int64_t)sm_count() * (sizeof(T) == 4 ? 2 : 3);
   const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
   SGLB_CUDA(launch_pdl(kern, grid, kStreamThreads, smem, stream, static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
-                                               total_elems, groups_per_row, s_stride_token, s_stride_group, contiguous,
-                                               eps, qmin, qmax, g_stream_wait_probes, trigger));
+                                               total_elems, sl.groups_per_row, sl.stride_token, sl.stride_group,
+                                               sl.contiguous, eps, qmin, qmax, g_stream_wait_probes, trigger));
   return SGLB200_OK;
+}
+
+template <typename T, int LPG, bool kStd>
+static int launch_quant_inst(const void* input, void* output_q, float* output_s, int64_t tokens, const ScaleLayout& sl,
+                             float eps, float qmin, float qmax, bool trigger, cudaStream_t stream) {
+  constexpr int G = LPG * kLaneElems;
+  const int64_t groups = tokens * sl.groups_per_row;
+  const bool wide_in = aligned_to(input, 32), wide_out = aligned_to(output_q, 16);
+  auto go = [&](auto kern, int64_t blocks) -> int {
+    SGLB_REQUIRE(blocks < (1ll << 31), "quantizer: input too large");
+    SGLB_CUDA(launch_pdl(kern, (unsigned)blocks, kQuantThreads, 0, stream, static_cast<const T*>(input),
+                         static_cast<uint8_t*>(output_q), output_s, tokens, sl, eps, qmin, qmax, wide_in, wide_out, trigger));
+    return SGLB200_OK;
+  };
+  const int64_t elems = groups * G, sms = sm_count();
+  // Up to four CTAs an SM the flat direct form: all of the input is requested at once and nothing is set up for it
+  // (64 x 7168 bf16: 1.8 us, ring 2.4; 257 x 8192: 2.6 and 3.1).  Beyond the two lines here the ring's deeper staging wins
+  // (4096 x 7168: 16.2 us, direct 16.9; 8192 x 18432: 73.9 and 84.4).  With dense row-major scales the direct form would
+  // still be ahead a little above the first line (777 x 4096: 2.8 us, ring 3.7); the ring keeps that range because the
+  // bounded wait of the ring is tested at that shape.
+  if (elems <= sms * 4 * kUnitElems)
+    return go(quant_kernel<T, LPG, kStd, 1, false>, (elems + kUnitElems - 1) / kUnitElems);
+  // M-major scales, up to 32 CTA-units an SM: the tiled direct form (1024 x 4096: 3.5 us, ring 4.0; 2048 x 4096: 5.2 and
+  // 6.0; 4096 x 4096: 9.0 and 10.1).  Its warps idle in the last tile of a row: not where that is more than a quarter.
+  const int64_t ktiles = (sl.groups_per_row + 7) / 8, tile_rows = 2 * (32 / LPG);
+  if (!sl.contiguous && sl.stride_token == 1 && sl.groups_per_row >= ktiles * 6 && elems <= sms * 32 * kUnitElems)
+    return go(quant_kernel<T, LPG, kStd, 2, true>, ktiles * ((tokens + tile_rows - 1) / tile_rows));
+  return launch_quant_ring<T, LPG / 2, kStd>(input, output_q, output_s, elems, sl, eps, qmin, qmax, trigger, stream);
 }
 
 template <typename T>
 static int launch_quant(const void* input, void* output_q, float* output_s, int64_t num_tokens, int64_t hidden,
                         int group_size, float eps, float qmin, float qmax, int64_t s_stride_token,
                         int64_t s_stride_group, bool trigger, cudaStream_t stream) {
-  const int64_t total = num_tokens * hidden;
   const int groups_per_row = (int)(hidden / group_size);
-  const bool contiguous = (s_stride_group == 1 && s_stride_token == groups_per_row);
-  if (total == 0) return SGLB200_OK;
+  const ScaleLayout sl{groups_per_row, s_stride_token, s_stride_group,
+                       s_stride_group == 1 && s_stride_token == groups_per_row};
   const bool std_range = (qmin == -448.0f && qmax == 448.0f);
-#define SGLB_LAUNCH_Q(LPG)                                                                                          \
-  return std_range ? launch_quant_inst<T, LPG, true>(input, output_q, output_s, total, groups_per_row,              \
-                                                     s_stride_token, s_stride_group, contiguous, eps, qmin, qmax, trigger,   \
-                                                     stream)                                                        \
-                   : launch_quant_inst<T, LPG, false>(input, output_q, output_s, total, groups_per_row,             \
-                                                      s_stride_token, s_stride_group, contiguous, eps, qmin, qmax, trigger,  \
-                                                      stream)
+#define SGLB_LAUNCH_Q(LPG)                                                                                        \
+  return std_range ? launch_quant_inst<T, LPG, true>(input, output_q, output_s, num_tokens, sl, eps, qmin, qmax,  \
+                                                     trigger, stream)                                             \
+                   : launch_quant_inst<T, LPG, false>(input, output_q, output_s, num_tokens, sl, eps, qmin, qmax, \
+                                                      trigger, stream)
   switch (group_size) {
-    case 32: SGLB_LAUNCH_Q(1);
-    case 64: SGLB_LAUNCH_Q(2);
-    case 128: SGLB_LAUNCH_Q(4);
-    case 256: SGLB_LAUNCH_Q(8);
+    case 32: SGLB_LAUNCH_Q(2);
+    case 64: SGLB_LAUNCH_Q(4);
+    case 128: SGLB_LAUNCH_Q(8);
+    case 256: SGLB_LAUNCH_Q(16);
     default: return fail(SGLB200_E_INVALID, "quantizer: group_size %d not in {32,64,128,256}", group_size);
   }
 #undef SGLB_LAUNCH_Q
 }
 
-template <typename T, int LPG, bool kMasked>
-static int launch_silu_mul_quant_kernel(const void* input, void* output_q, float* output_s, int64_t rows, int64_t d,
-                                        float eps, const int32_t* num_rows_dev, const int32_t* masked_m,
-                                        int num_experts, int64_t rows_per_expert, bool trigger, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)kSiluStages * 2 * kTileElems * sizeof(T);
-  auto kern = silu_mul_quant_stream_kernel<T, LPG, kMasked>;
-  SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // (masked: every expert's last tile may be partial, so the bound counts the experts' tiles one by one)
-  const int64_t tiles = kMasked ? (int64_t)num_experts * ((rows_per_expert * d + kTileElems - 1) / kTileElems)
-                                : (rows * d + kTileElems - 1) / kTileElems;
-  const int64_t resident = (int64_t)sm_count() * 3;
-  const unsigned grid = (unsigned)(tiles < resident ? tiles : resident);
-  SGLB_CUDA(launch_pdl(kern, grid, kStreamThreads, smem, stream, static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
-                                               rows, (int)d, num_rows_dev, eps, -448.0f, 448.0f, g_stream_wait_probes,
-                                               masked_m, num_experts, rows_per_expert, trigger));
+template <typename T, int LPG>
+static int launch_silu_mul_quant_inst(const void* input, void* output_q, float* output_s, int64_t rows, int64_t d,
+                                      float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t stream) {
+  // Two units a thread from 32 CTA-units an SM on: more loads in flight where occupancy no longer grows (131072 x 768
+  // bf16: 89 us, one unit 95, staged by bulk copies 104; 8192 x 3584: 29.0, 29.9 and 29.4), one below (256 x 768: 2.0, 2.9
+  // and 4.1; 16384 x 768: 12.2, 12.7 and 15.6; 1999 x 3584: 7.6, 7.8 and 8.5).
+  const int units = rows * d > (int64_t)sm_count() * 32 * kUnitElems ? 2 : 1;
+  const int64_t per = (int64_t)units * kUnitElems, blocks = (rows * d + per - 1) / per;
+  SGLB_REQUIRE(blocks < (1ll << 31), "silu_mul_quant: input too large");
+  SGLB_CUDA(launch_pdl(units == 2 ? silu_mul_quant_kernel<T, LPG, 2> : silu_mul_quant_kernel<T, LPG, 1>, (unsigned)blocks,
+                       kQuantThreads, 0, stream, static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s,
+                       rows, (int)d, num_rows_dev, eps, aligned_to(input, 32), aligned_to(output_q, 16), trigger));
   return SGLB200_OK;
 }
 
 template <typename T, int LPG>
-static int launch_silu_mul_quant_inst(const void* input, void* output_q, float* output_s, int64_t rows, int64_t d,
-                                      float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t stream,
-                                      const int32_t* masked_m = nullptr, int num_experts = 0,
-                                      int64_t rows_per_expert = 0) {
-  if (masked_m != nullptr)
-    return launch_silu_mul_quant_kernel<T, LPG, true>(input, output_q, output_s, rows, d, eps, nullptr, masked_m,
-                                                      num_experts, rows_per_expert, trigger, stream);
-  return launch_silu_mul_quant_kernel<T, LPG, false>(input, output_q, output_s, rows, d, eps, num_rows_dev, nullptr, 0, 0,
-                                                     trigger, stream);
+static int launch_silu_mul_quant_masked_inst(const void* input, void* output_q, float* output_s, int num_experts,
+                                             int64_t rows_per_expert, int64_t d, float eps, const int32_t* masked_m,
+                                             cudaStream_t stream) {
+  constexpr size_t smem = (size_t)kSiluStages * 2 * kTileElems * sizeof(T);
+  auto kern = silu_mul_quant_masked_kernel<T, LPG>;
+  SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (every expert's last tile may be partial, so the bound counts the experts' tiles one by one)
+  const int64_t tiles = (int64_t)num_experts * ((rows_per_expert * d + kTileElems - 1) / kTileElems);
+  const int64_t resident = (int64_t)sm_count() * 3;
+  SGLB_CUDA(launch_pdl(kern, (unsigned)(tiles < resident ? tiles : resident), kStreamThreads, smem, stream,
+                       static_cast<const T*>(input), static_cast<uint8_t*>(output_q), output_s, (int)d, eps, -448.0f, 448.0f,
+                       g_stream_wait_probes, masked_m, num_experts, rows_per_expert));
+  return SGLB200_OK;
 }
 
 template <typename T>
@@ -435,10 +625,10 @@ static int launch_silu_mul_quant(const void* input, void* output_q, float* outpu
   if (rows * d == 0) return SGLB200_OK;
   SGLB_REQUIRE(d < (1ll << 30), "silu_mul_quant: d %lld too large", (long long)d);
   switch (group_size) {
-    case 32: return launch_silu_mul_quant_inst<T, 1>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
-    case 64: return launch_silu_mul_quant_inst<T, 2>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
-    case 128: return launch_silu_mul_quant_inst<T, 4>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
-    case 256: return launch_silu_mul_quant_inst<T, 8>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
+    case 32: return launch_silu_mul_quant_inst<T, 2>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
+    case 64: return launch_silu_mul_quant_inst<T, 4>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
+    case 128: return launch_silu_mul_quant_inst<T, 8>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
+    case 256: return launch_silu_mul_quant_inst<T, 16>(input, output_q, output_s, rows, d, eps, num_rows_dev, trigger, stream);
     default: return fail(SGLB200_E_INVALID, "silu_mul_quant: group_size %d not in {32,64,128,256}", group_size);
   }
 }
@@ -447,10 +637,9 @@ template <typename T>
 static int launch_silu_mul_quant_masked(const void* input, void* output_q, float* output_s, int num_experts,
                                         int64_t rows_per_expert, int64_t d, int group_size, float eps,
                                         const int32_t* masked_m, cudaStream_t stream) {
-  const int64_t rows = (int64_t)num_experts * rows_per_expert;
 #define SGLB_MASKED(LPG)                                                                                         \
-  return launch_silu_mul_quant_inst<T, LPG>(input, output_q, output_s, rows, d, eps, nullptr, false, stream, masked_m, \
-                                            num_experts, rows_per_expert)
+  return launch_silu_mul_quant_masked_inst<T, LPG>(input, output_q, output_s, num_experts, rows_per_expert, d, eps, \
+                                                   masked_m, stream)
   switch (group_size) {
     case 32: SGLB_MASKED(1);
     case 64: SGLB_MASKED(2);

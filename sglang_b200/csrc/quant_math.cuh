@@ -127,12 +127,12 @@ __device__ __forceinline__ void quant_chunk_careful(const float* v, float scale,
   for (int i = 0; i < CE / 4; ++i) codes[i] = pack_e4m3x4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
 }
 
-// Scale and codes of the group this thread shares with LPG - 1 neighbouring lanes.  v holds the thread's 32
-// values (chunk-major), raw the bits they came from.  Every lane of the warp calls this together.
-template <typename T, int LPG, bool kStdRange>
+// Scale and codes of the group this thread shares with LPG - 1 neighbouring lanes.  v holds the thread's values
+// (NCH chunks, one after the other), raw the bits they came from.  Every lane of the warp calls this together.
+template <typename T, int LPG, bool kStdRange, int NCH = Chunk<T>::kPerThread>
 __device__ __forceinline__ float quant_group(const uint4* raw, const float* v, float eps, float qmin, float qmax,
                                              uint32_t (*codes)[Chunk<T>::kElems / 4]) {
-  constexpr int CE = Chunk<T>::kElems, NCH = Chunk<T>::kPerThread;
+  constexpr int CE = Chunk<T>::kElems;
   float m = eps;
 #pragma unroll
   for (int i = 0; i < NCH * CE; i += 2) m = max3_abs_nan(m, v[i], v[i + 1]);

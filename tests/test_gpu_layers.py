@@ -1,11 +1,13 @@
 """GPU parity of whole layers (quantised linear, routed experts) at the sizes where their dispatch or tiles can go wrong:
 edges of the 16/32/64-row tiles and of the step to 128-row tiles, K ranges that do not divide evenly over a cluster, N
 that does not fill a tile, experts with no rows and with many."""
+import numpy as np
 import pytest
 import torch
 
 from oracle import block_fp8_oracle as O
-from tests.util import assert_close_fp, codes_to_fp8, make_act, make_weight, to_f32_np
+from oracle import c_oracle as CO
+from tests.util import assert_close_fp, bf16_bits, codes_to_fp8, fp8_codes, make_act, make_weight, to_f32_np
 
 pytestmark = pytest.mark.gpu
 
@@ -68,3 +70,46 @@ def test_experts_one_slot_with_filtered_ids():
     ref = O.fused_experts_block_fp8(to_f32_np(x)[on], w13q, w13s, w2q, w2s, w.numpy()[on], ids.numpy()[on], 1.0)
     assert (got[~on] == 0).all()
     assert_close_fp(got[on], ref, rtol=2e-2, atol=2e-2)
+
+
+def _off(numel, dtype, nbytes):
+    """A buffer that starts `nbytes` after an aligned address."""
+    step = nbytes // torch.empty(0, dtype=dtype).element_size()
+    return torch.zeros(numel + step, device="cuda", dtype=dtype)[step:]
+
+
+# below, between and above the lines of the dispatch; rows that leave a tile's last rows and columns empty; inputs that
+# start 16 and codes that start 8 bytes after an aligned address
+@pytest.mark.parametrize("tokens,hidden,group", [(1, 128, 128), (3, 96, 32), (130, 1152, 64), (593, 4352, 128),
+                                                 (2401, 1024, 128), (1201, 2304, 256), (17001, 192, 32),
+                                                 (4097, 4864, 128)])
+@pytest.mark.parametrize("dtype,code,offset", [(torch.bfloat16, 0, False), (torch.float16, 1, True),
+                                               (torch.float32, 2, False)])
+@pytest.mark.parametrize("m_major", [False, True])
+def test_quant_forms(tokens, hidden, group, dtype, code, offset, m_major):
+    from sglang_b200 import ops
+    x = make_act(tokens, hidden, tokens + hidden, dtype=dtype)
+    xd = _off(x.numel(), dtype, 16 if offset else 0).view(tokens, hidden)
+    xd.copy_(x)
+    q = _off(x.numel(), torch.uint8, 8 if offset else 0).view(tokens, hidden).view(torch.float8_e4m3fn)
+    ld = (tokens + 3) // 4 * 4
+    guard = torch.full((hidden // group, ld) if m_major else (tokens, hidden // group), -7.0, device="cuda")
+    s = guard.t()[:tokens] if m_major else guard
+    ops.per_token_group_quant_fp8_out(xd, q, s, group)
+    rq, rs = CO.quant(x.numpy() if code == 2 else bf16_bits(x), code, group)
+    assert np.array_equal(s.cpu().numpy(), rs) and np.array_equal(fp8_codes(q), rq)
+    assert not m_major or bool((guard[:, tokens:] == -7.0).all())
+    assert ops.stream_status() == 0
+
+
+@pytest.mark.parametrize("rows,d,group", [(1, 32, 32), (5, 192, 64), (333, 768, 128), (25301, 768, 128), (9601, 2048, 256)])
+@pytest.mark.parametrize("dtype,offset", [(torch.bfloat16, False), (torch.float16, True)])
+def test_silu_mul_quant_forms(rows, d, group, dtype, offset):
+    from sglang_b200 import ops
+    x = _off(rows * 2 * d, dtype, 16 if offset else 0).view(rows, 2 * d)
+    x.copy_(make_act(rows, 2 * d, rows + d, dtype=dtype, outliers=False))
+    h = torch.empty(rows, d, device="cuda", dtype=dtype)
+    ops.silu_and_mul_out(h, x)
+    q_ref, s_ref = ops.per_token_group_quant_fp8(h, group)
+    q, s = ops.silu_and_mul_quant_fp8(x, group)
+    assert torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8)) and torch.equal(s, s_ref)
