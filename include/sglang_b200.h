@@ -270,7 +270,7 @@ int sglb200_gather_rows_fp8(const void* src_q, const float* src_s, void* dst_q, 
  *   w8a8_block_fp8_matmul (python/sglang/srt/layers/quantization/fp8_kernel.py:1072-1168, Triton kernel :695-777).
  * A [M,K] e4m3 row-major; B [N,K] e4m3 row-major (the checkpoint layout of `weight`);
  * a_s element (m,kb) at a_s[m*as_stride_m + kb*as_stride_k]; b_s [ceil(N/128), ceil(K/128)] row-major;
- * C [M,N] row-major, out_dtype 0 = bf16, 1 = fp16.  K % 16 == 0, K <= 65536, N % 8 == 0; A, B, C 16-byte aligned.
+ * C [M,N] row-major, out_dtype 0 = bf16, 1 = fp16.  K % 16 == 0, N % 8 == 0; A, B, C 16-byte aligned.
  * bias (optional, may be NULL): [N] of out_dtype, added in float32 before the final rounding.
  * workspace: only used for the split-K path chosen for small M; at least
  * sglb200_gemm_workspace_bytes(M,N,K) bytes (0 means none needed).
@@ -293,7 +293,7 @@ int sglb200_fp8_blockwise_scaled_mm(const void* A, const void* B, const float* a
  *   (python/sglang/srt/layers/moe/fused_moe_triton/fused_moe_triton_kernels.py:307-583, 586-790) and
  *   torch.ops.sgl_kernel.fp8_blockwise_scaled_grouped_mm (sgl-kernel/csrc/moe/fp8_blockwise_moe_kernel.cu:650-810).
  * A [max_rows, K] e4m3 (rows already in sorted order), a_s [max_rows, K/128] row-major,
- * B [E, N, K] e4m3, b_s [E, ceil(N/128), ceil(K/128)], block size of the sort must be 128.  K % 16 == 0, K <= 65536,
+ * B [E, N, K] e4m3, b_s [E, ceil(N/128), ceil(K/128)], block size of the sort must be 128.  K % 16 == 0,
  * N % 8 == 0.
  */
 int sglb200_fp8_blockwise_grouped_mm(const void* A, const float* a_s, const void* B, const float* b_s, void* C,

@@ -47,6 +47,10 @@ struct ExpertsPlan {
 
 constexpr int kRowsMaxExperts = 1024;  // experts of one call of the rows kernel
 
+// Rows per expert (tile height of the rows kernel, 0 = the 128-row kernel).  Only the average over the experts that can
+// be hit is known on the host; routing spreads around it, so a tile is taken up to an average below its height: an expert
+// with more rows reads its weights once per tile.  From 48 on the 128-row tiles are the faster ones: there the rows
+// kernel's promotion, which costs per column of 128 weight rows, outweighs the padding that it saves.
 static int experts_row_tile(int64_t numel, int64_t E) {
   if (E > kRowsMaxExperts) return 0;
   const int64_t avg = numel / std::min(numel, E);
