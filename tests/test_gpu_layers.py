@@ -31,6 +31,13 @@ def test_linear_row_counts(M, N, K, dtype, bias):
     assert_close_fp(to_f32_np(out), ref)
 
 
+# weights whose tiles are split over clusters of two to eight CTAs, with K ranges of unequal length, and not split at all
+@pytest.mark.parametrize("M", [20, 64])
+@pytest.mark.parametrize("N,K", [(4616, 1920), (3080, 1664), (2200, 2432), (4432, 1152), (8200, 640), (1032, 1152), (14848, 384)])
+def test_linear_cluster_splits(M, N, K):
+    test_linear_row_counts(M, N, K, torch.bfloat16, False)
+
+
 # (tokens, experts, topk): on average 1 to some hundred rows per expert, so that every tile height of the dispatch is taken;
 # the ids are skewed towards expert 0 and leave some experts without rows
 @pytest.mark.parametrize("T,E,topk", [(1, 8, 8), (5, 32, 2), (16, 8, 1), (40, 16, 4), (70, 6, 3), (160, 8, 2), (333, 4, 2)])
