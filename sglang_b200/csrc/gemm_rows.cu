@@ -416,8 +416,6 @@ static size_t rows_smem_bytes(int num_experts) {
   return (size_t)Cfg::kStages * Cfg::kStageBytes + sizeof(RowsCtl<Cfg>) + 1024 + (kGrouped ? sizeof(int) * (num_experts + 1) : 0);
 }
 
-constexpr int kSpreadSmem = 120 * 1024;  // of 227 KB: one CTA per SM
-
 // `pdl`: the launch may overlap the end of the kernel before it in the stream (the kernel waits by itself).
 template <class Cfg, bool kGrouped>
 static int launch_rows(const CUtensorMap& mw, const CUtensorMap& ma, const RowsParams& p, int64_t max_tiles, bool pdl,
@@ -428,10 +426,8 @@ static int launch_rows(const CUtensorMap& mw, const CUtensorMap& ma, const RowsP
   int dev = 0;
   SGLB_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-    // (the dense form's limit is also that of the occupancy question in spread_clusters)
-    const int most = (int)rows_smem_bytes<Cfg, kGrouped>(kMaxExperts);
     SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   !kGrouped && most < kSpreadSmem ? kSpreadSmem : most));
+                                   (int)rows_smem_bytes<Cfg, kGrouped>(kMaxExperts)));
     if (dev >= 0 && dev < 64) attr_set[dev] = true;
   }
   const int64_t slots = (int64_t)sm_count() * Cfg::kCtasPerSm;
@@ -458,26 +454,26 @@ static int launch_rows(const CUtensorMap& mw, const CUtensorMap& ma, const RowsP
   return SGLB200_OK;
 }
 
-// Clusters of `s` CTAs that the current GPU holds at once with one CTA on an SM: a cluster stays within a GPC, whose
-// number of SMs differs from GPC to GPC and from GPU to GPU, so the driver is asked (once per device and size).
-template <class Cfg>
-static int64_t spread_clusters(int s) {
+// Never launched: the occupancy question below is asked about it.
+__global__ void spread_probe_kernel() {}
+
+int64_t spread_clusters(int s) {
   if (s == 1) return sm_count();
-  static std::atomic<int> known[64][kMaxSplits + 1];
+  constexpr int kSmem = 120 * 1024;  // of 227 KB: one CTA per SM
+  static std::atomic<int> known[64][kMostClusterCtas + 1];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / s;
   int n = known[dev][s].load(std::memory_order_relaxed);
   if (n == 0) {
-    auto kern = fp8_rows_gemm_kernel<Cfg, false>;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = (unsigned)s, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)s, 1, 1), cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
-    cfg.dynamicSmemBytes = kSpreadSmem;  // more than half of an SM's
+    cfg.gridDim = dim3((unsigned)s, 1, 1), cfg.blockDim = dim3(256, 1, 1), cfg.dynamicSmemBytes = kSmem;
     cfg.attrs = &attr, cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaFuncSetAttribute(spread_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(spread_probe_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, spread_probe_kernel, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = sm_count() / s;
     }
@@ -485,25 +481,23 @@ static int64_t spread_clusters(int s) {
   }
   return n;
 }
+int64_t paired_clusters(int s) { return s % 2 == 0 ? spread_clusters(s / 2) : 2 * spread_clusters(s); }
 
 // CTAs per cluster for a dense problem of `tiles` tiles and `kb` slabs: the split that finishes first, counted in
 // quarters of the time of a slab in a CTA that has an SM to itself (0.41 us with 64 rows).  A CTA's start and end are three
 // slabs and the exchange of a cluster two more.  Where CTAs share SMs a slab takes 7/4 and start, end and exchange a little
 // longer (a cluster or two too many for one CTA an SM still count as alone); clusters beyond what two CTAs an SM hold
-// wait for a whole round.  A GPC holds as many clusters of 2s CTAs at two an SM as of s at one.
+// wait for a whole round.
 // Measured with 64 and 20 rows over splits of 1 to 8: 4096 x 4096 four CTAs 11.5 / 8.9 us, eight (sharing SMs) 12.4 / 9.6;
 // K 7168 with N 2112 six 11.8 / 9.1, eight 12.2 / 9.6; 4096 x 14336 eight 20.3, four 21.4; 10240 x 8192 three 23.9, two
 // 29.3, four 32.9 (a second round); 4616 x 1920 three 9.8, eight 14.5 (296 CTAs, but 37 clusters of eight do not fit);
 // 14944 x 768 one 9.4, two 11.5.
-template <class Cfg>
 static int rows_splits(int64_t tiles, int kb) {
-  static_assert(Cfg::kCtasPerSm == 2, "clusters that fit");
   int best = 1;
   int64_t best_cost = -1;
   for (int s = 1; s <= kMaxSplits && s <= kb; ++s) {
-    const int64_t per = (kb + s - 1) / s, spread = spread_clusters<Cfg>(s);
-    const int64_t fit = s % 2 == 0 ? spread_clusters<Cfg>(s / 2) : 2 * spread;
-    const int64_t rounds = (tiles + fit - 1) / fit;
+    const int64_t per = (kb + s - 1) / s, spread = spread_clusters(s);
+    const int64_t fit = paired_clusters(s), rounds = (tiles + fit - 1) / fit;
     const bool alone = tiles <= (s == 1 ? spread : spread + spread / 16);
     const int64_t cost = s == 1 ? rounds * per * (alone ? 4 : 7) + 12
                                 : (alone ? 4 * per + 20 : rounds * (7 * per + (s > 4 ? 28 : 22)));
@@ -522,7 +516,8 @@ static int rows_dense_cfg(const void* A, const void* B, RowsParams& p, int64_t K
   p.tiles_m = (int)((p.M + Cfg::NT - 1) / Cfg::NT);
   p.group_m = choose_group_m(p.M, K, Cfg::NT);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
-  p.splits = rows_splits<Cfg>(tiles, p.kb_total);
+  static_assert(Cfg::kCtasPerSm == 2, "rows_splits counts on two");
+  p.splits = rows_splits(tiles, p.kb_total);
   return launch_rows<Cfg, false>(mw, ma, p, tiles, pdl, st);
 }
 

@@ -12,6 +12,13 @@ constexpr uint32_t kWBytes = kRowsBM * kRowsBK;  // weight bytes per stage
 constexpr int kScBatch = 8;                      // slabs whose scales are prepared together
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxSplits = 8;                    // CTAs of a cluster
+constexpr int kMostClusterCtas = 16;
+
+// Clusters of `s` CTAs that the current GPU holds at once with one CTA on an SM: a cluster stays within a GPC, whose number
+// of SMs differs from GPC to GPC and from GPU to GPU, so the driver is asked (once per device and size).  And with two on
+// an SM: a GPC holds as many clusters of 2s CTAs at two an SM as of s at one; for odd sizes at least twice as many.
+int64_t spread_clusters(int s);
+int64_t paired_clusters(int s);
 
 struct RowsParams {
   const float* a_s;

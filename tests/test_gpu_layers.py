@@ -31,9 +31,9 @@ def test_linear_row_counts(M, N, K, dtype, bias):
     assert_close_fp(to_f32_np(out), ref)
 
 
-# weights whose tiles are split over clusters of two to eight CTAs, with K ranges of unequal length, and not split at all
-@pytest.mark.parametrize("M", [20, 64])
-@pytest.mark.parametrize("N,K", [(4616, 1920), (3080, 1664), (2200, 2432), (4432, 1152), (8200, 640), (1032, 1152), (14848, 384)])
+# weights whose tiles are split over clusters of two to sixteen CTAs, with K ranges of unequal length, and not split at all
+@pytest.mark.parametrize("M", [1, 16, 20, 64])
+@pytest.mark.parametrize("N,K", [(1024, 8192), (512, 512), (4616, 1920), (3080, 1664), (2200, 2432), (4432, 1152), (8200, 640), (1032, 1152), (14848, 384)])
 def test_linear_cluster_splits(M, N, K):
     test_linear_row_counts(M, N, K, torch.bfloat16, False)
 
