@@ -590,8 +590,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           auto hand_back = [&]() {
             ptx::tc_fence_before();
             ptx::mbar_arrive_relaxed_if(bar_tempty0 + kBuf * 8, lane == 0);
-            if (I == 0) {  // (every lane has used a scale of the slot: all four are in registers)
-              ptx::mbar_arrive_relaxed_if(bar_sempty0 + ss * 8, lane == 0);
+            if (I == 0) {  // (the slot's four scales have been read: every lane's read is ordered before lane 0's release)
+              __syncwarp();
+              ptx::mbar_arrive_if(bar_sempty0 + ss * 8, lane == 0);
               ss ^= 1u;
               sph ^= ss == 0 ? 1u : 0u;
             }

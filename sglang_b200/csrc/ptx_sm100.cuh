@@ -102,8 +102,9 @@ __device__ __forceinline__ bool mbar_wait_quiet(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// The same without ordering anything (a hand-back of tensor memory or of a slot that has been read: the reads have
-// completed, and a release would first wait for the thread's earlier accesses).
+// The same without ordering anything, for a hand-back of tensor memory only: there tcgen05.wait::ld and the fence before
+// it order the reads, and a release would first wait for the thread's earlier accesses.  Shared memory that has been read
+// goes back with a release (after a __syncwarp where one lane arrives for the warp).
 __device__ __forceinline__ void mbar_arrive_relaxed_if(uint32_t bar, uint32_t pred) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"

@@ -1,0 +1,20 @@
+"""Orderings between threads that a run cannot show, because a wrong order almost always gives the right result: checked in
+the kernels' sources."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sglang_b200", "csrc")
+
+
+def _code(name):
+    """The file without its comments."""
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", text, flags=re.S))
+
+
+def test_relaxed_arrivals_hand_back_tensor_memory_only():
+    """An arrival without a release orders no shared-memory read of any lane; the reads of tensor memory are ordered by
+    tcgen05.wait::ld and the fence in front of it."""
+    for name in sorted(f for f in os.listdir(CSRC) if f.endswith(".cu")):
+        for bar in re.findall(r"mbar_arrive_relaxed_if\(\s*(\w+)", _code(name)):
+            assert bar.startswith("bar_tempty"), (name, bar)
