@@ -587,6 +587,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             for (int jj = 0; jj < 32; jj += 2) ptx::fma2(acc[32 * i + jj], acc[32 * i + jj + 1], v[jj], v[jj + 1], sc);
           };
           bool ok = true;
+          uint32_t asked = 0;
           auto hand_back = [&]() {
             ptx::tc_fence_before();
             ptx::mbar_arrive_relaxed_if(bar_tempty0 + kBuf * 8, lane == 0);
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
               sph ^= ss == 0 ? 1u : 0u;
             }
             if (left > I + 1) {
-              ptx::mbar_ask(bar_tfull0 + kNext * 8, aph[kNext]);
+              asked = ptx::mbar_ask(bar_tfull0 + kNext * 8, aph[kNext]);
               if (I == 3) ok = fetch_scales();
             }
           };
@@ -619,7 +620,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             fma(2, r[0]);
             fma(3, r[1]);
           }
-          ready = ptx::mbar_answer();
+          ready = ptx::mbar_answer(asked);  // (not looked at where nothing was asked: the unit ends)
           return ok;
         };
         bool ok = fetch_scales();

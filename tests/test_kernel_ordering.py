@@ -18,3 +18,15 @@ def test_relaxed_arrivals_hand_back_tensor_memory_only():
     for name in sorted(f for f in os.listdir(CSRC) if f.endswith(".cu")):
         for bar in re.findall(r"mbar_arrive_relaxed_if\(\s*(\w+)", _code(name)):
             assert bar.startswith("bar_tempty"), (name, bar)
+
+
+def test_an_answer_depends_on_its_question():
+    """`mbar_ask` leaves its outcome in a predicate register that the compiler does not know: the value that it returns and
+    `mbar_answer` takes is what keeps the two in order."""
+    header = _code("ptx_sm100.cuh")
+    assert re.search(r"uint32_t mbar_ask\(", header) and re.search(r"bool mbar_answer\(uint32_t (\w+)\)", header)
+    assert re.search(r'"selp\.u32 %0, 1, %1, sglb_asked;" : "=r"\(ok\) : "r"\(asked\)', header)
+    asked = re.findall(r"(\w+) = ptx::mbar_ask\(", _code("gemm.cu"))
+    answered = re.findall(r"ptx::mbar_answer\((\w*)\)", _code("gemm.cu"))
+    assert len(asked) == 1 and answered == asked
+    assert _code("gemm.cu").count("SGLB_MBAR_ASK_DECL()") == 1
