@@ -4,9 +4,11 @@
 //   C[m,n] = out_t( sum_kb a_s[m,kb] * b_s[n/128,kb] * sum_{k in kb} q(x)[m,k] * B[n,k] ) (+ bias)
 //
 // A decoded token through a 2112 x 7168 layer is 2.3 us of HBM time.  As quantizer + GEMM it took 8.5 us: two launches, a
-// round trip of the codes through L2, a ring with per-slab hand-offs; in one launch 7.2 us, which is about what the host
-// takes to issue it.  The CTAs of a cluster share K and each holds its few slabs whole: one thread requests all of its
-// weight tiles at the start (they do not depend on the kernel before), meanwhile the other warps quantise the CTA's part
+// round trip of the codes through L2, a ring with per-slab hand-offs; in one launch 6.7 us, called or from a graph (6.2 with
+// the weights in L2, 7.1 with 15 MB of others per call), so the GPU and not the host is what it waits for.  The CTAs of a
+// cluster share K and each holds its few slabs whole: one thread requests all of its weight tiles as soon as the kernel
+// before is complete (0.1 to 0.5 us later than at the start of the launch, which is not safe: that kernel may have
+// written them; asking for them towards L2 at the start gained nothing), meanwhile the other warps quantise the CTA's part
 // of the activations straight into the swizzled MMA operand (every CTA of the same K range repeats that for itself: a few
 // kilobytes; with 64 rows it cost more than the launch it saves, 14.1 against 12.3 us), every slab has an accumulator of
 // its own, and there is one barrier between each two steps.  The cluster adds its partial sums through distributed
@@ -60,13 +62,6 @@ __global__ void __launch_bounds__(kSmallThreads, 2)
       ptx::mbar_init(ptx::smem_u32(&ctl->acc_full), 1);
       ctl->abort_flag = 0;
       ptx::mbar_fence_init();
-      // The weights: a kernel of this library that writes e4m3 codes for the caller lets nothing start before it is done
-      // (quant.cu), and other kernels let nothing start early at all.
-      for (int s = 0; s < slabs; ++s) {
-        const uint32_t bar = ptx::smem_u32(&ctl->w_full[s]);
-        ptx::mbar_arrive_expect_tx(bar, kWBytes);
-        ptx::tma_load_3d(ptx::smem_u32(weights) + s * kWBytes, &map_w, bar, (kb_begin + s) * kRowsBK, n_tile * kRowsBM, 0);
-      }
     }
     __syncwarp();
     ptx::tmem_alloc(ptx::smem_u32(&ctl->tmem_base), kSmallTmem);
@@ -84,6 +79,14 @@ __global__ void __launch_bounds__(kSmallThreads, 2)
       constexpr uint32_t idesc = ptx::make_idesc_e4m3_f32(kRowsBM, kSmallRows);
       const uint32_t w_lo = ((ptx::smem_u32(weights) & 0x3ffffu) >> 4) | (1u << 16);
       const uint32_t t_lo = ((ptx::smem_u32(tokens) & 0x3ffffu) >> 4) | (1u << 16);
+      // The weights too are read only after the wait: the kernel before this one may have written them, and a launch that
+      // may start early can start before such writes are visible even where that kernel triggers nothing.
+      ptx::grid_dependency_wait();
+      for (int s = 0; s < slabs; ++s) {
+        const uint32_t bar = ptx::smem_u32(&ctl->w_full[s]);
+        ptx::mbar_arrive_expect_tx(bar, kWBytes);
+        ptx::tma_load_3d(ptx::smem_u32(weights) + s * kWBytes, &map_w, bar, (kb_begin + s) * kRowsBK, n_tile * kRowsBM, 0);
+      }
       bool ok = ROWS_WAIT(bar_tok, 0);
       for (int s = 0; s < slabs && ok; ++s) {
         ok = ROWS_WAIT(ptx::smem_u32(&ctl->w_full[s]), 0);

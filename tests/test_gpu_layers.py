@@ -38,6 +38,25 @@ def test_linear_cluster_splits(M, N, K):
     test_linear_row_counts(M, N, K, torch.bfloat16, False)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 2112, 7168), (16, 512, 512), (16, 4368, 4352), (64, 2112, 7168)])
+def test_linear_after_its_weights_were_written(M, N, K):
+    """The kernel in front of the layer writes the weights it multiplies with."""
+    from sglang_b200.srt.layers.quantization.fp8_utils import b200_w8a8_block_fp8_linear
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    ws = torch.rand((N + 127) // 128, K // 128, device="cuda", generator=g) * 1e-3
+    kept = [(torch.randn(N, K, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for _ in range(2)]
+    want = [b200_w8a8_block_fp8_linear(x, w, [128, 128], ws) for w in kept]
+    torch.cuda.synchronize()
+    w = torch.empty_like(kept[0])
+    got = []
+    for i in range(40):
+        w.copy_(kept[i % 2])
+        got.append(b200_w8a8_block_fp8_linear(x, w, [128, 128], ws))
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2])
+
+
 # (tokens, experts, topk): on average 1 to some hundred rows per expert, so that every tile height of the dispatch is taken;
 # the ids are skewed towards expert 0 and leave some experts without rows
 @pytest.mark.parametrize("T,E,topk", [(1, 8, 8), (5, 32, 2), (16, 8, 1), (40, 16, 4), (70, 6, 3), (160, 8, 2), (333, 4, 2)])

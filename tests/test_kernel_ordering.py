@@ -30,3 +30,17 @@ def test_an_answer_depends_on_its_question():
     answered = re.findall(r"ptx::mbar_answer\((\w*)\)", _code("gemm.cu"))
     assert len(asked) == 1 and answered == asked
     assert _code("gemm.cu").count("SGLB_MBAR_ASK_DECL()") == 1
+
+
+def test_one_launch_linear_reads_nothing_before_its_wait():
+    """The launch may start before the writes of the kernel in front of it are visible, and that kernel may be the one that
+    wrote the weights: no load may stand in front of griddepcontrol.wait."""
+    kernel = _code("gemm_small.cu")
+    kernel = kernel[kernel.index("fp8_small_linear_kernel("):kernel.index("struct SmallPlan")]
+    weights = kernel.index("if (ptx::elect_one())")
+    assert "tma_load" not in kernel[:weights] and "ld_nc_16" not in kernel[:weights] and "__ldg" not in kernel[:weights]
+    rest = kernel[weights:]
+    wait = rest.index("grid_dependency_wait")
+    assert wait < rest.index("tma_load_3d")
+    second = rest.index("grid_dependency_wait", wait + 1)
+    assert rest.index("tma_load_3d") < second < min(rest.index("__ldg"), rest.index("ld_nc_16"))
