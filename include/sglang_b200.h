@@ -335,7 +335,8 @@ int sglb200_stream_status_clear(void); /* back to 0 on the current device; synch
  * Number of barrier probes (a few microseconds each) after which a streaming kernel gives up waiting for a staged
  * tile; 0 restores the default (seconds); UINT32_MAX makes every wait give up at once.  A diagnostic knob like
  * sglb200_gemm_set_wait_probes: with UINT32_MAX a healthy call gives up before its first tile has landed, sets the
- * status word and returns after its copies in flight have landed.  No counterpart in the reference.
+ * status word and returns after its copies in flight have landed.  While a limit other than the default is set, the
+ * quantizer stages its input at every size (by default only large inputs are staged).  No counterpart in the reference.
  */
 void sglb200_stream_set_wait_probes(uint32_t probes);
 

@@ -550,17 +550,21 @@ static int launch_quant_inst(const void* input, void* output_q, float* output_s,
     return SGLB200_OK;
   };
   const int64_t elems = groups * G, sms = sm_count();
-  // Up to four CTAs an SM the flat direct form: all of the input is requested at once and nothing is set up for it
-  // (64 x 7168 bf16: 1.8 us, ring 2.4; 257 x 8192: 2.6 and 3.1).  Beyond the two lines here the ring's deeper staging wins
-  // (4096 x 7168: 16.2 us, direct 16.9; 8192 x 18432: 73.9 and 84.4).  With dense row-major scales the direct form would
-  // still be ahead a little above the first line (777 x 4096: 2.8 us, ring 3.7); the ring keeps that range because the
-  // bounded wait of the ring is tested at that shape.
-  if (elems <= sms * 4 * kUnitElems)
+  // The flat direct form requests a CTA's whole input at once and sets nothing up for it; the ring's deeper staging wins
+  // where 16-bit inputs are many times what the SMs hold.  With dense row-major scales: 64 x 7168 bf16 1.8 us, ring 2.4;
+  // 781 x 4096 2.6 and 3.4; 2441 x 4096 5.6 and 5.9; 4882 x 4096 (33 CTAs an SM) 9.8 and 9.8; 7080 x 4096 14.9 and 13.8;
+  // 8192 x 18432 84.4 and 73.9; groups of 32 to 256 and fp16 cross between 30 and 65 CTAs an SM.  float32, whose ring has
+  // two CTAs an SM, never crosses: 585 x 4096 2.4 and 2.8, 8192 x 18432 106.4 and 129.7.  Other layouts leave the flat
+  // form earlier: its scales then go out one word per sector.  A limit on the ring's waits (the tests of its give-up)
+  // selects the ring at any size.
+  const bool ring = g_stream_wait_probes != ptx::kProbeLimit;
+  const bool flat = elems <= sms * (sl.contiguous ? 32 : 4) * kUnitElems || (sl.contiguous && sizeof(T) == 4);
+  if (!ring && flat)
     return go(quant_kernel<T, LPG, kStd, 1, false>, (elems + kUnitElems - 1) / kUnitElems);
   // M-major scales, up to 32 CTA-units an SM: the tiled direct form (1024 x 4096: 3.5 us, ring 4.0; 2048 x 4096: 5.2 and
   // 6.0; 4096 x 4096: 9.0 and 10.1).  Its warps idle in the last tile of a row: not where that is more than a quarter.
   const int64_t ktiles = (sl.groups_per_row + 7) / 8, tile_rows = 2 * (32 / LPG);
-  if (!sl.contiguous && sl.stride_token == 1 && sl.groups_per_row >= ktiles * 6 && elems <= sms * 32 * kUnitElems)
+  if (!ring && !sl.contiguous && sl.stride_token == 1 && sl.groups_per_row >= ktiles * 6 && elems <= sms * 32 * kUnitElems)
     return go(quant_kernel<T, LPG, kStd, 2, true>, ktiles * ((tokens + tile_rows - 1) / tile_rows));
   return launch_quant_ring<T, LPG / 2, kStd>(input, output_q, output_s, elems, sl, eps, qmin, qmax, trigger, stream);
 }

@@ -80,6 +80,28 @@ def test_stream_kernels_wait_runs_out_and_recover():
     assert torch.equal(hq.view(torch.uint8), good_hq.view(torch.uint8)) and torch.equal(hs, good_hs)
 
 
+@pytest.mark.parametrize("tokens,m_major", [(1, False), (64, False), (64, True), (777, True)])
+def test_quantizer_wait_runs_out_at_any_size(tokens, m_major):
+    """A limit on the waits of the ring selects the ring also where the quantizer would do without one."""
+    from sglang_b200 import ops
+    from sglang_b200._lib import check, lib
+    x = torch.randn(tokens, 4096, device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens)).bfloat16()
+    good_q, good_s = ops.per_token_group_quant_fp8(x, 128, column_major_scales=m_major)
+    torch.cuda.synchronize()
+    assert ops.stream_status() == 0
+    lib.sglb200_stream_set_wait_probes(GIVE_UP_AT_ONCE)
+    try:
+        ops.per_token_group_quant_fp8(x, 128, column_major_scales=m_major)
+        torch.cuda.synchronize()
+        assert ops.stream_status() == 1
+    finally:
+        lib.sglb200_stream_set_wait_probes(0)
+        check(lib.sglb200_stream_status_clear())
+    q, s = ops.per_token_group_quant_fp8(x, 128, column_major_scales=m_major)
+    torch.cuda.synchronize()
+    assert ops.stream_status() == 0 and torch.equal(q.view(torch.uint8), good_q.view(torch.uint8)) and torch.equal(s, good_s)
+
+
 def test_reduce_gather_peer_never_arrives_then_completes():
     from sglang_b200._lib import check, lib
     world, rank, M, N = 2, 0, 256, 512

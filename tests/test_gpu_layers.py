@@ -128,6 +128,28 @@ def test_quant_forms(tokens, hidden, group, dtype, code, offset, m_major):
     assert ops.stream_status() == 0
 
 
+# the ring of staged tiles (8192 elements), which a limit on its waits selects at any size: less than a tile, whole tiles
+# and one group more or less, more tiles than CTAs
+@pytest.mark.parametrize("tokens,hidden,group", [(1, 128, 128), (3, 96, 32), (64, 128, 128), (65, 128, 64), (63, 256, 256),
+                                                 (2401, 1024, 128), (1000, 7168, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("m_major", [False, True])
+def test_quant_ring_equals_direct(tokens, hidden, group, dtype, m_major):
+    from sglang_b200 import ops
+    from sglang_b200._lib import lib
+    x = make_act(tokens, hidden, tokens + hidden, dtype=dtype).cuda()
+    x[0, 0], x[0, 1], x[-1, -1] = float("nan"), -0.0, float("inf")
+    q, s = ops.per_token_group_quant_fp8(x, group, column_major_scales=m_major)
+    lib.sglb200_stream_set_wait_probes((1 << 22) - 1)  # (the default is one more)
+    try:
+        rq, rs = ops.per_token_group_quant_fp8(x, group, column_major_scales=m_major)
+        torch.cuda.synchronize()
+    finally:
+        lib.sglb200_stream_set_wait_probes(0)
+    assert ops.stream_status() == 0
+    assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(s, rs)
+
+
 @pytest.mark.parametrize("rows,d,group", [(1, 32, 32), (5, 192, 64), (333, 768, 128), (25301, 768, 128), (9601, 2048, 256)])
 @pytest.mark.parametrize("dtype,offset", [(torch.bfloat16, False), (torch.float16, True)])
 def test_silu_mul_quant_forms(rows, d, group, dtype, offset):
