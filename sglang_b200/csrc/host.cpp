@@ -77,6 +77,9 @@ PyObject* guarded(F&& f) {
   return nullptr;
 }
 
+// Truth as Python sees it (True, 1, numpy's bool); a failing __bool__ leaves its error for the caller's PyErr_Occurred.
+bool flag(PyObject* o) { return PyObject_IsTrue(o) == 1; }
+
 // ---- tensors --------------------------------------------------------------------------------------------------
 using at::Tensor;
 
@@ -117,7 +120,7 @@ PyObject* quant(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const Tensor* xp = cuda_contig(args[0]);
   const int64_t group = PyLong_AsLongLong(args[1]);
   const double eps = PyFloat_AsDouble(args[2]);
-  const bool colmajor = args[3] == Py_True, tma = args[4] == Py_True;
+  const bool colmajor = flag(args[3]), tma = flag(args[4]);
   if (PyErr_Occurred()) return nullptr;
   if (xp == nullptr || xp->dim() < 1 || (colmajor && xp->dim() != 2)) Py_RETURN_NONE;
   const Tensor& x = *xp;
@@ -254,13 +257,14 @@ PyObject* topk_softmax(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (nargs != 3) Py_RETURN_NONE;
   const Tensor* g = cuda_contig(args[0]);
   const int64_t k = PyLong_AsLongLong(args[1]);
+  const bool renormalize = flag(args[2]);
   if (PyErr_Occurred()) return nullptr;
   if (g == nullptr || g->dim() != 2 || k < 1) Py_RETURN_NONE;
   const int dt = dtype_code(g->scalar_type());
   if (dt < 0) Py_RETURN_NONE;
   return guarded([&]() -> PyObject* {
     Tensor w = make({g->size(0), k}, at::kFloat, g->device()), ids = make({g->size(0), k}, at::kInt, g->device());
-    const int rc = abi.sglb200_topk_softmax(g->data_ptr(), dt, g->size(0), (int)g->size(1), (int)k, args[2] == Py_True, 0.f, nullptr,
+    const int rc = abi.sglb200_topk_softmax(g->data_ptr(), dt, g->size(0), (int)g->size(1), (int)k, renormalize, 0.f, nullptr,
                                             static_cast<float*>(w.data_ptr()), static_cast<int32_t*>(ids.data_ptr()), stream_of(*g));
     if (rc) return raise_last(rc);
     return pair(std::move(w), std::move(ids));
@@ -274,6 +278,7 @@ PyObject* fused_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t groups = PyLong_AsLongLong(args[2]), kept = PyLong_AsLongLong(args[3]), k = PyLong_AsLongLong(args[4]),
                 shared = PyLong_AsLongLong(args[5]);
   const double factor = PyFloat_AsDouble(args[6]);
+  const bool scale_output = flag(args[7]);
   if (PyErr_Occurred()) return nullptr;
   if (g == nullptr || b == nullptr || g->dim() != 2 || b->numel() != g->size(1) || b->scalar_type() != g->scalar_type() || k < 1)
     Py_RETURN_NONE;
@@ -282,7 +287,7 @@ PyObject* fused_gate(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject* {
     Tensor w = make({g->size(0), k}, at::kFloat, g->device()), ids = make({g->size(0), k}, at::kInt, g->device());
     const int rc = abi.sglb200_moe_fused_gate(g->data_ptr(), b->data_ptr(), dt, g->size(0), (int)g->size(1), (int)groups, (int)kept,
-                                              (int)k, (int)shared, (float)factor, args[7] == Py_True,
+                                              (int)k, (int)shared, (float)factor, scale_output,
                                               static_cast<float*>(w.data_ptr()), static_cast<int32_t*>(ids.data_ptr()), stream_of(*g));
     if (rc) return raise_last(rc);
     return pair(std::move(w), std::move(ids));

@@ -161,3 +161,21 @@ def test_silu_mul_quant_forms(rows, d, group, dtype, offset):
     q_ref, s_ref = ops.per_token_group_quant_fp8(h, group)
     q, s = ops.silu_and_mul_quant_fp8(x, group)
     assert torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8)) and torch.equal(s, s_ref)
+
+
+@pytest.mark.parametrize("yes,no", [(1, 0), (np.True_, np.False_)])
+def test_flags_by_their_truth(yes, no):
+    """Options given as integers or numpy's truth values are those options."""
+    from sglang_b200 import ops
+    from sglang_b200.srt.layers.moe.topk import fused_topk
+    from sglang_b200.srt.layers.quantization.fp8_kernel import per_token_group_quant_fp8
+    x = make_act(6, 256, 1).cuda()
+    for quant in (ops.per_token_group_quant_fp8, per_token_group_quant_fp8):
+        for c, t in ((True, True), (True, False), (False, False)):
+            q, s = quant(x, 128, column_major_scales=yes if c else no, scale_tma_aligned=yes if t else no)
+            rq, rs = quant(x, 128, column_major_scales=c, scale_tma_aligned=t)
+            assert s.stride() == rs.stride() and torch.equal(s, rs) and torch.equal(q.view(torch.uint8), rq.view(torch.uint8))
+    logits = torch.randn(5, 16, generator=torch.Generator().manual_seed(3)).cuda()
+    for given, flag in ((yes, True), (no, False)):
+        for a, b in zip(fused_topk(logits, 4, given), fused_topk(logits, 4, flag)):
+            assert torch.equal(a, b)
