@@ -124,8 +124,7 @@ struct GemmParams {
   int full_units;              // dense: the first `full_units` tiles are one unit each ...
   int splits;                  // ... and every later tile is cut into `splits` units along K (1 = none)
   int kb_per_split;            // K slabs per unit of a split tile
-  float* partial;              // float32 partial sums of the split tiles: [slot][BM x BN block]
-  int partial_rowmajor;        // layout of a block: 1 = [row][BN] (few rows), 0 = [column / 4][row][4] (full tiles)
+  float* partial;              // float32 partial sums of the split tiles: [slot][column / 4][row][4]
   int nb_total;                // ceil(N/128): weight scale blocks along N
   int tiles_n;                 // ceil(N/BN)
   int scatter;
@@ -650,21 +649,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // this unit's float32 partial sums, tile-local layout; a second kernel adds the units of a tile in a
         // fixed order, adds the bias and rounds once
         if (row < rows) {  // (rows past M are never read back)
-          // Layout of a block: with full tiles [column / 4][row][4], so that the 32 lanes of a warp (32 consecutive
-          // rows) write 512 contiguous bytes per store; with a handful of rows (weight streaming) [row][BN], where
-          // a row's columns stay together.  The reduction kernel reads it the same way.
-          if (p.partial_rowmajor) {
-            float* dst = p.partial + (int64_t)un.slot * (BM * BN) + row_in_tile * BN + cgrp * kEpiCols;
+          // [column / 4][row][4]: the 32 lanes of a warp (32 consecutive rows) write 512 contiguous bytes per store.
+          float* dst = p.partial + (int64_t)un.slot * (BM * BN) + ((int64_t)(cgrp * kEpiCols / 4) * BM + row_in_tile) * 4;
 #pragma unroll
-            for (int j = 0; j < kEpiCols / 4; ++j)
-              *reinterpret_cast<float4*>(dst + j * 4) = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-          } else {
-            float* dst = p.partial + (int64_t)un.slot * (BM * BN) + ((int64_t)(cgrp * kEpiCols / 4) * BM + row_in_tile) * 4;
-#pragma unroll
-            for (int j = 0; j < kEpiCols / 4; ++j)
-              *reinterpret_cast<float4*>(dst + (int64_t)j * BM * 4) =
-                  make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-          }
+          for (int j = 0; j < kEpiCols / 4; ++j)
+            *reinterpret_cast<float4*>(dst + (int64_t)j * BM * 4) =
+                make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
         }
         continue;
       }
@@ -791,23 +781,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
 }
 
-// Offset of element (row r of the tile, column c, a multiple of 4) inside a unit's partial sums: 128-row blocks one
-// after the other, each laid out [column / 4][row][4] or, with `rowmajor`, [row][BN]; `step` = distance between
-// the two float4 halves of an 8-column group.
-__device__ __forceinline__ int64_t partial_offset(int r, int c, int BN, int rowmajor) {
-  const int64_t blk = (int64_t)(r / BM) * (BM * BN);
-  return rowmajor ? blk + (int64_t)(r % BM) * BN + c : blk + ((int64_t)(c >> 2) * BM + (r % BM)) * 4;
-}
-// Thread i of a tile's reduction -> (row, first of 8 columns): columns fastest for the row-major layout, rows
-// fastest for the other, so that neighbouring threads read neighbouring words either way.
-__device__ __forceinline__ void reduce_coord(int i, int tile_rows, int BN, int rowmajor, int& r, int& c8) {
-  if (rowmajor) {
-    r = i / (BN / 8);
-    c8 = (i - r * (BN / 8)) * 8;
-  } else {
-    c8 = (i / tile_rows) * 8;
-    r = i - (i / tile_rows) * tile_rows;
-  }
+// Thread i of a tile's reduction -> (row, first of 8 columns), rows fastest, so that neighbouring threads read neighbouring
+// words of a unit's partial sums ([column / 4][row][4]; the two halves of the eight columns lie BM float4 apart).
+__device__ __forceinline__ void reduce_coord(int i, int& r, int& c8) {
+  c8 = (i / BM) * 8;
+  r = i % BM;
 }
 
 // Sums the partial tiles of every split output tile in ascending split order (deterministic), adds the bias,
@@ -816,24 +794,21 @@ __device__ __forceinline__ void reduce_coord(int i, int tile_rows, int BN, int r
 template <typename OutT>
 __global__ void __launch_bounds__(256)
     split_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ C, const OutT* __restrict__ bias,
-                        int64_t M, int64_t N, int BN, int tile_rows, int tiles_m, int tiles_n, int group_m,
-                        int full_units, int splits, int rowmajor) {
+                        int64_t M, int64_t N, int BN, int tiles_m, int tiles_n, int group_m, int full_units, int splits) {
   ptx::grid_dependency_wait();  // the GEMM's partial sums are complete and visible
   const int tile = full_units + blockIdx.x;
   int m_tile, n_tile;
   tile_coord(tile, tiles_m, tiles_n, group_m, m_tile, n_tile);
   // one thread per (row, 8-column group)
   int r, c8;
-  reduce_coord(blockIdx.y * 256 + threadIdx.x, tile_rows, BN, rowmajor, r, c8);
-  const int half = rowmajor ? 4 : BM * 4;
-  const int64_t row = (int64_t)m_tile * tile_rows + r;
+  reduce_coord(blockIdx.y * 256 + threadIdx.x, r, c8);
+  const int64_t row = (int64_t)m_tile * BM + r;
   const int64_t col = (int64_t)n_tile * BN + c8;
-  if (c8 >= BN || r >= tile_rows || row >= M || col >= N) return;  // N is a multiple of 8: a group is inside or outside as a whole
+  if (c8 >= BN || row >= M || col >= N) return;  // N is a multiple of 8: a group is inside or outside as a whole
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  const int64_t tile_elems = (int64_t)tile_rows * BN;  // (a pair's unit = two 128-row blocks one after the other)
-  const float* src = partial + (int64_t)blockIdx.x * splits * tile_elems + partial_offset(r, c8, BN, rowmajor);
-  for (int s = 0; s < splits; ++s, src += tile_elems) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src + half));
+  const float4* src = reinterpret_cast<const float4*>(partial) + (int64_t)blockIdx.x * splits * (BM * BN / 4) + (c8 >> 2) * BM + r;
+  for (int s = 0; s < splits; ++s, src += BM * BN / 4) {
+    const float4 a = __ldg(src), b = __ldg(src + BM);
     acc[0] += a.x, acc[1] += a.y, acc[2] += a.z, acc[3] += a.w;
     acc[4] += b.x, acc[5] += b.y, acc[6] += b.z, acc[7] += b.w;
   }
@@ -854,24 +829,24 @@ __global__ void __launch_bounds__(256)
 template <typename OutT>
 __global__ void __launch_bounds__(256)
     streamk_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ C, const OutT* __restrict__ bias,
-                          int64_t M, int64_t N, int BN, int tile_rows, int tiles_m, int tiles_n, int group_m,
-                          int kb_total, int share, int ctas, int rowmajor) {
+                          int64_t M, int64_t N, int BN, int tiles_m, int tiles_n, int group_m, int kb_total, int share,
+                          int ctas) {
   ptx::grid_dependency_wait();  // the GEMM's partial sums are complete and visible
   const int tile = blockIdx.x;
   int m_tile, n_tile;
   tile_coord(tile, tiles_m, tiles_n, group_m, m_tile, n_tile);
   int r, c8;
-  reduce_coord(blockIdx.y * 256 + threadIdx.x, tile_rows, BN, rowmajor, r, c8);
-  const int half = rowmajor ? 4 : BM * 4;
-  const int64_t row = (int64_t)m_tile * tile_rows + r;
+  reduce_coord(blockIdx.y * 256 + threadIdx.x, r, c8);
+  const int64_t row = (int64_t)m_tile * BM + r;
   const int64_t col = (int64_t)n_tile * BN + c8;
-  if (c8 >= BN || r >= tile_rows || row >= M || col >= N) return;
+  if (c8 >= BN || row >= M || col >= N) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const float4* mine = reinterpret_cast<const float4*>(partial) + (c8 >> 2) * BM + r;
   const int c_first = tile * kb_total / share, c_last = ((tile + 1) * kb_total - 1) / share;
   for (int c = c_first; c <= c_last; ++c) {
     const int slot = c + ctas * (tile - c * share / kb_total);
-    const float* src = partial + (int64_t)slot * tile_rows * BN + partial_offset(r, c8, BN, rowmajor);
-    const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src + half));
+    const float4* src = mine + (int64_t)slot * (BM * BN / 4);
+    const float4 a = __ldg(src), b = __ldg(src + BM);
     acc[0] += a.x, acc[1] += a.y, acc[2] += a.z, acc[3] += a.w;
     acc[4] += b.x, acc[5] += b.y, acc[6] += b.z, acc[7] += b.w;
   }
@@ -907,10 +882,9 @@ struct UnitPlan {
   int sk_share, sk_ctas, sk_pieces;  // stream-K (sk_share > 0): supersedes the fields above
   int64_t scratch_blocks() const { return sk_share > 0 ? (int64_t)sk_pieces * sk_ctas : split_tiles * splits; }
 };
-// `tile_rows` x BN tiles shared among `sms` workers (SMs, or pairs of SMs for 256-row tiles).
-static UnitPlan plan_units(int64_t M, int64_t N, int64_t K, int BN, int tile_rows, int sms) {
+static UnitPlan plan_units(int64_t M, int64_t N, int64_t K, int BN, int sms) {
   const int kb_total = (int)((K + BK - 1) / BK);
-  const int64_t tiles = ((M + tile_rows - 1) / tile_rows) * ((N + BN - 1) / BN);
+  const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   UnitPlan pl{(int)tiles, 1, kb_total, 0, 0, 0, 2};
   int64_t s = 1, split_tiles = 0;
   if (kStreamK && tiles < 2 * sms && kb_total >= 8 && kb_total % 4 == 0) {
@@ -920,7 +894,7 @@ static UnitPlan plan_units(int64_t M, int64_t N, int64_t K, int BN, int tile_row
     int64_t share = (total + sms - 1) / sms;
     share = (share + 3) / 4 * 4;  // runs start on multiples of four slabs: aligned 128-bit loads of the activation scales
     const int64_t ctas = (total + share - 1) / share;
-    const int64_t rows = M < tile_rows ? M : tile_rows;
+    const int64_t rows = M < BM ? M : BM;
     const int pieces = share <= kb_total ? 2 : 3;
     bool take = false;
     if (tiles * 2 <= sms && pieces == 2) {
@@ -931,7 +905,7 @@ static UnitPlan plan_units(int64_t M, int64_t N, int64_t K, int BN, int tile_row
       // Compared in slab times (about 0.45 us each): the run plus the partial sums (one piece per run and per
       // tile boundary, written and read back at about 4 TB/s, plus the second launch) against the whole waves.
       const int64_t waves = (tiles + sms - 1) / sms;
-      const double partial_bytes = (double)(ctas + tiles) * tile_rows * BN * 4 * 2;
+      const double partial_bytes = (double)(ctas + tiles) * BM * BN * 4 * 2;
       const double cost = (double)share + partial_bytes / 1.8e6 + 6.0;
       take = cost < 0.9 * (double)(waves * kb_total);
     }
@@ -1076,7 +1050,7 @@ int choose_group_m(int64_t rows, int64_t K, int tile_rows) {
 // Compared as waves x tile width, the 128-wide tile charged 156 instead of 128 (it takes 0.61 of a wide tile's time).
 static int choose_bn(int64_t M, int64_t N, int64_t K) {
   const int sms = sm_count();
-  if (plan_units(M, N, K, 256, BM, sms).scratch_blocks() > 0) return 256;
+  if (plan_units(M, N, K, 256, sms).scratch_blocks() > 0) return 256;
   const int64_t tiles_m = (M + BM - 1) / BM;
   const int64_t waves256 = (tiles_m * ((N + 255) / 256) + sms - 1) / sms;
   const int64_t waves128 = (tiles_m * ((N + 127) / 128) + sms - 1) / sms;
@@ -1097,7 +1071,7 @@ struct DensePlan {
 static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
   DensePlan d;
   d.bn = choose_bn(M, N, K);
-  d.units = plan_units(M, N, K, d.bn, BM, sm_count());
+  d.units = plan_units(M, N, K, d.bn, sm_count());
   return d;
 }
 
@@ -1138,7 +1112,6 @@ template <int BN>
 static int dense_mm(const DensePlan& dp, const void* A, const void* B, const float* a_s, const float* b_s, void* C,
                     const void* bias, int64_t M, int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k,
                     int out_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t st) {
-  constexpr int kTileRows = BM;
   CUtensorMap ma, mb;
   int rc = get_tensor_map(A, (uint64_t)K, (uint64_t)M, 1, BM, 2, &ma);
   if (rc) return rc;
@@ -1151,18 +1124,17 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
   p.as_stride_m = as_stride_m, p.as_stride_k = as_stride_k;
   p.kb_total = (int)((K + BK - 1) / BK), p.nb_total = (int)((N + kScaleBlockN - 1) / kScaleBlockN);
   p.tiles_n = (int)((N + BN - 1) / BN);
-  p.group_m = choose_group_m(M, K, kTileRows);
+  p.group_m = choose_group_m(M, K, BM);
   p.out_fp16 = out_dtype;
   p.wait_probes = g_gemm_wait_probes;
   UnitPlan pl = dp.units;
-  const int64_t tiles = ((M + kTileRows - 1) / kTileRows) * p.tiles_n;
+  const int64_t tiles = ((M + BM - 1) / BM) * p.tiles_n;
   if (pl.scratch_blocks() > 0 &&
       (workspace == nullptr || !aligned16(workspace) || workspace_bytes < dp.scratch_bytes()))
     pl = UnitPlan{(int)tiles, 1, p.kb_total, 0, 0, 0, 2};  // no scratch offered: one unit per tile
   p.full_units = pl.full_units, p.splits = pl.splits, p.kb_per_split = pl.kb_per_split;
   p.sk_share = pl.sk_share, p.sk_ctas = pl.sk_ctas, p.sk_pieces = pl.sk_pieces, p.sk_total = (int)(tiles * p.kb_total);
   p.partial = static_cast<float*>(workspace);
-  p.partial_rowmajor = M <= 32 ? 1 : 0;
   CUtensorMap mc{};
   p.tma_out = pl.sk_share == 0 && pl.full_units > 0;
   if (p.tma_out) {
@@ -1171,8 +1143,8 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
   }
   rc = launch_gemm<false, BN>(ma, mb, mc, p, pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits, st);
   if (rc != SGLB200_OK || pl.scratch_blocks() == 0) return rc;
-  const int tiles_m = (int)((M + kTileRows - 1) / kTileRows);
-  const unsigned ygrid = (unsigned)((kTileRows * BN / 8 + 255) / 256);
+  const int tiles_m = (int)((M + BM - 1) / BM);
+  const unsigned ygrid = (unsigned)((BM * BN / 8 + 255) / 256);
   // The reduction is launched programmatically (it may be scheduled while the GEMM's last CTAs drain).
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(256, 1, 1);
@@ -1183,28 +1155,28 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const int rowmajor = p.partial_rowmajor, bn = BN, tile_rows = kTileRows;
+  const int bn = BN;
   if (pl.sk_share > 0) {
     cfg.gridDim = dim3((unsigned)tiles, ygrid, 1);
     if (out_dtype == 0)
       SGLB_CUDA(cudaLaunchKernelEx(&cfg, streamk_reduce_kernel<__nv_bfloat16>, (const float*)p.partial,
                                    static_cast<__nv_bfloat16*>(C), static_cast<const __nv_bfloat16*>(bias), M, N, bn,
-                                   tile_rows, tiles_m, p.tiles_n, p.group_m, p.kb_total, pl.sk_share, pl.sk_ctas, rowmajor));
+                                   tiles_m, p.tiles_n, p.group_m, p.kb_total, pl.sk_share, pl.sk_ctas));
     else
       SGLB_CUDA(cudaLaunchKernelEx(&cfg, streamk_reduce_kernel<__half>, (const float*)p.partial, static_cast<__half*>(C),
-                                   static_cast<const __half*>(bias), M, N, bn, tile_rows, tiles_m, p.tiles_n, p.group_m,
-                                   p.kb_total, pl.sk_share, pl.sk_ctas, rowmajor));
+                                   static_cast<const __half*>(bias), M, N, bn, tiles_m, p.tiles_n, p.group_m,
+                                   p.kb_total, pl.sk_share, pl.sk_ctas));
     return SGLB200_OK;
   }
   cfg.gridDim = dim3((unsigned)pl.split_tiles, ygrid, 1);
   if (out_dtype == 0)
     SGLB_CUDA(cudaLaunchKernelEx(&cfg, split_reduce_kernel<__nv_bfloat16>, (const float*)p.partial,
-                                 static_cast<__nv_bfloat16*>(C), static_cast<const __nv_bfloat16*>(bias), M, N, bn, tile_rows,
-                                 tiles_m, p.tiles_n, p.group_m, pl.full_units, pl.splits, rowmajor));
+                                 static_cast<__nv_bfloat16*>(C), static_cast<const __nv_bfloat16*>(bias), M, N, bn, tiles_m,
+                                 p.tiles_n, p.group_m, pl.full_units, pl.splits));
   else
     SGLB_CUDA(cudaLaunchKernelEx(&cfg, split_reduce_kernel<__half>, (const float*)p.partial, static_cast<__half*>(C),
-                                 static_cast<const __half*>(bias), M, N, bn, tile_rows, tiles_m, p.tiles_n, p.group_m,
-                                 pl.full_units, pl.splits, rowmajor));
+                                 static_cast<const __half*>(bias), M, N, bn, tiles_m, p.tiles_n, p.group_m,
+                                 pl.full_units, pl.splits));
   return SGLB200_OK;
 }
 
@@ -1371,7 +1343,6 @@ template <int BN>
 static int push_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* const* stage_ptrs, int world,
                    int rank, int64_t M, int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype,
                    int sm_margin, cudaStream_t st) {
-  constexpr int kTileRows = BM;
   CUtensorMap ma, mb;
   int rc = get_tensor_map(A, (uint64_t)K, (uint64_t)M, 1, BM, 2, &ma);
   if (rc) return rc;
@@ -1383,10 +1354,10 @@ static int push_mm(const void* A, const void* B, const float* a_s, const float* 
   p.as_stride_m = as_stride_m, p.as_stride_k = as_stride_k;
   p.kb_total = (int)((K + BK - 1) / BK), p.nb_total = (int)((N + kScaleBlockN - 1) / kScaleBlockN);
   p.tiles_n = (int)((N + BN - 1) / BN);
-  p.group_m = choose_group_m(M, K, kTileRows);
+  p.group_m = choose_group_m(M, K, BM);
   p.out_fp16 = out_dtype;
   p.wait_probes = g_gemm_wait_probes;
-  const int64_t tiles = ((M + kTileRows - 1) / kTileRows) * p.tiles_n;
+  const int64_t tiles = ((M + BM - 1) / BM) * p.tiles_n;
   p.full_units = (int)tiles, p.splits = 1, p.kb_per_split = p.kb_total, p.partial = nullptr;  // one unit per tile
   p.sk_pieces = 2;
   p.tma_out = 1;
