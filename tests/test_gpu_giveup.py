@@ -1,8 +1,9 @@
 """The bounded waits of the kernels, made to run out on a healthy GPU (nothing faults, traps or hangs): each kernel
 must return promptly with its status word set, leave the context usable, and the next ordinary call must be right.
 
-* GEMM and streaming kernels: the probe limit is set to "give up at once" (`*_set_wait_probes(UINT32_MAX)`), so every
-  pipeline wait expires before anything was loaded.
+* GEMMs (the 128-row kernel, the rows kernel dense and grouped, the one-launch linear) and streaming kernels (the
+  quantizer's ring, the masked activation): the probe limit is set to "give up at once"
+  (`*_set_wait_probes(UINT32_MAX)`), so every pipeline wait expires before its data has landed.
 * reduce-and-gather kernel of the fused all-reduce: one process plays rank 0 of a two-rank group whose "peer" buffers
   are this GPU's own memory; nothing ever writes the peer's flag, so the wait for it runs out after a small number of
   probes.  Then the flags the peer would have written are set from the host and the same call completes: rank 0's
@@ -78,6 +79,96 @@ def test_stream_kernels_wait_runs_out_and_recover():
     assert ops.stream_status() == 0
     assert torch.equal(q.view(torch.uint8), good_q.view(torch.uint8)) and torch.equal(s, good_s)
     assert torch.equal(hq.view(torch.uint8), good_hq.view(torch.uint8)) and torch.equal(hs, good_hs)
+
+
+# 1 x 1024 and 16 x 4352: quantise and multiply in one launch; 20 and 64 rows: the rows kernel behind the quantizer, with
+# its weights requested early, K split over a cluster or whole; 300: the 128-row kernel
+@pytest.mark.parametrize("M,N,K", [(1, 512, 1024), (16, 4368, 4352), (20, 1024, 8192), (64, 14848, 384), (300, 512, 1024)])
+def test_linear_wait_runs_out_and_recovers(M, N, K):
+    from sglang_b200 import ops
+    from sglang_b200._lib import check, lib
+    from sglang_b200.srt.layers.quantization.fp8_utils import b200_w8a8_block_fp8_linear
+    x, _, _, wq, ws = _inputs(M, N, K)
+    good = b200_w8a8_block_fp8_linear(x, wq, [128, 128], ws)
+    torch.cuda.synchronize()
+    assert ops.gemm_status() == 0
+    lib.sglb200_gemm_set_wait_probes(GIVE_UP_AT_ONCE)
+    try:
+        t0 = time.perf_counter()
+        b200_w8a8_block_fp8_linear(x, wq, [128, 128], ws)
+        torch.cuda.synchronize()
+        assert time.perf_counter() - t0 < 5.0
+        assert ops.gemm_status() == 1
+    finally:
+        lib.sglb200_gemm_set_wait_probes(0)
+        check(lib.sglb200_gemm_status_clear())
+    again = b200_w8a8_block_fp8_linear(x, wq, [128, 128], ws)
+    torch.cuda.synchronize()
+    assert ops.gemm_status() == 0 and torch.equal(again, good)
+
+
+# on average 1, 8 and 40 rows an expert: the rows kernel with tiles of 16, 32 and 64 rows; 150: the 128-row kernel
+@pytest.mark.parametrize("tokens", [4, 32, 160, 600])
+def test_experts_wait_runs_out_and_recovers(tokens):
+    from sglang_b200 import ops
+    from sglang_b200._lib import check, lib
+    from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
+    E, H, I, topk = 8, 384, 256, 2
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, H, device="cuda", generator=g).bfloat16()
+    w13, w2 = ((torch.randn(*s, device="cuda", generator=g) * 20).clamp(-448, 448).to(torch.float8_e4m3fn)
+               for s in ((E, 2 * I, H), (E, H, I)))
+    s13, s2 = (torch.rand(*s, device="cuda", generator=g) * 1e-3 for s in ((E, 2 * I // 128, H // 128), (E, H // 128, I // 128)))
+    wt, ids = torch.topk(torch.softmax(torch.randn(tokens, E, device="cuda", generator=g), -1), topk)
+
+    def call():
+        out = fused_experts_impl(x, w13, w2, wt, ids.to(torch.int32), use_fp8_w8a8=True, w1_scale=s13, w2_scale=s2,
+                                 block_shape=[128, 128])
+        torch.cuda.synchronize()
+        return out
+
+    good = call()
+    assert ops.gemm_status() == 0
+    lib.sglb200_gemm_set_wait_probes(GIVE_UP_AT_ONCE)
+    try:
+        t0 = time.perf_counter()
+        call()
+        assert time.perf_counter() - t0 < 5.0
+        assert ops.gemm_status() == 1
+    finally:
+        lib.sglb200_gemm_set_wait_probes(0)
+        check(lib.sglb200_gemm_status_clear())
+    assert torch.equal(call(), good) and ops.gemm_status() == 0
+
+
+def test_masked_activation_wait_runs_out_and_recovers():
+    """The masked form of the fused activation is the one that stages its input."""
+    from sglang_b200 import ops
+    from sglang_b200._lib import check, lib
+    E, T, d = 3, 70, 1024
+    x = torch.randn(E, T, 2 * d, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).bfloat16()
+    masked_m = torch.tensor([70, 0, 13], device="cuda", dtype=torch.int32)
+
+    def call():
+        q = torch.zeros(E, T, d, device="cuda", dtype=torch.uint8).view(torch.float8_e4m3fn)
+        s = torch.zeros(E, T, d // 128, device="cuda")
+        ops.silu_and_mul_masked_quant_fp8_out(x, q, s, masked_m)
+        torch.cuda.synchronize()
+        return q.view(torch.uint8), s
+
+    good = call()
+    assert ops.stream_status() == 0
+    lib.sglb200_stream_set_wait_probes(GIVE_UP_AT_ONCE)
+    try:
+        t0 = time.perf_counter()
+        call()
+        assert time.perf_counter() - t0 < 5.0
+        assert ops.stream_status() == 1
+    finally:
+        lib.sglb200_stream_set_wait_probes(0)
+        check(lib.sglb200_stream_status_clear())
+    again = call()
+    assert ops.stream_status() == 0 and torch.equal(again[0], good[0]) and torch.equal(again[1], good[1])
 
 
 @pytest.mark.parametrize("tokens,m_major", [(1, False), (64, False), (64, True), (777, True)])
