@@ -272,7 +272,7 @@ int sglb200_gather_rows_fp8(const void* src_q, const float* src_s, void* dst_q, 
  * a_s element (m,kb) at a_s[m*as_stride_m + kb*as_stride_k]; b_s [ceil(N/128), ceil(K/128)] row-major;
  * C [M,N] row-major, out_dtype 0 = bf16, 1 = fp16.  K % 16 == 0, N % 8 == 0; A, B, C 16-byte aligned.
  * bias (optional, may be NULL): [N] of out_dtype, added in float32 before the final rounding.
- * workspace: only used for the split-K path chosen for small M; at least
+ * workspace: partial sums where K is split over units (above 64 rows); at least
  * sglb200_gemm_workspace_bytes(M,N,K) bytes (0 means none needed).
  */
 int64_t sglb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K);
@@ -322,8 +322,8 @@ int sglb200_gemm_status_clear(void);
 void sglb200_gemm_set_wait_probes(uint32_t probes);
 
 /*
- * Health of the streaming kernels (the quantizer and the fused silu_and_mul + quantizer stage their input
- * through shared memory with bulk copies that complete on mbarriers): 0, or 1 if a bounded wait for a staged
+ * Health of the streaming kernels (the quantizer on large inputs and the masked silu_and_mul + quantizer stage their
+ * input through shared memory with bulk copies that complete on mbarriers): 0, or 1 if a bounded wait for a staged
  * tile expired since the library was loaded (the CTA then returns and leaves its output incomplete).
  * Synchronises the device.  Stands in for the CUDA error a failed run of the reference's quantizer launcher
  * (sgl-kernel/csrc/gemm/per_token_group_quant_8bit.cu:116-217) would surface at the next synchronisation.

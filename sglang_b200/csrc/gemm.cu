@@ -24,13 +24,14 @@
 // read 48 KB of it, 768 clocks at 128 bytes a clock for 512 clocks of MMA; measured 860 without any promotion and about
 // 900 with it.  On the way there, same box, back to back (power-limited) in microseconds: 1310 with a 192-wide tile; 1165
 // with 256 columns, setmaxnreg and waits that ask before the FMAs and look after them; 1088 with the scales from the
-// scout's ring, relaxed hand-backs and the two-step question; 1034 with the promotion loop unrolled by four, so that
-// buffers, barriers and scales are compile-time (its bookkeeping was a chain of dependent instructions as long as the
-// FMAs).  Keeping one TMEM load in flight across the FMAs, chunk by chunk, was slower (1250): every extra wait for a load
-// costs more than the overlap gives.
+// scout's ring, relaxed hand-backs of tensor memory and the two-step question; 1056 to 1077 (the spread over boxes) with
+// the promotion loop unrolled by four, so that buffers, barriers and scales are compile-time (its bookkeeping was a chain
+// of dependent instructions as long as the FMAs).  Keeping one TMEM load in flight across the FMAs, chunk by chunk, was
+// slower (1250): every extra wait for a load costs more than the overlap gives.  ptxas spills at 168 registers a thread: 12
+// to 16 bytes of stores in every instance, 40 to 44 bytes of loads in the 256-wide ones, 248 to 264 in the 128-wide ones.
 // The epilogue rounds to bf16/fp16, parks the tile in swizzled shared memory, from where TMA stores drain it
-// during the next tile; in grouped "scatter" mode it multiplies by the routing
-// weight and writes 16 bytes at a time to the token-major row named by sorted_token_ids.
+// during the next tile; in grouped "scatter" mode it multiplies by the routing weight, parks likewise and writes 128
+// contiguous bytes at a time to the token-major row named by sorted_token_ids.
 // Scheduling: with fewer than two waves of tiles and a long K the tiles x slabs space is cut into one equal run
 // of slabs per SM (stream-K; a run covers the end of one tile, possibly a whole tile, and the start of the next);
 // otherwise the tiles of a short last wave are split along K.  Split work writes float32 partial sums that a
@@ -862,7 +863,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // How a dense problem is cut into units.
-//  * Few tiles, long K, M <= 128 (weight streaming): stream-K over all SMs while the partial sums cost less than a
+//  * Few tiles, long K, M of 65 to 128 (weight streaming): stream-K over all SMs while the partial sums cost less than a
 //    quarter of the weight bytes.
 //  * Fewer than two waves of tiles with a long K otherwise (M = 256 or so): stream-K when its run of slabs plus
 //    the cost of the partial sums is shorter than the whole waves it replaces.

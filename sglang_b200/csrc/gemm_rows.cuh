@@ -13,6 +13,10 @@ constexpr int kScBatch = 8;                      // slabs whose scales are prepa
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxSplits = 8;                    // CTAs of a cluster
 constexpr int kMostClusterCtas = 16;
+// Tensor memory: a CTA of these kernels takes 128 or 256 of an SM's 512 columns and may find CTAs of the kernel in front
+// of it or behind it there, of which the latter wait for this one.  No allocation can wait for them in turn: with 256 or
+// 288 threads of 94 to 128 registers at most two such CTAs fit an SM, whatever kernels they belong to, and the 128-row
+// kernel, which takes all columns, leaves no registers for another CTA.
 
 // Clusters of `s` CTAs that the current GPU holds at once with one CTA on an SM: a cluster stays within a GPC, whose number
 // of SMs differs from GPC to GPC and from GPU to GPU, so the driver is asked (once per device and size).  And with two on

@@ -3,7 +3,7 @@
 //
 // Both are bound by HBM, and have two forms.  Direct: a thread loads 16 elements of one group straight into registers
 // (one 256-bit load for 16-bit types), the group maximum takes log2(G / 16) shuffles, and the 16 codes leave in one
-// 128-bit store; no shared memory and no barrier, so no warp waits for another.  Ring (large inputs of the quantizer,
+// 128-bit store; no shared memory and no barrier, so no warp waits for another.  Ring (large 16-bit inputs of the quantizer,
 // masked expert batches of the activation): persistent CTAs walk tiles of 8192 elements that one thread stages with bulk
 // copies (cp.async.bulk) into a ring of shared-memory buffers completing on mbarriers, so the bytes in flight per SM do
 // not depend on registers or occupancy; a thread owns 32 elements of one group per tile.

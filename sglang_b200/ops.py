@@ -443,6 +443,6 @@ def gemm_status() -> int:
 
 
 def stream_status() -> int:
-    """0, or 1 if a wait for a staged tile inside a streaming kernel (quantizer, fused silu_and_mul + quantizer)
+    """0, or 1 if a wait for a staged tile inside a streaming kernel (quantizer, masked silu_and_mul + quantizer)
     expired since the library was loaded (synchronises)."""
     return lib.sglb200_stream_status()

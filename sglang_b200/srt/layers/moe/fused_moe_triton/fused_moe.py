@@ -13,6 +13,9 @@ expert-sorted order so that both GEMMs read plain TMA tiles:
     silu_and_mul+quantise -> A2 [P,I] e4m3 + scales
     grouped GEMM #2       -> ic3 [T*topk,H] bf16, scattered to token-major order, x top-k weight
     moe_sum_reduce        -> out [T,H]
+
+The plain form (16-bit rows, every id local) is one native call that runs these steps; with few rows per expert it sorts
+in blocks of 16 and GEMM #1 fetches its rows itself (csrc/layers.cu).
 """
 from __future__ import annotations
 
