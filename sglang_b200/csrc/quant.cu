@@ -99,9 +99,9 @@ __global__ void __launch_bounds__(kStreamThreads, 3)
     for (int s = 0; s < kStreamStages; ++s) ptx::mbar_init(ptx::smem_u32(&bars[s]), 1);
     ptx::mbar_fence_init();
   }
-  // In this order: what is launched on the trigger may then count on everything before this kernel being complete
-  // (the GEMM of a linear layer reads its weights at once).  A kernel that writes e4m3 codes or block scales for the
-  // caller does not trigger: the codes could be the weights of the layer that follows.
+  // In this order: what is launched on the trigger may then count on everything before this kernel being complete and
+  // visible (the rows kernel of the same linear layer reads its weights at once).  Only a call whose next launch is its own
+  // triggers; what follows a kernel that writes for the caller starts when that is done.
   ptx::grid_dependency_wait();
   if (trigger) ptx::launch_dependents();
   if (tid == 0) {
@@ -217,9 +217,9 @@ __global__ void __launch_bounds__(kQuantThreads)
   constexpr int CE = Chunk<T>::kElems, NCH = kLaneElems / CE, G = LPG * kLaneElems;
   constexpr int kWarpGroups = 32 / LPG;
   static_assert(U <= LPG, "one lane of the group stores each unit's scale");
-  // In this order: what is launched on the trigger may then count on everything before this kernel being complete
-  // (the GEMM of a linear layer reads its weights at once).  A kernel that writes e4m3 codes or block scales for the
-  // caller does not trigger: the codes could be the weights of the layer that follows.
+  // In this order: what is launched on the trigger may then count on everything before this kernel being complete and
+  // visible (the rows kernel of the same linear layer reads its weights at once).  Only a call whose next launch is its own
+  // triggers; what follows a kernel that writes for the caller starts when that is done.
   ptx::grid_dependency_wait();
   if (trigger) ptx::launch_dependents();
   const int l = threadIdx.x % LPG, slot = (threadIdx.x & 31) / LPG, warp = threadIdx.x >> 5;
