@@ -48,7 +48,7 @@ int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, 
 // gemm_rows.cu: the dense product for few activation rows, and the expert-grouped one on rows sorted with a padding of
 // 16 (`cumsum` = padded starts of the buckets, as the sort writes them; bucket 0 = filtered ids is skipped).
 // `gather_topk` > 0: A and a_s have a row per token, fetched by sorted slot / gather_topk; 0: a row per sorted row.
-// `nt` = activation rows per tile: 16, 32 or 64.
+// `nt` = activation rows per tile: 32 or 64.
 int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
                   int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, bool after_quantizer,
                   cudaStream_t st);

@@ -17,7 +17,9 @@
 //
 // Roles (one CTA): warp 0 issues the TMA loads (all lanes: one box of 16 rows, or one gather of 4 rows, per lane and
 // slab), warp 1 issues the MMAs, warp 2 prepares the scales (a_s * b_s of eight slabs at a time, one product per
-// column, in shared memory), warps 4.. promote: TMEM -> registers, acc += partial * scale, then store.
+// column, in shared memory), warps 4.. promote: TMEM -> registers, acc += partial * scale, then store.  Next to HBM the
+// shared-memory port is the limit: 64 rows stage 24 KB a slab and the MMA reads them back, 384 clocks at 128 bytes a
+// clock; see the promotion for what the scales add.
 // Every mbarrier wait is bounded as in gemm.cu (status word, no trap).
 #include <atomic>
 #include <cuda.h>
@@ -32,14 +34,12 @@ struct RowsCfg {
   static constexpr int NT = NT_, kPromoWarps = kPromoWarps_, kStages = kStages_, kAccBufs = kAccBufs_,
                        kCtasPerSm = kCtasPerSm_;
   static constexpr int kThreads = 128 + kPromoWarps * 32;
-  static constexpr int kColGroups = kPromoWarps / 4;      // promotion warps per TMEM lane quadrant
-  static constexpr int kWarpCols = NT / kColGroups;       // columns one promotion warp owns
-  static constexpr int kCW = kWarpCols < 32 ? kWarpCols : 32;  // columns per tcgen05.ld
-  static constexpr int kChunks = kWarpCols / kCW;         // chunk i of group h: columns (h + i * kColGroups) * kCW ..
+  static constexpr int kCW = NT < 32 ? NT : 32;           // columns that a promotion warp takes out of TMEM at once
+  static constexpr int kChunks = NT / kCW;
   static constexpr uint32_t kStageBytes = kWBytes + NT * kRowsBK;
   static constexpr int kTmemCols = kAccBufs * NT;
   static_assert((kTmemCols & (kTmemCols - 1)) == 0 && kTmemCols >= 32 && kTmemCols * kCtasPerSm <= 512, "TMEM columns");
-  static_assert(NT % 16 == 0 && kStageBytes % 1024 == 0, "tile layout");
+  static_assert(NT % 16 == 0 && kStageBytes % 1024 == 0 && kPromoWarps == 4, "tile layout");
 };
 using Rows16 = RowsCfg<16, 4, 6, 8, 2>;
 using Rows32 = RowsCfg<32, 4, 5, 8, 2>;
@@ -53,7 +53,7 @@ struct RowsCtl {
   uint32_t tmem_base;
   int abort_flag;
   int warp_sum[32];
-  alignas(16) float sc[2][kScBatch][Cfg::NT];  // a_s * b_s per slab and column
+  alignas(16) float sc[2][kScBatch][Cfg::NT];  // a_s * b_s per slab and column (columns in the order of frag_column)
   // (grouped: followed by tiles_before[experts + 1], the token tiles of the experts before e)
 };
 
@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     fp8_rows_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                          const RowsParams p) {
   constexpr int NT = Cfg::NT, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs, kCW = Cfg::kCW, kChunks = Cfg::kChunks;
+  static_assert(NT * kPartPitch * 4 <= kStages * Cfg::kStageBytes, "the partial sums fit the ring");
   constexpr uint32_t kStageBytes = Cfg::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
         for (int b = 0; b < kScBatch; ++b)
 #pragma unroll
           for (int i = 0; i < kPer; ++i)
-            if (lane + 32 * i < NT) ctl->sc[d][b][lane + 32 * i] = v[i][b];
+            if (lane + 32 * i < NT) ctl->sc[d][b][frag_column(lane + 32 * i)] = v[i][b];
         ptx::mbar_arrive(bar_full0 + d * 8);
         d ^= 1u;
         if (d == 0) dph ^= 1u;
@@ -257,25 +258,29 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     }
   } else if (warp >= 4) {
     // ------------------------------ promotion + store ------------------------------
-    const int q = warp & 3, h = (warp - 4) >> 2;
-    constexpr int G = Cfg::kColGroups;
+    // The accumulator is read as fragments of 16 lanes x 8 columns: a thread holds four of the warp's 32 weight rows
+    // (lane / 4 + 8 i) in two neighbouring columns (2 (lane % 4), + 1) of every eight, so that a scale it reads serves four
+    // values.  With a lane per weight row every lane needs every column's scale, and a shared-memory read delivers 128
+    // bytes a clock however many lanes ask for the same word: 256 clocks a slab for 64 rows beside 384 of operands, 64 this
+    // way.  64 rows by 36864 x 7168, with the quantizer: 52.2 us with a lane per weight row, 49.7 so; 4096 x 4096 11.5
+    // and 11.3.
+    const int q = warp & 3;
     const uint32_t bar_tfull0 = ptx::smem_u32(&ctl->tmem_full[0]), bar_tempty0 = ptx::smem_u32(&ctl->tmem_empty[0]);
     const uint32_t bar_sfull0 = ptx::smem_u32(&ctl->sc_full[0]), bar_sempty0 = ptx::smem_u32(&ctl->sc_empty[0]);
-    const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16) + h * kCW;
+    const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16);
+    const uint32_t sc0 = ptx::smem_u32(&ctl->sc[0][0][0]) + (lane & 3) * 16;
+    constexpr int kBlocks = kCW / 16, kRegs = 8 * kBlocks;  // 16-column blocks of a chunk; values of half a chunk (16 lanes)
     ptx::grid_dependency_wait();
     uint32_t buf = 0, aph = 0, d = 0, dph = 0;
     bool alive = true;
     for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
       const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
-      const int n = x.n_tile * kRowsBM + q * 32 + lane;  // this thread's output column of C
-      int active = 0;                                    // chunks of this warp that hold columns of the tile
-#pragma unroll
-      for (int i = 0; i < kChunks; ++i) active += (h + i * G) * kCW < x.n_eff ? 1 : 0;
-      float acc[kChunks][kCW];
+      const int active = (x.n_eff + kCW - 1) / kCW;  // chunks that hold columns of the tile
+      float acc[kChunks][2][kRegs];                  // chunk, 16-lane half, [block][8 columns of it][row lane / 4, + 8][2]
 #pragma unroll
       for (int i = 0; i < kChunks; ++i)
 #pragma unroll
-        for (int j = 0; j < kCW; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < kRegs; ++j) acc[i][0][j] = acc[i][1][j] = 0.f;
       const int slabs = kb_stop - kb_begin;
       for (int g = 0; g < slabs; ++g) {
         const int b = g & (kScBatch - 1);
@@ -285,26 +290,32 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
           break;
         }
         ptx::tc_fence_after();
-        const uint32_t taddr = taddr0 + buf * NT;
-        const float4* sc = reinterpret_cast<const float4*>(&ctl->sc[d][b][h * kCW]);
-        if (active == 0 && lane == 0) ptx::mbar_arrive(bar_tempty0 + buf * 8);
+        const uint32_t taddr = taddr0 + buf * NT, sc = sc0 + (d * kScBatch + b) * (NT * 4);
 #pragma unroll
         for (int i = 0; i < kChunks; ++i) {
           if (i < active) {
-            uint32_t r[kCW];
-            if constexpr (kCW == 32) ptx::tmem_ld_32x32(taddr + i * (G * kCW), r);
-            else ptx::tmem_ld_32x16(taddr + i * (G * kCW), r);
+            uint32_t r[2][kRegs];
+            float4 s4[kBlocks];
+            ptx::tmem_ld_16x256<2 * kBlocks>(taddr + i * kCW, r[0]);
+            ptx::tmem_ld_16x256<2 * kBlocks>(taddr + i * kCW + (16u << 16), r[1]);
+#pragma unroll
+            for (int w = 0; w < kBlocks; ++w) s4[w] = ptx::lds_f32x4(sc + (i * kBlocks + w) * 64);
             ptx::tmem_ld_wait();
             if (i == active - 1) {
               ptx::tc_fence_before();
               ptx::mbar_arrive_if(bar_tempty0 + buf * 8, lane == 0);
             }
 #pragma unroll
-            for (int j = 0; j < kCW; j += 4) {
-              const float4 s4 = sc[(i * (G * kCW) + j) / 4];
-              ptx::fma2(acc[i][j], acc[i][j + 1], r[j], r[j + 1], s4.x, s4.y);
-              ptx::fma2(acc[i][j + 2], acc[i][j + 3], r[j + 2], r[j + 3], s4.z, s4.w);
-            }
+            for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+              for (int w = 0; w < kBlocks; ++w) {
+                float* a = acc[i][hf] + 8 * w;
+                const uint32_t* v = r[hf] + 8 * w;
+                ptx::fma2(a[0], a[1], v[0], v[1], s4[w].x, s4[w].y);
+                ptx::fma2(a[2], a[3], v[2], v[3], s4[w].x, s4[w].y);
+                ptx::fma2(a[4], a[5], v[4], v[5], s4[w].z, s4[w].w);
+                ptx::fma2(a[6], a[7], v[6], v[7], s4[w].z, s4[w].w);
+              }
           }
         }
         if (b == kScBatch - 1 || g == slabs - 1) {
@@ -322,63 +333,74 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
       if (splits > 1) {
         // this CTA's partial sums, [column][weight row], over its ring: every slab has been consumed, and a cluster
         // works on one tile only
-        float* part = reinterpret_cast<float*>(tiles) + q * 32 + lane;
+        float* part = reinterpret_cast<float*>(tiles) + 2 * (lane & 3) * kPartPitch + q * 32 + (lane >> 2);
 #pragma unroll
         for (int i = 0; i < kChunks; ++i)
           if (i < active) {
 #pragma unroll
-            for (int j = 0; j < kCW; ++j) part[((h + i * G) * kCW + j) * kRowsBM] = acc[i][j];
+            for (int j = 0; j < kRegs; ++j) {
+              float* at = part + (i * kCW + (j >> 2) * 8 + (j & 1)) * kPartPitch + ((j >> 1) & 1) * 8;
+              at[0] = acc[i][0][j];
+              at[16] = acc[i][1][j];
+            }
           }
         continue;
       }
-      // Two lanes (weight rows n, n + 1) exchange one value per pair of columns, so that each of them stores one
-      // 32-bit word: 64 bytes of one output row per 16 lanes.
-      const bool n_ok = n < p.N;  // (N is even: a pair is inside or outside as a whole)
-      float bias = 0.f;
-      if (!kGrouped && p.bias != nullptr && n_ok)
-        bias = p.out_fp16 ? __half2float(static_cast<const __half*>(p.bias)[n])
-                          : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n]);
+      // Eight columns (output rows) at a time: rounded and transposed in registers, so that a lane has eight neighbouring
+      // values of one output row and four lanes write 64 contiguous bytes.
+      const int n0 = x.n_tile * kRowsBM + q * 32;
+      float bias[4] = {0.f, 0.f, 0.f, 0.f};
+      if (!kGrouped && p.bias != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int n = min(n0 + 8 * i + (lane >> 2), (int)p.N - 1);
+          bias[i] = p.out_fp16 ? __half2float(static_cast<const __half*>(p.bias)[n])
+                               : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n]);
+        }
+      }
+      const int n = n0 + (lane & 3) * 8;  // first of the eight values this lane writes (N is a multiple of 8)
 #pragma unroll
       for (int i = 0; i < kChunks; ++i) {
-        if (i < active) {
-          const int col0 = (h + i * G) * kCW;
-          // destination row and routing weight of column col0 + lane; -1 = not stored
-          int dst = -1;
-          float w = 1.f;
-          if (lane < kCW && col0 + lane < x.n_eff) {
-            const int row = x.row0 + col0 + lane;
-            dst = row;
+#pragma unroll
+        for (int w = 0; w < kBlocks; ++w) {
+          const int col0 = i * kCW + w * 16;
+          if (col0 < x.n_eff) {
+            // destination row and routing weight of column col0 + lane % 16; -1 = not stored
+            int dst = x.row0 + col0 + (lane & 15);
+            float wt = 1.f;
             if (kGrouped) {
               if (p.scatter) {
-                const int id = p.sorted_ids[row];
+                const int id = p.sorted_ids[dst];
                 dst = id < p.numel ? id : -1;
-                if (p.row_weights != nullptr && dst >= 0) w = __ldg(p.row_weights + id);
+                if (p.row_weights != nullptr && dst >= 0) wt = __ldg(p.row_weights + id);
               }
-            } else if (row >= p.M) {
+            } else if (dst >= p.M) {
               dst = -1;
             }
-          }
 #pragma unroll
-          for (int j = 0; j < kCW; j += 2) {
-            float v0 = acc[i][j] + bias, v1 = acc[i][j + 1] + bias;
-            if (kGrouped) {
-              v0 *= __shfl_sync(0xffffffffu, w, j);
-              v1 *= __shfl_sync(0xffffffffu, w, j + 1);
+            for (int u = 0; u < 2; ++u) {
+              const int c = 8 * u + 2 * (lane & 3);
+              const float w0 = kGrouped ? __shfl_sync(0xffffffffu, wt, c) : 1.f;
+              const float w1 = kGrouped ? __shfl_sync(0xffffffffu, wt, c + 1) : 1.f;
+              uint32_t m[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {  // weight rows lane / 4 + 8 k
+                const float* a = acc[i][k >> 1] + 8 * w + 4 * u + 2 * (k & 1);
+                float v0 = a[0], v1 = a[1];
+                if (kGrouped) v0 *= w0, v1 *= w1;
+                else v0 += bias[k], v1 += bias[k];
+                if (p.out_fp16) {
+                  const __half2 o = __floats2half2_rn(v0, v1);
+                  m[k] = *reinterpret_cast<const uint32_t*>(&o);
+                } else {
+                  const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
+                  m[k] = *reinterpret_cast<const uint32_t*>(&o);
+                }
+              }
+              const int row = __shfl_sync(0xffffffffu, dst, 8 * u + (lane >> 2));
+              const uint4 v = ptx::transpose_frags(m, lane);
+              if (row >= 0 && n < p.N) *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + n) = v;
             }
-            const bool odd = lane & 1;
-            const float other = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-            const float lo = odd ? other : v0, hi = odd ? v1 : other;
-            const int row = __shfl_sync(0xffffffffu, dst, j + (lane & 1));
-            uint32_t word;
-            if (p.out_fp16) {
-              const __half2 o = __floats2half2_rn(lo, hi);
-              word = *reinterpret_cast<const uint32_t*>(&o);
-            } else {
-              const __nv_bfloat162 o = __floats2bfloat162_rn(lo, hi);
-              word = *reinterpret_cast<const uint32_t*>(&o);
-            }
-            if (row >= 0 && n_ok)
-              *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + (n & ~1)) = word;
           }
         }
       }
@@ -564,7 +586,6 @@ int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const floa
   p.gather_topk = gather_topk, p.scatter = scatter, p.row_weights = row_weights;
   p.wait_probes = g_gemm_wait_probes;
   switch (nt) {
-    case 16: return rows_grouped_cfg<Rows16>(A, a_rows, B, p, max_rows, K, pdl, st);
     case 32: return rows_grouped_cfg<Rows32>(A, a_rows, B, p, max_rows, K, pdl, st);
     case 64: return rows_grouped_cfg<Rows64>(A, a_rows, B, p, max_rows, K, pdl, st);
     default: return fail(SGLB200_E_INVALID, "rows GEMM: %d rows per tile", nt);

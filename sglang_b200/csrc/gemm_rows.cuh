@@ -13,10 +13,17 @@ constexpr int kScBatch = 8;                      // slabs whose scales are prepa
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxSplits = 8;                    // CTAs of a cluster
 constexpr int kMostClusterCtas = 16;
+constexpr int kPartPitch = kRowsBM + 4;          // floats between the columns of a CTA's partial sums
+
+// Where the scale of column j of a tile lies, so that one 16-byte read gives a thread those of the four columns that it
+// holds of 16 (2 c, 2 c + 1, 2 c + 8, 2 c + 9 with c = lane % 4, see ptx::tmem_ld_16x256).
+__device__ __forceinline__ int frag_column(int j) { return (j & ~15) + ((j & 7) >> 1) * 4 + ((j >> 3) & 1) * 2 + (j & 1); }
 // Tensor memory: a CTA of these kernels takes 128 or 256 of an SM's 512 columns and may find CTAs of the kernel in front
-// of it or behind it there, of which the latter wait for this one.  No allocation can wait for them in turn: with 256 or
-// 288 threads of 94 to 128 registers at most two such CTAs fit an SM, whatever kernels they belong to, and the 128-row
-// kernel, which takes all columns, leaves no registers for another CTA.
+// of it or behind it there, of which the latter wait for this one.  No allocation can wait for them in turn, as an SM that has
+// registers for a set of such CTAs has columns for it too: a CTA with 256 columns has 256 threads of at least 110 registers
+// (43 % of the file), one with 128 columns 256 threads of at least 74 (31 %) or 288 of 96 (42 %), so that beside one
+// with 256 columns there is room for one other of either kind, without one for three of 128.  The 128-row kernel, which takes
+// all columns, leaves no registers for another CTA.
 
 // Clusters of `s` CTAs that the current GPU holds at once with one CTA on an SM: a cluster stays within a GPC, whose number
 // of SMs differs from GPC to GPC and from GPU to GPU, so the driver is asked (once per device and size).  And with two on
@@ -111,7 +118,7 @@ __device__ __forceinline__ void rows_count_tiles(const RowsParams& p, int* tiles
 }
 
 // The output of a tile whose K range was split over the CTAs of a cluster (at most kMost): sums their partial sums
-// ([column][weight row] of float32 at `part` in every CTA's shared memory) in ascending K order, adds the bias, rounds once.
+// ([column][kPartPitch weight rows] of float32 at `part` in every CTA's shared memory) in ascending K order, adds the bias, rounds once.
 template <int kMost>
 __device__ __forceinline__ void rows_cluster_sum(const RowsParams& p, const RowsTile& x, int rank, uint32_t part, int tid,
                                                  int threads) {
@@ -125,7 +132,7 @@ __device__ __forceinline__ void rows_cluster_sum(const RowsParams& p, const Rows
     float2 v[kMost];
 #pragma unroll
     for (int s = 0; s < kMost; ++s)  // all requested before the first is added
-      if (s < splits) v[s] = ptx::lds_cluster_f32x2(ptx::cluster_map(part + (col * kRowsBM + pair * 2) * 4, s));
+      if (s < splits) v[s] = ptx::lds_cluster_f32x2(ptx::cluster_map(part + (col * kPartPitch + pair * 2) * 4, s));
     float a = v[0].x, b = v[0].y;
 #pragma unroll
     for (int s = 1; s < kMost; ++s)

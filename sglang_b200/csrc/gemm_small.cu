@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2)
         // partial sums [column][weight row] over the weights, which have been consumed
         float* part = reinterpret_cast<float*>(weights) + warp * 32 + lane;
 #pragma unroll
-        for (int j = 0; j < kSmallRows; ++j) part[j * kRowsBM] = acc[j];
+        for (int j = 0; j < kSmallRows; ++j) part[j * kPartPitch] = acc[j];
       }
     }
   }

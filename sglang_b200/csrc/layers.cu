@@ -49,13 +49,15 @@ constexpr int kRowsMaxExperts = 1024;  // experts of one call of the rows kernel
 
 // Rows per expert (tile height of the rows kernel, 0 = the 128-row kernel).  Only the average over the experts that can
 // be hit is known on the host; routing spreads around it, so a tile is taken up to an average below its height: an expert
-// with more rows reads its weights once per tile.  From 48 on the 128-row tiles are the faster ones: there the rows
-// kernel's promotion, which costs per column of 128 weight rows, outweighs the padding that it saves.
+// with more rows reads its weights once per tile.  Work follows the rows that a tile has, so a height above them costs
+// nothing but depth of the operand ring: 32 against 64 rows a tile, 256 experts of 7168 x 2048, in us: 0.1 rows an
+// expert 242 / 242, two 1 445 / 1 441, four 1 640 / 1 609, 24 1 935 / 1 875; 128 experts of 2048 x 768 with 0.2 rows
+// 53 / 55.  From 48 on the 128-row tiles are the faster ones (64 against 128 rows a tile: 48 rows 2 573 / 2 457 and
+// 175 / 206, 64 rows 3 470 / 2 550 and 241 / 210): experts above 64 rows read their weights twice.
 static int experts_row_tile(int64_t numel, int64_t E) {
   if (E > kRowsMaxExperts) return 0;
   const int64_t avg = numel / std::min(numel, E);
-  if (avg <= 3) return 16;
-  if (avg <= 24) return 32;
+  if (avg <= 3) return 32;
   if (avg <= 48) return 64;
   return 0;
 }

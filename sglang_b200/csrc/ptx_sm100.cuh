@@ -300,6 +300,61 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// 16 lanes x 8 N columns: per 8 columns a thread receives columns 2 (lane % 4), + 1 of lane (lane / 4) in r[0], r[1] and of
+// lane (lane / 4 + 8) in r[2], r[3].
+__device__ __forceinline__ void tmem_ld_16x256_x2(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_16x256_x8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+               : "r"(taddr)
+               : "memory");
+}
+template <int N>
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t* r) {
+  if constexpr (N >= 8) {
+    tmem_ld_16x256_x8(taddr, r);
+    if constexpr (N > 8) tmem_ld_16x256<N - 8>(taddr + 64, r + 32);
+  } else if constexpr (N >= 4) {
+    tmem_ld_16x256_x4(taddr, r);
+    if constexpr (N > 4) tmem_ld_16x256<N - 4>(taddr + 32, r + 16);
+  } else {
+    static_assert(N == 2, "even numbers of 8-column units");
+    tmem_ld_16x256_x2(taddr, r);
+  }
+}
+
+// Four 8 x 8 fragments of 16-bit values, one below the other (word k of a lane: row 8 k + lane / 4, columns 2 (lane % 4),
+// + 1), transposed: the lane receives rows 8 (lane % 4) .. + 7 of column lane / 4.
+__device__ __forceinline__ uint4 transpose_frags(const uint32_t (&m)[4], int lane) {
+  uint32_t t[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)  // word k: column lane / 4, rows 8 k + 2 (lane % 4), + 1
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(t[k]) : "r"(m[k]));
+  // the four lanes of a column exchange words: lane c keeps block c
+#pragma unroll
+  for (int k = 0; k < 4; k += 2) {
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? t[k] : t[k + 1], 1);
+    if (lane & 1) t[k] = got; else t[k + 1] = got;
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, (lane & 2) ? t[k] : t[k + 2], 2);
+    if (lane & 2) t[k] = got; else t[k + 2] = got;
+  }
+  return make_uint4(t[0], t[1], t[2], t[3]);
+}
+
 // Instruction descriptor for kind::f8f6f4: e4m3 x e4m3 (formats 0/0), f32 accumulate (1 at bit 4),
 // both operands K-major, N/8 at bit 17, M/16 at bit 24.
 __host__ __device__ constexpr uint32_t make_idesc_e4m3_f32(int m, int n) {

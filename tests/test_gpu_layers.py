@@ -38,6 +38,13 @@ def test_linear_cluster_splits(M, N, K):
     test_linear_row_counts(M, N, K, torch.bfloat16, False)
 
 
+# blocks of 16 rows of a 32- and a 64-row tile, each with its last block part filled, and eight-column remainders of N
+@pytest.mark.parametrize("M", [18, 31, 47, 48, 49])
+@pytest.mark.parametrize("N,K", [(136, 384), (1000, 256)])
+def test_linear_row_blocks(M, N, K):
+    test_linear_row_counts(M, N, K, torch.float16, True)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 2112, 7168), (16, 512, 512), (16, 4368, 4352), (64, 2112, 7168)])
 def test_linear_after_its_weights_were_written(M, N, K):
     """The kernel in front of the layer writes the weights it multiplies with."""
