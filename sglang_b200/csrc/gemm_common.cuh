@@ -39,6 +39,13 @@ int quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s, 
 int silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s, int64_t rows, int64_t d, int group_size,
                        float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t st);
 
+// moe_align.cu: the sort of few ids (as sglb200_moe_align_block_size, padding written) and the quantizer of the same layer's
+// activations (groups of 128) in one launch, where `align_quant_fits`.
+bool align_quant_fits(const void* x, int64_t numel, int buckets);
+int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
+                int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
+                int64_t hidden, float eps, float fp8_max, cudaStream_t st);
+
 // gemm.cu: the dense product (arguments as sglb200_fp8_blockwise_scaled_mm).  `after_quantizer`: the kernel before it in
 // the stream is this library's quantizer, launched by the same call, so that the weights may be fetched while that runs.
 int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M, int64_t N,

@@ -147,10 +147,16 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   void* ic3 = p.direct ? out : base + p.ic3;
   const int64_t hb = H / 128, ib = I / 128;
-  int rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
-  if (rc) return rc;
-  rc = sglb200_moe_align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
-                                    p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, stream);
+  int rc;
+  if (align_quant_fits(x, numel, (int)E + 1)) {
+    rc = align_quant(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), x, dtype, base + p.q, f(p.s), T,
+                     H, kQuantEps, kFp8Max, st);
+  } else {
+    rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
+    if (rc) return rc;
+    rc = sglb200_moe_align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
+                                      p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, stream);
+  }
   if (rc) return rc;
   if (p.tile > 0) {
     if (p.direct) SGLB_CUDA(cudaMemsetAsync(out, 0, T * Ho * 2, st));  // rows of negative ids are not written below

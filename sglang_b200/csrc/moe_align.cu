@@ -22,7 +22,9 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gemm_common.cuh"
 #include "ptx_sm100.cuh"
+#include "quant_math.cuh"
 
 namespace sglb200 {
 
@@ -193,11 +195,10 @@ __device__ __forceinline__ void fill_meta(int B, int block_size, int64_t numel, 
 }
 
 // ---- numel <= kChunk: everything in one CTA -------------------------------------------------
-__global__ void __launch_bounds__(kAlignThreads)
-    moe_align_single_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
-                            int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
-                            int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted) {
-  extern __shared__ int smem[];
+__device__ __forceinline__ void align_single(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
+                                             int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
+                                             int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
+                                             int* smem) {
   int* wc = smem;                       // [32][B]
   int* tot = wc + kAlignWarps * B;      // [B]
   int* prefix = tot + B;                // [B+1]
@@ -216,6 +217,47 @@ __global__ void __launch_bounds__(kAlignThreads)
   if (threadIdx.x == 0) *post_pad = prefix[B];
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, 0, 1);
   scatter_chunk(ids, 0, numel, span, B, wc, prefix, sorted);
+}
+__global__ void __launch_bounds__(kAlignThreads)
+    moe_align_single_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
+                            int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
+                            int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted) {
+  extern __shared__ int smem[];
+  align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, pad_sorted, smem);
+}
+
+// The sort of one CTA beside the quantizer of the same layer's activations (groups of 128, 16-bit input, dense row-major
+// scales): CTA 0 sorts, the others quantise, a group to eight lanes of 16 values.  Both are a few microseconds of latency
+// with little work, and neither needs the other.  A layer of 128 experts of 2048 x 768 from a graph, two launches and one: 1
+// token 29.0 -> 28.1 us, 8 tokens 68.2 -> 66.5, 32 tokens 120.6 -> 119.2; 8 experts of 4096 x 1408, 64 tokens 48.9 -> 47.6.
+constexpr int kAlignQuantGroups = kAlignThreads / 8;  // groups of one CTA
+template <typename T>
+__global__ void __launch_bounds__(kAlignThreads)
+    moe_align_quant_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
+                           int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids, int32_t* __restrict__ post_pad,
+                           int32_t* __restrict__ cumsum, const T* __restrict__ x, uint8_t* __restrict__ out_q,
+                           float* __restrict__ out_s, int64_t groups, float eps, float qmax) {
+  extern __shared__ int smem[];
+  if (blockIdx.x == 0) {
+    align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, true, smem);
+    return;
+  }
+  ptx::grid_dependency_wait();
+  ptx::launch_dependents();
+  const int l = threadIdx.x & 7;
+  const int64_t g = (int64_t)(blockIdx.x - 1) * kAlignQuantGroups + (threadIdx.x >> 3);
+  const int64_t e = g * 128 + l * 16;
+  uint4 raw[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+  if (g < groups) raw[0] = ld_nc_16(x + e), raw[1] = ld_nc_16(x + e + 8);
+  float v[16];
+  unpack_chunk<T>(raw[0], v);
+  unpack_chunk<T>(raw[1], v + 8);
+  uint32_t codes[2][2];
+  const float scale = quant_group<T, 8, true, 2>(raw, v, eps, -qmax, qmax, codes);
+  if (g < groups) {
+    *reinterpret_cast<uint4*>(out_q + e) = make_uint4(codes[0][0], codes[0][1], codes[1][0], codes[1][1]);
+    if (l == 0) out_s[g] = scale;
+  }
 }
 
 // ---- numel > kChunk: histogram per chunk -> scan over chunks -> scatter ----------------------
@@ -520,6 +562,29 @@ static void align_plan(int64_t numel, int64_t* chunks, int* span) {
 }
 
 static size_t align_smem_bytes(int B) { return sizeof(int) * ((size_t)kAlignWarps * B + 3 * (size_t)B + 1 + 33 + 8); }
+
+bool align_quant_fits(const void* x, int64_t numel, int buckets) {
+  return numel <= kSingleMax && align_smem_bytes(buckets) <= 48 * 1024 && aligned16(x);
+}
+
+int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
+                int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
+                int64_t hidden, float eps, float fp8_max, cudaStream_t st) {
+  int64_t chunks = 0;
+  int span = 0;
+  align_plan(numel, &chunks, &span);
+  const int64_t groups = tokens * (hidden / 128);
+  const unsigned grid = 1 + (unsigned)((groups + kAlignQuantGroups - 1) / kAlignQuantGroups);
+  const size_t smem = align_smem_bytes(buckets);
+  uint8_t* q = static_cast<uint8_t*>(out_q);
+  if (dtype == 0)
+    SGLB_CUDA(launch_pdl(moe_align_quant_kernel<__nv_bfloat16>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size,
+                         sorted, expert_ids, post_pad, cumsum, static_cast<const __nv_bfloat16*>(x), q, out_s, groups, eps, fp8_max));
+  else
+    SGLB_CUDA(launch_pdl(moe_align_quant_kernel<__half>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size, sorted,
+                         expert_ids, post_pad, cumsum, static_cast<const __half*>(x), q, out_s, groups, eps, fp8_max));
+  return SGLB200_OK;
+}
 
 }  // namespace sglb200
 
