@@ -64,7 +64,9 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     fp8_rows_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                          const RowsParams p) {
   constexpr int NT = Cfg::NT, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs, kCW = Cfg::kCW, kChunks = Cfg::kChunks;
-  static_assert(NT * kPartPitch * 4 <= kStages * Cfg::kStageBytes, "the partial sums fit the ring");
+  constexpr bool kPush = !kGrouped && NT == 64;  // how a cluster exchanges its partial sums
+  static_assert(NT * kPartPitch <= kStages * Cfg::kStageBytes / 4 && (NT / 2 + kMaxSplits - 1) * kPartPair <= kStages * Cfg::kStageBytes / 4,
+                "the partial sums fit the ring");
   constexpr uint32_t kStageBytes = Cfg::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     constexpr int kBlocks = kCW / 16, kRegs = 8 * kBlocks;  // 16-column blocks of a chunk; values of half a chunk (16 lanes)
     ptx::grid_dependency_wait();
     uint32_t buf = 0, aph = 0, d = 0, dph = 0;
-    bool alive = true;
+    bool alive = true, arrived = false, waited = false;
     for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
       const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
       const int active = (x.n_eff + kCW - 1) / kCW;  // chunks that hold columns of the tile
@@ -290,6 +292,10 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
           break;
         }
         ptx::tc_fence_after();
+        if (kPush && splits > 1 && g == slabs - 1) {  // the operands have been consumed: the ring may be written
+          ptx::cluster_arrive();
+          arrived = true;
+        }
         const uint32_t taddr = taddr0 + buf * NT, sc = sc0 + (d * kScBatch + b) * (NT * 4);
 #pragma unroll
         for (int i = 0; i < kChunks; ++i) {
@@ -330,7 +336,15 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
         }
       }
       if (!alive) break;
-      if (splits > 1) {
+      if (kPush && splits > 1) {
+        ptx::cluster_wait();
+        waited = true;
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i)
+          if (i < active) rows_cluster_put<2 * kBlocks>(p, x, rank, ptx::smem_u32(tiles), acc[i][0], acc[i][1], i * kCW, q, lane);
+        continue;
+      }
+      if (!kPush && splits > 1) {
         // this CTA's partial sums, [column][weight row], over its ring: every slab has been consumed, and a cluster
         // works on one tile only
         float* part = reinterpret_cast<float*>(tiles) + 2 * (lane & 3) * kPartPitch + q * 32 + (lane >> 2);
@@ -405,10 +419,24 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
         }
       }
     }
+    if (kPush && splits > 1 && !waited) {  // (a wait expired: the others must not wait for this warp)
+      if (!arrived) ptx::cluster_arrive();
+      ptx::cluster_wait();
+    }
   }
 
   // ------------------------------ sum over the CTAs of a cluster ------------------------------
-  if (!kGrouped && splits > 1) {
+  if (kPush && splits > 1) {
+    __syncwarp();
+    if (warp < 4) {
+      ptx::cluster_arrive();
+      ptx::cluster_wait();
+    }
+    ptx::cluster_arrive();
+    ptx::cluster_wait();  // (nothing crosses the cluster after this: a CTA may leave)
+    const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, tile_first);
+    if (ctl->abort_flag == 0) rows_cluster_get(p, x, rank, ptx::smem_u32(tiles), warp, Cfg::kThreads / 32, lane);
+  } else if (!kGrouped && splits > 1) {
     __syncwarp();
     ptx::cluster_sync();
     const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, tile_first);

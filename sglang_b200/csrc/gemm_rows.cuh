@@ -14,6 +14,7 @@ constexpr int kMaxExperts = 1024;
 constexpr int kMaxSplits = 8;                    // CTAs of a cluster
 constexpr int kMostClusterCtas = 16;
 constexpr int kPartPitch = kRowsBM + 4;          // floats between the columns of a CTA's partial sums
+constexpr int kPartPair = 2 * kRowsBM + 8;       // the same between pairs of columns in the pushed form
 
 // Where the scale of column j of a tile lies, so that one 16-byte read gives a thread those of the four columns that it
 // holds of 16 (2 c, 2 c + 1, 2 c + 8, 2 c + 9 with c = lane % 4, see ptx::tmem_ld_16x256).
@@ -154,6 +155,75 @@ __device__ __forceinline__ void rows_cluster_sum(const RowsParams& p, const Rows
       word = *reinterpret_cast<const uint32_t*>(&o);
     }
     *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + n) = word;
+  }
+}
+
+// The same for tiles of 64 columns, pushed instead of fetched: a CTA owns the pairs of neighbouring columns rank, rank +
+// splits, .., every CTA writes the others' partial sums straight into their shared memory ([source CTA][owned pair][2][128
+// rows] at `part`), and after a barrier all that is left is local.  Fetched (written, barrier, read across the cluster, barrier
+// before anyone may leave) the exchange takes 3.4 of the kernel's 8.6 us of 64 x 4096 x 4096; the layer with its quantizer
+// 10.9 us so and 10.1 pushed, 512 x 512 7.2 and 6.4, 4096 x 14336 17.5 and 16.2.  With 16 or 32 columns there is little
+// to exchange and the barrier before the first remote write costs more than that saves (32 x 1024 x 8192 7.6 and 8.0).
+//
+// Every thread of the cluster arrives and waits twice: the first time when its CTA's operands, which `part` lies over, have
+// been consumed, the second time when its partial sums are written.
+__device__ __forceinline__ int cluster_pairs(const RowsTile& x, int splits) { return (x.n_eff / 2 + splits - 1) / splits; }
+
+// One thread's part of `kUnits` times eight columns from `col0` on: acc[half][4 u ..] as tmem_ld_16x256 has them, of quadrant q.
+template <int kUnits>
+__device__ __forceinline__ void rows_cluster_put(const RowsParams& p, const RowsTile& x, int rank, uint32_t part, const float* acc0,
+                                                 const float* acc1, int col0, int q, int lane) {
+  const int splits = p.splits, pairs = cluster_pairs(x, splits), rows = min(x.n_eff, (int)p.M - x.row0);
+  const uint32_t mine = part + (uint32_t)(rank * pairs * kPartPair + q * 32 + (lane >> 2) * 4) * 4;
+#pragma unroll
+  for (int u = 0; u < kUnits; ++u) {
+    const int pair = col0 / 2 + 4 * u + (lane & 3);
+    if (2 * pair < rows) {
+      const int idx = pair / splits;
+      const uint32_t to = ptx::cluster_map(mine + (uint32_t)(idx * kPartPair) * 4, pair - idx * splits);
+      ptx::sts_cluster_f32x4(to, acc0[4 * u], acc0[4 * u + 2], acc1[4 * u], acc1[4 * u + 2]);
+      ptx::sts_cluster_f32x4(to + kRowsBM * 4, acc0[4 * u + 1], acc0[4 * u + 3], acc1[4 * u + 1], acc1[4 * u + 3]);
+    }
+  }
+}
+
+// The owned columns: partial sums in ascending K order, bias, one rounding.  A warp takes 32 weight rows of four pairs.
+__device__ __forceinline__ void rows_cluster_get(const RowsParams& p, const RowsTile& x, int rank, uint32_t part, int warp, int warps,
+                                                 int lane) {
+  const int splits = p.splits, pairs = cluster_pairs(x, splits);
+  for (int t = warp; t < 4 * ((pairs + 3) / 4); t += warps) {  // (uniform over the warp)
+    const int q = t & 3, first = (t >> 2) * 4, idx = first + (lane & 3);
+    float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
+    if (idx < pairs && 2 * (rank + splits * idx) < (int)p.M - x.row0) {  // (pairs past the last row are not written)
+      uint32_t from = part + (uint32_t)(idx * kPartPair + q * 32 + (lane >> 2) * 4) * 4;
+#pragma unroll 4
+      for (int s = 0; s < splits; ++s, from += (uint32_t)(pairs * kPartPair) * 4) {
+        const float4 v = ptx::lds_f32x4(from), w = ptx::lds_f32x4(from + kRowsBM * 4);
+        a[0] += v.x, a[1] += v.y, a[2] += v.z, a[3] += v.w;
+        b[0] += w.x, b[1] += w.y, b[2] += w.z, b[3] += w.w;
+      }
+    }
+    const int n0 = x.n_tile * kRowsBM + q * 32;
+    uint32_t m[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float bias = 0.f;
+      const int n = min(n0 + 8 * k + (lane >> 2), (int)p.N - 1);
+      if (p.out_fp16) {
+        if (p.bias != nullptr) bias = __half2float(static_cast<const __half*>(p.bias)[n]);
+        const __half2 o = __floats2half2_rn(a[k] + bias, b[k] + bias);
+        m[k] = *reinterpret_cast<const uint32_t*>(&o);
+      } else {
+        if (p.bias != nullptr) bias = __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[n]);
+        const __nv_bfloat162 o = __floats2bfloat162_rn(a[k] + bias, b[k] + bias);
+        m[k] = *reinterpret_cast<const uint32_t*>(&o);
+      }
+    }
+    const uint4 v = ptx::transpose_frags(m, lane);
+    const int c = lane >> 2, mine = first + (c >> 1), col = 2 * (rank + splits * mine) + (c & 1), row = x.row0 + col;
+    const int n = n0 + (lane & 3) * 8;  // (N is a multiple of 8)
+    if (mine < pairs && col < x.n_eff && row < p.M && n < p.N)
+      *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.C) + (int64_t)row * p.N + n) = v;
   }
 }
 
