@@ -440,7 +440,10 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     __syncwarp();
     ptx::cluster_sync();
     const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, tile_first);
-    if (ctl->abort_flag == 0) rows_cluster_sum<kMaxSplits>(p, x, rank, ptx::smem_u32(tiles), tid, Cfg::kThreads);
+    if (ctl->abort_flag == 0) {
+      if (splits <= 8) rows_cluster_sum<8>(p, x, rank, ptx::smem_u32(tiles), tid, Cfg::kThreads);
+      else rows_cluster_sum<kMaxSplits>(p, x, rank, ptx::smem_u32(tiles), tid, Cfg::kThreads);
+    }
     ptx::cluster_sync();  // no CTA leaves while another reads its shared memory
   }
 
@@ -478,6 +481,7 @@ static int launch_rows(const CUtensorMap& mw, const CUtensorMap& ma, const RowsP
   if (dev < 0 || dev >= 64 || !attr_set[dev]) {
     SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)rows_smem_bytes<Cfg, kGrouped>(kMaxExperts)));
+    if (!kGrouped) SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (dev >= 0 && dev < 64) attr_set[dev] = true;
   }
   const int64_t slots = (int64_t)sm_count() * Cfg::kCtasPerSm;
@@ -512,7 +516,7 @@ int64_t spread_clusters(int s) {
   constexpr int kSmem = 120 * 1024;  // of 227 KB: one CTA per SM
   static std::atomic<int> known[64][kMostClusterCtas + 1];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sm_count() / s;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return s <= 8 ? sm_count() / s : 0;
   int n = known[dev][s].load(std::memory_order_relaxed);
   if (n == 0) {
     cudaLaunchAttribute attr;
@@ -525,11 +529,11 @@ int64_t spread_clusters(int s) {
         cudaFuncSetAttribute(spread_probe_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, spread_probe_kernel, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
-      n = sm_count() / s;
+      n = s <= 8 ? sm_count() / s : -1;
     }
     known[dev][s].store(n, std::memory_order_relaxed);
   }
-  return n;
+  return n > 0 ? n : 0;
 }
 int64_t paired_clusters(int s) { return s % 2 == 0 ? spread_clusters(s / 2) : 2 * spread_clusters(s); }
 
@@ -541,16 +545,22 @@ int64_t paired_clusters(int s) { return s % 2 == 0 ? spread_clusters(s / 2) : 2 
 // Measured with 64 and 20 rows over splits of 1 to 8: 4096 x 4096 four CTAs 11.5 / 8.9 us, eight (sharing SMs) 12.4 / 9.6;
 // K 7168 with N 2112 six 11.8 / 9.1, eight 12.2 / 9.6; 4096 x 14336 eight 20.3, four 21.4; 10240 x 8192 three 23.9, two
 // 29.3, four 32.9 (a second round); 4616 x 1920 three 9.8, eight 14.5 (296 CTAs, but 37 clusters of eight do not fit);
-// 14944 x 768 one 9.4, two 11.5.
-static int rows_splits(int64_t tiles, int kb) {
+// 14944 x 768 one 9.4, two 11.5.  More than eight CTAs, for few tiles and a long K: 512 x 8192 sixteen 8.6, eight 9.5; 768 x
+// 18432 sixteen 11.1, eight 14.0; 1024 x 8192 ten 9.6, eight 9.9, sixteen 10.8; where that gains no whole slab, eight
+// (1536 x 7168 with 20 rows eight 7.3, nine 7.5).  With up to 32 rows, which are not pushed, they have to gain more
+// than one (32 rows: 1280 x 5120 eight 7.0, ten 7.2; 576 x 7168 eight 7.4, fourteen 7.2; 640 x 12288 eight 8.6, sixteen 7.8).
+static int rows_splits(int64_t tiles, int kb, bool pushed) {
+  const int large = pushed ? 1 : 5;
   int best = 1;
   int64_t best_cost = -1;
   for (int s = 1; s <= kMaxSplits && s <= kb; ++s) {
     const int64_t per = (kb + s - 1) / s, spread = spread_clusters(s);
-    const int64_t fit = paired_clusters(s), rounds = (tiles + fit - 1) / fit;
+    const int64_t fit = paired_clusters(s);
+    if (fit == 0) continue;
+    const int64_t rounds = (tiles + fit - 1) / fit;
     const bool alone = tiles <= (s == 1 ? spread : spread + spread / 16);
     const int64_t cost = s == 1 ? rounds * per * (alone ? 4 : 7) + 12
-                                : (alone ? 4 * per + 20 : rounds * (7 * per + (s > 4 ? 28 : 22)));
+                                : (alone ? 4 * per + 20 + (s > 8 ? large : 0) : rounds * (7 * per + (s > 4 ? 28 : 22)));
     if (best_cost < 0 || cost <= best_cost) best = s, best_cost = cost;
   }
   return best;
@@ -567,7 +577,7 @@ static int rows_dense_cfg(const void* A, const void* B, RowsParams& p, int64_t K
   p.group_m = choose_group_m(p.M, K, Cfg::NT);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
   static_assert(Cfg::kCtasPerSm == 2, "rows_splits counts on two");
-  p.splits = rows_splits(tiles, p.kb_total);
+  p.splits = rows_splits(tiles, p.kb_total, Cfg::NT == 64);
   return launch_rows<Cfg, false>(mw, ma, p, tiles, pdl, st);
 }
 

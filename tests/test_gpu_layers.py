@@ -45,6 +45,14 @@ def test_linear_row_blocks(M, N, K):
     test_linear_row_counts(M, N, K, torch.float16, True)
 
 
+# clusters of more than eight CTAs: K ranges of one slab and of unequal length, pairs of columns that the CTAs share unequally,
+# CTAs that own none of the rows there are
+@pytest.mark.parametrize("M", [17, 32, 34, 63, 64])
+@pytest.mark.parametrize("N,K", [(136, 2048), (520, 4480), (768, 8320)])
+def test_linear_large_clusters(M, N, K):
+    test_linear_row_counts(M, N, K, torch.float16, True)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 2112, 7168), (16, 512, 512), (16, 4368, 4352), (64, 2112, 7168)])
 def test_linear_after_its_weights_were_written(M, N, K):
     """The kernel in front of the layer writes the weights it multiplies with."""
