@@ -40,11 +40,11 @@ int silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* outp
                        float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t st);
 
 // moe_align.cu: the sort of few ids (as sglb200_moe_align_block_size, padding written) and the quantizer of the same layer's
-// activations (groups of 128) in one launch, where `align_quant_fits`.
+// activations (groups of 128) in one launch, where `align_quant_fits`.  zeros[0] and zeros[1] are set to 0.
 bool align_quant_fits(const void* x, int64_t numel, int buckets);
 int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                 int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
-                int64_t hidden, float eps, float fp8_max, cudaStream_t st);
+                int64_t hidden, float eps, float fp8_max, int32_t* zeros, cudaStream_t st);
 
 // gemm.cu: the dense product (arguments as sglb200_fp8_blockwise_scaled_mm).  `after_quantizer`: the kernel before it in
 // the stream is this library's quantizer, launched by the same call, so that the weights may be fetched while that runs.
@@ -55,14 +55,14 @@ int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, 
 // gemm_rows.cu: the dense product for few activation rows, and the expert-grouped one on rows sorted with a padding of
 // 16 (`cumsum` = padded starts of the buckets, as the sort writes them; bucket 0 = filtered ids is skipped).
 // `gather_topk` > 0: A and a_s have a row per token, fetched by sorted slot / gather_topk; 0: a row per sorted row.
-// `nt` = activation rows per tile: 32 or 64.
+// `nt` = activation rows per tile: 32 or 64.  `next_tile`: a zero (or nullptr), see RowsParams.
 int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
                   int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, bool after_quantizer,
                   cudaStream_t st);
 int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const float* a_s, const void* B, const float* b_s, void* C,
                     const int32_t* cumsum, const int32_t* sorted_ids, const float* row_weights, int64_t max_rows,
                     int64_t numel, int num_experts, int64_t N, int64_t K, int gather_topk, int scatter, int out_dtype, int nt,
-                    bool pdl, cudaStream_t st);
+                    int32_t* next_tile, bool pdl, cudaStream_t st);
 
 // gemm_small.cu: quantise + multiply in one launch; whether a problem is one for it.
 bool small_linear_fits(int64_t M, int64_t N, int64_t K);

@@ -45,16 +45,20 @@ using Rows16 = RowsCfg<16, 4, 6, 8, 2>;
 using Rows32 = RowsCfg<32, 4, 5, 8, 2>;
 using Rows64 = RowsCfg<64, 4, 4, 4, 2>;
 
+constexpr int kTileSlots = 4;
+
 template <class Cfg>
 struct RowsCtl {
   uint64_t full[Cfg::kStages], empty[Cfg::kStages];
   uint64_t tmem_full[Cfg::kAccBufs], tmem_empty[Cfg::kAccBufs];
   uint64_t sc_full[2], sc_empty[2];
+  uint64_t tile_full[kTileSlots], tile_empty[kTileSlots];  // the tiles that the producer took, for the other roles
+  RowsTile tile[kTileSlots];                               // n_eff = 0: there is none left
   uint32_t tmem_base;
   int abort_flag;
   int warp_sum[32];
   alignas(16) float sc[2][kScBatch][Cfg::NT];  // a_s * b_s per slab and column (columns in the order of frag_column)
-  // (grouped: followed by tiles_before[experts + 1], the token tiles of the experts before e)
+  // (grouped: followed by tiles_before[experts + 1], the token tiles of the experts before e, and row_begin[experts + 1])
 };
 
 __device__ int g_rows_status = 0;  // 0 ok, 1 = a pipeline wait expired
@@ -71,7 +75,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   RowsCtl<Cfg>* ctl = reinterpret_cast<RowsCtl<Cfg>*>(tiles + kStages * kStageBytes);
-  int* tiles_before = reinterpret_cast<int*>(ctl + 1);
+  int* tiles_before = reinterpret_cast<int*>(ctl + 1);  // grouped: token tiles before, then first row of, every expert
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int* abort_flag = &ctl->abort_flag;
 
@@ -88,6 +92,10 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     for (int d = 0; d < 2; ++d) {
       ptx::mbar_init(ptx::smem_u32(&ctl->sc_full[d]), 32);
       ptx::mbar_init(ptx::smem_u32(&ctl->sc_empty[d]), Cfg::kPromoWarps);
+    }
+    for (int d = 0; d < kTileSlots; ++d) {
+      ptx::mbar_init(ptx::smem_u32(&ctl->tile_full[d]), 1);
+      ptx::mbar_init(ptx::smem_u32(&ctl->tile_empty[d]), Cfg::kPromoWarps + 2);
     }
     ctl->abort_flag = 0;
     ptx::mbar_fence_init();
@@ -113,6 +121,36 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
   const int num_tiles = (kGrouped ? tiles_before[p.num_experts] : p.tiles_m) * p.tiles_n;
   const int kb_begin = rank * p.kb_total / splits, kb_stop = (rank + 1) * p.kb_total / splits;
 
+  // The tiles of this CTA, one call after the other: in the dense form every role counts for itself, in the grouped one the
+  // producer takes them (from a counter that the CTAs share, where there is one) and hands them to the other roles through
+  // a ring.  `t` and `x` are the caller's; false = none left, or a wait expired.
+  // The counter is for experts with more tiles than CTAs: those that HBM serves faster then take more of them, and a last
+  // round that is part full spreads over all SMs.  Dealt out in turn, the CTAs of 256 experts of 7168 x 2048 with 64 tokens
+  // ended between 849 and 940 us of the first product; the layer took 1 419 us and takes 1 369; 128 experts of 2048 x 768
+  // from a graph, 32 tokens 117.5 and 108.7, 16 tokens 86.3 and 84.2.  What the ring costs shows where a CTA has a tile or
+  // none (8 experts of 4096 x 1408, one token 30.6 and 31.5).  Weights of the first tile asked for before its row ids, so that
+  // these wait behind them, cost another 1 to 2 us; the experts' first rows in shared memory 0.6.
+  const uint32_t bar_tile_full0 = ptx::smem_u32(&ctl->tile_full[0]), bar_tile_empty0 = ptx::smem_u32(&ctl->tile_empty[0]);
+  uint32_t ts = 0, tph = 0;
+  auto take_tile = [&](int& t, RowsTile& x, bool first, bool one_thread) -> bool {
+    if constexpr (kGrouped) {
+      if (!ROWS_WAIT(bar_tile_full0 + ts * 8, tph)) {
+        *abort_flag = 1;
+        return false;
+      }
+      x = ctl->tile[ts];
+      if (!one_thread) __syncwarp();  // (every lane has read it)
+      if (one_thread || lane == 0) ptx::mbar_arrive(bar_tile_empty0 + ts * 8);
+      if (++ts == (uint32_t)kTileSlots) ts = 0, tph ^= 1u;
+      return x.n_eff > 0;
+    } else {
+      t = first ? tile_first : t + tile_step;
+      if (t >= num_tiles) return false;
+      x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+      return true;
+    }
+  };
+
   if (warp == 0) {
     // ------------------------------ TMA producer (all lanes) ------------------------------
     const uint32_t bar_empty0 = ptx::smem_u32(&ctl->empty[0]), bar_full0 = ptx::smem_u32(&ctl->full[0]);
@@ -134,8 +172,22 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     }
     uint32_t s = 0, ph = 0;
     bool alive = true;
-    for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
+    auto publish = [&](const RowsTile& x) -> bool {
+      if (!ROWS_WAIT(bar_tile_empty0 + ts * 8, tph ^ 1u)) {
+        *abort_flag = 1;
+        return false;
+      }
+      if (lane == 0) {
+        ctl->tile[ts] = x;
+        ptx::mbar_arrive(bar_tile_full0 + ts * 8);
+      }
+      if (++ts == (uint32_t)kTileSlots) ts = 0, tph ^= 1u;
+      return true;
+    };
+    int t_next = 0;
+    for (int t = tile_first; t < num_tiles && alive; t = kGrouped ? __shfl_sync(0xffffffffu, t_next, 0) : t + tile_step) {
       const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+      if (kGrouped && !publish(x)) break;
       const bool gather = kGrouped && p.gather_topk > 0;
       int r[4] = {0, 0, 0, 0};
       if (gather && lane * 4 < x.n_eff) {
@@ -149,6 +201,9 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
       for (int kb = kb_begin; kb < kb_stop; ++kb) {
         const uint32_t bar = bar_full0 + s * 8, dst = tiles0 + s * kStageBytes;
         const int k0 = kb * kRowsBK;
+        // (late enough that the next tile is taken by a CTA that can start it, early enough that the answer is not waited for)
+        if (kGrouped && lane == 0 && kb == max(kb_begin, kb_stop - kStages))
+          t_next = p.next_tile != nullptr && num_tiles > (int)gridDim.x ? atomicAdd(p.next_tile, 1) + (int)gridDim.x : t + tile_step;
         if (ahead > 0) {
           --ahead;
         } else {
@@ -170,6 +225,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
         }
       }
     }
+    if (kGrouped && alive) publish(RowsTile{0, 0, 0, 0});
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     if (ptx::elect_one()) {
@@ -179,8 +235,9 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
       const uint32_t bar_tfull0 = ptx::smem_u32(&ctl->tmem_full[0]), bar_tempty0 = ptx::smem_u32(&ctl->tmem_empty[0]);
       uint32_t s = 0, ph = 0, buf = 0, aph = 0;
       bool alive = true;
-      for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
-        const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+      int t = 0;
+      RowsTile x;
+      for (bool first = true; alive && take_tile(t, x, first, true); first = false) {
         const uint32_t idesc = ptx::make_idesc_e4m3_f32(kRowsBM, x.n_eff);
         for (int kb = kb_begin; kb < kb_stop; ++kb) {
           if (!ROWS_WAIT(bar_tempty0 + buf * 8, aph ^ 1u) || !ROWS_WAIT(bar_full0 + s * 8, ph)) {
@@ -217,8 +274,9 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     ptx::grid_dependency_wait();
     uint32_t d = 0, dph = 0;
     bool alive = true;
-    for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
-      const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+    int t = 0;
+    RowsTile x;
+    for (bool first = true; alive && take_tile(t, x, first, false); first = false) {
       const float* b_row = p.b_s + ((int64_t)x.expert * p.nb_total + x.n_tile) * p.kb_total;
       const float* a_row[kPer];
       bool on[kPer];
@@ -275,8 +333,9 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     ptx::grid_dependency_wait();
     uint32_t buf = 0, aph = 0, d = 0, dph = 0;
     bool alive = true, arrived = false, waited = false;
-    for (int t = tile_first; t < num_tiles && alive; t += tile_step) {
-      const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
+    int t = 0;
+    RowsTile x;
+    for (bool first = true; alive && take_tile(t, x, first, false); first = false) {
       const int active = (x.n_eff + kCW - 1) / kCW;  // chunks that hold columns of the tile
       float acc[kChunks][2][kRegs];                  // chunk, 16-lane half, [block][8 columns of it][row lane / 4, + 8][2]
 #pragma unroll
@@ -615,13 +674,13 @@ static int rows_grouped_cfg(const void* A, int64_t a_rows, const void* B, RowsPa
 int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const float* a_s, const void* B, const float* b_s, void* C,
                     const int32_t* cumsum, const int32_t* sorted_ids, const float* row_weights, int64_t max_rows,
                     int64_t numel, int num_experts, int64_t N, int64_t K, int gather_topk, int scatter, int out_dtype, int nt,
-                    bool pdl, cudaStream_t st) {
+                    int32_t* next_tile, bool pdl, cudaStream_t st) {
   RowsParams p{};
   p.a_s = a_s, p.b_s = b_s, p.C = C;
   p.M = a_rows, p.N = N, p.as_stride_m = as_stride, p.as_stride_k = 1;
   p.kb_total = (int)((K + kRowsBK - 1) / kRowsBK), p.nb_total = (int)((N + 127) / 128), p.tiles_n = p.nb_total;
   p.out_fp16 = out_dtype, p.num_experts = num_experts, p.cumsum = cumsum, p.sorted_ids = sorted_ids, p.numel = numel;
-  p.gather_topk = gather_topk, p.scatter = scatter, p.row_weights = row_weights;
+  p.gather_topk = gather_topk, p.scatter = scatter, p.row_weights = row_weights, p.next_tile = next_tile;
   p.wait_probes = g_gemm_wait_probes;
   switch (nt) {
     case 32: return rows_grouped_cfg<Rows32>(A, a_rows, B, p, max_rows, K, pdl, st);

@@ -54,10 +54,11 @@ struct RowsParams {
   int gather_topk;                 // > 0: A has a row per token, fetched by slot / gather_topk; 0: A is in expert order
   int scatter;                     // write row sorted_ids[r] instead of row r
   const float* row_weights;        // scatter, optional
+  int32_t* next_tile;              // optional, zero: tiles beyond the first of every CTA are taken from this counter
   uint32_t wait_probes;
 };
 
-struct RowsTile {
+struct alignas(16) RowsTile {
   int n_tile, row0, n_eff, expert;
 };
 
@@ -87,8 +88,8 @@ __device__ __forceinline__ RowsTile rows_tile(const RowsParams& p, const int* ti
   return x;
 }
 
-// Token tiles (of NT rows) of every expert and their exclusive scan into tiles_before[0 .. experts]: four experts per
-// thread, all NTHREADS threads of the block.  The scan is visible after the next __syncthreads.
+// Token tiles (of NT rows) of every expert and their exclusive scan into tiles_before[0 .. experts], the experts' first rows
+// behind it (a tile is then located without a round trip to L2): four experts per thread, all NTHREADS threads of the block.  The scan is visible after the next __syncthreads.
 template <int NT, int NTHREADS>
 __device__ __forceinline__ void rows_count_tiles(const RowsParams& p, int* tiles_before, int* warp_sum) {
   static_assert(NTHREADS * 4 >= kMaxExperts, "four experts per thread");

@@ -41,7 +41,7 @@ static LinearParts linear_parts(int64_t M, int64_t N, int64_t K) {
 struct ExpertsPlan {
   int tile, block;
   int64_t cap, rows;  // entries of the sort's output; rows that can be in use
-  int64_t q, s, sorted, eid, post, cum, sort, sort_bytes, a1, a1s, ic1, a2, a2s, ic3, total;
+  int64_t q, s, sorted, eid, post, next, cum, sort, sort_bytes, a1, a1s, ic1, a2, a2s, ic3, total;
   bool direct;        // one expert per token and no factor: the second GEMM writes the result itself
 };
 
@@ -73,7 +73,7 @@ static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int6
   p.sort_bytes = sglb200_moe_align_workspace_bytes(numel, (int)E + 1);
   Carver c;
   p.q = c.take(T * H), p.s = c.take(T * (H / 128) * 4);
-  p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4);
+  p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4), p.next = c.take(8);
   p.cum = c.take((E + 2) * 4), p.sort = c.take(p.sort_bytes);
   if (p.tile == 0) p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
   p.ic1 = c.take(p.rows * 2 * I * 2);
@@ -148,9 +148,11 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   void* ic3 = p.direct ? out : base + p.ic3;
   const int64_t hb = H / 128, ib = I / 128;
   int rc;
+  int32_t* next = nullptr;  // counters of the two products' tiles
   if (align_quant_fits(x, numel, (int)E + 1)) {
     rc = align_quant(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), x, dtype, base + p.q, f(p.s), T,
-                     H, kQuantEps, kFp8Max, st);
+                     H, kQuantEps, kFp8Max, i(p.next), st);
+    next = i(p.next);
   } else {
     rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
     if (rc) return rc;
@@ -161,12 +163,12 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   if (p.tile > 0) {
     if (p.direct) SGLB_CUDA(cudaMemsetAsync(out, 0, T * Ho * 2, st));  // rows of negative ids are not written below
     rc = rows_grouped_mm(base + p.q, T, hb, f(p.s), w13, w13_s, base + p.ic1, i(p.cum), i(p.sorted), nullptr, p.rows, numel, (int)E,
-                         2 * I, H, (int)k, 0, dtype, p.tile, true, st);
+                         2 * I, H, (int)k, 0, dtype, p.tile, next, true, st);
     if (rc) return rc;
     rc = silu_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), true, st);
     if (rc) return rc;
     rc = rows_grouped_mm(base + p.a2, p.rows, ib, f(p.a2s), w2, w2_s, ic3, i(p.cum), i(p.sorted), topk_weights, p.rows, numel,
-                         (int)E, Ho, I, 0, 1, dtype, p.tile, true, st);
+                         (int)E, Ho, I, 0, 1, dtype, p.tile, next ? next + 1 : nullptr, true, st);
   } else {
     rc = sglb200_gather_rows_fp8(base + p.q, f(p.s), base + p.a1, f(p.a1s), i(p.sorted), i(p.post), p.rows, numel, (int)k, H, hb,
                                  stream);

@@ -236,10 +236,11 @@ __global__ void __launch_bounds__(kAlignThreads)
     moe_align_quant_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                            int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids, int32_t* __restrict__ post_pad,
                            int32_t* __restrict__ cumsum, const T* __restrict__ x, uint8_t* __restrict__ out_q,
-                           float* __restrict__ out_s, int64_t groups, float eps, float qmax) {
+                           float* __restrict__ out_s, int64_t groups, float eps, float qmax, int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   if (blockIdx.x == 0) {
     align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, true, smem);
+    if (threadIdx.x < 2) zeros[threadIdx.x] = 0;
     return;
   }
   ptx::grid_dependency_wait();
@@ -569,7 +570,7 @@ bool align_quant_fits(const void* x, int64_t numel, int buckets) {
 
 int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                 int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
-                int64_t hidden, float eps, float fp8_max, cudaStream_t st) {
+                int64_t hidden, float eps, float fp8_max, int32_t* zeros, cudaStream_t st) {
   int64_t chunks = 0;
   int span = 0;
   align_plan(numel, &chunks, &span);
@@ -579,10 +580,11 @@ int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, 
   uint8_t* q = static_cast<uint8_t*>(out_q);
   if (dtype == 0)
     SGLB_CUDA(launch_pdl(moe_align_quant_kernel<__nv_bfloat16>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size,
-                         sorted, expert_ids, post_pad, cumsum, static_cast<const __nv_bfloat16*>(x), q, out_s, groups, eps, fp8_max));
+                         sorted, expert_ids, post_pad, cumsum, static_cast<const __nv_bfloat16*>(x), q, out_s, groups, eps, fp8_max,
+                         zeros));
   else
     SGLB_CUDA(launch_pdl(moe_align_quant_kernel<__half>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size, sorted,
-                         expert_ids, post_pad, cumsum, static_cast<const __half*>(x), q, out_s, groups, eps, fp8_max));
+                         expert_ids, post_pad, cumsum, static_cast<const __half*>(x), q, out_s, groups, eps, fp8_max, zeros));
   return SGLB200_OK;
 }
 

@@ -94,6 +94,26 @@ def test_experts_row_counts(T, E, topk):
     assert_close_fp(to_f32_np(out), ref, rtol=2e-2, atol=2e-2)
 
 
+# more tiles than CTAs, taken from a counter (up to 2048 ids) and in turn; experts without rows among them
+@pytest.mark.parametrize("T,E,topk", [(40, 64, 2), (700, 96, 3)])
+def test_experts_many_tiles(T, E, topk):
+    from sglang_b200 import ops
+    from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
+    H, I = 256, 640
+    x = make_act(T, H, T, outliers=False)
+    w13q, w13s = make_weight(2 * I, H, 1, std=0.05, experts=E)
+    w2q, w2s = make_weight(H, I, 2, std=0.05, experts=E)
+    w, ids = torch.topk(torch.softmax(torch.randn(T, E, generator=torch.Generator().manual_seed(T)), -1), topk, dim=-1)
+    ids = ids.to(torch.int32)
+    ref = O.fused_experts_block_fp8(to_f32_np(x), w13q, w13s, w2q, w2s, w.numpy(), ids.numpy(), 1.0)
+    args = (x.cuda(), codes_to_fp8(w13q), codes_to_fp8(w2q), w.cuda(), ids.cuda())
+    for _ in range(3):
+        out = fused_experts_impl(*args, use_fp8_w8a8=True, w1_scale=torch.from_numpy(w13s).cuda(),
+                                 w2_scale=torch.from_numpy(w2s).cuda(), block_shape=[128, 128])
+        assert_close_fp(to_f32_np(out), ref, rtol=2e-2, atol=2e-2)
+    assert ops.gemm_status() == 0 and ops.stream_status() == 0
+
+
 # sort and quantizer in one launch (up to 2048 ids) and in two: a single group of CTAs part filled, the last size of the one, the
 # first of the other
 @pytest.mark.parametrize("T,E,topk", [(1, 4, 2), (43, 8, 3), (1024, 8, 2), (1025, 8, 2)])
