@@ -39,6 +39,12 @@ int quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s, 
 int silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s, int64_t rows, int64_t d, int group_size,
                        float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t st);
 
+// moe_align.cu: the sort (arguments as sglb200_moe_align_block_size); zeros[0] and zeros[1] are set to 0 where the ids take
+// more than one CTA and are at most 2^20 (otherwise left alone).
+int align_block_size(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size, int32_t* sorted_token_ids,
+                     int32_t* expert_ids, int32_t* num_tokens_post_pad, int32_t* cumsum_buffer, int pad_sorted_token_ids,
+                     void* workspace, int64_t workspace_bytes, int32_t* zeros, cudaStream_t st);
+
 // moe_align.cu: the sort of few ids (as sglb200_moe_align_block_size, padding written) and the quantizer of the same layer's
 // activations (groups of 128) in one launch, where `align_quant_fits`.  zeros[0] and zeros[1] are set to 0.
 bool align_quant_fits(const void* x, int64_t numel, int buckets);

@@ -156,8 +156,9 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   } else {
     rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
     if (rc) return rc;
-    rc = sglb200_moe_align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
-                                      p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, stream);
+    rc = align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
+                          p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, i(p.next), st);
+    if (p.sort_bytes > 0 && numel <= (1 << 20)) next = i(p.next);
   }
   if (rc) return rc;
   if (p.tile > 0) {

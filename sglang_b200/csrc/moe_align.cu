@@ -301,7 +301,8 @@ __global__ void __launch_bounds__(kAlignThreads)
     moe_align_scatter_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                              const int* __restrict__ chunk_hist, const int* __restrict__ totals,
                              int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
-                             int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted) {
+                             int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
+                             int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   int* wc = smem;                       // [32][B]
   int* tot = wc + kAlignWarps * B;      // [B]   this chunk's totals (unused after scan) / all-chunk totals
@@ -316,6 +317,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   if (blockIdx.x == 0) {
     for (int b = threadIdx.x; b <= B; b += kAlignThreads) cumsum[b] = prefix[b];
     if (threadIdx.x == 0) *post_pad = prefix[B];
+    if (zeros != nullptr && threadIdx.x < 2) zeros[threadIdx.x] = 0;
   }
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, blockIdx.x, gridDim.x);
   __syncthreads();  // fill_meta is done with tot[] before it is reused below
@@ -338,7 +340,8 @@ template <int NBITS>
 __global__ void __launch_bounds__(kAlignThreads)
     moe_align_coop_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                           int* __restrict__ chunk_hist, int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
-                          int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted) {
+                          int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
+                          int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   int* wc = smem;                       // [32][B]
   int* tot = wc + kAlignWarps * B;      // [B]   this chunk's totals, then the totals over all chunks
@@ -388,6 +391,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   if (blockIdx.x == 0) {
     for (int b = threadIdx.x; b <= B; b += kAlignThreads) cumsum[b] = prefix[b];
     if (threadIdx.x == 0) *post_pad = prefix[B];
+    if (zeros != nullptr && threadIdx.x < 2) zeros[threadIdx.x] = 0;
   }
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, blockIdx.x, gridDim.x);
   __syncthreads();
@@ -396,7 +400,8 @@ __global__ void __launch_bounds__(kAlignThreads)
 
 static bool g_align_coop_enabled = true;  // sglb200_moe_align_set_cooperative
 
-using CoopKernel = void (*)(const int32_t*, int64_t, int, int, int, int*, int32_t*, int32_t*, int32_t*, int32_t*, bool);
+using CoopKernel = void (*)(const int32_t*, int64_t, int, int, int, int*, int32_t*, int32_t*, int32_t*, int32_t*, bool,
+                              int32_t*);
 static CoopKernel coop_kernel_for(int B) {
   switch (32 - __builtin_clz((unsigned)(B + 31))) {  // keys run up to B + 31
     case 6: return moe_align_coop_kernel<6>;
@@ -607,11 +612,10 @@ extern "C" int64_t sglb200_moe_align_workspace_bytes(int64_t numel, int num_expe
   return (chunks + 1) * (int64_t)num_experts * (int64_t)sizeof(int);
 }
 
-extern "C" int sglb200_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size,
-                                            int32_t* sorted_token_ids, int32_t* expert_ids,
-                                            int32_t* num_tokens_post_pad, int32_t* cumsum_buffer,
-                                            int pad_sorted_token_ids, void* workspace, int64_t workspace_bytes,
-                                            void* stream) {
+int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size, int32_t* sorted_token_ids,
+                              int32_t* expert_ids, int32_t* num_tokens_post_pad, int32_t* cumsum_buffer,
+                              int pad_sorted_token_ids, void* workspace, int64_t workspace_bytes, int32_t* zeros,
+                              cudaStream_t st) {
   SGLB_REQUIRE(numel >= 0 && numel < (1ll << 31) - (int64_t)num_experts * block_size, "moe_align: numel %lld too large",
                (long long)numel);
   SGLB_REQUIRE(num_experts >= 1 && block_size >= 1, "moe_align: num_experts %d, block_size %d", num_experts, block_size);
@@ -620,7 +624,6 @@ extern "C" int sglb200_moe_align_block_size(const int32_t* topk_ids, int64_t num
   const int B = num_experts;
   const size_t smem = align_smem_bytes(B);
   SGLB_REQUIRE(smem <= 200 * 1024, "moe_align: %d buckets need %zu bytes of shared memory (limit 200 KiB)", B, smem);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (smem > 48 * 1024) {
     // opt in to more than 48 KiB of dynamic shared memory (a per-function, per-device attribute; cheap to repeat)
     SGLB_CUDA(cudaFuncSetAttribute(moe_align_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -689,7 +692,7 @@ extern "C" int sglb200_moe_align_block_size(const int32_t* topk_ids, int64_t num
     if (coop_fits(kern, chunks, smem)) {
       bool pad = pad_sorted_token_ids != 0;
       void* args[] = {&topk_ids, &numel, &span, (void*)&B, &block_size, &chunk_hist, &sorted_token_ids, &expert_ids,
-                      &num_tokens_post_pad, &cumsum_buffer, &pad};
+                      &num_tokens_post_pad, &cumsum_buffer, &pad, &zeros};
       SGLB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern),
                                             dim3((unsigned)chunks), dim3(kAlignThreads), args, smem, st));
       return SGLB200_OK;
@@ -701,9 +704,19 @@ extern "C" int sglb200_moe_align_block_size(const int32_t* topk_ids, int64_t num
   moe_align_scatter_kernel<<<(unsigned)chunks, kAlignThreads, smem, st>>>(topk_ids, numel, span, B, block_size, chunk_hist,
                                                                           totals, sorted_token_ids, expert_ids,
                                                                           num_tokens_post_pad, cumsum_buffer,
-                                                                          pad_sorted_token_ids != 0);
+                                                                          pad_sorted_token_ids != 0, zeros);
   SGLB_CUDA(cudaGetLastError());
   return SGLB200_OK;
+}
+
+extern "C" int sglb200_moe_align_block_size(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size,
+                                            int32_t* sorted_token_ids, int32_t* expert_ids,
+                                            int32_t* num_tokens_post_pad, int32_t* cumsum_buffer,
+                                            int pad_sorted_token_ids, void* workspace, int64_t workspace_bytes,
+                                            void* stream) {
+  return align_block_size(topk_ids, numel, num_experts, block_size, sorted_token_ids, expert_ids, num_tokens_post_pad,
+                          cumsum_buffer, pad_sorted_token_ids, workspace, workspace_bytes, nullptr,
+                          static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------------------
