@@ -601,10 +601,9 @@ int64_t paired_clusters(int s) { return s % 2 == 0 ? spread_clusters(s / 2) : 2 
 // slabs and the exchange of a cluster two more.  Where CTAs share SMs a slab takes 7/4 and start, end and exchange a little
 // longer (a cluster or two too many for one CTA an SM still count as alone); clusters beyond what two CTAs an SM hold
 // wait for a whole round.
-// Measured with 64 and 20 rows over splits of 1 to 8: 4096 x 4096 four CTAs 11.5 / 8.9 us, eight (sharing SMs) 12.4 / 9.6;
-// K 7168 with N 2112 six 11.8 / 9.1, eight 12.2 / 9.6; 4096 x 14336 eight 20.3, four 21.4; 10240 x 8192 three 23.9, two
-// 29.3, four 32.9 (a second round); 4616 x 1920 three 9.8, eight 14.5 (296 CTAs, but 37 clusters of eight do not fit);
-// 14944 x 768 one 9.4, two 11.5.  More than eight CTAs, for few tiles and a long K: 512 x 8192 sixteen 8.6, eight 9.5; 768 x
+// Measured with 64 rows over splits of 1 to 8: 4096 x 4096 four CTAs 10.0 us, eight (sharing SMs) 10.9; K 7168 with N 2112
+// six 10.7, eight 11.0; 4096 x 14336 eight 16.1, four 18.1; 10240 x 8192 three 19.8, two 23.4, four 26.8 (a second round);
+// 4616 x 1920 three 9.0, eight 14.1 (296 CTAs, but 37 clusters of eight do not fit); 14944 x 768 one 7.2, two 8.8.  More than eight CTAs, for few tiles and a long K: 512 x 8192 sixteen 8.6, eight 9.5; 768 x
 // 18432 sixteen 11.1, eight 14.0; 1024 x 8192 ten 9.6, eight 9.9, sixteen 10.8; where that gains no whole slab, eight
 // (1536 x 7168 with 20 rows eight 7.3, nine 7.5).  With up to 32 rows, which are not pushed, they have to gain more
 // than one (32 rows: 1280 x 5120 eight 7.0, ten 7.2; 576 x 7168 eight 7.4, fourteen 7.2; 640 x 12288 eight 8.6, sixteen 7.8).

@@ -304,6 +304,8 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
       : "r"(taddr)
       : "memory");
 }
+// For the loads in front of it in straight-line code: with a branch between the loads and the wait a buffer of tensor memory
+// was handed back, and written by the next MMA, before the last load had read it.
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // 16 lanes x 8 N columns: per 8 columns a thread receives columns 2 (lane % 4), + 1 of lane (lane / 4) in r[0], r[1] and of
