@@ -33,7 +33,7 @@ def sources():
 
 
 def _headers():
-    return glob.glob(os.path.join(PKG, "..", "include", "*.h"))
+    return glob.glob(os.path.join(PKG, "..", "include", "*.h")) + glob.glob(os.path.join(CSRC, "*.h"))
 
 
 def _stale(target: str, deps) -> bool:

@@ -21,8 +21,9 @@
 // shared-memory port is the limit: 64 rows stage 24 KB a slab and the MMA reads them back, 384 clocks at 128 bytes a
 // clock; see the promotion for what the scales add.
 // Every mbarrier wait is bounded as in gemm.cu (status word, no trap).
-#include <atomic>
 #include <cuda.h>
+
+#include <mutex>
 
 #include "common.cuh"
 #include "gemm_rows.cuh"
@@ -567,61 +568,37 @@ static int launch_rows(const CUtensorMap& mw, const CUtensorMap& ma, const RowsP
   return SGLB200_OK;
 }
 
-// Never launched: the occupancy question below is asked about it.
-__global__ void spread_probe_kernel() {}
+// Never launched: the occupancy questions below are asked about it.
+__global__ void cluster_probe_kernel() {}
 
-int64_t spread_clusters(int s) {
-  if (s == 1) return sm_count();
-  constexpr int kSmem = 120 * 1024;  // of 227 KB: one CTA per SM
-  static std::atomic<int> known[64][kMostClusterCtas + 1];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return s <= 8 ? sm_count() / s : 0;
-  int n = known[dev][s].load(std::memory_order_relaxed);
-  if (n == 0) {
+const ClusterFits& cluster_fits() {
+  constexpr int kAlone = 120 * 1024, kPaired = 104 * 1024;  // of 227 KB: one and two CTAs per SM
+  const auto ask = [](int s, int per_sm) -> int64_t {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = (unsigned)s, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)s, 1, 1), cfg.blockDim = dim3(256, 1, 1), cfg.dynamicSmemBytes = kSmem;
+    cfg.gridDim = dim3((unsigned)s, 1, 1), cfg.blockDim = dim3(256, 1, 1);
+    cfg.dynamicSmemBytes = per_sm == 1 ? kAlone : kPaired;
     cfg.attrs = &attr, cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(spread_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(spread_probe_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, spread_probe_kernel, &cfg) != cudaSuccess || n <= 0) {
+    int n = 0;
+    if (cudaFuncSetAttribute(cluster_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlone) != cudaSuccess ||
+        cudaFuncSetAttribute(cluster_probe_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, cluster_probe_kernel, &cfg) != cudaSuccess) {
       cudaGetLastError();
-      n = s <= 8 ? sm_count() / s : -1;
+      return 0;
     }
-    known[dev][s].store(n, std::memory_order_relaxed);
+    return n;
+  };
+  static std::once_flag once[64];
+  static ClusterFits known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    static const ClusterFits portable = cluster_fits_of([](int, int) -> int64_t { return 0; }, 148);
+    return portable;
   }
-  return n > 0 ? n : 0;
-}
-int64_t paired_clusters(int s) { return s % 2 == 0 ? spread_clusters(s / 2) : 2 * spread_clusters(s); }
-
-// CTAs per cluster for a dense problem of `tiles` tiles and `kb` slabs: the split that finishes first, counted in
-// quarters of the time of a slab in a CTA that has an SM to itself (0.41 us with 64 rows).  A CTA's start and end are three
-// slabs and the exchange of a cluster two more.  Where CTAs share SMs a slab takes 7/4 and start, end and exchange a little
-// longer (a cluster or two too many for one CTA an SM still count as alone); clusters beyond what two CTAs an SM hold
-// wait for a whole round.
-// Measured with 64 rows over splits of 1 to 8: 4096 x 4096 four CTAs 10.0 us, eight (sharing SMs) 10.9; K 7168 with N 2112
-// six 10.7, eight 11.0; 4096 x 14336 eight 16.1, four 18.1; 10240 x 8192 three 19.8, two 23.4, four 26.8 (a second round);
-// 4616 x 1920 three 9.0, eight 14.1 (296 CTAs, but 37 clusters of eight do not fit); 14944 x 768 one 7.2, two 8.8.  More than eight CTAs, for few tiles and a long K: 512 x 8192 sixteen 8.6, eight 9.5; 768 x
-// 18432 sixteen 11.1, eight 14.0; 1024 x 8192 ten 9.6, eight 9.9, sixteen 10.8; where that gains no whole slab, eight
-// (1536 x 7168 with 20 rows eight 7.3, nine 7.5).  With up to 32 rows, which are not pushed, they have to gain more
-// than one (32 rows: 1280 x 5120 eight 7.0, ten 7.2; 576 x 7168 eight 7.4, fourteen 7.2; 640 x 12288 eight 8.6, sixteen 7.8).
-static int rows_splits(int64_t tiles, int kb, bool pushed) {
-  const int large = pushed ? 1 : 5;
-  int best = 1;
-  int64_t best_cost = -1;
-  for (int s = 1; s <= kMaxSplits && s <= kb; ++s) {
-    const int64_t per = (kb + s - 1) / s, spread = spread_clusters(s);
-    const int64_t fit = paired_clusters(s);
-    if (fit == 0) continue;
-    const int64_t rounds = (tiles + fit - 1) / fit;
-    const bool alone = tiles <= (s == 1 ? spread : spread + spread / 16);
-    const int64_t cost = s == 1 ? rounds * per * (alone ? 4 : 7) + 12
-                                : (alone ? 4 * per + 20 + (s > 8 ? large : 0) : rounds * (7 * per + (s > 4 ? 28 : 22)));
-    if (best_cost < 0 || cost <= best_cost) best = s, best_cost = cost;
-  }
-  return best;
+  std::call_once(once[dev], [&] { known[dev] = cluster_fits_of(ask, sm_count()); });
+  return known[dev];
 }
 
 template <class Cfg>
@@ -635,7 +612,7 @@ static int rows_dense_cfg(const void* A, const void* B, RowsParams& p, int64_t K
   p.group_m = choose_group_m(p.M, K, Cfg::NT);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
   static_assert(Cfg::kCtasPerSm == 2, "rows_splits counts on two");
-  p.splits = rows_splits(tiles, p.kb_total, Cfg::NT == 64);
+  p.splits = rows_splits(tiles, p.kb_total, Cfg::NT == 64, cluster_fits());
   return launch_rows<Cfg, false>(mw, ma, p, tiles, pdl, st);
 }
 

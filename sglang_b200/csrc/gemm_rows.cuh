@@ -1,5 +1,6 @@
 // Shared by the kernels with the weights on the M side (gemm_rows.cu, gemm_small.cu): launch parameters, the walk over tiles, the count of the experts' token tiles.
 #pragma once
+#include "cluster_rule.h"
 #include "common.cuh"
 #include "gemm_common.cuh"
 #include "ptx_sm100.cuh"
@@ -11,7 +12,6 @@ constexpr int kRowsBK = 128;                     // K slab: one scale block
 constexpr uint32_t kWBytes = kRowsBM * kRowsBK;  // weight bytes per stage
 constexpr int kScBatch = 8;                      // slabs whose scales are prepared together
 constexpr int kMaxExperts = 1024;
-constexpr int kMostClusterCtas = 16;
 constexpr int kMaxSplits = kMostClusterCtas;     // CTAs of a cluster
 constexpr int kPartPitch = kRowsBM + 4;          // floats between the columns of a CTA's partial sums
 constexpr int kPartPair = 2 * kRowsBM + 8;       // the same between pairs of columns in the pushed form
@@ -26,12 +26,8 @@ __device__ __forceinline__ int frag_column(int j) { return (j & ~15) + ((j & 7) 
 // with 256 columns there is room for one other of either kind, without one for three of 128.  The 128-row kernel, which takes
 // all columns, leaves no registers for another CTA.
 
-// Clusters of `s` CTAs that the current GPU holds at once with one CTA on an SM: a cluster stays within a GPC, whose number
-// of SMs differs from GPC to GPC and from GPU to GPU, so the driver is asked (once per device and size).  And with two on
-// an SM: a GPC holds as many clusters of 2s CTAs at two an SM as of s at one; for odd sizes at least twice as many.
-// Where the driver does not say, eight CTAs or fewer (the portable sizes) are taken to fit everywhere and more not at all.
-int64_t spread_clusters(int s);
-int64_t paired_clusters(int s);
+// What the current GPU holds of clusters (the driver is asked once per device).
+const ClusterFits& cluster_fits();
 
 struct RowsParams {
   const float* a_s;

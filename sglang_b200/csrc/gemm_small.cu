@@ -25,7 +25,6 @@ constexpr int kSmallRows = 16;
 constexpr int kSmallWarps = 8;                            // quantise (the first four then promote); one more loads and multiplies
 constexpr int kSmallThreads = (kSmallWarps + 1) * 32;
 constexpr int kSmallMaxSlabs = 8;
-constexpr int kSmallMaxSplits = kMostClusterCtas;
 constexpr int kSmallTmem = kSmallMaxSlabs * kSmallRows;
 constexpr uint32_t kSmallTokBytes = kSmallRows * kRowsBK;
 constexpr int64_t kSmallSmem = 111 * 1024;                // two CTAs per SM
@@ -165,7 +164,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2)
   __syncwarp();
   ptx::cluster_sync();
   const RowsTile t{n_tile, 0, kSmallRows, 0};
-  if (ctl->abort_flag == 0) rows_cluster_sum<kSmallMaxSplits>(p, t, rank, ptx::smem_u32(weights), tid, kSmallThreads);
+  if (ctl->abort_flag == 0) rows_cluster_sum<kMostClusterCtas>(p, t, rank, ptx::smem_u32(weights), tid, kSmallThreads);
   ptx::cluster_sync();  // no CTA leaves while another reads its shared memory
 
   // ------------------------------ teardown ------------------------------
@@ -191,25 +190,16 @@ struct SmallPlan {
 static int64_t small_smem_bytes(int slabs) {
   return 1024 + (int64_t)slabs * (kWBytes + kSmallTokBytes + kSmallRows * 4) + (int64_t)sizeof(SmallCtl);
 }
-// CTAs per cluster: the cheapest split with which a CTA's slabs fit in half an SM and all clusters run at once, in
-// hundredths of a microsecond: 45 for a slab of a CTA, one for a CTA of the grid (they share the SMs, the L2 and the
-// launch), 60 for a CTA without a cluster, 20 for an odd cluster (half of a pair of SMs idles), 15 for a cluster of more
-// than eight and ten for each of its CTAs beyond the eighth.  Measured with 16 rows over all splits: 512 x 512 one CTA 5.2 us, four 3.6; 4096 x 1024 two 5.3, four
-// 4.8, eight 6.1; 7168 x 2048 three 8.0, four 6.9, five 8.2; 2048 x 2048 four 5.0, eight 4.8; 1024 x 8192 eleven 7.1,
-// sixteen 5.8; 4368 x 4352 six 8.7, eight 12.8 (35 clusters of eight do not fit), quantised in a launch of its own 10.6.
 static SmallPlan small_plan(int64_t M, int64_t N, int64_t K) {
   SmallPlan pl{0, 0};
   if (M > kSmallRows || K % kRowsBK != 0) return pl;
-  const int kb = (int)(K / kRowsBK);
   const int64_t tiles = (N + kRowsBM - 1) / kRowsBM;
-  if (kb > kSmallMaxSlabs * kSmallMaxSplits || tiles > 2 * (int64_t)sm_count()) return pl;
-  int64_t best_cost = -1;
-  for (int s = 1; s <= kSmallMaxSplits && s <= kb; ++s) {
-    const int slabs = (kb + s - 1) / s;
-    if (slabs > kSmallMaxSlabs || small_smem_bytes(slabs) > kSmallSmem || tiles > paired_clusters(s)) continue;
-    const int64_t cost = 45 * slabs + tiles * s + (s == 1 ? 60 : s % 2 != 0 ? 20 : 0) + (s > 8 ? 15 + 10 * (s - 8) : 0);
-    if (best_cost < 0 || cost < best_cost) pl.splits = s, pl.slabs = slabs, best_cost = cost;
-  }
+  if (K / kRowsBK > kSmallMaxSlabs * kMostClusterCtas || tiles > 2 * (int64_t)sm_count()) return pl;
+  int most = kSmallMaxSlabs;
+  while (small_smem_bytes(most) > kSmallSmem) --most;
+  const int kb = (int)(K / kRowsBK);
+  pl.splits = small_splits(tiles, kb, most, cluster_fits());
+  if (pl.splits > 0) pl.slabs = (kb + pl.splits - 1) / pl.splits;
   return pl;
 }
 

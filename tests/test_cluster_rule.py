@@ -1,0 +1,73 @@
+"""Over how many CTAs K is split (csrc/cluster_rule.h), compiled for the CPU and asked about GPUs of different kinds."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sglang_b200", "csrc")
+SHIM = """
+#include "cluster_rule.h"
+using namespace sglb200;
+extern "C" void fits(const int64_t* one, const int64_t* two, int64_t sms, ClusterFits* f) {
+  *f = cluster_fits_of([&](int s, int per_sm) { return per_sm == 1 ? one[s] : two[s]; }, sms);
+}
+extern "C" int rows(int64_t tiles, int kb, int pushed, const ClusterFits* f) { return rows_splits(tiles, kb, pushed != 0, *f); }
+extern "C" int one_launch(int64_t tiles, int kb, int most, const ClusterFits* f) { return small_splits(tiles, kb, most, *f); }
+"""
+ROW = ctypes.c_int64 * 17
+# clusters of 0, 1, .. 16 CTAs that a B200 holds, as its driver says: one CTA on an SM, two on an SM
+B200 = ([0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7],
+        [0, 296, 148, 93, 71, 56, 45, 37, 33, 30, 26, 21, 21, 17, 14, 14, 14])
+# the same where sizes above eight are refused, and where the driver says nothing
+PORTABLE = tuple(r[:9] + [0] * 8 for r in B200)
+SILENT = ([0] * 17, [-1] * 17)
+
+
+class Fits(ctypes.Structure):
+    _fields_ = [("alone", ROW), ("paired", ROW)]
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    d = tmp_path_factory.mktemp("cluster_rule")
+    (d / "shim.cpp").write_text(SHIM)
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", CSRC, "-o", str(d / "shim.so"), str(d / "shim.cpp")])
+    lib = ctypes.CDLL(str(d / "shim.so"))
+    lib.rows.argtypes = lib.one_launch.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.POINTER(Fits)]
+
+    def fits(gpu):
+        f = Fits()
+        lib.fits(ROW(*gpu[0]), ROW(*gpu[1]), ctypes.c_int64(148), ctypes.byref(f))
+        return f
+
+    lib.of = fits
+    return lib
+
+
+TILES, SLABS = range(1, 300, 3), range(1, 148, 3)
+
+
+def test_no_more_clusters_are_counted_than_the_driver_says(rule):
+    f = rule.of(B200)
+    for s in range(1, 17):
+        assert 0 < f.alone[s] <= B200[0][s] and 0 < f.paired[s] <= B200[1][s], s
+
+
+def test_the_one_launch_linear_takes_only_clusters_that_run_at_once(rule):
+    for gpu in (B200, PORTABLE):
+        f = rule.of(gpu)
+        for tiles in range(1, 297):
+            for kb in range(1, 129):
+                s = rule.one_launch(tiles, kb, 6, f)
+                assert s == 0 or tiles <= gpu[1][s], (tiles, kb, s)
+
+
+@pytest.mark.parametrize("gpu", [PORTABLE, SILENT])
+def test_a_size_that_the_driver_refuses_is_never_taken(rule, gpu):
+    f = rule.of(gpu)
+    for tiles in TILES:
+        for kb in SLABS:
+            for pushed in (0, 1):
+                assert 1 <= rule.rows(tiles, kb, pushed, f) <= 8, (tiles, kb, pushed)
+            assert rule.one_launch(tiles, kb, 6, f) <= 8, (tiles, kb)
