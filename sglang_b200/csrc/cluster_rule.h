@@ -46,10 +46,14 @@ inline ClusterFits cluster_fits_of(const Ask& ask, int64_t sms) {
 // 4616 x 1920 three 9.0, eight 14.1 (296 CTAs, but 37 clusters of eight do not fit); 14944 x 768 one 7.2, two 8.8.  More than
 // eight CTAs, for few tiles and a long K: 512 x 8192 sixteen 8.6, eight 9.5; 768 x 18432 sixteen 11.1, eight 14.0; 1024 x
 // 8192 ten 9.6, eight 9.9, sixteen 10.8; where that gains no whole slab, eight (1536 x 7168 with 20 rows eight 7.3, nine
-// 7.5).  With up to 32 rows, whose partial sums are not `pushed`, they have to gain more than one (32 rows: 1280 x 5120 eight
-// 7.0, ten 7.2; 576 x 7168 eight 7.4, fourteen 7.2; 640 x 12288 eight 8.6, sixteen 7.8).
-inline int rows_splits(int64_t tiles, int kb, bool pushed, const ClusterFits& fits) {
-  const int large = pushed ? 1 : 5;
+// 7.5).  With up to 32 rows, whose partial sums are not pushed, they have to gain more than one (32 rows: 1280 x 5120 eight
+// 7.0, ten 7.2; 576 x 7168 eight 7.4, fourteen 7.2; 640 x 12288 eight 8.6, sixteen 7.8).  Both hold where CTAs share SMs as well
+// (64 rows: 19200 x 16128 five CTAs 68.2, nine 80.7; 3840 x 4352 four 11.5, nine 12.3; 3200 x 9856 five 14.4, ten 15.5; 32
+// rows: 2560 x 13696 six 12.6, twelve 13.2), but for even clusters with 33 to 48 rows, which exchange less (35 rows: 3072 x
+// 10240 five 13.9, ten 13.3; 39 rows: 2688 x 12288 six 14.1, twelve 13.7).  Still the better ones: ten for 3072 x 14720 with
+// 52 rows (16.7, five 17.2) and 3072 x 10240 with 49 (13.7, five 14.1).
+inline int rows_splits(int64_t tiles, int kb, int64_t rows, const ClusterFits& fits) {
+  const int large = rows > 32 ? 1 : 5;  // (more than 32 rows: partial sums are pushed)
   int best = 1;
   int64_t best_cost = -1;
   for (int s = 1; s <= kMostClusterCtas && s <= kb; ++s) {
@@ -57,8 +61,9 @@ inline int rows_splits(int64_t tiles, int kb, bool pushed, const ClusterFits& fi
     if (fit == 0) continue;
     const int64_t rounds = (tiles + fit - 1) / fit;
     const bool alone = tiles <= (s == 1 ? spread : spread + spread / 16);
+    const bool charged = s > 8 && (alone || s % 2 != 0 || rows <= 32 || rows > 48);
     const int64_t cost = s == 1 ? rounds * per * (alone ? 4 : 7) + 12
-                                : (alone ? 4 * per + 20 + (s > 8 ? large : 0) : rounds * (7 * per + (s > 4 ? 28 : 22)));
+                                : (alone ? 4 * per + 20 : rounds * (7 * per + (s > 4 ? 28 : 22))) + (charged ? large : 0);
     if (best_cost < 0 || cost <= best_cost) best = s, best_cost = cost;
   }
   return best;

@@ -612,7 +612,7 @@ static int rows_dense_cfg(const void* A, const void* B, RowsParams& p, int64_t K
   p.group_m = choose_group_m(p.M, K, Cfg::NT);
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
   static_assert(Cfg::kCtasPerSm == 2, "rows_splits counts on two");
-  p.splits = rows_splits(tiles, p.kb_total, Cfg::NT == 64, cluster_fits());
+  p.splits = rows_splits(tiles, p.kb_total, p.M, cluster_fits());
   return launch_rows<Cfg, false>(mw, ma, p, tiles, pdl, st);
 }
 

@@ -12,7 +12,7 @@ using namespace sglb200;
 extern "C" void fits(const int64_t* one, const int64_t* two, int64_t sms, ClusterFits* f) {
   *f = cluster_fits_of([&](int s, int per_sm) { return per_sm == 1 ? one[s] : two[s]; }, sms);
 }
-extern "C" int rows(int64_t tiles, int kb, int pushed, const ClusterFits* f) { return rows_splits(tiles, kb, pushed != 0, *f); }
+extern "C" int rows(int64_t tiles, int kb, int m, const ClusterFits* f) { return rows_splits(tiles, kb, m, *f); }
 extern "C" int one_launch(int64_t tiles, int kb, int most, const ClusterFits* f) { return small_splits(tiles, kb, most, *f); }
 """
 ROW = ctypes.c_int64 * 17
@@ -68,6 +68,15 @@ def test_a_size_that_the_driver_refuses_is_never_taken(rule, gpu):
     f = rule.of(gpu)
     for tiles in TILES:
         for kb in SLABS:
-            for pushed in (0, 1):
-                assert 1 <= rule.rows(tiles, kb, pushed, f) <= 8, (tiles, kb, pushed)
+            for m in (17, 40, 64):
+                assert 1 <= rule.rows(tiles, kb, m, f) <= 8, (tiles, kb, m)
             assert rule.one_launch(tiles, kb, 6, f) <= 8, (tiles, kb)
+
+
+# (tiles, slabs, rows, CTAs measured as the faster ones): more than eight, sharing SMs, save less than they cost, but for even
+# clusters with 33 to 48 rows
+@pytest.mark.parametrize("tiles,kb,m,want", [(150, 126, 64, 5), (150, 126, 34, 5), (18, 91, 61, 6), (25, 77, 64, 5), (30, 34, 61, 4),
+                                             (29, 35, 43, 4), (24, 80, 35, 10), (21, 96, 39, 12), (20, 107, 32, 6),
+                                             (25, 78, 20, 5), (30, 64, 30, 8), (12, 127, 17, 8)])
+def test_large_clusters_that_share_sms_have_to_gain_too(rule, tiles, kb, m, want):
+    assert rule.rows(tiles, kb, m, rule.of(B200)) == want
