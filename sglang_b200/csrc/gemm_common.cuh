@@ -39,14 +39,13 @@ int quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s, 
 int silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s, int64_t rows, int64_t d, int group_size,
                        float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t st);
 
-// moe_align.cu: the sort (arguments as sglb200_moe_align_block_size); zeros[0] and zeros[1] are set to 0 where the ids take
-// more than one CTA and are at most 2^20 (otherwise left alone).
+// moe_align.cu: the sort (arguments as sglb200_moe_align_block_size).  `zeros` (or nullptr): zeros[0] and zeros[1] are set to 0.
 int align_block_size(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size, int32_t* sorted_token_ids,
                      int32_t* expert_ids, int32_t* num_tokens_post_pad, int32_t* cumsum_buffer, int pad_sorted_token_ids,
                      void* workspace, int64_t workspace_bytes, int32_t* zeros, cudaStream_t st);
 
 // moe_align.cu: the sort of few ids (as sglb200_moe_align_block_size, padding written) and the quantizer of the same layer's
-// activations (groups of 128) in one launch, where `align_quant_fits`.  zeros[0] and zeros[1] are set to 0.
+// activations (groups of 128) in one launch, where `align_quant_fits`.  `zeros` as above.
 bool align_quant_fits(const void* x, int64_t numel, int buckets);
 int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                 int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
@@ -61,7 +60,7 @@ int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, 
 // gemm_rows.cu: the dense product for few activation rows, and the expert-grouped one on rows sorted with a padding of
 // 16 (`cumsum` = padded starts of the buckets, as the sort writes them; bucket 0 = filtered ids is skipped).
 // `gather_topk` > 0: A and a_s have a row per token, fetched by sorted slot / gather_topk; 0: a row per sorted row.
-// `nt` = activation rows per tile: 32 or 64.  `next_tile`: a zero (or nullptr), see RowsParams.
+// `nt` = activation rows per tile: 32 or 64.  `next_tile`: a zero, see RowsParams.
 int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
                   int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, bool after_quantizer,
                   cudaStream_t st);

@@ -123,8 +123,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
   const int kb_begin = rank * p.kb_total / splits, kb_stop = (rank + 1) * p.kb_total / splits;
 
   // The tiles of this CTA, one call after the other: in the dense form every role counts for itself, in the grouped one the
-  // producer takes them (from a counter that the CTAs share, where there is one) and hands them to the other roles through
-  // a ring.  `t` and `x` are the caller's; false = none left, or a wait expired.
+  // producer takes them (from a counter that the CTAs share) and hands them to the other roles through a ring.  `t` and `x` are the caller's; false = none left, or a wait expired.
   // The counter is for experts with more tiles than CTAs: those that HBM serves faster then take more of them, and a last
   // round that is part full spreads over all SMs.  Dealt out in turn, the CTAs of 256 experts of 7168 x 2048 with 64 tokens
   // ended between 849 and 940 us of the first product; the layer took 1 419 us and takes 1 369; 128 experts of 2048 x 768
@@ -204,7 +203,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
         const int k0 = kb * kRowsBK;
         // (late enough that the next tile is taken by a CTA that can start it, early enough that the answer is not waited for)
         if (kGrouped && lane == 0 && kb == max(kb_begin, kb_stop - kStages))
-          t_next = p.next_tile != nullptr && num_tiles > (int)gridDim.x ? atomicAdd(p.next_tile, 1) + (int)gridDim.x : t + tile_step;
+          t_next = num_tiles > (int)gridDim.x ? atomicAdd(p.next_tile, 1) + (int)gridDim.x : num_tiles;
         if (ahead > 0) {
           --ahead;
         } else {

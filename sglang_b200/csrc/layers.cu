@@ -148,17 +148,15 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   void* ic3 = p.direct ? out : base + p.ic3;
   const int64_t hb = H / 128, ib = I / 128;
   int rc;
-  int32_t* next = nullptr;  // counters of the two products' tiles
+  int32_t* next = i(p.next);  // counters of the two products' tiles, which the sort sets to zero
   if (align_quant_fits(x, numel, (int)E + 1)) {
     rc = align_quant(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), x, dtype, base + p.q, f(p.s), T,
-                     H, kQuantEps, kFp8Max, i(p.next), st);
-    next = i(p.next);
+                     H, kQuantEps, kFp8Max, next, st);
   } else {
     rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
     if (rc) return rc;
     rc = align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
-                          p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, i(p.next), st);
-    if (p.sort_bytes > 0 && numel <= (1 << 20)) next = i(p.next);
+                          p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, next, st);
   }
   if (rc) return rc;
   if (p.tile > 0) {
@@ -169,7 +167,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     rc = silu_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), true, st);
     if (rc) return rc;
     rc = rows_grouped_mm(base + p.a2, p.rows, ib, f(p.a2s), w2, w2_s, ic3, i(p.cum), i(p.sorted), topk_weights, p.rows, numel,
-                         (int)E, Ho, I, 0, 1, dtype, p.tile, next ? next + 1 : nullptr, true, st);
+                         (int)E, Ho, I, 0, 1, dtype, p.tile, next + 1, true, st);
   } else {
     rc = sglb200_gather_rows_fp8(base + p.q, f(p.s), base + p.a1, f(p.a1s), i(p.sorted), i(p.post), p.rows, numel, (int)k, H, hb,
                                  stream);

@@ -134,6 +134,16 @@ __device__ __forceinline__ void padded_prefix(int B, int block_size, const int* 
   __syncthreads();
 }
 
+// What every sort leaves beside the order, from the one CTA that does it: the padded starts of the buckets, their total, and
+// where there are `zeros`, two counters set to 0.
+template <int NT = kAlignThreads>
+__device__ __forceinline__ void write_starts(int B, const int* prefix, int32_t* __restrict__ cumsum, int32_t* __restrict__ post_pad,
+                                             int32_t* __restrict__ zeros) {
+  for (int b = threadIdx.x; b <= B; b += NT) cumsum[b] = prefix[b];
+  if (threadIdx.x == 0) *post_pad = prefix[B];
+  if (zeros != nullptr && threadIdx.x < 2) zeros[threadIdx.x] = 0;
+}
+
 // Writes sorted_token_ids for the chunk.  base[b] = padded start of bucket b + entries in earlier chunks.
 template <int NBITS = 0>  // > 0: the number of key bits is known at compile time (unrolled ballots)
 __device__ __forceinline__ void scatter_chunk(const int32_t* __restrict__ ids, int64_t chunk_begin, int64_t chunk_end,
@@ -198,7 +208,7 @@ __device__ __forceinline__ void fill_meta(int B, int block_size, int64_t numel, 
 __device__ __forceinline__ void align_single(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                                              int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
                                              int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
-                                             int* smem) {
+                                             int32_t* __restrict__ zeros, int* smem) {
   int* wc = smem;                       // [32][B]
   int* tot = wc + kAlignWarps * B;      // [B]
   int* prefix = tot + B;                // [B+1]
@@ -213,17 +223,17 @@ __device__ __forceinline__ void align_single(const int32_t* __restrict__ ids, in
   scan_over_warps(B, wc, tot);
   __syncthreads();
   padded_prefix(B, block_size, tot, prefix, scratch);
-  for (int b = threadIdx.x; b <= B; b += kAlignThreads) cumsum[b] = prefix[b];
-  if (threadIdx.x == 0) *post_pad = prefix[B];
+  write_starts(B, prefix, cumsum, post_pad, zeros);
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, 0, 1);
   scatter_chunk(ids, 0, numel, span, B, wc, prefix, sorted);
 }
 __global__ void __launch_bounds__(kAlignThreads)
     moe_align_single_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                             int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
-                            int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted) {
+                            int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
+                            int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
-  align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, pad_sorted, smem);
+  align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, pad_sorted, zeros, smem);
 }
 
 // The sort of one CTA beside the quantizer of the same layer's activations (groups of 128, 16-bit input, dense row-major
@@ -239,8 +249,7 @@ __global__ void __launch_bounds__(kAlignThreads)
                            float* __restrict__ out_s, int64_t groups, float eps, float qmax, int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   if (blockIdx.x == 0) {
-    align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, true, smem);
-    if (threadIdx.x < 2) zeros[threadIdx.x] = 0;
+    align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, true, zeros, smem);
     return;
   }
   ptx::grid_dependency_wait();
@@ -314,11 +323,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   __syncthreads();
   padded_prefix(B, block_size, tot, prefix, scratch);
   for (int b = threadIdx.x; b < B; b += kAlignThreads) base[b] = prefix[b] + chunk_hist[(int64_t)blockIdx.x * B + b];
-  if (blockIdx.x == 0) {
-    for (int b = threadIdx.x; b <= B; b += kAlignThreads) cumsum[b] = prefix[b];
-    if (threadIdx.x == 0) *post_pad = prefix[B];
-    if (zeros != nullptr && threadIdx.x < 2) zeros[threadIdx.x] = 0;
-  }
+  if (blockIdx.x == 0) write_starts(B, prefix, cumsum, post_pad, zeros);
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, blockIdx.x, gridDim.x);
   __syncthreads();  // fill_meta is done with tot[] before it is reused below
   const int64_t chunk_len = (int64_t)span * kAlignWarps;
@@ -388,11 +393,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   __syncthreads();
   padded_prefix(B, block_size, tot, prefix, scratch);
   for (int b = threadIdx.x; b < B; b += kAlignThreads) base[b] += prefix[b];
-  if (blockIdx.x == 0) {
-    for (int b = threadIdx.x; b <= B; b += kAlignThreads) cumsum[b] = prefix[b];
-    if (threadIdx.x == 0) *post_pad = prefix[B];
-    if (zeros != nullptr && threadIdx.x < 2) zeros[threadIdx.x] = 0;
-  }
+  if (blockIdx.x == 0) write_starts(B, prefix, cumsum, post_pad, zeros);
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, blockIdx.x, gridDim.x);
   __syncthreads();
   scatter_chunk<NBITS>(ids, begin, end, span, B, wc, base, sorted);
@@ -451,7 +452,8 @@ __global__ void __launch_bounds__(kTsThreads, 2)
     moe_align_tile_scatter_kernel(const int32_t* __restrict__ ids, int64_t numel, int64_t chunk_len, int B,
                                   int block_size, const int* __restrict__ chunk_hist, const int* __restrict__ totals,
                                   int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
-                                  int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted) {
+                                  int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
+                                  int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   int* wc = smem;                        // [16][B]  per-warp counts of the tile, then exclusive over warps
   int* tot_all = wc + kTsWarps * B;      // [B]      totals over all chunks
@@ -467,10 +469,7 @@ __global__ void __launch_bounds__(kTsThreads, 2)
   __syncthreads();
   padded_prefix<kTsThreads>(B, block_size, tot_all, prefix, scratch);
   for (int b = tid; b < B; b += kTsThreads) base[b] = prefix[b] + chunk_hist[(int64_t)blockIdx.x * B + b];
-  if (blockIdx.x == 0) {
-    for (int b = tid; b <= B; b += kTsThreads) cumsum[b] = prefix[b];
-    if (tid == 0) *post_pad = prefix[B];
-  }
+  if (blockIdx.x == 0) write_starts<kTsThreads>(B, prefix, cumsum, post_pad, zeros);
   fill_meta<kTsThreads>(B, block_size, numel, prefix, tot_all, expert_ids, sorted, pad_sorted, blockIdx.x, gridDim.x);
 
   const int64_t begin = (int64_t)blockIdx.x * chunk_len;
@@ -655,7 +654,7 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
                                      200 * 1024));                                                                  \
     moe_align_tile_scatter_kernel<NB><<<(unsigned)lchunks, kTsThreads, ts_smem, st>>>(                              \
         topk_ids, numel, chunk_len, B, block_size, hist, tot, sorted_token_ids, expert_ids, num_tokens_post_pad,    \
-        cumsum_buffer, pad_sorted_token_ids != 0);                                                                  \
+        cumsum_buffer, pad_sorted_token_ids != 0, zeros);                                                           \
     break
     switch (nbits) {
       SGLB_TILE_SCATTER(6);
@@ -676,7 +675,7 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
   align_plan(numel, &chunks, &span);
   if (chunks == 1) {
     SGLB_CUDA(launch_pdl(moe_align_single_kernel, 1, kAlignThreads, smem, st, topk_ids, numel, span, B, block_size,
-                         sorted_token_ids, expert_ids, num_tokens_post_pad, cumsum_buffer, pad_sorted_token_ids != 0));
+                         sorted_token_ids, expert_ids, num_tokens_post_pad, cumsum_buffer, pad_sorted_token_ids != 0, zeros));
     return SGLB200_OK;
   }
   const int64_t need = sglb200_moe_align_workspace_bytes(numel, num_experts);

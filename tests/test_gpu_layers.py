@@ -114,6 +114,44 @@ def test_experts_many_tiles(T, E, topk):
     assert ops.gemm_status() == 0 and ops.stream_status() == 0
 
 
+# (tokens, experts, topk, cooperative launches): the sort in one CTA beside the quantizer and alone (more experts than fit beside
+# it), in one cooperative launch and in three; both products have more tiles than CTAs, whose counters start from whatever the
+# workspace held
+@pytest.mark.parametrize("T,E,topk,coop", [(80, 64, 2, True), (60, 400, 4, True), (700, 96, 3, True), (700, 96, 3, False)])
+def test_experts_tile_counters_start_from_zero(T, E, topk, coop):
+    from sglang_b200 import ops
+    from sglang_b200._lib import check, lib
+    H, I = 1024, 384
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    w13, w2 = ((torch.randn(*s, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+               for s in ((E, 2 * I, H), (E, H, I)))
+    s13, s2 = (torch.rand(*s, device="cuda", generator=g) * 1e-3 for s in ((E, 2 * I // 128, H // 128), (E, H // 128, I // 128)))
+    w, ids = torch.topk(torch.softmax(torch.randn(T, E, device="cuda", generator=g), -1), topk)
+    ids = ids.to(torch.int32)
+    tiles = int(sum((c + 63) // 64 for c in torch.bincount(ids.flatten().long(), minlength=E).tolist()))
+    slots = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert tiles * (H // 128) > slots and tiles * (2 * I // 128) > slots
+    outs = []
+    for fill in (0, 0x7F):
+        ws = torch.full((lib.sglb200_fused_experts_workspace_bytes(T, topk, E, H, I, H, 1.0),), fill, device="cuda", dtype=torch.uint8)
+        out = torch.zeros(T, H, device="cuda", dtype=torch.bfloat16)
+        lib.sglb200_moe_align_set_cooperative(int(coop))
+        try:
+            check(lib.sglb200_fused_experts(x.data_ptr(), 0, w13.data_ptr(), s13.data_ptr(), w2.data_ptr(), s2.data_ptr(), w.data_ptr(),
+                                            ids.data_ptr(), out.data_ptr(), T, topk, E, H, I, H, 1.0, ws.data_ptr(), ws.numel(),
+                                            torch.cuda.current_stream().cuda_stream))
+        finally:
+            lib.sglb200_moe_align_set_cooperative(1)
+        outs.append(out)
+    n = 4  # rows against the oracle
+    ref = O.fused_experts_block_fp8(to_f32_np(x[:n].cpu()), fp8_codes(w13), s13.cpu().numpy(), fp8_codes(w2), s2.cpu().numpy(),
+                                    w[:n].cpu().numpy(), ids[:n].cpu().numpy(), 1.0)
+    assert ops.gemm_status() == 0 and ops.stream_status() == 0
+    assert torch.equal(outs[0], outs[1])
+    assert_close_fp(to_f32_np(outs[1][:n]), ref, rtol=2e-2, atol=2e-2)
+
+
 # sort and quantizer in one launch (up to 2048 ids) and in two: a single group of CTAs part filled, the last size of the one, the
 # first of the other
 @pytest.mark.parametrize("T,E,topk", [(1, 4, 2), (43, 8, 3), (1024, 8, 2), (1025, 8, 2)])

@@ -44,3 +44,20 @@ def test_one_launch_linear_reads_nothing_before_its_wait():
     assert wait < rest.index("tma_load_3d")
     second = rest.index("grid_dependency_wait", wait + 1)
     assert rest.index("tma_load_3d") < second < min(rest.index("__ldg"), rest.index("ld_nc_16"))
+
+
+def test_every_sort_zeroes_the_tile_counters():
+    """The rows kernel takes its tiles from counters that the sort of the same call sets to zero; one that is left alone skips
+    tiles silently.  So there is one function that ends a sort, and the layer hands its counters on whatever the sizes are."""
+    sort = _code("moe_align.cu")
+    ends = re.findall(r"void write_starts\(.*?\n}\n", sort, flags=re.S)
+    assert len(ends) == 1 and "zeros[threadIdx.x] = 0" in ends[0]
+    assert len(re.findall(r"\bcumsum\[\w+\] =", sort)) == len(re.findall(r"\*post_pad =", sort)) == 1
+    kernels = re.findall(r"__global__ void[^;{]*?(moe_align_\w+)\((.*?)\n}\n", sort, flags=re.S)
+    for name, body in kernels:
+        if "post_pad" in body:
+            assert re.search(r"write_starts(<\w+>)?\([^;]*zeros\)|align_single\([^;]*zeros, smem\)", body), name
+    assert sum("post_pad" in body for _, body in kernels) == 5
+    layer = _code("layers.cu")
+    layer = layer[layer.index("int sglb200_fused_experts("):]
+    assert re.search(r"int32_t\* next = i\(p\.next\);", layer) and not re.search(r"\bnext = (?!i\(p\.next\);)|\bnext \?", layer)
