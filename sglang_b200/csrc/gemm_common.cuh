@@ -60,7 +60,8 @@ int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, 
 // gemm_rows.cu: the dense product for few activation rows, and the expert-grouped one on rows sorted with a padding of
 // 16 (`cumsum` = padded starts of the buckets, as the sort writes them; bucket 0 = filtered ids is skipped).
 // `gather_topk` > 0: A and a_s have a row per token, fetched by sorted slot / gather_topk; 0: a row per sorted row.
-// `nt` = activation rows per tile: 32 or 64.  `next_tile`: a zero, see RowsParams.
+// `nt` = activation rows per tile: 32 or 64.  `next_tile`: a zero (or nullptr), see RowsParams.
+// `rows_grouped_single`: such a product has no more tiles than CTAs.
 int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
                   int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, bool after_quantizer,
                   cudaStream_t st);
@@ -68,6 +69,7 @@ int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const floa
                     const int32_t* cumsum, const int32_t* sorted_ids, const float* row_weights, int64_t max_rows,
                     int64_t numel, int num_experts, int64_t N, int64_t K, int gather_topk, int scatter, int out_dtype, int nt,
                     int32_t* next_tile, bool pdl, cudaStream_t st);
+bool rows_grouped_single(int64_t max_rows, int num_experts, int64_t N, int nt);
 
 // gemm_small.cu: quantise + multiply in one launch; whether a problem is one for it.
 bool small_linear_fits(int64_t M, int64_t N, int64_t K);

@@ -23,6 +23,7 @@
 // Every mbarrier wait is bounded as in gemm.cu (status word, no trap).
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -64,7 +65,8 @@ struct RowsCtl {
 
 __device__ int g_rows_status = 0;  // 0 ok, 1 = a pipeline wait expired
 
-template <class Cfg, bool kGrouped>
+// kCounter (grouped): there may be more tiles than CTAs, see take_tile.
+template <class Cfg, bool kGrouped, bool kCounter>
 __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
     fp8_rows_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                          const RowsParams p) {
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
       ptx::mbar_init(ptx::smem_u32(&ctl->sc_full[d]), 32);
       ptx::mbar_init(ptx::smem_u32(&ctl->sc_empty[d]), Cfg::kPromoWarps);
     }
-    for (int d = 0; d < kTileSlots; ++d) {
+    for (int d = 0; kCounter && d < kTileSlots; ++d) {
       ptx::mbar_init(ptx::smem_u32(&ctl->tile_full[d]), 1);
       ptx::mbar_init(ptx::smem_u32(&ctl->tile_empty[d]), Cfg::kPromoWarps + 2);
     }
@@ -122,18 +124,21 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
   const int num_tiles = (kGrouped ? tiles_before[p.num_experts] : p.tiles_m) * p.tiles_n;
   const int kb_begin = rank * p.kb_total / splits, kb_stop = (rank + 1) * p.kb_total / splits;
 
-  // The tiles of this CTA, one call after the other: in the dense form every role counts for itself, in the grouped one the
-  // producer takes them (from a counter that the CTAs share) and hands them to the other roles through a ring.  `t` and `x` are the caller's; false = none left, or a wait expired.
+  // The tiles of this CTA, one call after the other.  With kCounter the producer takes them, from a counter that the CTAs
+  // share, and hands them to the other roles through a ring; otherwise they are dealt out in turn and every role counts for
+  // itself.  `t` and `x` are the caller's; false = none left, or a wait expired.
   // The counter is for experts with more tiles than CTAs: those that HBM serves faster then take more of them, and a last
   // round that is part full spreads over all SMs.  Dealt out in turn, the CTAs of 256 experts of 7168 x 2048 with 64 tokens
   // ended between 849 and 940 us of the first product; the layer took 1 419 us and takes 1 369; 128 experts of 2048 x 768
-  // from a graph, 32 tokens 117.5 and 108.7, 16 tokens 86.3 and 84.2.  What the ring costs shows where a CTA has a tile or
-  // none (8 experts of 4096 x 1408, one token 30.6 and 31.5).  Weights of the first tile asked for before its row ids, so that
-  // these wait behind them, cost another 1 to 2 us; the experts' first rows in shared memory 0.6.
+  // from a graph, 32 tokens 117.5 and 108.7, 16 tokens 86.3 and 84.2.  Where a CTA has a tile or none the ring only costs (one
+  // token, 8 experts of 4096 x 1408 30.0 us, in turn 29.1; 16 experts of 2048 x 768 23.0 and 22.6), so the host leaves it out
+  // where the number of rows bounds the tiles.  Both ways in one kernel, chosen by the tiles there are, 31.1 and 23.7: its
+  // code is fetched anew in every launch.  Weights of the first tile asked for before its row ids, so that these wait behind
+  // them, cost another 1 to 2 us.
   const uint32_t bar_tile_full0 = ptx::smem_u32(&ctl->tile_full[0]), bar_tile_empty0 = ptx::smem_u32(&ctl->tile_empty[0]);
   uint32_t ts = 0, tph = 0;
   auto take_tile = [&](int& t, RowsTile& x, bool first, bool one_thread) -> bool {
-    if constexpr (kGrouped) {
+    if constexpr (kCounter) {
       if (!ROWS_WAIT(bar_tile_full0 + ts * 8, tph)) {
         *abort_flag = 1;
         return false;
@@ -185,9 +190,9 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
       return true;
     };
     int t_next = 0;
-    for (int t = tile_first; t < num_tiles && alive; t = kGrouped ? __shfl_sync(0xffffffffu, t_next, 0) : t + tile_step) {
+    for (int t = tile_first; t < num_tiles && alive; t = kCounter ? __shfl_sync(0xffffffffu, t_next, 0) : t + tile_step) {
       const RowsTile x = rows_tile<NT, kGrouped>(p, tiles_before, t);
-      if (kGrouped && !publish(x)) break;
+      if (kCounter && !publish(x)) break;
       const bool gather = kGrouped && p.gather_topk > 0;
       int r[4] = {0, 0, 0, 0};
       if (gather && lane * 4 < x.n_eff) {
@@ -202,7 +207,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
         const uint32_t bar = bar_full0 + s * 8, dst = tiles0 + s * kStageBytes;
         const int k0 = kb * kRowsBK;
         // (late enough that the next tile is taken by a CTA that can start it, early enough that the answer is not waited for)
-        if (kGrouped && lane == 0 && kb == max(kb_begin, kb_stop - kStages))
+        if (kCounter && lane == 0 && kb == max(kb_begin, kb_stop - kStages))
           t_next = num_tiles > (int)gridDim.x ? atomicAdd(p.next_tile, 1) + (int)gridDim.x : num_tiles;
         if (ahead > 0) {
           --ahead;
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
         }
       }
     }
-    if (kGrouped && alive) publish(RowsTile{0, 0, 0, 0});
+    if (kCounter && alive) publish(RowsTile{0, 0, 0, 0});
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     if (ptx::elect_one()) {
@@ -529,10 +534,10 @@ static size_t rows_smem_bytes(int num_experts) {
 }
 
 // `pdl`: the launch may overlap the end of the kernel before it in the stream (the kernel waits by itself).
-template <class Cfg, bool kGrouped>
+template <class Cfg, bool kGrouped, bool kCounter>
 static int launch_rows(const CUtensorMap& mw, const CUtensorMap& ma, const RowsParams& p, int64_t max_tiles, bool pdl,
                        cudaStream_t st) {
-  auto kern = fp8_rows_gemm_kernel<Cfg, kGrouped>;
+  auto kern = fp8_rows_gemm_kernel<Cfg, kGrouped, kCounter>;
   const size_t smem = rows_smem_bytes<Cfg, kGrouped>(p.num_experts);
   static thread_local bool attr_set[64] = {false};  // the opt-in is per function and per device
   int dev = 0;
@@ -612,7 +617,7 @@ static int rows_dense_cfg(const void* A, const void* B, RowsParams& p, int64_t K
   const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
   static_assert(Cfg::kCtasPerSm == 2, "rows_splits counts on two");
   p.splits = rows_splits(tiles, p.kb_total, p.M, cluster_fits());
-  return launch_rows<Cfg, false>(mw, ma, p, tiles, pdl, st);
+  return launch_rows<Cfg, false, false>(mw, ma, p, tiles, pdl, st);
 }
 
 int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b_s, void* C, const void* bias, int64_t M,
@@ -630,6 +635,14 @@ int rows_dense_mm(const void* A, const void* B, const float* a_s, const float* b
   return rows_dense_cfg<Rows64>(A, B, p, K, after_quantizer, st);
 }
 
+// Most token tiles there can be: every expert has at most one partial tile.
+static int64_t rows_grouped_tiles(int64_t max_rows, int num_experts, int nt) {
+  return std::min(max_rows / nt + num_experts, max_rows / 16);
+}
+bool rows_grouped_single(int64_t max_rows, int num_experts, int64_t N, int nt) {
+  return rows_grouped_tiles(max_rows, num_experts, nt) * ((N + 127) / 128) <= 2 * (int64_t)sm_count();
+}
+
 template <class Cfg>
 static int rows_grouped_cfg(const void* A, int64_t a_rows, const void* B, RowsParams& p, int64_t max_rows, int64_t K, bool pdl,
                             cudaStream_t st) {
@@ -640,10 +653,9 @@ static int rows_grouped_cfg(const void* A, int64_t a_rows, const void* B, RowsPa
   if (rc) return rc;
   p.group_m = choose_group_m(max_rows, K, Cfg::NT);
   p.splits = 1;
-  // every expert has at most one partial tile
-  int64_t tiles = max_rows / Cfg::NT + p.num_experts;
-  if (tiles > max_rows / 16) tiles = max_rows / 16;
-  return launch_rows<Cfg, true>(mw, ma, p, tiles * p.tiles_n, pdl, st);
+  const int64_t tiles = rows_grouped_tiles(max_rows, p.num_experts, Cfg::NT) * p.tiles_n;
+  return p.next_tile != nullptr ? launch_rows<Cfg, true, true>(mw, ma, p, tiles, pdl, st)
+                                : launch_rows<Cfg, true, false>(mw, ma, p, tiles, pdl, st);
 }
 
 int rows_grouped_mm(const void* A, int64_t a_rows, int64_t as_stride, const float* a_s, const void* B, const float* b_s, void* C,

@@ -50,7 +50,7 @@ struct RowsParams {
   int gather_topk;                 // > 0: A has a row per token, fetched by slot / gather_topk; 0: A is in expert order
   int scatter;                     // write row sorted_ids[r] instead of row r
   const float* row_weights;        // scatter, optional
-  int32_t* next_tile;              // a zero: tiles beyond the first of every CTA are taken from this counter
+  int32_t* next_tile;              // a zero: tiles beyond the first of every CTA are taken from this counter; nullptr: in turn
   uint32_t wait_probes;
 };
 

@@ -107,13 +107,14 @@ def test_linear_wait_runs_out_and_recovers(M, N, K):
     assert ops.gemm_status() == 0 and torch.equal(again, good)
 
 
-# on average 1, 8 and 40 rows an expert: the rows kernel with tiles of 16, 32 and 64 rows; 150: the 128-row kernel
-@pytest.mark.parametrize("tokens", [4, 32, 160, 600])
-def test_experts_wait_runs_out_and_recovers(tokens):
+# on average 1, 8 and 40 rows an expert: the rows kernel with tiles of 32 and 64 rows, a tile a CTA or none; 5120: more tiles than
+# CTAs, handed on through a ring; 150 rows: the 128-row kernel
+@pytest.mark.parametrize("tokens,H", [(4, 384), (32, 384), (160, 384), (4, 5120), (32, 5120), (600, 384)])
+def test_experts_wait_runs_out_and_recovers(tokens, H):
     from sglang_b200 import ops
     from sglang_b200._lib import check, lib
     from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
-    E, H, I, topk = 8, 384, 256, 2
+    E, I, topk = 8, 256, 2
     g = torch.Generator(device="cuda").manual_seed(tokens)
     x = torch.randn(tokens, H, device="cuda", generator=g).bfloat16()
     w13, w2 = ((torch.randn(*s, device="cuda", generator=g) * 20).clamp(-448, 448).to(torch.float8_e4m3fn)

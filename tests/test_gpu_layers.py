@@ -75,10 +75,9 @@ def test_linear_after_its_weights_were_written(M, N, K):
 # (tokens, experts, topk): on average 1 to some hundred rows per expert, so that every tile height of the dispatch is taken;
 # the ids are skewed towards expert 0 and leave some experts without rows
 @pytest.mark.parametrize("T,E,topk", [(1, 8, 8), (5, 32, 2), (16, 8, 1), (40, 16, 4), (70, 6, 3), (160, 8, 2), (333, 4, 2)])
-def test_experts_row_counts(T, E, topk):
+def test_experts_row_counts(T, E, topk, H=384, I=256):
     from sglang_b200 import ops
     from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
-    H, I = 384, 256
     g = torch.Generator().manual_seed(T + E)
     x = make_act(T, H, T, outliers=False)
     w13q, w13s = make_weight(2 * I, H, 1, std=0.05, experts=E)
@@ -150,6 +149,12 @@ def test_experts_tile_counters_start_from_zero(T, E, topk, coop):
     assert ops.gemm_status() == 0 and ops.stream_status() == 0
     assert torch.equal(outs[0], outs[1])
     assert_close_fp(to_f32_np(outs[1][:n]), ref, rtol=2e-2, atol=2e-2)
+
+
+# the second product has as many tiles as CTAs (no counter), and eight more (its tiles, and the first product's, come from one)
+@pytest.mark.parametrize("H", [4736, 4864])
+def test_experts_as_many_tiles_as_ctas(H):
+    test_experts_row_counts(1, 8, 8, H, 128)
 
 
 # sort and quantizer in one launch (up to 2048 ids) and in two: a single group of CTAs part filled, the last size of the one, the
