@@ -38,6 +38,8 @@ constexpr int kMidMaxChunks = 128;                 // CTAs of the multi-CTA path
 #endif
 constexpr bool kAlignCoop = SGLB_ALIGN_COOP != 0;  // one cooperative launch instead of three for 8192 < ids <= 1 M
 constexpr int kMaxChunks = 296;                    // about two CTAs per SM; longer inputs get longer chunks
+// Dynamic shared memory that a kernel has without asking, and that the sorts ask for at most (1461 buckets).
+constexpr size_t kSmemDefault = 48 * 1024, kAlignSmemMax = 200 * 1024;
 
 __device__ __forceinline__ int warp_incl_scan(int v) {
   const int lane = threadIdx.x & 31;
@@ -238,8 +240,11 @@ __global__ void __launch_bounds__(kAlignThreads)
 
 // The sort of one CTA beside the quantizer of the same layer's activations (groups of 128, 16-bit input, dense row-major
 // scales): CTA 0 sorts, the others quantise, a group to eight lanes of 16 values.  Both are a few microseconds of latency
-// with little work, and neither needs the other.  A layer of 128 experts of 2048 x 768 from a graph, two launches and one: 1
-// token 29.0 -> 28.1 us, 8 tokens 68.2 -> 66.5, 32 tokens 120.6 -> 119.2; 8 experts of 4096 x 1408, 64 tokens 48.9 -> 47.6.
+// with little work, and neither needs the other.  Two launches and one, from a graph of nothing else: 64 tokens of 2048, 128
+// experts 6.3 -> 4.9 us; at the upper end, 1024 tokens of 7168 to two of 64 experts 10.0 -> 5.9, 2048 tokens of 7168 to one of
+// 64 13.0 -> 9.7.  Every CTA has the sort's shared memory, though only the first uses it: with 1000 experts 137 KB, so one CTA
+// an SM, and still 1024 tokens of 7168 18.5 -> 14.1, one token 8.9 -> 7.4.  A layer of 128 experts of 2048 x 768: 1 token 29.0 ->
+// 28.1 us, 32 tokens 120.6 -> 119.2; 512 experts of 2048 x 512: 1 token 26.9 -> 25.5, 64 tokens 186.6 -> 181.0.
 constexpr int kAlignQuantGroups = kAlignThreads / 8;  // groups of one CTA
 template <typename T>
 __global__ void __launch_bounds__(kAlignThreads)
@@ -569,27 +574,34 @@ static void align_plan(int64_t numel, int64_t* chunks, int* span) {
 static size_t align_smem_bytes(int B) { return sizeof(int) * ((size_t)kAlignWarps * B + 3 * (size_t)B + 1 + 33 + 8); }
 
 bool align_quant_fits(const void* x, int64_t numel, int buckets) {
-  return numel <= kSingleMax && align_smem_bytes(buckets) <= 48 * 1024 && aligned16(x);
+  return numel <= kSingleMax && align_smem_bytes(buckets) <= kAlignSmemMax && aligned16(x);
+}
+
+template <typename T>
+static int launch_align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
+                              int32_t* post_pad, int32_t* cumsum, const void* x, void* out_q, float* out_s, int64_t groups,
+                              float eps, float fp8_max, int32_t* zeros, cudaStream_t st) {
+  int64_t chunks = 0;
+  int span = 0;
+  align_plan(numel, &chunks, &span);
+  const unsigned grid = 1 + (unsigned)((groups + kAlignQuantGroups - 1) / kAlignQuantGroups);
+  const size_t smem = align_smem_bytes(buckets);
+  if (smem > kSmemDefault)
+    SGLB_CUDA(cudaFuncSetAttribute(moe_align_quant_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmemMax));
+  SGLB_CUDA(launch_pdl(moe_align_quant_kernel<T>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size, sorted,
+                       expert_ids, post_pad, cumsum, static_cast<const T*>(x), static_cast<uint8_t*>(out_q), out_s, groups, eps,
+                       fp8_max, zeros));
+  return SGLB200_OK;
 }
 
 int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                 int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
                 int64_t hidden, float eps, float fp8_max, int32_t* zeros, cudaStream_t st) {
-  int64_t chunks = 0;
-  int span = 0;
-  align_plan(numel, &chunks, &span);
   const int64_t groups = tokens * (hidden / 128);
-  const unsigned grid = 1 + (unsigned)((groups + kAlignQuantGroups - 1) / kAlignQuantGroups);
-  const size_t smem = align_smem_bytes(buckets);
-  uint8_t* q = static_cast<uint8_t*>(out_q);
-  if (dtype == 0)
-    SGLB_CUDA(launch_pdl(moe_align_quant_kernel<__nv_bfloat16>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size,
-                         sorted, expert_ids, post_pad, cumsum, static_cast<const __nv_bfloat16*>(x), q, out_s, groups, eps, fp8_max,
-                         zeros));
-  else
-    SGLB_CUDA(launch_pdl(moe_align_quant_kernel<__half>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size, sorted,
-                         expert_ids, post_pad, cumsum, static_cast<const __half*>(x), q, out_s, groups, eps, fp8_max, zeros));
-  return SGLB200_OK;
+  return dtype == 0 ? launch_align_quant<__nv_bfloat16>(ids, numel, buckets, block_size, sorted, expert_ids, post_pad, cumsum, x,
+                                                        out_q, out_s, groups, eps, fp8_max, zeros, st)
+                    : launch_align_quant<__half>(ids, numel, buckets, block_size, sorted, expert_ids, post_pad, cumsum, x, out_q,
+                                                 out_s, groups, eps, fp8_max, zeros, st);
 }
 
 }  // namespace sglb200
@@ -622,17 +634,17 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
                "moe_align: null pointer");
   const int B = num_experts;
   const size_t smem = align_smem_bytes(B);
-  SGLB_REQUIRE(smem <= 200 * 1024, "moe_align: %d buckets need %zu bytes of shared memory (limit 200 KiB)", B, smem);
-  if (smem > 48 * 1024) {
+  SGLB_REQUIRE(smem <= kAlignSmemMax, "moe_align: %d buckets need %zu bytes of shared memory (limit 200 KiB)", B, smem);
+  if (smem > kSmemDefault) {
     // opt in to more than 48 KiB of dynamic shared memory (a per-function, per-device attribute; cheap to repeat)
-    SGLB_CUDA(cudaFuncSetAttribute(moe_align_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    SGLB_CUDA(cudaFuncSetAttribute(moe_align_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    SGLB_CUDA(cudaFuncSetAttribute(moe_align_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    SGLB_CUDA(cudaFuncSetAttribute(moe_align_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmemMax));
+    SGLB_CUDA(cudaFuncSetAttribute(moe_align_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmemMax));
+    SGLB_CUDA(cudaFuncSetAttribute(moe_align_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmemMax));
   }
   if (numel > kLargeMin) {
     SGLB_REQUIRE(B <= 8160, "moe_align: %d buckets exceed the bucket field of the large-input path", B);
     const size_t ts_smem = tile_scatter_smem_bytes(B);
-    SGLB_REQUIRE(ts_smem <= 200 * 1024, "moe_align: %d buckets need %zu bytes of shared memory (limit 200 KiB)", B,
+    SGLB_REQUIRE(ts_smem <= kAlignSmemMax, "moe_align: %d buckets need %zu bytes of shared memory (limit 200 KiB)", B,
                  ts_smem);
     const int nbits = 32 - __builtin_clz((unsigned)(B + 31));  // keys run up to B + 31
     int64_t lchunks = 0, chunk_len = 0;
@@ -649,9 +661,9 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
                                                                                                      (int)lchunks, B);
 #define SGLB_TILE_SCATTER(NB)                                                                                       \
   case NB:                                                                                                          \
-    if (ts_smem > 48 * 1024)                                                                                        \
+    if (ts_smem > kSmemDefault)                                                                                     \
       SGLB_CUDA(cudaFuncSetAttribute(moe_align_tile_scatter_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                     200 * 1024));                                                                  \
+                                     (int)kAlignSmemMax));                                                          \
     moe_align_tile_scatter_kernel<NB><<<(unsigned)lchunks, kTsThreads, ts_smem, st>>>(                              \
         topk_ids, numel, chunk_len, B, block_size, hist, tot, sorted_token_ids, expert_ids, num_tokens_post_pad,    \
         cumsum_buffer, pad_sorted_token_ids != 0, zeros);                                                           \
@@ -686,8 +698,8 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
   int* totals = chunk_hist + chunks * B;
   if (kAlignCoop && g_align_coop_enabled) {
     const CoopKernel kern = coop_kernel_for(B);
-    if (smem > 48 * 1024)
-      SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    if (smem > kSmemDefault)
+      SGLB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmemMax));
     if (coop_fits(kern, chunks, smem)) {
       bool pad = pad_sorted_token_ids != 0;
       void* args[] = {&topk_ids, &numel, &span, (void*)&B, &block_size, &chunk_hist, &sorted_token_ids, &expert_ids,

@@ -113,9 +113,8 @@ def test_experts_many_tiles(T, E, topk):
     assert ops.gemm_status() == 0 and ops.stream_status() == 0
 
 
-# (tokens, experts, topk, cooperative launches): the sort in one CTA beside the quantizer and alone (more experts than fit beside
-# it), in one cooperative launch and in three; both products have more tiles than CTAs, whose counters start from whatever the
-# workspace held
+# (tokens, experts, topk, cooperative launches): the sort in one CTA beside the quantizer, with few and with many experts, in one
+# cooperative launch and in three; both products have more tiles than CTAs, whose counters start from whatever the workspace held
 @pytest.mark.parametrize("T,E,topk,coop", [(80, 64, 2, True), (60, 400, 4, True), (700, 96, 3, True), (700, 96, 3, False)])
 def test_experts_tile_counters_start_from_zero(T, E, topk, coop):
     from sglang_b200 import ops
@@ -158,8 +157,8 @@ def test_experts_as_many_tiles_as_ctas(H):
 
 
 # sort and quantizer in one launch (up to 2048 ids) and in two: a single group of CTAs part filled, the last size of the one, the
-# first of the other
-@pytest.mark.parametrize("T,E,topk", [(1, 4, 2), (43, 8, 3), (1024, 8, 2), (1025, 8, 2)])
+# first of the other; the last number of experts whose counts fit the shared memory every kernel has, the first beyond it, and many
+@pytest.mark.parametrize("T,E,topk", [(1, 4, 2), (43, 8, 3), (1024, 8, 2), (1025, 8, 2), (9, 348, 2), (9, 349, 2), (3, 1000, 8)])
 def test_experts_sort_beside_quantizer(T, E, topk):
     from sglang_b200 import ops
     from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
