@@ -81,9 +81,11 @@ def test_stream_kernels_wait_runs_out_and_recover():
     assert torch.equal(hq.view(torch.uint8), good_hq.view(torch.uint8)) and torch.equal(hs, good_hs)
 
 
-# 1 x 1024 and 16 x 4352: quantise and multiply in one launch; 20 and 64 rows: the rows kernel behind the quantizer, with
-# its weights requested early, K split over a cluster or whole; 300: the 128-row kernel
-@pytest.mark.parametrize("M,N,K", [(1, 512, 1024), (16, 4368, 4352), (20, 1024, 8192), (64, 14848, 384), (300, 512, 1024)])
+# one and 16 rows: quantise and multiply in one launch; 20 and 64: the rows kernel behind the quantizer, with its weights
+# requested early, K split over a cluster whose CTAs fetch the partial sums (20) or push them (64 x 1024 x 8192: two barriers of
+# the cluster, at which every warp arrives whether its waits expired or not) or whole; 300: the 128-row kernel
+@pytest.mark.parametrize("M,N,K", [(1, 512, 1024), (16, 4368, 4352), (20, 1024, 8192), (64, 1024, 8192), (64, 14848, 384),
+                                   (300, 512, 1024)])
 def test_linear_wait_runs_out_and_recovers(M, N, K):
     from sglang_b200 import ops
     from sglang_b200._lib import check, lib

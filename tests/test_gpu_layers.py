@@ -31,9 +31,11 @@ def test_linear_row_counts(M, N, K, dtype, bias):
     assert_close_fp(to_f32_np(out), ref)
 
 
-# weights whose tiles are split over clusters of two to sixteen CTAs, with K ranges of unequal length, and not split at all
+# weights whose tiles are split over clusters of two to sixteen CTAs, with K ranges of unequal length, and not split at all; the
+# last has more tiles than two CTAs an SM, which are dealt out in turn
 @pytest.mark.parametrize("M", [1, 16, 20, 64])
-@pytest.mark.parametrize("N,K", [(1024, 8192), (512, 512), (4616, 1920), (3080, 1664), (2200, 2432), (4432, 1152), (8200, 640), (1032, 1152), (14848, 384)])
+@pytest.mark.parametrize("N,K", [(1024, 8192), (512, 512), (4616, 1920), (3080, 1664), (2200, 2432), (4432, 1152), (8200, 640),
+                                 (1032, 1152), (14848, 384), (38408, 256)])
 def test_linear_cluster_splits(M, N, K):
     test_linear_row_counts(M, N, K, torch.bfloat16, False)
 
@@ -93,7 +95,7 @@ def test_experts_row_counts(T, E, topk, H=384, I=256):
     assert_close_fp(to_f32_np(out), ref, rtol=2e-2, atol=2e-2)
 
 
-# more tiles than CTAs, taken from a counter (up to 2048 ids) and in turn; experts without rows among them
+# more tiles of the first product than CTAs, behind the sort of up to 2048 ids and of more; experts without rows among them
 @pytest.mark.parametrize("T,E,topk", [(40, 64, 2), (700, 96, 3)])
 def test_experts_many_tiles(T, E, topk):
     from sglang_b200 import ops
