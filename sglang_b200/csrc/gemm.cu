@@ -1112,9 +1112,10 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // A single wave is launched programmatically: 257 x 10240 x 8192 with its quantizer 49.0 -> 48.0 us.  With several waves
-  // the CTAs, which then start wherever an SM falls free, no longer share L2 as their numbers suggest: 4096 x 32768 x 512
-  // 114.4 -> 120.9.  Push mode, which other streams take part in: an ordinary launch.
+  // A single wave is launched programmatically.  With their quantizer, both ways in turn on one box: 100 x 4096 x 4096 15.1 ->
+  // 14.4 us, 512 x 4096 x 4096 16.9 -> 16.1, 200 x 8192 x 1024 9.7 -> 9.0; 257 x 10240 x 8192 40.4 -> 39.6, which is less than
+  // boxes and runs differ by.  With several waves the CTAs, which then start wherever an SM falls free, no longer share L2 as
+  // their numbers suggest: 4096 x 32768 x 512 114.4 -> 120.9.  Push mode, which other streams take part in: an ordinary launch.
   cfg.numAttrs = max_units <= sms && p.push_maps == nullptr ? 1 : 0;
   SGLB_CUDA(cudaLaunchKernelEx(&cfg, fp8_blockscale_gemm_kernel<kGrouped, BN>, ma, mb, mc, p));
   return SGLB200_OK;

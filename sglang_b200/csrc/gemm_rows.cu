@@ -60,7 +60,7 @@ struct RowsCtl {
   int abort_flag;
   int warp_sum[32];
   alignas(16) float sc[2][kScBatch][Cfg::NT];  // a_s * b_s per slab and column (columns in the order of frag_column)
-  // (grouped: followed by tiles_before[experts + 1], the token tiles of the experts before e, and row_begin[experts + 1])
+  // (grouped: followed by tiles_before[experts + 1], the token tiles of the experts before e)
 };
 
 __device__ int g_rows_status = 0;  // 0 ok, 1 = a pipeline wait expired
@@ -72,13 +72,14 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kCtasPerSm)
                          const RowsParams p) {
   constexpr int NT = Cfg::NT, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs, kCW = Cfg::kCW, kChunks = Cfg::kChunks;
   constexpr bool kPush = !kGrouped && NT == 64;  // how a cluster exchanges its partial sums
-  static_assert(NT * kPartPitch <= kStages * Cfg::kStageBytes / 4 && (NT / 2 + kMaxSplits - 1) * kPartPair <= kStages * Cfg::kStageBytes / 4,
+  static_assert(NT * kPartPitch <= kStages * Cfg::kStageBytes / 4 &&
+                    (NT / 2 + kMaxSplits - 1) * kPartPair <= kStages * Cfg::kStageBytes / 4,
                 "the partial sums fit the ring");
   constexpr uint32_t kStageBytes = Cfg::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   RowsCtl<Cfg>* ctl = reinterpret_cast<RowsCtl<Cfg>*>(tiles + kStages * kStageBytes);
-  int* tiles_before = reinterpret_cast<int*>(ctl + 1);  // grouped: token tiles before, then first row of, every expert
+  int* tiles_before = reinterpret_cast<int*>(ctl + 1);  // grouped: token tiles before every expert
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int* abort_flag = &ctl->abort_flag;
 

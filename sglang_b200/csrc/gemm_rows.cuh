@@ -1,4 +1,5 @@
-// Shared by the kernels with the weights on the M side (gemm_rows.cu, gemm_small.cu): launch parameters, the walk over tiles, the count of the experts' token tiles.
+// Shared by the kernels with the weights on the M side (gemm_rows.cu, gemm_small.cu): launch parameters, the walk over
+// tiles, the count of the experts' token tiles, the sum over the CTAs of a cluster.
 #pragma once
 #include "cluster_rule.h"
 #include "common.cuh"
@@ -84,8 +85,9 @@ __device__ __forceinline__ RowsTile rows_tile(const RowsParams& p, const int* ti
   return x;
 }
 
-// Token tiles (of NT rows) of every expert and their exclusive scan into tiles_before[0 .. experts], the experts' first rows
-// behind it (a tile is then located without a round trip to L2): four experts per thread, all NTHREADS threads of the block.  The scan is visible after the next __syncthreads.
+// Token tiles (of NT rows) of every expert and their exclusive scan into tiles_before[0 .. experts]: four experts per thread,
+// all NTHREADS threads of the block.  The scan is visible after the next __syncthreads.  An expert's first row is read from
+// p.cumsum where a tile is located: in shared memory beside the scan, it cost a layer of 128 experts 0.6 us.
 template <int NT, int NTHREADS>
 __device__ __forceinline__ void rows_count_tiles(const RowsParams& p, int* tiles_before, int* warp_sum) {
   static_assert(NTHREADS * 4 >= kMaxExperts, "four experts per thread");
@@ -117,7 +119,8 @@ __device__ __forceinline__ void rows_count_tiles(const RowsParams& p, int* tiles
 }
 
 // The output of a tile whose K range was split over the CTAs of a cluster (at most kMost): sums their partial sums
-// ([column][kPartPitch weight rows] of float32 at `part` in every CTA's shared memory) in ascending K order, adds the bias, rounds once.
+// ([column][kPartPitch weight rows] of float32 at `part` in every CTA's shared memory) in ascending K order, adds the bias,
+// rounds once.
 template <int kMost>
 __device__ __forceinline__ void rows_cluster_sum(const RowsParams& p, const RowsTile& x, int rank, uint32_t part, int tid,
                                                  int threads) {

@@ -36,7 +36,7 @@ constexpr int kMidMaxChunks = 128;                 // CTAs of the multi-CTA path
 #ifndef SGLB_ALIGN_COOP
 #define SGLB_ALIGN_COOP 1
 #endif
-constexpr bool kAlignCoop = SGLB_ALIGN_COOP != 0;  // one cooperative launch instead of three for 8192 < ids <= 1 M
+constexpr bool kAlignCoop = SGLB_ALIGN_COOP != 0;  // one cooperative launch instead of three for 2048 < ids <= 1 M
 constexpr int kMaxChunks = 296;                    // about two CTAs per SM; longer inputs get longer chunks
 // Dynamic shared memory that a kernel has without asking, and that the sorts ask for at most (1461 buckets).
 constexpr size_t kSmemDefault = 48 * 1024, kAlignSmemMax = 200 * 1024;
@@ -206,7 +206,7 @@ __device__ __forceinline__ void fill_meta(int B, int block_size, int64_t numel, 
   }
 }
 
-// ---- numel <= kChunk: everything in one CTA -------------------------------------------------
+// ---- numel <= kSingleMax: everything in one CTA ---------------------------------------------
 __device__ __forceinline__ void align_single(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                                              int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
                                              int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   }
 }
 
-// ---- numel > kChunk: histogram per chunk -> scan over chunks -> scatter ----------------------
+// ---- numel > kSingleMax: histogram per chunk -> scan over chunks -> scatter ------------------
 __global__ void __launch_bounds__(kAlignThreads)
     moe_align_hist_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B,
                           int* __restrict__ chunk_hist) {
