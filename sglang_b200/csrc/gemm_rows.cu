@@ -641,7 +641,8 @@ static int64_t rows_grouped_tiles(int64_t max_rows, int num_experts, int nt) {
   return std::min(max_rows / nt + num_experts, max_rows / 16);
 }
 bool rows_grouped_single(int64_t max_rows, int num_experts, int64_t N, int nt) {
-  return rows_grouped_tiles(max_rows, num_experts, nt) * ((N + 127) / 128) <= 2 * (int64_t)sm_count();
+  static_assert(Rows32::kCtasPerSm == Rows64::kCtasPerSm, "one number of CTAs for both heights");
+  return rows_grouped_tiles(max_rows, num_experts, nt) * ((N + 127) / 128) <= (int64_t)sm_count() * Rows64::kCtasPerSm;
 }
 
 template <class Cfg>
