@@ -22,7 +22,7 @@
 //     part of a tile in shared memory and arrive on an mbarrier, never waiting for each other or for a store.
 // What bounds it (M = 4096, N = 36864, K = 7168): the shared-memory port.  A 128 x 256 slab stages 48 KB and the MMAs
 // read 48 KB of it, 768 clocks at 128 bytes a clock for 512 clocks of MMA; measured 860 without any promotion and about
-// 900 with it.  On the way there, same box, back to back (power-limited) in microseconds: 1310 with a 192-wide tile; 1165
+// 900 with it.  On the way there, same GPU, back to back (power-limited) in microseconds: 1310 with a 192-wide tile; 1165
 // with 256 columns, setmaxnreg and waits that ask before the FMAs and look after them; 1088 with the scales from the
 // scout's ring, relaxed hand-backs of tensor memory and the two-step question; 1056 to 1077 (the spread over boxes) with
 // the promotion loop unrolled by four, so that buffers, barriers and scales are compile-time (its bookkeeping was a chain
@@ -1112,9 +1112,9 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // A single wave is launched programmatically.  With their quantizer, both ways in turn on one box: 100 x 4096 x 4096 15.1 ->
+  // A single wave is launched programmatically.  With their quantizer, both ways in turn on one GPU: 100 x 4096 x 4096 15.1 ->
   // 14.4 us, 512 x 4096 x 4096 16.9 -> 16.1, 200 x 8192 x 1024 9.7 -> 9.0; 257 x 10240 x 8192 40.4 -> 39.6, which is less than
-  // boxes and runs differ by.  With several waves the CTAs, which then start wherever an SM falls free, no longer share L2 as
+  // GPUs and runs differ by.  With several waves the CTAs, which then start wherever an SM falls free, no longer share L2 as
   // their numbers suggest: 4096 x 32768 x 512 114.4 -> 120.9.  Push mode, which other streams take part in: an ordinary launch.
   cfg.numAttrs = max_units <= sms && p.push_maps == nullptr ? 1 : 0;
   SGLB_CUDA(cudaLaunchKernelEx(&cfg, fp8_blockscale_gemm_kernel<kGrouped, BN>, ma, mb, mc, p));
