@@ -67,6 +67,21 @@ __device__ __forceinline__ void chunk_signs(const uint4& raw, uint32_t* s) {
   }
 }
 
+// q0 = RN(x r), e = fma(-q0, scale, x), q = fma(e, r, q0) of two elements (packed float32: half the issue slots.  Cold inputs, 8192 x 18432
+// bf16: 83.8 us -> 79.7).
+__device__ __forceinline__ void quotient2(float x0, float x1, float scale, float r, float& q0, float& q1) {
+  asm("{\n\t.reg .b64 x, s, r, a, e;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 s, {%4, %4};\n\t"
+      "mov.b64 r, {%5, %5};\n\t"
+      "mul.rn.f32x2 a, x, r;\n\t"
+      "fma.rn.f32x2 e, a, s, x;\n\t"
+      "fma.rn.f32x2 a, e, r, a;\n\t"
+      "mov.b64 {%0, %1}, a;\n\t}"
+      : "=f"(q0), "=f"(q1)
+      : "f"(x0), "f"(x1), "f"(-scale), "f"(r));
+}
+
 // Codes of one chunk when every element of the group is finite and the scale is in the range where the
 // division-free quotient is exact (see quant_chunk_careful).  With the standard range no clamp is needed: a quotient can
 // exceed 448 only by rounding and the conversion saturates; the sign of a zero quotient is taken from the
@@ -77,11 +92,12 @@ __device__ __forceinline__ void quant_chunk_fast(const uint4& raw, const float* 
   constexpr int CE = Chunk<T>::kElems;
   float q[CE];
 #pragma unroll
-  for (int i = 0; i < CE; ++i) {
-    const float q0 = __fmul_rn(v[i], r);
-    const float e = __fmaf_rn(-q0, scale, v[i]);
-    q[i] = __fmaf_rn(e, r, q0);
-    if (!kStdRange) q[i] = fminf(fmaxf(copysignf(q[i], v[i]), qmin), qmax);
+  for (int i = 0; i < CE; i += 2) {
+    quotient2(v[i], v[i + 1], scale, r, q[i], q[i + 1]);
+    if (!kStdRange) {
+      q[i] = fminf(fmaxf(copysignf(q[i], v[i]), qmin), qmax);
+      q[i + 1] = fminf(fmaxf(copysignf(q[i + 1], v[i + 1]), qmin), qmax);
+    }
   }
 #pragma unroll
   for (int i = 0; i < CE / 4; ++i) codes[i] = pack_e4m3x4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
