@@ -87,8 +87,15 @@ __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
 
 // silu(x) = x / (1 + e^-x) in float32 with the hardware exponential and reciprocal.  The result is rounded to
 // bf16/fp16 by every caller, so the few-ulp float32 error of the approximations shows only at rounding ties
-// (the unfused and fused activation kernels share this function and stay bit-identical to each other).
-__device__ __forceinline__ float silu_f32(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+// (the unfused and fused activation kernels share this function and stay bit-identical to each other).  Flushing
+// subnormals changes nothing that can be seen: e^-x below 2^-126 vanishes beside 1, and 1 / (1 + e^-x) is subnormal only
+// for x < -87.3, where the quotient was 0 before too (a divisor above 2^126).
+__device__ __forceinline__ float silu_f32(float x) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.44269504f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return x * r;
+}
 
 // Four float32 -> four e4m3 codes packed little-endian (a in bits 0-7 ... d in bits 24-31).
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {

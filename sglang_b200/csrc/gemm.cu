@@ -51,6 +51,7 @@
 #include "common.cuh"
 #include "gemm_common.cuh"
 #include "ptx_sm100.cuh"
+#include "quant_math.cuh"
 
 namespace sglb200 {
 
@@ -82,9 +83,18 @@ __device__ long long g_trace[2][kTraceUnits][kTraceStamps];
 #define SGLB_WAIT(bar, parity) \
   (p.wait_probes != ptx::kProbesNone && (ptx::mbar_test(bar, parity) || ptx::mbar_wait_quiet(bar, parity)))
 
+// What a launch computes.  kActivated: the gate and up projections of the experts, of which a tile takes 128 columns each
+// (columns 0-127 of its accumulators and 128-255), so that the epilogue has both factors of 128 activated values and a whole
+// quantisation group of every row, and writes codes and scales instead of 16-bit products that another launch reads back.
+// 131072 rows through 128 experts of 2048 x 768 (Zipf routing, sustained, both ways on one GPU): product 493 us + activation 117
+// -> 550; 32768 rows, 256 experts of 7168 x 2048: 1 970 + 147 -> 1 979.  The epilogue's exponentials and reciprocals are 2 048
+// clocks a tile of the special-function units, which the next tile's first two slabs hide in part.  Four stages of operands,
+// for which there is room: 562 and 2 063.
+enum class Form { kDense, kGrouped, kActivated };
+
 // Tile width BN: 256 columns with two TMEM accumulator buffers, or 128 columns with four (more tiles for the same
 // problem: where one wave of wide tiles would leave SMs idle).
-template <int BN_>
+template <int BN_, Form kForm = Form::kDense>
 struct TileCfg {
   static constexpr int BN = BN_;
   static constexpr int kStages = BN_ >= 256 ? 3 : 5;
@@ -100,7 +110,8 @@ struct TileCfg {
   // output staging for the TMA store: per 64 columns a [128 rows][64 columns] 2-byte tile in the 128-byte swizzle
   static constexpr int kOutGroups = BN_ / 64;
   static constexpr uint32_t kOutGroupBytes = BM * 64 * 2;
-  static constexpr uint32_t kOutBytes = kOutGroups * kOutGroupBytes;
+  static constexpr uint32_t kOutBytes = kForm == Form::kActivated ? BM * 128 : kOutGroups * kOutGroupBytes;
+  static constexpr int kHalfRows = kForm == Form::kActivated ? BM : 1;
   static_assert(kEpiWarps % 4 == 0 && BN_ % kColGroups == 0 && kEpiCols % 32 == 0 && BN_ % 64 == 0 &&
                     kAccBufs * kAccStride <= kTmemCols && BN_ <= 256 && kStageBytes % 1024 == 0,
                 "accumulator layout");
@@ -145,6 +156,7 @@ struct GemmParams {
   int sk_pieces;                 // 2 or 3
   int sk_total;                  // tiles * kb_total
   uint32_t wait_probes;          // probes after which a pipeline wait gives up
+  float* act_s;                  // activated form: C holds codes [row][N / 2], this their scales [row][N / 256]
 };
 
 // What the scout warp prepares for the promotion warps while they work on the previous unit: where the unit lies, so that
@@ -170,6 +182,9 @@ struct SharedCtl {
   uint64_t tmem_empty[Cfg::kAccBufs];
   uint64_t out_full;  // the output staging holds a rounded tile (every promotion thread arrives)
   uint64_t out_free;  // the TMA stores of the previous tile have read the staging (the storing thread arrives)
+  // activated form: the two warps of a row quadrant exchange the maxima of their halves of a group
+  alignas(16) float2 half_max[2][kColGroups][Cfg::kHalfRows];  // units in turn, column group, row: with NaNs, without
+  uint64_t half_full[4];                           // a quadrant's maxima of the unit are written (one lane of each warp)
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -215,11 +230,80 @@ __device__ __forceinline__ Unit decode_unit(const GemmParams& p, int u) {
   return x;
 }
 
-template <bool kGrouped, int BN_>
+// Epilogue of the activated form for one row: acc holds 64 gate and 64 up values, columns cgrp * 64 .. of group `n_tile`.
+// Rounded to T as a stored product would be, silu(gate) rounded to T, times up rounded to T, then the quantizer: the
+// arithmetic of silu_mul_quant_kernel, bit for bit.  The other half of the group is in the same lane of the other warp of
+// the quadrant, so the two warps exchange their maxima; `half` is this row's place of column group 0.  False when the wait
+// for the other warp expired.  The 64 codes come back in `codes`.
+template <typename T>
+__device__ __forceinline__ bool activate_row(const GemmParams& p, const float (&acc)[128], int cgrp, float2* half, uint32_t bar,
+                                             uint32_t parity, uint4 (&codes)[4], float& scale) {
+  constexpr float kEps = 1e-10f;  // as the quantizer of the layer's activations
+  uint4 h[8];
+  uint32_t top = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = 8 * j + 2 * k;
+      float g[2];
+      Packed2<T>::unpack(Packed2<T>::pack(acc[c], acc[c + 1]), g);
+      w[k] = Packed2<T>::round_mul(silu_f32(g[0]), silu_f32(g[1]), Packed2<T>::pack(acc[64 + c], acc[64 + c + 1]));
+      top = Packed2<T>::max_abs_nan(top, w[k]);
+    }
+    h[j] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  float t2[2];
+  Packed2<T>::unpack(top, t2);
+  float most = max3_abs_nan(kEps, t2[0], t2[1]), finite = most;  // (finite: the maximum of what is a number)
+  if (most != most) {
+    finite = kEps;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float v[8];
+      unpack_chunk<T>(h[j], v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) finite = fmaxf(finite, fabsf(v[k]));
+    }
+  }
+  ptx::sts_64(ptx::smem_u32(half + cgrp * BM), __float_as_uint(most), __float_as_uint(finite));
+  __syncwarp();
+  ptx::mbar_arrive_if(bar, (threadIdx.x & 31) == 0);
+  if (!SGLB_WAIT(bar, parity)) return false;
+  const float2 other = ptx::lds_f32x2(ptx::smem_u32(half + (cgrp ^ 1) * BM));
+  most = max_nan(most, other.x), finite = fmaxf(finite, other.y);
+  scale = __fdiv_rn(most, 448.0f);
+  uint32_t out[8][2];
+  if (most < __int_as_float(0x7f800000) && scale >= 1e-30f && scale <= 1e36f) {
+    const float r = __frcp_rn(scale);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float v[8];
+      unpack_chunk<T>(h[j], v);
+      quant_chunk_fast<T, true>(h[j], v, scale, r, -448.0f, 448.0f, out[j]);
+    }
+  } else {
+    scale = __fdiv_rn(finite, 448.0f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float v[8];
+      unpack_chunk<T>(h[j], v);
+      quant_chunk_careful<T>(v, scale, -448.0f, 448.0f, out[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) codes[j] = make_uint4(out[2 * j][0], out[2 * j][1], out[2 * j + 1][0], out[2 * j + 1][1]);
+  return true;
+}
+
+template <Form kForm, int BN_>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     fp8_blockscale_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
-  using Cfg = TileCfg<BN_>;
+  constexpr bool kGrouped = kForm != Form::kDense, kAct = kForm == Form::kActivated;
+  static_assert(!kAct || BN_ == 256, "a tile of 128 gate and 128 up columns");
+  using Cfg = TileCfg<BN_, kForm>;
   constexpr int BN = Cfg::BN, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs, kAccStride = Cfg::kAccStride,
                 kEpiCols = Cfg::kEpiCols, kOutGroups = Cfg::kOutGroups;
   constexpr uint32_t kStageBytes = Cfg::kStageBytes, kOutGroupBytes = Cfg::kOutGroupBytes, kOutBytes = Cfg::kOutBytes;
@@ -251,6 +335,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     ptx::mbar_init(ptx::smem_u32(&ctl->out_full), kEpiThreads);
     ptx::mbar_init(ptx::smem_u32(&ctl->out_free), 1);
+    for (int i = 0; i < 4; ++i) ptx::mbar_init(ptx::smem_u32(&ctl->half_full[i]), kColGroups);
     ctl->abort_flag = 0;
     ptx::mbar_fence_init();
     ptx::tma_prefetch_desc(&map_a);
@@ -316,7 +401,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         // this thread shares its scheduler with promotion warps that always have work: every instruction it
         // spends per slab delays the loads, so the loop keeps only 32-bit counters that step
-        const int row_a = m_tile * BM, row_b = n_tile * BN;
+        const int row_a = m_tile * BM, row_b = n_tile * (kAct ? BN / 2 : BN), row_up = kAct ? (int)(p.N / 2) + row_b : 0;
         for (int k0 = kb_begin * BK; k0 < kb_stop * BK; k0 += BK) {
           if (!SGLB_WAIT(bar_empty0 + s * 8, ph ^ 1u)) { *abort_flag = 1; alive = false; break; }
           const uint32_t bar = bar_full0 + s * 8;
@@ -324,6 +409,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           const uint32_t dst_a = tiles0 + s * kStageBytes;
           ptx::tma_load_2d(dst_a, &map_a, bar, k0, row_a);
           ptx::tma_load_3d(dst_a + kTileBytesA, &map_b, bar, k0, row_b, e);
+          if (kAct) ptx::tma_load_3d(dst_a + kTileBytesA + Cfg::kTileBytesB / 2, &map_b, bar, k0, row_up, e);
           if (++s == (uint32_t)kStages) {
             s = 0;
             ph ^= 1u;
@@ -408,10 +494,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             cmap = p.push_maps + owner;
             out_row0 += (p.push_rank - owner) * p.push_rows_per_owner;
           }
+          if constexpr (kAct) {
+            ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage), n_tile * 128, out_row0);
+          } else {
 #pragma unroll
-          for (int g = 0; g < kOutGroups; ++g) {
-            if (n_tile * BN + g * 64 < n_end)
-              ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage) + g * kOutGroupBytes, n_tile * BN + g * 64, out_row0);
+            for (int g = 0; g < kOutGroups; ++g) {
+              if (n_tile * BN + g * 64 < n_end)
+                ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage) + g * kOutGroupBytes, n_tile * BN + g * 64, out_row0);
+            }
           }
           ptx::tma_store_commit();
         }
@@ -457,9 +547,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         dph ^= 1u;
       }
       if (!work || e < 0) continue;
-      const int nb_tile = min(n_tile * BN / kScaleBlockN, p.nb_total - 1);
+      const int nb_tile = kAct ? n_tile : min(n_tile * BN / kScaleBlockN, p.nb_total - 1);
+      const int nb_next = kAct ? p.nb_total / 2 + n_tile : min(nb_tile + 1, p.nb_total - 1);
       const float* b_row0 = p.b_s + ((int64_t)e * p.nb_total + nb_tile) * kb_total;
-      const float* b_row1 = p.b_s + ((int64_t)e * p.nb_total + min(nb_tile + 1, p.nb_total - 1)) * kb_total;
+      const float* b_row1 = p.b_s + ((int64_t)e * p.nb_total + nb_next) * kb_total;
       for (int kb = un.kb_begin; kb < un.kb_stop; kb += kScSlabs) {
         float b0[kScSlabs], b1[kScSlabs];
 #pragma unroll
@@ -508,13 +599,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     constexpr int kPiecesMax = kEpiCols / 32;
     const int row_in_tile = q * 32 + lane;
     const uint32_t bar_tfull0 = ptx::smem_u32(&ctl->tmem_full[0]), bar_tempty0 = ptx::smem_u32(&ctl->tmem_empty[0]);
-    const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16) + cgrp * kEpiCols;
+    // (activated form: a warp's columns are cgrp * 64 .. of the gate half and the same of the up half)
+    const uint32_t taddr0 = tmem_base + ((uint32_t)(q * 32) << 16) + cgrp * (kAct ? kEpiCols / 2 : kEpiCols);
+    constexpr int kPiece2 = kAct ? BN / 2 : 64;  // TMEM columns from a warp's first to its 64th
     const uint32_t bar_out_full = ptx::smem_u32(&ctl->out_full), bar_out_free = ptx::smem_u32(&ctl->out_free);
     const uint32_t bar_dfull0 = ptx::smem_u32(&ctl->desc_full[0]), bar_dempty0 = ptx::smem_u32(&ctl->desc_empty[0]);
     const uint32_t desc_addr0 = ptx::smem_u32(&ctl->desc[0]);
     const uint32_t bar_sfull0 = ptx::smem_u32(&ctl->sc_full[0]), bar_sempty0 = ptx::smem_u32(&ctl->sc_empty[0]);
     SGLB_MBAR_ASK_DECL();
-    uint32_t oph = 0, ds = 0, dph = 0, ss = 0, sph = 0;
+    uint32_t oph = 0, ds = 0, dph = 0, ss = 0, sph = 0, half_ph = 0;
     uint32_t aph[kAccBufs];  // phase of every accumulator buffer
 #pragma unroll
     for (int b = 0; b < kAccBufs; ++b) aph[b] = 0;
@@ -558,12 +651,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // Scales of four slabs at a time from the scout's ring, requested a slab ahead.  A warp's columns lie in one weight
         // block; columns wholly past N take the last block's.
         static_assert(kScaleBlockN % kEpiCols == 0 && kAccBufs <= 4 && 4 % kAccBufs == 0, "one weight block per warp");
-        const bool second = BN > kScaleBlockN && n0 / kScaleBlockN != n_tile * BN / kScaleBlockN && n0 / kScaleBlockN < p.nb_total;
+        const bool second = !kAct && BN > kScaleBlockN && n0 / kScaleBlockN != n_tile * BN / kScaleBlockN && n0 / kScaleBlockN < p.nb_total;
         const uint32_t sc_addr0 = ptx::smem_u32(&ctl->sc[0][second ? 1 : 0][row_in_tile][0]);
-        float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f), s4_up = s4;
         auto fetch_scales = [&]() -> bool {
           if (!SGLB_WAIT(bar_sfull0 + ss * 8, sph)) return false;
           s4 = ptx::lds_f32x4(sc_addr0 + ss * (2 * BM * 16));
+          if (kAct) s4_up = ptx::lds_f32x4(sc_addr0 + ss * (2 * BM * 16) + BM * 16);
           return true;
         };
         int left = kb_stop - kb_begin;  // slabs from the current group of four on
@@ -582,8 +676,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           ptx::tc_fence_after();
           aph[kBuf] ^= 1u;
           const uint32_t taddr = taddr0 + kBuf * kAccStride;
-          const float sc = I == 0 ? s4.x : I == 1 ? s4.y : I == 2 ? s4.z : s4.w;
+          const float sc_lo = I == 0 ? s4.x : I == 1 ? s4.y : I == 2 ? s4.z : s4.w;
+          const float sc_up = I == 0 ? s4_up.x : I == 1 ? s4_up.y : I == 2 ? s4_up.z : s4_up.w;
           auto fma = [&](int i, const uint32_t (&v)[32]) {
+            const float sc = kAct && i >= 2 ? sc_up : sc_lo;
             // two columns per instruction (packed float32 FMA: the same two IEEE operations): half the issue slots
 #pragma unroll
             for (int jj = 0; jj < 32; jj += 2) ptx::fma2(acc[32 * i + jj], acc[32 * i + jj + 1], v[jj], v[jj + 1], sc);
@@ -614,9 +710,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             fma(1, r[1]);
           } else {  // (128 accumulators leave room for two pieces at a time)
             fma(0, r[0]);
-            ptx::tmem_ld_32x32(taddr + 64, r[0]);
+            ptx::tmem_ld_32x32(taddr + kPiece2, r[0]);
             fma(1, r[1]);
-            ptx::tmem_ld_32x32(taddr + 96, r[1]);
+            ptx::tmem_ld_32x32(taddr + kPiece2 + 32, r[1]);
             ptx::tmem_ld_wait();
             hand_back();
             fma(2, r[0]);
@@ -659,6 +755,27 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             *reinterpret_cast<float4*>(dst + (int64_t)j * BM * 4) =
                 make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
         }
+        continue;
+      }
+      if constexpr (kAct) {  // codes of this row's half group into the staging area (128-byte rows, swizzled), as below
+        const uint32_t bar_half = ptx::smem_u32(&ctl->half_full[q]);
+        float2* half = &ctl->half_max[half_ph][0][row_in_tile];
+        uint4 codes[4];
+        float scale;
+        if (!(p.out_fp16 ? activate_row<__half>(p, acc, cgrp, half, bar_half, half_ph, codes, scale)
+                         : activate_row<__nv_bfloat16>(p, acc, cgrp, half, bar_half, half_ph, codes, scale)) ||
+            !SGLB_WAIT(bar_out_free, oph ^ 1u)) {
+          *abort_flag = 1;
+          break;
+        }
+        oph ^= 1u;
+        const uint32_t stage = ptx::smem_u32(out_stage) + row_in_tile * 128;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ptx::sts_128(stage + (((cgrp * 4 + j) ^ (row_in_tile & 7)) << 4), codes[j]);
+        if (cgrp == 0 && row < rows) p.act_s[row * (p.N / 256) + n_tile] = scale;
+        ptx::fence_async_smem();
+        ptx::mbar_arrive(bar_out_full);
+        half_ph ^= 1u;
         continue;
       }
       if (!kGrouped || p.tma_out) {  // (dense tiles always leave this way)
@@ -718,7 +835,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       // Grouped scatter: the rows go to the token-major slots that sorted_token_ids names.  Through this warp's part of the
       // staging area (same layout), so that every store instruction writes 128 contiguous bytes of four rows; stored
       // row by row from the accumulators, each lane wrote 16 bytes of its own row at a time, half a sector.
-      if constexpr (kGrouped) {
+      if constexpr (kForm == Form::kGrouped) {
         int dst = -1;
         if (row < rows) {
           const int32_t id = p.sorted_ids[row];
@@ -1091,15 +1208,15 @@ static size_t gemm_smem_bytes() {
   return (size_t)Cfg::kStages * Cfg::kStageBytes + Cfg::kOutBytes + sizeof(SharedCtl<Cfg>) + 1024;
 }
 
-template <bool kGrouped, int BN>
+template <Form kForm, int BN>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const GemmParams& p,
                        int64_t max_units, cudaStream_t st, int sm_margin = 0) {
-  const size_t smem = gemm_smem_bytes<TileCfg<BN>>();
+  const size_t smem = gemm_smem_bytes<TileCfg<BN, kForm>>();
   static thread_local bool attr_set[64] = {false};  // the opt-in is per function and per device
   int dev = 0;
   SGLB_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-    SGLB_CUDA(cudaFuncSetAttribute(fp8_blockscale_gemm_kernel<kGrouped, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    SGLB_CUDA(cudaFuncSetAttribute(fp8_blockscale_gemm_kernel<kForm, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem));
     if (dev >= 0 && dev < 64) attr_set[dev] = true;
   }
@@ -1117,7 +1234,7 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   // GPUs and runs differ by.  With several waves the CTAs, which then start wherever an SM falls free, no longer share L2 as
   // their numbers suggest: 4096 x 32768 x 512 114.4 -> 120.9.  Push mode, which other streams take part in: an ordinary launch.
   cfg.numAttrs = max_units <= sms && p.push_maps == nullptr ? 1 : 0;
-  SGLB_CUDA(cudaLaunchKernelEx(&cfg, fp8_blockscale_gemm_kernel<kGrouped, BN>, ma, mb, mc, p));
+  SGLB_CUDA(cudaLaunchKernelEx(&cfg, fp8_blockscale_gemm_kernel<kForm, BN>, ma, mb, mc, p));
   return SGLB200_OK;
 }
 
@@ -1154,7 +1271,7 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
     rc = get_out_map(C, (uint64_t)N, (uint64_t)M, out_dtype, BM, &mc);
     if (rc) return rc;
   }
-  rc = launch_gemm<false, BN>(ma, mb, mc, p, pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits, st);
+  rc = launch_gemm<Form::kDense, BN>(ma, mb, mc, p, pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits, st);
   if (rc != SGLB200_OK || pl.scratch_blocks() == 0) return rc;
   const int tiles_m = (int)((M + BM - 1) / BM);
   const unsigned ygrid = (unsigned)((BM * BN / 8 + 255) / 256);
@@ -1223,7 +1340,34 @@ static int grouped_mm(const void* A, const float* a_s, const void* B, const floa
     if (rc) return rc;
   }
   const int64_t tiles = ((max_rows + BM - 1) / BM) * p.tiles_n;
-  return launch_gemm<true, BN>(ma, mb, mc, p, tiles, st);
+  return launch_gemm<Form::kGrouped, BN>(ma, mb, mc, p, tiles, st);
+}
+
+// The first product of the routed experts with the activation and its quantizer in the epilogue (rows as grouped_mm):
+// codes [max_rows][I] and scales [max_rows][I / 128] of silu(A w_gate) * (A w_up), w13 = [E][2 I][K].
+int grouped_act_mm(const void* A, const float* a_s, const void* w13, const float* b_s, void* out_q, float* out_s,
+                   const int32_t* expert_ids, const int32_t* num_rows_dev, int64_t max_rows, int num_experts, int64_t I,
+                   int64_t K, int dtype, cudaStream_t st) {
+  CUtensorMap ma, mb, mc;
+  int rc = get_tensor_map(A, (uint64_t)K, (uint64_t)max_rows, 1, BM, 2, &ma);
+  if (rc) return rc;
+  rc = get_tensor_map(w13, (uint64_t)K, (uint64_t)(2 * I), (uint64_t)num_experts, 128, 3, &mb);
+  if (rc) return rc;
+  rc = get_tensor_map(out_q, (uint64_t)I, (uint64_t)max_rows, 1, BM, 2, &mc);
+  if (rc) return rc;
+  GemmParams p{};
+  p.a_s = a_s, p.b_s = b_s, p.C = out_q, p.act_s = out_s;
+  p.tma_out = 1;
+  p.expert_ids = expert_ids, p.num_rows_dev = num_rows_dev;
+  p.M = max_rows, p.N = 2 * I, p.K = K;
+  p.kb_total = (int)(K / BK), p.nb_total = (int)(2 * I / kScaleBlockN);
+  p.tiles_n = (int)(I / 128);
+  p.group_m = choose_group_m(max_rows, K, BM);
+  p.as_stride_m = p.kb_total, p.as_stride_k = 1;
+  p.out_fp16 = dtype;
+  p.wait_probes = g_gemm_wait_probes;
+  p.splits = 1, p.kb_per_split = p.kb_total, p.sk_pieces = 2;
+  return launch_gemm<Form::kActivated, 256>(ma, mb, mc, p, (max_rows + BM - 1) / BM * p.tiles_n, st);
 }
 
 }  // namespace sglb200
@@ -1383,7 +1527,7 @@ static int push_mm(const void* A, const void* B, const float* a_s, const float* 
   CUtensorMap mc = {};
   rc = get_out_map(stage_ptrs[rank], (uint64_t)N, (uint64_t)(rpo * world), out_dtype, BM, &mc);  // unused by the stores; keeps map_c valid
   if (rc) return rc;
-  return launch_gemm<false, BN>(ma, mb, mc, p, tiles, st, sm_margin);
+  return launch_gemm<Form::kDense, BN>(ma, mb, mc, p, tiles, st, sm_margin);
 }
 
 }  // namespace sglb200

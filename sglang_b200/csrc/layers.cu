@@ -76,7 +76,7 @@ static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int6
   p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4), p.next = c.take(8);
   p.cum = c.take((E + 2) * 4), p.sort = c.take(p.sort_bytes);
   if (p.tile == 0) p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
-  p.ic1 = c.take(p.rows * 2 * I * 2);
+  else p.ic1 = c.take(p.rows * 2 * I * 2);
   p.a2 = c.take(p.rows * I), p.a2s = c.take(p.rows * (I / 128) * 4);
   if (!p.direct) p.ic3 = c.take(numel * Ho * 2);
   p.total = c.bytes;
@@ -175,10 +175,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     rc = sglb200_gather_rows_fp8(base + p.q, f(p.s), base + p.a1, f(p.a1s), i(p.sorted), i(p.post), p.rows, numel, (int)k, H, hb,
                                  stream);
     if (rc) return rc;
-    rc = sglb200_fp8_blockwise_grouped_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.ic1, i(p.sorted), i(p.eid), i(p.post), nullptr,
-                                          p.rows, numel, (int)E, 2 * I, H, 0, dtype, stream);
-    if (rc) return rc;
-    rc = silu_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), true, st);
+    rc = grouped_act_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.a2, f(p.a2s), i(p.eid), i(p.post), p.rows, (int)E, I, H, dtype, st);
     if (rc) return rc;
     rc = sglb200_fp8_blockwise_grouped_mm(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights,
                                           p.rows, numel, (int)E, Ho, I, 1, dtype, stream);

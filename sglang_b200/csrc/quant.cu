@@ -289,25 +289,6 @@ __global__ void __launch_bounds__(kQuantThreads)
 // segments.  h = T(T(silu(gate)) * up): silu in float32 rounded to T, then one packed multiply (the product of
 // two 16-bit floats is exact in float32, so its single rounding equals rounding the float32 product), then
 // the quantizer arithmetic on h in registers.
-template <typename T>
-struct Packed2;
-template <>
-struct Packed2<__nv_bfloat16> {
-  static __device__ __forceinline__ uint32_t round_mul(float a, float b, uint32_t up) {
-    const __nv_bfloat162 act = __floats2bfloat162_rn(a, b);
-    const __nv_bfloat162 h = __hmul2(act, *reinterpret_cast<const __nv_bfloat162*>(&up));
-    return *reinterpret_cast<const uint32_t*>(&h);
-  }
-};
-template <>
-struct Packed2<__half> {
-  static __device__ __forceinline__ uint32_t round_mul(float a, float b, uint32_t up) {
-    const __half2 act = __floats2half2_rn(a, b);
-    const __half2 h = __hmul2(act, *reinterpret_cast<const __half2*>(&up));
-    return *reinterpret_cast<const uint32_t*>(&h);
-  }
-};
-
 // Direct form: as the quantizer, 16 gate and 16 up values a thread and unit.
 template <typename T, int LPG, int U>
 __global__ void __launch_bounds__(kQuantThreads)

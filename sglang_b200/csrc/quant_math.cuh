@@ -56,6 +56,44 @@ __device__ __forceinline__ void unpack_chunk<float>(const uint4& raw, float* v) 
   v[2] = __uint_as_float(raw.z), v[3] = __uint_as_float(raw.w);
 }
 
+// Pairs of 16-bit values in one word.  round_mul: the rounded pair (a, b) times `up`, rounded again (the product of two 16-bit
+// floats is exact in float32, so a single packed multiply does); max_abs_nan: per half, NaN if either is.
+template <typename T>
+struct Packed2;
+template <>
+struct Packed2<__nv_bfloat16> {
+  typedef __nv_bfloat162 Pair;
+  static __device__ __forceinline__ void unpack(uint32_t w, float (&v)[2]) {
+    v[0] = __uint_as_float(w << 16), v[1] = __uint_as_float(w & 0xffff0000u);
+  }
+  static __device__ __forceinline__ uint32_t pack(float a, float b) { return bits(__floats2bfloat162_rn(a, b)); }
+  static __device__ __forceinline__ uint32_t round_mul(float a, float b, uint32_t up) {
+    return bits(__hmul2(__floats2bfloat162_rn(a, b), pair(up)));
+  }
+  static __device__ __forceinline__ uint32_t max_abs_nan(uint32_t m, uint32_t w) {
+    return bits(__hmax2_nan(pair(m), pair(w & 0x7fff7fffu)));
+  }
+  static __device__ __forceinline__ Pair pair(uint32_t w) { return *reinterpret_cast<const Pair*>(&w); }
+  static __device__ __forceinline__ uint32_t bits(Pair h) { return *reinterpret_cast<const uint32_t*>(&h); }
+};
+template <>
+struct Packed2<__half> {
+  typedef __half2 Pair;
+  static __device__ __forceinline__ void unpack(uint32_t w, float (&v)[2]) {
+    const float2 f = __half22float2(pair(w));
+    v[0] = f.x, v[1] = f.y;
+  }
+  static __device__ __forceinline__ uint32_t pack(float a, float b) { return bits(__floats2half2_rn(a, b)); }
+  static __device__ __forceinline__ uint32_t round_mul(float a, float b, uint32_t up) {
+    return bits(__hmul2(__floats2half2_rn(a, b), pair(up)));
+  }
+  static __device__ __forceinline__ uint32_t max_abs_nan(uint32_t m, uint32_t w) {
+    return bits(__hmax2_nan(pair(m), pair(w & 0x7fff7fffu)));
+  }
+  static __device__ __forceinline__ Pair pair(uint32_t w) { return *reinterpret_cast<const Pair*>(&w); }
+  static __device__ __forceinline__ uint32_t bits(Pair h) { return *reinterpret_cast<const uint32_t*>(&h); }
+};
+
 // Sign bits of the chunk's elements, one per byte (bit 7), in element order.
 template <typename T>
 __device__ __forceinline__ void chunk_signs(const uint4& raw, uint32_t* s) {
@@ -67,8 +105,8 @@ __device__ __forceinline__ void chunk_signs(const uint4& raw, uint32_t* s) {
   }
 }
 
-// q0 = RN(x r), e = fma(-q0, scale, x), q = fma(e, r, q0) of two elements (packed float32: half the issue slots.  Cold inputs, 8192 x 18432
-// bf16: 83.8 us -> 79.7).
+// q0 = RN(x r), e = fma(-q0, scale, x), q = fma(e, r, q0) of two elements (packed float32: half the issue slots.  Cold
+// inputs, 8192 x 18432 bf16: 83.8 us -> 79.7).
 __device__ __forceinline__ void quotient2(float x0, float x1, float scale, float r, float& q0, float& q1) {
   asm("{\n\t.reg .b64 x, s, r, a, e;\n\t"
       "mov.b64 x, {%2, %3};\n\t"

@@ -95,6 +95,42 @@ def test_experts_row_counts(T, E, topk, H=384, I=256):
     assert_close_fp(to_f32_np(out), ref, rtol=2e-2, atol=2e-2)
 
 
+# the one-call layer against its steps one by one, bit for bit, where experts have more than 48 rows on average: rows that end in
+# every part of a 128-row tile, one and several groups of hidden and intermediate columns, one slot a token, more ids than one
+# CTA sorts; `ids`: some of them negative, and a weight scale that overflows one expert to infinities and NaN
+@pytest.mark.parametrize("T,E,topk,H,I,dtype,odd", [
+    (97, 1, 1, 128, 128, torch.bfloat16, False), (150, 4, 2, 384, 256, torch.float16, False),
+    (333, 4, 2, 1152, 384, torch.bfloat16, True), (700, 9, 3, 256, 640, torch.float16, True),
+    (2000, 16, 8, 512, 128, torch.bfloat16, False), (5000, 7, 2, 2048, 768, torch.bfloat16, False)])
+def test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd):
+    from sglang_b200 import ops
+    from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, H, device="cuda", generator=g).to(dtype)
+    w13, w2 = ((torch.randn(*s, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+               for s in ((E, 2 * I, H), (E, H, I)))
+    s13, s2 = (torch.rand(*s, device="cuda", generator=g) * 1e-3 for s in ((E, 2 * I // 128, H // 128), (E, H // 128, I // 128)))
+    logits = torch.randn(T, E, device="cuda", generator=g) - 0.2 * torch.arange(E, device="cuda")
+    wt, ids = torch.topk(torch.softmax(logits, -1), topk)
+    ids = ids.to(torch.int32)
+    if odd:
+        ids[torch.rand(T, topk, device="cuda", generator=g) < 0.1] = -1
+        s13[1] *= 1e38
+    got = fused_experts_impl(x, w13, w2, wt, ids, use_fp8_w8a8=True, w1_scale=s13, w2_scale=s2, block_shape=[128, 128])
+    xq, xs = ops.per_token_group_quant_fp8(x, 128)
+    order, eid, post = ops.moe_align_block_size(ids, 128, E)
+    a1, a1s = ops.gather_rows_fp8(xq, xs, order, post, T * topk, topk, order.numel() // 128 * 128)
+    ic1 = ops.grouped_block_fp8_matmul(a1, a1s, w13, s13, order, eid, post, numel=T * topk, scatter=False, output_dtype=dtype)
+    a2, a2s = ops.silu_and_mul_quant_fp8(ic1, 128, num_rows=post)
+    ic3 = ops.grouped_block_fp8_matmul(a2, a2s, w2, s2, order, eid, post, numel=T * topk, scatter=True, row_weights=wt,
+                                       output_dtype=dtype)
+    want = torch.empty_like(x)
+    ops.moe_sum_reduce_out(ic3.view(T, topk, H), want, 1.0)
+    assert ops.gemm_status() == 0
+    assert odd == bool(want.isnan().any())
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(), want.nan_to_num())
+
+
 # more tiles of the first product than CTAs, behind the sort of up to 2048 ids and of more; experts without rows among them
 @pytest.mark.parametrize("T,E,topk", [(40, 64, 2), (700, 96, 3)])
 def test_experts_many_tiles(T, E, topk):
