@@ -156,6 +156,7 @@ struct GemmParams {
   int sk_pieces;                 // 2 or 3
   int sk_total;                  // tiles * kb_total
   uint32_t wait_probes;          // probes after which a pipeline wait gives up
+  int skip_padding;              // grouped: nobody reads the rows of a 32-row quadrant that is all padding (sorted_ids >= numel)
   float* act_s;                  // activated form: C holds codes [row][N / 2], this their scales [row][N / 256]
 };
 
@@ -164,7 +165,7 @@ struct GemmParams {
 // own, the slabs' scales.
 struct UnitDesc {
   int m_tile, n_tile, expert, kb_begin;
-  int kb_stop, split, slot, pad;
+  int kb_stop, split, slot, live;  // live: leading 32-row quadrants of the tile with rows that count
 };
 constexpr int kScSlabs = 4;  // slabs per slot of the scale ring: one 16-byte read per promotion thread and weight block
 
@@ -192,6 +193,13 @@ struct SharedCtl {
 struct TileCoord {
   int m_tile, n_tile, expert;
 };
+
+// Leading 32-row quadrants of a tile that hold rows.  An expert's rows come first and its padding last, and a tile has a row.
+__device__ __forceinline__ int live_quadrants(const GemmParams& p, int m_tile) {
+  const int32_t* id = p.sorted_ids + (int64_t)m_tile * BM;
+  const int a = id[32], b = id[64], c = id[96];
+  return 1 + (a < p.numel) + (b < p.numel) + (c < p.numel);
+}
 
 // A unit of work = one output tile x one K range.  Dense problems number their units: the tiles
 // [0, full_units) whole, then `splits` consecutive units per remaining tile.
@@ -300,7 +308,8 @@ __device__ __forceinline__ bool activate_row(const GemmParams& p, const float (&
 template <Form kForm, int BN_>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     fp8_blockscale_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                               const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
+                               const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_a32,
+                               const GemmParams p) {
   constexpr bool kGrouped = kForm != Form::kDense, kAct = kForm == Form::kActivated;
   static_assert(!kAct || BN_ == 256, "a tile of 128 gate and 128 up columns");
   using Cfg = TileCfg<BN_, kForm>;
@@ -394,9 +403,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (kb_begin >= kb_stop) continue;  // (an empty piece of a stream-K run)
         int m_tile, n_tile;
         tile_coord(t, tiles_m, tiles_n, p.group_m, m_tile, n_tile);
-        int e = 0;
+        int e = 0, live = 4;
         if (kGrouped) {
           e = p.expert_ids[m_tile];
+          if (p.skip_padding) live = live_quadrants(p, m_tile);
           if (e < 0) continue;
         }
         // this thread shares its scheduler with promotion warps that always have work: every instruction it
@@ -407,7 +417,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           const uint32_t bar = bar_full0 + s * 8;
           ptx::mbar_arrive_expect_tx(bar, kStageBytes);
           const uint32_t dst_a = tiles0 + s * kStageBytes;
-          ptx::tma_load_2d(dst_a, &map_a, bar, k0, row_a);
+          if (!kGrouped || live == 4) {
+            ptx::tma_load_2d(dst_a, &map_a, bar, k0, row_a);
+          } else {  // quadrants of padding come from beyond the last row: zeros, without a byte of memory traffic
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              ptx::tma_load_2d(dst_a + i * (kTileBytesA / 4), &map_a32, bar, k0, i < live ? row_a + 32 * i : (int)p.M);
+          }
           ptx::tma_load_3d(dst_a + kTileBytesA, &map_b, bar, k0, row_b, e);
           if (kAct) ptx::tma_load_3d(dst_a + kTileBytesA + Cfg::kTileBytesB / 2, &map_b, bar, k0, row_up, e);
           if (++s == (uint32_t)kStages) {
@@ -495,7 +511,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             out_row0 += (p.push_rank - owner) * p.push_rows_per_owner;
           }
           if constexpr (kAct) {
-            ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage), n_tile * 128, out_row0);
+            const int live = p.skip_padding ? live_quadrants(p, m_tile) : 4;
+            for (int i = 0; i < live; ++i)
+              ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage) + i * (32 * 128), n_tile * 128, out_row0 + 32 * i);
           } else {
 #pragma unroll
             for (int g = 0; g < kOutGroups; ++g) {
@@ -531,15 +549,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       const Unit un = decode_unit<kGrouped>(p, u);
       UnitDesc* d = &ctl->desc[ds];
-      int m_tile = 0, n_tile = 0, e = 0;
+      int m_tile = 0, n_tile = 0, e = 0, live = 4;
       const bool work = un.kb_begin < un.kb_stop;
       if (work) {
         tile_coord(un.tile, tiles_m, tiles_n, p.group_m, m_tile, n_tile);
         if (kGrouped) e = p.expert_ids[m_tile];
+        if (kGrouped && p.skip_padding) live = live_quadrants(p, m_tile);
       }
       if (lane == 0) {
         d->m_tile = m_tile, d->n_tile = n_tile, d->expert = e, d->kb_begin = un.kb_begin;
-        d->kb_stop = un.kb_stop, d->split = un.split ? 1 : 0, d->slot = un.slot, d->pad = 0;
+        d->kb_stop = un.kb_stop, d->split = un.split ? 1 : 0, d->slot = un.slot, d->live = live;
       }
       ptx::mbar_arrive(bar_dfull0 + ds * 8);  // every lane: its own writes are released with its arrival
       if (++ds == 2u) {
@@ -638,6 +657,40 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const int kb_stop = __float_as_int(ptx::lds_f32(desc_addr + (uint32_t)offsetof(UnitDesc, kb_stop)));
       if (kb_begin >= kb_stop) {  // (an empty piece of a stream-K run; uniform over the CTA)
         release_desc();
+        continue;
+      }
+      if (kGrouped && q >= __float_as_int(ptx::lds_f32(desc_addr + (uint32_t)offsetof(UnitDesc, live)))) {
+        // None of this warp's rows counts: it hands everything on unread and stores nothing.  About 128 rows an expert, of
+        // which every second one then has a second tile with a few rows (32768 rows, 256 experts of 7168 x 2048, sustained):
+        // layer 3 491 -> 3 405 us, mostly by the power that the other warps and the MMAs (zeros) no longer share.  In dense
+        // products, which have one such row of tiles, the test cost more than it gave (4096 x 36864 x 7168 1 036 -> 1 041).
+        int left = __float_as_int(h0.z) < 0 ? 0 : kb_stop - kb_begin;
+        release_desc();
+        bool ok = true;
+        for (; left > 0 && ok; left -= 4) {
+          ok = SGLB_WAIT(bar_sfull0 + ss * 8, sph);
+          if (ok) ptx::mbar_arrive_if(bar_sempty0 + ss * 8, lane == 0);
+          ss ^= 1u;
+          sph ^= ss == 0 ? 1u : 0u;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int b = i % kAccBufs;
+            if (i < left && ok) {
+              ok = SGLB_WAIT(bar_tfull0 + b * 8, aph[b]);
+              aph[b] ^= 1u;
+              if (ok) ptx::mbar_arrive_if(bar_tempty0 + b * 8, lane == 0);
+            }
+          }
+        }
+        if (ok && p.tma_out) {  // (the staging area takes part in turn, so that no arrival counts for the tile before)
+          ok = SGLB_WAIT(bar_out_free, oph ^ 1u);
+          oph ^= 1u;
+          if (ok) ptx::mbar_arrive(bar_out_full);
+        }
+        if (!ok) {
+          *abort_flag = 1;
+          break;
+        }
         continue;
       }
       const int64_t row = (int64_t)m_tile * BM + row_in_tile;
@@ -1209,8 +1262,8 @@ static size_t gemm_smem_bytes() {
 }
 
 template <Form kForm, int BN>
-static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const GemmParams& p,
-                       int64_t max_units, cudaStream_t st, int sm_margin = 0) {
+static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const CUtensorMap& ma32,
+                       const GemmParams& p, int64_t max_units, cudaStream_t st, int sm_margin = 0) {
   const size_t smem = gemm_smem_bytes<TileCfg<BN, kForm>>();
   static thread_local bool attr_set[64] = {false};  // the opt-in is per function and per device
   int dev = 0;
@@ -1234,7 +1287,7 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   // GPUs and runs differ by.  With several waves the CTAs, which then start wherever an SM falls free, no longer share L2 as
   // their numbers suggest: 4096 x 32768 x 512 114.4 -> 120.9.  Push mode, which other streams take part in: an ordinary launch.
   cfg.numAttrs = max_units <= sms && p.push_maps == nullptr ? 1 : 0;
-  SGLB_CUDA(cudaLaunchKernelEx(&cfg, fp8_blockscale_gemm_kernel<kForm, BN>, ma, mb, mc, p));
+  SGLB_CUDA(cudaLaunchKernelEx(&cfg, fp8_blockscale_gemm_kernel<kForm, BN>, ma, mb, mc, ma32, p));
   return SGLB200_OK;
 }
 
@@ -1271,7 +1324,7 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
     rc = get_out_map(C, (uint64_t)N, (uint64_t)M, out_dtype, BM, &mc);
     if (rc) return rc;
   }
-  rc = launch_gemm<Form::kDense, BN>(ma, mb, mc, p, pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits, st);
+  rc = launch_gemm<Form::kDense, BN>(ma, mb, mc, ma, p, pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits, st);
   if (rc != SGLB200_OK || pl.scratch_blocks() == 0) return rc;
   const int tiles_m = (int)((M + BM - 1) / BM);
   const unsigned ygrid = (unsigned)((BM * BN / 8 + 255) / 256);
@@ -1314,9 +1367,11 @@ template <int BN>
 static int grouped_mm(const void* A, const float* a_s, const void* B, const float* b_s, void* C,
                       const int32_t* sorted_token_ids, const int32_t* expert_ids, const int32_t* num_rows_dev,
                       const float* row_weights, int64_t max_rows, int64_t numel, int num_experts, int64_t N, int64_t K,
-                      int scatter, int out_dtype, cudaStream_t st) {
-  CUtensorMap ma, mb;
+                      int scatter, int out_dtype, bool skip_padding, cudaStream_t st) {
+  CUtensorMap ma, mb, ma32;
   int rc = get_tensor_map(A, (uint64_t)K, (uint64_t)max_rows, 1, BM, 2, &ma);
+  if (rc) return rc;
+  rc = get_tensor_map(A, (uint64_t)K, (uint64_t)max_rows, 1, 32, 2, &ma32);
   if (rc) return rc;
   rc = get_tensor_map(B, (uint64_t)K, (uint64_t)N, (uint64_t)num_experts, BN, 3, &mb);
   if (rc) return rc;
@@ -1329,7 +1384,7 @@ static int grouped_mm(const void* A, const float* a_s, const void* B, const floa
   p.tiles_n = (int)((N + BN - 1) / BN);
   p.group_m = choose_group_m(max_rows, K, BM);
   p.as_stride_m = p.kb_total, p.as_stride_k = 1;
-  p.numel = numel, p.scatter = scatter, p.out_fp16 = out_dtype;
+  p.numel = numel, p.scatter = scatter, p.out_fp16 = out_dtype, p.skip_padding = skip_padding;
   p.wait_probes = g_gemm_wait_probes;
   p.full_units = 0, p.splits = 1, p.kb_per_split = p.kb_total, p.partial = nullptr;  // grouped: one unit per tile
   p.sk_pieces = 2;
@@ -1340,25 +1395,29 @@ static int grouped_mm(const void* A, const float* a_s, const void* B, const floa
     if (rc) return rc;
   }
   const int64_t tiles = ((max_rows + BM - 1) / BM) * p.tiles_n;
-  return launch_gemm<Form::kGrouped, BN>(ma, mb, mc, p, tiles, st);
+  return launch_gemm<Form::kGrouped, BN>(ma, mb, mc, ma32, p, tiles, st);
 }
 
 // The first product of the routed experts with the activation and its quantizer in the epilogue (rows as grouped_mm):
-// codes [max_rows][I] and scales [max_rows][I / 128] of silu(A w_gate) * (A w_up), w13 = [E][2 I][K].
+// codes [max_rows][I] and scales [max_rows][I / 128] of silu(A w_gate) * (A w_up), w13 = [E][2 I][K].  Quadrants of padding are
+// not written.
 int grouped_act_mm(const void* A, const float* a_s, const void* w13, const float* b_s, void* out_q, float* out_s,
-                   const int32_t* expert_ids, const int32_t* num_rows_dev, int64_t max_rows, int num_experts, int64_t I,
-                   int64_t K, int dtype, cudaStream_t st) {
-  CUtensorMap ma, mb, mc;
+                   const int32_t* sorted_ids, const int32_t* expert_ids, const int32_t* num_rows_dev, int64_t max_rows,
+                   int64_t numel, int num_experts, int64_t I, int64_t K, int dtype, cudaStream_t st) {
+  CUtensorMap ma, mb, mc, ma32;
   int rc = get_tensor_map(A, (uint64_t)K, (uint64_t)max_rows, 1, BM, 2, &ma);
   if (rc) return rc;
   rc = get_tensor_map(w13, (uint64_t)K, (uint64_t)(2 * I), (uint64_t)num_experts, 128, 3, &mb);
   if (rc) return rc;
-  rc = get_tensor_map(out_q, (uint64_t)I, (uint64_t)max_rows, 1, BM, 2, &mc);
+  rc = get_tensor_map(A, (uint64_t)K, (uint64_t)max_rows, 1, 32, 2, &ma32);
+  if (rc) return rc;
+  rc = get_tensor_map(out_q, (uint64_t)I, (uint64_t)max_rows, 1, 32, 2, &mc);
   if (rc) return rc;
   GemmParams p{};
   p.a_s = a_s, p.b_s = b_s, p.C = out_q, p.act_s = out_s;
   p.tma_out = 1;
-  p.expert_ids = expert_ids, p.num_rows_dev = num_rows_dev;
+  p.sorted_ids = sorted_ids, p.expert_ids = expert_ids, p.num_rows_dev = num_rows_dev;
+  p.numel = numel, p.skip_padding = 1;
   p.M = max_rows, p.N = 2 * I, p.K = K;
   p.kb_total = (int)(K / BK), p.nb_total = (int)(2 * I / kScaleBlockN);
   p.tiles_n = (int)(I / 128);
@@ -1367,7 +1426,7 @@ int grouped_act_mm(const void* A, const float* a_s, const void* w13, const float
   p.out_fp16 = dtype;
   p.wait_probes = g_gemm_wait_probes;
   p.splits = 1, p.kb_per_split = p.kb_total, p.sk_pieces = 2;
-  return launch_gemm<Form::kActivated, 256>(ma, mb, mc, p, (max_rows + BM - 1) / BM * p.tiles_n, st);
+  return launch_gemm<Form::kActivated, 256>(ma, mb, mc, ma32, p, (max_rows + BM - 1) / BM * p.tiles_n, st);
 }
 
 }  // namespace sglb200
@@ -1431,6 +1490,14 @@ extern "C" int sglb200_fp8_blockwise_grouped_mm(const void* A, const float* a_s,
                                                 const int32_t* num_rows_dev, const float* row_weights,
                                                 int64_t max_rows, int64_t numel, int num_experts, int64_t N, int64_t K,
                                                 int scatter, int out_dtype, void* stream) {
+  return sglb200::grouped_mm_any(A, a_s, B, b_s, C, sorted_token_ids, expert_ids, num_rows_dev, row_weights, max_rows, numel,
+                                 num_experts, N, K, scatter, out_dtype, false, static_cast<cudaStream_t>(stream));
+}
+
+int sglb200::grouped_mm_any(const void* A, const float* a_s, const void* B, const float* b_s, void* C,
+                            const int32_t* sorted_token_ids, const int32_t* expert_ids, const int32_t* num_rows_dev,
+                            const float* row_weights, int64_t max_rows, int64_t numel, int num_experts, int64_t N, int64_t K,
+                            int scatter, int out_dtype, bool skip_padding, cudaStream_t st) {
   SGLB_REQUIRE(max_rows >= 0 && N > 0 && K > 0 && num_experts >= 1, "grouped_mm: bad shape rows=%lld N=%lld K=%lld E=%d",
                (long long)max_rows, (long long)N, (long long)K, num_experts);
   SGLB_REQUIRE(K % 16 == 0 && N % 8 == 0, "grouped_mm: K must be a multiple of 16 and N of 8");
@@ -1439,12 +1506,11 @@ extern "C" int sglb200_fp8_blockwise_grouped_mm(const void* A, const float* a_s,
   SGLB_REQUIRE(A && a_s && B && b_s && C && expert_ids && num_rows_dev, "grouped_mm: null pointer");
   SGLB_REQUIRE(!scatter || sorted_token_ids, "grouped_mm: scatter mode needs sorted_token_ids");
   SGLB_REQUIRE(aligned16(A) && aligned16(B) && aligned16(C), "grouped_mm: A, B and C must be 16-byte aligned");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (choose_bn_grouped(numel) == 128)
     return grouped_mm<128>(A, a_s, B, b_s, C, sorted_token_ids, expert_ids, num_rows_dev, row_weights, max_rows, numel,
-                           num_experts, N, K, scatter, out_dtype, st);
+                           num_experts, N, K, scatter, out_dtype, skip_padding, st);
   return grouped_mm<256>(A, a_s, B, b_s, C, sorted_token_ids, expert_ids, num_rows_dev, row_weights, max_rows, numel,
-                         num_experts, N, K, scatter, out_dtype, st);
+                         num_experts, N, K, scatter, out_dtype, skip_padding, st);
 }
 
 
@@ -1527,7 +1593,7 @@ static int push_mm(const void* A, const void* B, const float* a_s, const float* 
   CUtensorMap mc = {};
   rc = get_out_map(stage_ptrs[rank], (uint64_t)N, (uint64_t)(rpo * world), out_dtype, BM, &mc);  // unused by the stores; keeps map_c valid
   if (rc) return rc;
-  return launch_gemm<Form::kDense, BN>(ma, mb, mc, p, tiles, st, sm_margin);
+  return launch_gemm<Form::kDense, BN>(ma, mb, mc, ma, p, tiles, st, sm_margin);
 }
 
 }  // namespace sglb200

@@ -175,10 +175,11 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     rc = sglb200_gather_rows_fp8(base + p.q, f(p.s), base + p.a1, f(p.a1s), i(p.sorted), i(p.post), p.rows, numel, (int)k, H, hb,
                                  stream);
     if (rc) return rc;
-    rc = grouped_act_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.a2, f(p.a2s), i(p.eid), i(p.post), p.rows, (int)E, I, H, dtype, st);
+    rc = grouped_act_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.a2, f(p.a2s), i(p.sorted), i(p.eid), i(p.post),
+                        p.rows, numel, (int)E, I, H, dtype, st);
     if (rc) return rc;
-    rc = sglb200_fp8_blockwise_grouped_mm(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights,
-                                          p.rows, numel, (int)E, Ho, I, 1, dtype, stream);
+    rc = grouped_mm_any(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights, p.rows, numel, (int)E,
+                        Ho, I, 1, dtype, true, st);
   }
   if (rc || p.direct) return rc;
   // (the rows kernel leaves the slots of negative ids unwritten)
