@@ -39,17 +39,25 @@ int quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s, 
 int silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s, int64_t rows, int64_t d, int group_size,
                        float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t st);
 
-// moe_align.cu: the sort (arguments as sglb200_moe_align_block_size).  `zeros` (or nullptr): zeros[0] and zeros[1] are set to 0.
+// quant.cu: the quantizer (groups of 128) of a layer's activations with every row's codes and scales written to its `topk`
+// places in the sorted order (`inverse` of the sort, -1 = nowhere), and zeros to the padding rows of 32-row quadrants that
+// hold rows; other padding is not written.
+int quant_sorted(const void* x, int dtype, void* out_q, float* out_s, const int32_t* inverse, const int32_t* sorted_ids,
+                 const int32_t* num_rows_dev, int64_t max_rows, int64_t tokens, int topk, int64_t hidden, float eps,
+                 cudaStream_t st);
+
+// moe_align.cu: the sort (arguments as sglb200_moe_align_block_size).  `inverse` (or nullptr): the place of every flat index in
+// the order, -1 for an id that is no bucket's.  `zeros` (or nullptr): zeros[0] and zeros[1] are set to 0.
 int align_block_size(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size, int32_t* sorted_token_ids,
                      int32_t* expert_ids, int32_t* num_tokens_post_pad, int32_t* cumsum_buffer, int pad_sorted_token_ids,
-                     void* workspace, int64_t workspace_bytes, int32_t* zeros, cudaStream_t st);
+                     void* workspace, int64_t workspace_bytes, int32_t* inverse, int32_t* zeros, cudaStream_t st);
 
 // moe_align.cu: the sort of few ids (as sglb200_moe_align_block_size, padding written) and the quantizer of the same layer's
-// activations (groups of 128) in one launch, where `align_quant_fits`.  `zeros` as above.
+// activations (groups of 128) in one launch, where `align_quant_fits`.  `inverse` and `zeros` as above.
 bool align_quant_fits(const void* x, int64_t numel, int buckets);
 int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                 int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
-                int64_t hidden, float eps, float fp8_max, int32_t* zeros, cudaStream_t st);
+                int64_t hidden, float eps, float fp8_max, int32_t* inverse, int32_t* zeros, cudaStream_t st);
 
 // gemm.cu: the dense product (arguments as sglb200_fp8_blockwise_scaled_mm).  `after_quantizer`: the kernel before it in
 // the stream is this library's quantizer, launched by the same call, so that the weights may be fetched while that runs.

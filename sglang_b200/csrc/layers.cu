@@ -41,7 +41,7 @@ static LinearParts linear_parts(int64_t M, int64_t N, int64_t K) {
 struct ExpertsPlan {
   int tile, block;
   int64_t cap, rows;  // entries of the sort's output; rows that can be in use
-  int64_t q, s, sorted, eid, post, next, cum, sort, sort_bytes, a1, a1s, ic1, a2, a2s, ic3, total;
+  int64_t q, s, sorted, inv, eid, post, next, cum, sort, sort_bytes, a1, a1s, ic1, a2, a2s, ic3, total;
   bool direct;        // one expert per token and no factor: the second GEMM writes the result itself
 };
 
@@ -75,7 +75,7 @@ static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int6
   p.q = c.take(T * H), p.s = c.take(T * (H / 128) * 4);
   p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4), p.next = c.take(8);
   p.cum = c.take((E + 2) * 4), p.sort = c.take(p.sort_bytes);
-  if (p.tile == 0) p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
+  if (p.tile == 0) p.inv = c.take(numel * 4), p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
   else p.ic1 = c.take(p.rows * 2 * I * 2);
   p.a2 = c.take(p.rows * I), p.a2s = c.take(p.rows * (I / 128) * 4);
   if (!p.direct) p.ic3 = c.take(numel * Ho * 2);
@@ -149,14 +149,20 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   const int64_t hb = H / 128, ib = I / 128;
   int rc;
   int32_t* next = i(p.next);  // counters of the two products' tiles, which the sort sets to zero
-  if (align_quant_fits(x, numel, (int)E + 1)) {
+  const bool beside = align_quant_fits(x, numel, (int)E + 1), sorted_rows = p.tile == 0 && !beside;
+  if (beside) {
     rc = align_quant(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), x, dtype, base + p.q, f(p.s), T,
-                     H, kQuantEps, kFp8Max, next, st);
+                     H, kQuantEps, kFp8Max, nullptr, next, st);
+  } else if (sorted_rows) {
+    rc = align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
+                          p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, i(p.inv), next, st);
+    if (rc) return rc;
+    rc = quant_sorted(x, dtype, base + p.a1, f(p.a1s), i(p.inv), i(p.sorted), i(p.post), p.rows, T, (int)k, H, kQuantEps, st);
   } else {
     rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
     if (rc) return rc;
     rc = align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
-                          p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, next, st);
+                          p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, nullptr, next, st);
   }
   if (rc) return rc;
   if (p.tile > 0) {
@@ -172,9 +178,11 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     rc = rows_grouped_mm(base + p.a2, p.rows, ib, f(p.a2s), w2, w2_s, ic3, i(p.cum), i(p.sorted), topk_weights, p.rows, numel,
                          (int)E, Ho, I, 0, 1, dtype, p.tile, single ? nullptr : next + 1, true, st);
   } else {
-    rc = sglb200_gather_rows_fp8(base + p.q, f(p.s), base + p.a1, f(p.a1s), i(p.sorted), i(p.post), p.rows, numel, (int)k, H, hb,
-                                 stream);
-    if (rc) return rc;
+    if (!sorted_rows) {
+      rc = sglb200_gather_rows_fp8(base + p.q, f(p.s), base + p.a1, f(p.a1s), i(p.sorted), i(p.post), p.rows, numel, (int)k, H, hb,
+                                   stream);
+      if (rc) return rc;
+    }
     rc = grouped_act_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.a2, f(p.a2s), i(p.sorted), i(p.eid), i(p.post),
                         p.rows, numel, (int)E, I, H, dtype, st);
     if (rc) return rc;

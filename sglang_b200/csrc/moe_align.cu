@@ -146,10 +146,12 @@ __device__ __forceinline__ void write_starts(int B, const int* prefix, int32_t* 
   if (zeros != nullptr && threadIdx.x < 2) zeros[threadIdx.x] = 0;
 }
 
-// Writes sorted_token_ids for the chunk.  base[b] = padded start of bucket b + entries in earlier chunks.
+// Writes sorted_token_ids for the chunk.  base[b] = padded start of bucket b + entries in earlier chunks.  Every scatter also
+// writes, where asked to, the inverse: the place of each flat index in the order (-1: its id is no bucket's).
 template <int NBITS = 0>  // > 0: the number of key bits is known at compile time (unrolled ballots)
 __device__ __forceinline__ void scatter_chunk(const int32_t* __restrict__ ids, int64_t chunk_begin, int64_t chunk_end,
-                                              int span, int B, int* wc, const int* base, int32_t* __restrict__ sorted) {
+                                              int span, int B, int* wc, const int* base, int32_t* __restrict__ sorted,
+                                              int32_t* __restrict__ inverse) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t seg = chunk_begin + (int64_t)warp * span;
   const int64_t seg_end = seg + span < chunk_end ? seg + span : chunk_end;
@@ -173,8 +175,10 @@ __device__ __forceinline__ void scatter_chunk(const int32_t* __restrict__ ids, i
       int start = 0;
       if (b >= 0) start = wc[warp * B + b];
       __syncwarp();
+      const int place = b >= 0 ? base[b] + start + rank : -1;
+      if (inverse != nullptr && s0 + j * 32 + lane < seg_end) inverse[s0 + j * 32 + lane] = place;
       if (b >= 0) {
-        sorted[(int64_t)base[b] + start + rank] = (int32_t)(s0 + j * 32 + lane);
+        sorted[place] = (int32_t)(s0 + j * 32 + lane);
         if (lane == 31 - __clz(peers)) wc[warp * B + b] = start + __popc(peers);
       }
       __syncwarp();
@@ -210,7 +214,7 @@ __device__ __forceinline__ void fill_meta(int B, int block_size, int64_t numel, 
 __device__ __forceinline__ void align_single(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                                              int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
                                              int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
-                                             int32_t* __restrict__ zeros, int* smem) {
+                                             int32_t* __restrict__ inverse, int32_t* __restrict__ zeros, int* smem) {
   int* wc = smem;                       // [32][B]
   int* tot = wc + kAlignWarps * B;      // [B]
   int* prefix = tot + B;                // [B+1]
@@ -227,15 +231,15 @@ __device__ __forceinline__ void align_single(const int32_t* __restrict__ ids, in
   padded_prefix(B, block_size, tot, prefix, scratch);
   write_starts(B, prefix, cumsum, post_pad, zeros);
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, 0, 1);
-  scatter_chunk(ids, 0, numel, span, B, wc, prefix, sorted);
+  scatter_chunk(ids, 0, numel, span, B, wc, prefix, sorted, inverse);
 }
 __global__ void __launch_bounds__(kAlignThreads)
     moe_align_single_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                             int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
                             int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
-                            int32_t* __restrict__ zeros) {
+                            int32_t* __restrict__ inverse, int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
-  align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, pad_sorted, zeros, smem);
+  align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, pad_sorted, inverse, zeros, smem);
 }
 
 // The sort of one CTA beside the quantizer of the same layer's activations (groups of 128, 16-bit input, dense row-major
@@ -251,10 +255,11 @@ __global__ void __launch_bounds__(kAlignThreads)
     moe_align_quant_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                            int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids, int32_t* __restrict__ post_pad,
                            int32_t* __restrict__ cumsum, const T* __restrict__ x, uint8_t* __restrict__ out_q,
-                           float* __restrict__ out_s, int64_t groups, float eps, float qmax, int32_t* __restrict__ zeros) {
+                           float* __restrict__ out_s, int64_t groups, float eps, float qmax, int32_t* __restrict__ inverse,
+                           int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   if (blockIdx.x == 0) {
-    align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, true, zeros, smem);
+    align_single(ids, numel, span, B, block_size, sorted, expert_ids, post_pad, cumsum, true, inverse, zeros, smem);
     return;
   }
   ptx::grid_dependency_wait();
@@ -316,7 +321,7 @@ __global__ void __launch_bounds__(kAlignThreads)
                              const int* __restrict__ chunk_hist, const int* __restrict__ totals,
                              int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
                              int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
-                             int32_t* __restrict__ zeros) {
+                             int32_t* __restrict__ inverse, int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   int* wc = smem;                       // [32][B]
   int* tot = wc + kAlignWarps * B;      // [B]   this chunk's totals (unused after scan) / all-chunk totals
@@ -338,7 +343,7 @@ __global__ void __launch_bounds__(kAlignThreads)
   __syncthreads();
   scan_over_warps(B, wc, tot);
   __syncthreads();
-  scatter_chunk(ids, begin, end, span, B, wc, base, sorted);
+  scatter_chunk(ids, begin, end, span, B, wc, base, sorted, inverse);
 }
 
 // ---- kSingleMax < numel <= kLargeMin, one launch ------------------------------------------------
@@ -351,7 +356,7 @@ __global__ void __launch_bounds__(kAlignThreads)
     moe_align_coop_kernel(const int32_t* __restrict__ ids, int64_t numel, int span, int B, int block_size,
                           int* __restrict__ chunk_hist, int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
                           int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
-                          int32_t* __restrict__ zeros) {
+                          int32_t* __restrict__ inverse, int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   int* wc = smem;                       // [32][B]
   int* tot = wc + kAlignWarps * B;      // [B]   this chunk's totals, then the totals over all chunks
@@ -401,13 +406,13 @@ __global__ void __launch_bounds__(kAlignThreads)
   if (blockIdx.x == 0) write_starts(B, prefix, cumsum, post_pad, zeros);
   fill_meta(B, block_size, numel, prefix, tot, expert_ids, sorted, pad_sorted, blockIdx.x, gridDim.x);
   __syncthreads();
-  scatter_chunk<NBITS>(ids, begin, end, span, B, wc, base, sorted);
+  scatter_chunk<NBITS>(ids, begin, end, span, B, wc, base, sorted, inverse);
 }
 
 static bool g_align_coop_enabled = true;  // sglb200_moe_align_set_cooperative
 
 using CoopKernel = void (*)(const int32_t*, int64_t, int, int, int, int*, int32_t*, int32_t*, int32_t*, int32_t*, bool,
-                              int32_t*);
+                              int32_t*, int32_t*);
 static CoopKernel coop_kernel_for(int B) {
   switch (32 - __builtin_clz((unsigned)(B + 31))) {  // keys run up to B + 31
     case 6: return moe_align_coop_kernel<6>;
@@ -458,7 +463,7 @@ __global__ void __launch_bounds__(kTsThreads, 2)
                                   int block_size, const int* __restrict__ chunk_hist, const int* __restrict__ totals,
                                   int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
                                   int32_t* __restrict__ post_pad, int32_t* __restrict__ cumsum, bool pad_sorted,
-                                  int32_t* __restrict__ zeros) {
+                                  int32_t* __restrict__ inverse, int32_t* __restrict__ zeros) {
   extern __shared__ int smem[];
   int* wc = smem;                        // [16][B]  per-warp counts of the tile, then exclusive over warps
   int* tot_all = wc + kTsWarps * B;      // [B]      totals over all chunks
@@ -490,6 +495,7 @@ __global__ void __launch_bounds__(kTsThreads, 2)
       int b = i < end ? ids[i] + 1 : -1;
       if (b >= B) b = -1;
       key[j] = b;
+      if (inverse != nullptr && b < 0 && i < end) inverse[i] = -1;
     }
     __syncwarp();
 #pragma unroll
@@ -534,8 +540,9 @@ __global__ void __launch_bounds__(kTsThreads, 2)
     const int n = tstart[B];
     const int t_lo = (int)t0;  // numel < 2^31
     for (int p = tid; p < n; p += kTsThreads) {
-      const int e = val[p];
-      sorted[ttot[e >> 12] + p] = t_lo + (e & (kTsTile - 1));
+      const int e = val[p], place = ttot[e >> 12] + p, id = t_lo + (e & (kTsTile - 1));
+      sorted[place] = id;
+      if (inverse != nullptr) inverse[id] = place;
     }
     __syncthreads();
   }
@@ -580,7 +587,7 @@ bool align_quant_fits(const void* x, int64_t numel, int buckets) {
 template <typename T>
 static int launch_align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                               int32_t* post_pad, int32_t* cumsum, const void* x, void* out_q, float* out_s, int64_t groups,
-                              float eps, float fp8_max, int32_t* zeros, cudaStream_t st) {
+                              float eps, float fp8_max, int32_t* inverse, int32_t* zeros, cudaStream_t st) {
   int64_t chunks = 0;
   int span = 0;
   align_plan(numel, &chunks, &span);
@@ -590,18 +597,18 @@ static int launch_align_quant(const int32_t* ids, int64_t numel, int buckets, in
     SGLB_CUDA(cudaFuncSetAttribute(moe_align_quant_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmemMax));
   SGLB_CUDA(launch_pdl(moe_align_quant_kernel<T>, grid, kAlignThreads, smem, st, ids, numel, span, buckets, block_size, sorted,
                        expert_ids, post_pad, cumsum, static_cast<const T*>(x), static_cast<uint8_t*>(out_q), out_s, groups, eps,
-                       fp8_max, zeros));
+                       fp8_max, inverse, zeros));
   return SGLB200_OK;
 }
 
 int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                 int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
-                int64_t hidden, float eps, float fp8_max, int32_t* zeros, cudaStream_t st) {
+                int64_t hidden, float eps, float fp8_max, int32_t* inverse, int32_t* zeros, cudaStream_t st) {
   const int64_t groups = tokens * (hidden / 128);
   return dtype == 0 ? launch_align_quant<__nv_bfloat16>(ids, numel, buckets, block_size, sorted, expert_ids, post_pad, cumsum, x,
-                                                        out_q, out_s, groups, eps, fp8_max, zeros, st)
+                                                        out_q, out_s, groups, eps, fp8_max, inverse, zeros, st)
                     : launch_align_quant<__half>(ids, numel, buckets, block_size, sorted, expert_ids, post_pad, cumsum, x, out_q,
-                                                 out_s, groups, eps, fp8_max, zeros, st);
+                                                 out_s, groups, eps, fp8_max, inverse, zeros, st);
 }
 
 }  // namespace sglb200
@@ -625,8 +632,8 @@ extern "C" int64_t sglb200_moe_align_workspace_bytes(int64_t numel, int num_expe
 
 int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_experts, int block_size, int32_t* sorted_token_ids,
                               int32_t* expert_ids, int32_t* num_tokens_post_pad, int32_t* cumsum_buffer,
-                              int pad_sorted_token_ids, void* workspace, int64_t workspace_bytes, int32_t* zeros,
-                              cudaStream_t st) {
+                              int pad_sorted_token_ids, void* workspace, int64_t workspace_bytes, int32_t* inverse,
+                              int32_t* zeros, cudaStream_t st) {
   SGLB_REQUIRE(numel >= 0 && numel < (1ll << 31) - (int64_t)num_experts * block_size, "moe_align: numel %lld too large",
                (long long)numel);
   SGLB_REQUIRE(num_experts >= 1 && block_size >= 1, "moe_align: num_experts %d, block_size %d", num_experts, block_size);
@@ -666,7 +673,7 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
                                      (int)kAlignSmemMax));                                                          \
     moe_align_tile_scatter_kernel<NB><<<(unsigned)lchunks, kTsThreads, ts_smem, st>>>(                              \
         topk_ids, numel, chunk_len, B, block_size, hist, tot, sorted_token_ids, expert_ids, num_tokens_post_pad,    \
-        cumsum_buffer, pad_sorted_token_ids != 0, zeros);                                                           \
+        cumsum_buffer, pad_sorted_token_ids != 0, inverse, zeros);                                                  \
     break
     switch (nbits) {
       SGLB_TILE_SCATTER(6);
@@ -687,7 +694,8 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
   align_plan(numel, &chunks, &span);
   if (chunks == 1) {
     SGLB_CUDA(launch_pdl(moe_align_single_kernel, 1, kAlignThreads, smem, st, topk_ids, numel, span, B, block_size,
-                         sorted_token_ids, expert_ids, num_tokens_post_pad, cumsum_buffer, pad_sorted_token_ids != 0, zeros));
+                         sorted_token_ids, expert_ids, num_tokens_post_pad, cumsum_buffer, pad_sorted_token_ids != 0, inverse,
+                         zeros));
     return SGLB200_OK;
   }
   const int64_t need = sglb200_moe_align_workspace_bytes(numel, num_experts);
@@ -703,7 +711,7 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
     if (coop_fits(kern, chunks, smem)) {
       bool pad = pad_sorted_token_ids != 0;
       void* args[] = {&topk_ids, &numel, &span, (void*)&B, &block_size, &chunk_hist, &sorted_token_ids, &expert_ids,
-                      &num_tokens_post_pad, &cumsum_buffer, &pad, &zeros};
+                      &num_tokens_post_pad, &cumsum_buffer, &pad, &inverse, &zeros};
       SGLB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern),
                                             dim3((unsigned)chunks), dim3(kAlignThreads), args, smem, st));
       return SGLB200_OK;
@@ -715,7 +723,7 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
   moe_align_scatter_kernel<<<(unsigned)chunks, kAlignThreads, smem, st>>>(topk_ids, numel, span, B, block_size, chunk_hist,
                                                                           totals, sorted_token_ids, expert_ids,
                                                                           num_tokens_post_pad, cumsum_buffer,
-                                                                          pad_sorted_token_ids != 0, zeros);
+                                                                          pad_sorted_token_ids != 0, inverse, zeros);
   SGLB_CUDA(cudaGetLastError());
   return SGLB200_OK;
 }
@@ -726,7 +734,7 @@ extern "C" int sglb200_moe_align_block_size(const int32_t* topk_ids, int64_t num
                                             int pad_sorted_token_ids, void* workspace, int64_t workspace_bytes,
                                             void* stream) {
   return align_block_size(topk_ids, numel, num_experts, block_size, sorted_token_ids, expert_ids, num_tokens_post_pad,
-                          cumsum_buffer, pad_sorted_token_ids, workspace, workspace_bytes, nullptr,
+                          cumsum_buffer, pad_sorted_token_ids, workspace, workspace_bytes, nullptr, nullptr,
                           static_cast<cudaStream_t>(stream));
 }
 

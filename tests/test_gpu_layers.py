@@ -96,14 +96,17 @@ def test_experts_row_counts(T, E, topk, H=384, I=256):
 
 
 # the one-call layer against its steps one by one, bit for bit, where experts have more than 48 rows on average: rows that end in
-# every part of a 128-row tile, one and several groups of hidden and intermediate columns, one slot a token, more ids than one
-# CTA sorts; `ids`: some of them negative, and a weight scale that overflows one expert to infinities and NaN
+# every part of a 128-row tile, one and several groups of hidden and intermediate columns, one slot a token, ids that one CTA
+# sorts, a cooperative launch, three launches and the tile-sorted path (which all write the inverse order); odd: some ids
+# negative, and a weight scale that overflows one expert to infinities and NaN
 @pytest.mark.parametrize("T,E,topk,H,I,dtype,odd", [
     (97, 1, 1, 128, 128, torch.bfloat16, False), (150, 4, 2, 384, 256, torch.float16, False),
     (333, 4, 2, 1152, 384, torch.bfloat16, True), (700, 9, 3, 256, 640, torch.float16, True),
-    (2000, 16, 8, 512, 128, torch.bfloat16, False), (5000, 7, 2, 2048, 768, torch.bfloat16, False)])
+    (2000, 16, 8, 512, 128, torch.bfloat16, False), (5000, 7, 2, 2048, 768, torch.bfloat16, False),
+    (4100, 40, 33, 128, 128, torch.bfloat16, True), (53000, 32, 20, 128, 128, torch.float16, True)])
 def test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd):
     from sglang_b200 import ops
+    from sglang_b200._lib import lib
     from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
     g = torch.Generator(device="cuda").manual_seed(T)
     x = torch.randn(T, H, device="cuda", generator=g).to(dtype)
@@ -117,6 +120,11 @@ def test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd):
         ids[torch.rand(T, topk, device="cuda", generator=g) < 0.1] = -1
         s13[1] *= 1e38
     got = fused_experts_impl(x, w13, w2, wt, ids, use_fp8_w8a8=True, w1_scale=s13, w2_scale=s2, block_shape=[128, 128])
+    lib.sglb200_moe_align_set_cooperative(0)
+    try:
+        again = fused_experts_impl(x, w13, w2, wt, ids, use_fp8_w8a8=True, w1_scale=s13, w2_scale=s2, block_shape=[128, 128])
+    finally:
+        lib.sglb200_moe_align_set_cooperative(1)
     xq, xs = ops.per_token_group_quant_fp8(x, 128)
     order, eid, post = ops.moe_align_block_size(ids, 128, E)
     a1, a1s = ops.gather_rows_fp8(xq, xs, order, post, T * topk, topk, order.numel() // 128 * 128)
@@ -127,8 +135,10 @@ def test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd):
     want = torch.empty_like(x)
     ops.moe_sum_reduce_out(ic3.view(T, topk, H), want, 1.0)
     assert ops.gemm_status() == 0
-    assert odd == bool(want.isnan().any())
-    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(), want.nan_to_num())
+    assert odd != bool(want.isfinite().all())
+    kept = dict(nan=0.0, posinf=float("inf"), neginf=float("-inf"))
+    for out in (got, again):
+        assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.nan_to_num(**kept), want.nan_to_num(**kept))
 
 
 # more tiles of the first product than CTAs, behind the sort of up to 2048 ids and of more; experts without rows among them
