@@ -111,6 +111,7 @@ struct TileCfg {
   static constexpr int kOutGroups = BN_ / 64;
   static constexpr uint32_t kOutGroupBytes = BM * 64 * 2;
   static constexpr uint32_t kOutBytes = kForm == Form::kActivated ? BM * 128 : kOutGroups * kOutGroupBytes;
+  static constexpr int kWeightRows = kForm == Form::kGrouped ? BM : 1;
   static constexpr int kHalfRows = kForm == Form::kActivated ? BM : 1;
   static_assert(kEpiWarps % 4 == 0 && BN_ % kColGroups == 0 && kEpiCols % 32 == 0 && BN_ % 64 == 0 &&
                     kAccBufs * kAccStride <= kTmemCols && BN_ <= 256 && kStageBytes % 1024 == 0,
@@ -173,6 +174,7 @@ template <class Cfg>
 struct SharedCtl {
   alignas(16) float sc[2][2][BM][kScSlabs];  // a_s * b_s: slot, weight block of the tile (at most two), tile row, slab
   UnitDesc desc[2];
+  float row_w[2][Cfg::kWeightRows];  // grouped, rows stored in sorted order: their routing weights, a slot as the descriptor's
   uint64_t sc_full[2];     // the slot is written (every scout lane arrives)
   uint64_t sc_empty[2];    // every promotion warp has read it
   uint64_t desc_full[2];   // the descriptor is written (every scout lane arrives)
@@ -515,10 +517,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             for (int i = 0; i < live; ++i)
               ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage) + i * (32 * 128), n_tile * 128, out_row0 + 32 * i);
           } else {
+            // (with padding to skip, the map's box is a quadrant)
+            const int parts = kGrouped && p.skip_padding ? live_quadrants(p, m_tile) : 1;
 #pragma unroll
             for (int g = 0; g < kOutGroups; ++g) {
               if (n_tile * BN + g * 64 < n_end)
-                ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage) + g * kOutGroupBytes, n_tile * BN + g * 64, out_row0);
+                for (int i = 0; i < parts; ++i)
+                  ptx::tma_store_2d(cmap, ptx::smem_u32(out_stage) + g * kOutGroupBytes + i * (32 * 128), n_tile * BN + g * 64,
+                                    out_row0 + 32 * i);
             }
           }
           ptx::tma_store_commit();
@@ -559,6 +565,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (lane == 0) {
         d->m_tile = m_tile, d->n_tile = n_tile, d->expert = e, d->kb_begin = un.kb_begin;
         d->kb_stop = un.kb_stop, d->split = un.split ? 1 : 0, d->slot = un.slot, d->live = live;
+      }
+      if (kForm == Form::kGrouped && p.tma_out && p.row_weights != nullptr) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int32_t id = p.sorted_ids[(int64_t)m_tile * BM + 32 * k + lane];
+          ctl->row_w[ds][32 * k + lane] = id >= 0 && id < p.numel ? __ldg(p.row_weights + id) : 0.f;
+        }
       }
       ptx::mbar_arrive(bar_dfull0 + ds * 8);  // every lane: its own writes are released with its arrival
       if (++ds == 2u) {
@@ -793,6 +806,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const float4 h1 = ptx::lds_f32x4(desc_addr + (uint32_t)offsetof(UnitDesc, kb_stop));
         un.tile = 0, un.kb_begin = kb_begin, un.kb_stop = kb_stop;
         un.split = __float_as_int(h1.y) != 0, un.slot = __float_as_int(h1.z);
+      }
+      if constexpr (kForm == Form::kGrouped) {
+        if (p.tma_out && p.row_weights != nullptr) {
+          const float w = ptx::lds_f32(ptx::smem_u32(&ctl->row_w[ds][row_in_tile]));
+#pragma unroll
+          for (int j = 0; j < kEpiCols; ++j) acc[j] *= w;
+        }
       }
       release_desc();
       // ---- store ----
@@ -1391,7 +1411,7 @@ static int grouped_mm(const void* A, const float* a_s, const void* B, const floa
   CUtensorMap mc{};
   p.tma_out = !scatter;  // sorted-row output is contiguous; the scatter form writes token-major rows one by one
   if (p.tma_out) {
-    rc = get_out_map(C, (uint64_t)N, (uint64_t)max_rows, out_dtype, BM, &mc);
+    rc = get_out_map(C, (uint64_t)N, (uint64_t)max_rows, out_dtype, skip_padding ? 32 : BM, &mc);
     if (rc) return rc;
   }
   const int64_t tiles = ((max_rows + BM - 1) / BM) * p.tiles_n;

@@ -39,6 +39,10 @@ int quant_fp8(const void* input, int in_dtype, void* output_q, float* output_s, 
 int silu_mul_quant_fp8(const void* input, int dtype, void* output_q, float* output_s, int64_t rows, int64_t d, int group_size,
                        float eps, const int32_t* num_rows_dev, bool trigger, cudaStream_t st);
 
+// moe_misc.cu: out[t] = factor * sum over k of the row of `src` at inverse[t * topk + k], where that is not negative.
+int sum_sorted(const void* src, const int32_t* inverse, void* out, int dtype, int64_t tokens, int64_t topk, int64_t hidden,
+               float factor, cudaStream_t st);
+
 // quant.cu: the quantizer (groups of 128) of a layer's activations with every row's codes and scales written to its `topk`
 // places in the sorted order (`inverse` of the sort, -1 = nowhere), and zeros to the padding rows of 32-row quadrants that
 // hold rows; other padding is not written.
@@ -66,7 +70,8 @@ int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, 
               bool after_quantizer, cudaStream_t st);
 
 // gemm.cu: the product of sorted rows with their experts (arguments as sglb200_fp8_blockwise_grouped_mm).  `skip_padding`: the
-// rows are as the sort leaves them, every expert's padding after its rows, and nobody reads what belongs to a padding row.
+// rows are as the sort leaves them, every expert's padding after its rows, and nobody reads what belongs to a padding row;
+// without `scatter`, `row_weights` then apply to the sorted rows.
 int grouped_mm_any(const void* A, const float* a_s, const void* B, const float* b_s, void* C, const int32_t* sorted_token_ids,
                    const int32_t* expert_ids, const int32_t* num_rows_dev, const float* row_weights, int64_t max_rows,
                    int64_t numel, int num_experts, int64_t N, int64_t K, int scatter, int out_dtype, bool skip_padding,

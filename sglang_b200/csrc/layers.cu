@@ -78,7 +78,7 @@ static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int6
   if (p.tile == 0) p.inv = c.take(numel * 4), p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
   else p.ic1 = c.take(p.rows * 2 * I * 2);
   p.a2 = c.take(p.rows * I), p.a2s = c.take(p.rows * (I / 128) * 4);
-  if (!p.direct) p.ic3 = c.take(numel * Ho * 2);
+  if (!p.direct) p.ic3 = c.take((p.tile == 0 ? p.rows : numel) * Ho * 2);
   p.total = c.bytes;
   return p;
 }
@@ -152,7 +152,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
   const bool beside = align_quant_fits(x, numel, (int)E + 1), sorted_rows = p.tile == 0 && !beside;
   if (beside) {
     rc = align_quant(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), x, dtype, base + p.q, f(p.s), T,
-                     H, kQuantEps, kFp8Max, nullptr, next, st);
+                     H, kQuantEps, kFp8Max, p.tile == 0 ? i(p.inv) : nullptr, next, st);
   } else if (sorted_rows) {
     rc = align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
                           p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, i(p.inv), next, st);
@@ -187,10 +187,10 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
                         p.rows, numel, (int)E, I, H, dtype, st);
     if (rc) return rc;
     rc = grouped_mm_any(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights, p.rows, numel, (int)E,
-                        Ho, I, 1, dtype, true, st);
+                        Ho, I, p.direct, dtype, true, st);
   }
   if (rc || p.direct) return rc;
   // (the rows kernel leaves the slots of negative ids unwritten)
   if (p.tile > 0) return sglb200_moe_sum_reduce_masked(ic3, topk_ids, out, dtype, T, k, Ho, factor, stream);
-  return sglb200_moe_sum_reduce(ic3, out, dtype, T, k, Ho, factor, stream);
+  return sum_sorted(ic3, i(p.inv), out, dtype, T, k, Ho, factor, st);
 }
