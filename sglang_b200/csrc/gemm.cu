@@ -90,14 +90,20 @@ __device__ long long g_trace[2][kTraceUnits][kTraceStamps];
 // -> 550; 32768 rows, 256 experts of 7168 x 2048: 1 970 + 147 -> 1 979.  The epilogue's exponentials and reciprocals are 2 048
 // clocks a tile of the special-function units, which the next tile's first two slabs hide in part.  Four stages of operands,
 // for which there is room: 562 and 2 063.
-enum class Form { kDense, kGrouped, kActivated };
+// kOnce: a dense product whose CTAs store at most one tile each, when its last slab has been multiplied (a single wave), or none
+// (partial sums only): the staging area then lies in the operand ring, which has room for one stage more.  A slab of a single
+// wave takes 1 100 clocks, most of them the way from DRAM and L2 to shared memory (of many waves 850: other rows' CTAs have
+// brought the weights), so it is bytes in flight that count.  Us with the quantizer, ring of three stages -> four, both in turn
+// on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 256 x 7168 x 16384 55.4 -> 53.0, 100 x 4096 x 7168 23.1 -> 21.2, 512 x 7168 x
+// 16384 86.3 -> 82.1; below 32 slabs the ring is filled too few times: 7168 x 2048 with 65 to 512 rows 10.2-15.2 -> 0.1 more.
+enum class Form { kDense, kGrouped, kActivated, kOnce };
 
 // Tile width BN: 256 columns with two TMEM accumulator buffers, or 128 columns with four (more tiles for the same
 // problem: where one wave of wide tiles would leave SMs idle).
 template <int BN_, Form kForm = Form::kDense>
 struct TileCfg {
   static constexpr int BN = BN_;
-  static constexpr int kStages = BN_ >= 256 ? 3 : 5;
+  static constexpr int kStages = (BN_ >= 256 ? 3 : 5) + (kForm == Form::kOnce ? 1 : 0);
   // registers per thread after the split: promotion warps / the others.  The block is launched with 168 x 384 threads:
   // 256 * kPromoRegs + 128 * kOtherRegs <= 64512.
   static constexpr int kPromoRegs = BN_ >= 256 ? 224 : 200;
@@ -111,6 +117,8 @@ struct TileCfg {
   static constexpr int kOutGroups = BN_ / 64;
   static constexpr uint32_t kOutGroupBytes = BM * 64 * 2;
   static constexpr uint32_t kOutBytes = kForm == Form::kActivated ? BM * 128 : kOutGroups * kOutGroupBytes;
+  static constexpr uint32_t kOutOffset = kForm == Form::kOnce ? 0 : kStages * kStageBytes;  // of the staging area, from the ring
+  static constexpr uint32_t kTileArea = kForm == Form::kOnce ? kStages * kStageBytes : kOutOffset + kOutBytes;
   static constexpr int kWeightRows = kForm == Form::kGrouped ? BM : 1;
   static constexpr int kHalfRows = kForm == Form::kActivated ? BM : 1;
   static_assert(kEpiWarps % 4 == 0 && BN_ % kColGroups == 0 && kEpiCols % 32 == 0 && BN_ % 64 == 0 &&
@@ -312,17 +320,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     fp8_blockscale_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_a32,
                                const GemmParams p) {
-  constexpr bool kGrouped = kForm != Form::kDense, kAct = kForm == Form::kActivated;
+  constexpr bool kGrouped = kForm == Form::kGrouped || kForm == Form::kActivated, kAct = kForm == Form::kActivated;
   static_assert(!kAct || BN_ == 256, "a tile of 128 gate and 128 up columns");
   using Cfg = TileCfg<BN_, kForm>;
   constexpr int BN = Cfg::BN, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs, kAccStride = Cfg::kAccStride,
                 kEpiCols = Cfg::kEpiCols, kOutGroups = Cfg::kOutGroups;
-  constexpr uint32_t kStageBytes = Cfg::kStageBytes, kOutGroupBytes = Cfg::kOutGroupBytes, kOutBytes = Cfg::kOutBytes;
+  constexpr uint32_t kStageBytes = Cfg::kStageBytes, kOutGroupBytes = Cfg::kOutGroupBytes;
   extern __shared__ uint8_t smem_raw[];
   // tiles need 1024-byte alignment for the 128-byte swizzle
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* out_stage = tiles + kStages * kStageBytes;
-  SharedCtl<Cfg>* ctl = reinterpret_cast<SharedCtl<Cfg>*>(out_stage + kOutBytes);
+  uint8_t* out_stage = tiles + Cfg::kOutOffset;
+  SharedCtl<Cfg>* ctl = reinterpret_cast<SharedCtl<Cfg>*>(tiles + Cfg::kTileArea);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &ctl->abort_flag;
 
@@ -1278,7 +1286,7 @@ uint32_t g_gemm_wait_probes = ptx::kProbeLimit;
 
 template <class Cfg>
 static size_t gemm_smem_bytes() {
-  return (size_t)Cfg::kStages * Cfg::kStageBytes + Cfg::kOutBytes + sizeof(SharedCtl<Cfg>) + 1024;
+  return (size_t)Cfg::kTileArea + sizeof(SharedCtl<Cfg>) + 1024;
 }
 
 template <Form kForm, int BN>
@@ -1344,7 +1352,9 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
     rc = get_out_map(C, (uint64_t)N, (uint64_t)M, out_dtype, BM, &mc);
     if (rc) return rc;
   }
-  rc = launch_gemm<Form::kDense, BN>(ma, mb, mc, ma, p, pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits, st);
+  const int64_t units = pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits;
+  const bool once = p.kb_total >= 32 && (!p.tma_out || units <= sm_count());
+  rc = once ? launch_gemm<Form::kOnce, BN>(ma, mb, mc, ma, p, units, st) : launch_gemm<Form::kDense, BN>(ma, mb, mc, ma, p, units, st);
   if (rc != SGLB200_OK || pl.scratch_blocks() == 0) return rc;
   const int tiles_m = (int)((M + BM - 1) / BM);
   const unsigned ygrid = (unsigned)((BM * BN / 8 + 255) / 256);
