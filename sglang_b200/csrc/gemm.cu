@@ -211,6 +211,27 @@ __device__ __forceinline__ int live_quadrants(const GemmParams& p, int m_tile) {
   return 1 + (a < p.numel) + (b < p.numel) + (c < p.numel);
 }
 
+// Where a unit lies, and what its tile's rows are: looked up a unit ahead by the roles that must not stall between two tiles.
+// The ids stay as they came from memory until the tile is begun, so that nothing waits for them before.
+struct TileInfo {
+  int m_tile, n_tile, expert, id1, id2, id3;
+  // Leading 32-row quadrants that hold rows.  An expert's rows come first and its padding last, and a tile has a row.
+  __device__ __forceinline__ int live(const GemmParams& p) const { return 1 + (id1 < p.numel) + (id2 < p.numel) + (id3 < p.numel); }
+};
+template <bool kGrouped>
+__device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int tile, int tiles_m, int tiles_n) {
+  TileInfo x{0, 0, 0, 0, 0, 0};
+  tile_coord(tile, tiles_m, tiles_n, p.group_m, x.m_tile, x.n_tile);
+  if (kGrouped) {
+    x.expert = ptx::ldg_here_s32(p.expert_ids + x.m_tile);
+    if (p.skip_padding) {
+      const int32_t* id = p.sorted_ids + (int64_t)x.m_tile * BM;
+      x.id1 = ptx::ldg_here_s32(id + 32), x.id2 = ptx::ldg_here_s32(id + 64), x.id3 = ptx::ldg_here_s32(id + 96);
+    }
+  }
+  return x;
+}
+
 // A unit of work = one output tile x one K range.  Dense problems number their units: the tiles
 // [0, full_units) whole, then `splits` consecutive units per remaining tile.
 struct Unit {
@@ -383,7 +404,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-  const bool vec_scales = p.as_stride_k == 1 && (p.as_stride_m & 3) == 0 &&
+  const int64_t as_stride_k = kGrouped ? 1 : p.as_stride_k;  // (experts: dense rows)
+  const bool vec_scales = as_stride_k == 1 && ((kGrouped ? kb_total : p.as_stride_m) & 3) == 0 &&
                           (reinterpret_cast<uintptr_t>(p.a_s) & 15u) == 0;
   // activation scales of slabs kb .. kb+3 of the row `a_row` points at (zero past the last slab)
   auto load_a4_row = [&](const float* a_row, int kb) {
@@ -391,10 +413,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (vec_scales && kb + 3 < kb_total && (kb & 3) == 0) {
       v = __ldg(reinterpret_cast<const float4*>(a_row + kb));
     } else {
-      if (kb + 0 < kb_total) v.x = __ldg(a_row + (int64_t)(kb + 0) * p.as_stride_k);
-      if (kb + 1 < kb_total) v.y = __ldg(a_row + (int64_t)(kb + 1) * p.as_stride_k);
-      if (kb + 2 < kb_total) v.z = __ldg(a_row + (int64_t)(kb + 2) * p.as_stride_k);
-      if (kb + 3 < kb_total) v.w = __ldg(a_row + (int64_t)(kb + 3) * p.as_stride_k);
+      if (kb + 0 < kb_total) v.x = __ldg(a_row + (int64_t)(kb + 0) * as_stride_k);
+      if (kb + 1 < kb_total) v.y = __ldg(a_row + (int64_t)(kb + 1) * as_stride_k);
+      if (kb + 2 < kb_total) v.z = __ldg(a_row + (int64_t)(kb + 2) * as_stride_k);
+      if (kb + 3 < kb_total) v.w = __ldg(a_row + (int64_t)(kb + 3) * as_stride_k);
     }
     return v;
   };
@@ -407,18 +429,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const uint32_t tiles0 = ptx::smem_u32(tiles);
       uint32_t s = 0, ph = 0;
       bool alive = true;
+      // With experts the next tile is looked up behind the first loads of this one: between two tiles the ring would otherwise
+      // run dry for a round trip to L2.  (Dense tiles, whose coordinates are two divisions: 4096 x 32768 x 512 113.6 -> 115.9.)
+      TileInfo next{};
+      auto look_ahead = [&](int u) {
+        if (kGrouped && u < num_units) next = tile_info<kGrouped>(p, u, tiles_m, tiles_n);
+      };
+      look_ahead(blockIdx.x);
       for (int u = blockIdx.x; u < num_units && alive; u += gridDim.x) {
         const Unit un = decode_unit<kGrouped>(p, u);
-        const int t = un.tile, kb_begin = un.kb_begin, kb_stop = un.kb_stop;
+        const int kb_begin = un.kb_begin, kb_stop = un.kb_stop;
         if (kb_begin >= kb_stop) continue;  // (an empty piece of a stream-K run)
-        int m_tile, n_tile;
-        tile_coord(t, tiles_m, tiles_n, p.group_m, m_tile, n_tile);
-        int e = 0, live = 4;
-        if (kGrouped) {
-          e = p.expert_ids[m_tile];
-          if (p.skip_padding) live = live_quadrants(p, m_tile);
-          if (e < 0) continue;
+        const TileInfo at = kGrouped ? next : tile_info<kGrouped>(p, un.tile, tiles_m, tiles_n);
+        const int m_tile = at.m_tile, n_tile = at.n_tile, e = at.expert;
+        if (e < 0) {
+          look_ahead(u + gridDim.x);
+          continue;
         }
+        int live = 4;
+        if (kGrouped && p.skip_padding) live = at.live(p);
         // this thread shares its scheduler with promotion warps that always have work: every instruction it
         // spends per slab delays the loads, so the loop keeps only 32-bit counters that step
         const int row_a = m_tile * BM, row_b = n_tile * (kAct ? BN / 2 : BN), row_up = kAct ? (int)(p.N / 2) + row_b : 0;
@@ -436,6 +465,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
           ptx::tma_load_3d(dst_a + kTileBytesA, &map_b, bar, k0, row_b, e);
           if (kAct) ptx::tma_load_3d(dst_a + kTileBytesA + Cfg::kTileBytesB / 2, &map_b, bar, k0, row_up, e);
+          if (kGrouped && k0 == 0) look_ahead(u + gridDim.x);
           if (++s == (uint32_t)kStages) {
             s = 0;
             ph ^= 1u;
@@ -456,15 +486,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const uint32_t bar_tfull0 = ptx::smem_u32(&ctl->tmem_full[0]), bar_tempty0 = ptx::smem_u32(&ctl->tmem_empty[0]);
       uint32_t s = 0, ph = 0, aph = 0;  // aph: phase of every accumulator buffer, one bit each
       bool alive = true;
+      // (whether a tile has an expert is asked a unit ahead: the answer is a round trip to L2)
+      auto expert_of = [&](int u) -> int {
+        if (!kGrouped || u >= num_units) return 0;
+        int m_tile, n_tile;
+        tile_coord(u, tiles_m, tiles_n, p.group_m, m_tile, n_tile);
+        return ptx::ldg_here_s32(p.expert_ids + m_tile);
+      };
+      int e_next = expert_of(blockIdx.x);
       for (int u = blockIdx.x; u < num_units && alive; u += gridDim.x) {
         const Unit un = decode_unit<kGrouped>(p, u);
-        const int t = un.tile, kb_begin = un.kb_begin, kb_stop = un.kb_stop;
-        if (kb_begin >= kb_stop) continue;
-        if (kGrouped) {
-          int m_tile, n_tile;
-          tile_coord(t, tiles_m, tiles_n, p.group_m, m_tile, n_tile);
-          if (p.expert_ids[m_tile] < 0) continue;
-        }
+        const int kb_begin = un.kb_begin, kb_stop = un.kb_stop, e = e_next;
+        e_next = expert_of(u + gridDim.x);
+        if (kb_begin >= kb_stop || e < 0) continue;
         uint32_t buf = 0;  // (every unit starts with buffer 0, as the promotion does)
         for (int kb = kb_begin; kb < kb_stop; ++kb) {
           // (the buffer last: it is what the MMAs wait for, and a wait that finds its barrier ready takes 80 clocks too)
@@ -556,6 +590,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t bar_sfull0 = ptx::smem_u32(&ctl->sc_full[0]), bar_sempty0 = ptx::smem_u32(&ctl->sc_empty[0]);
     uint32_t ds = 0, dph = 0, ss = 0, sph = 0;
     bool alive = true;
+    // With experts a tile's ids are asked for a tile ahead, and the scales of its rows all at once: looked up one after the
+    // other, its expert, its rows' ids, their weights and two halves of the scales, twice, took as long as a tile of six slabs,
+    // and the promotion warps waited 2 500 to 3 600 of 9 000 clocks a tile for them (dense: 410 in all before the first slab;
+    // so 750).  Second product of 131072 rows through 128 experts of 2048 x 768: 393 -> 334 us, layer 1 219 -> 1 148.
+    constexpr int kRowsAhead = kForm == Form::kGrouped ? 4 : 2;  // (the others have no registers left for four)
+    const bool sorted_weights = kForm == Form::kGrouped && p.tma_out && p.row_weights != nullptr;
+    TileInfo next{};
+    int next_id[4] = {0, 0, 0, 0};
+    auto look_ahead = [&](int u) {
+      if (!kGrouped || u >= num_units) return;
+      next = tile_info<kGrouped>(p, u, tiles_m, tiles_n);
+      if (sorted_weights) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) next_id[k] = ptx::ldg_here_s32(p.sorted_ids + (int64_t)next.m_tile * BM + 32 * k + lane);
+      }
+    };
+    look_ahead(blockIdx.x);
     for (int u = blockIdx.x; u < num_units && alive; u += gridDim.x) {
       if (!SGLB_WAIT(bar_dempty0 + ds * 8, dph ^ 1u)) {
         *abort_flag = 1;
@@ -565,23 +616,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       UnitDesc* d = &ctl->desc[ds];
       int m_tile = 0, n_tile = 0, e = 0, live = 4;
       const bool work = un.kb_begin < un.kb_stop;
-      if (work) {
+      if (kGrouped) {
+        m_tile = next.m_tile, n_tile = next.n_tile, e = next.expert;
+        if (p.skip_padding) live = next.live(p);
+      } else if (work) {
         tile_coord(un.tile, tiles_m, tiles_n, p.group_m, m_tile, n_tile);
-        if (kGrouped) e = p.expert_ids[m_tile];
-        if (kGrouped && p.skip_padding) live = live_quadrants(p, m_tile);
       }
       if (lane == 0) {
         d->m_tile = m_tile, d->n_tile = n_tile, d->expert = e, d->kb_begin = un.kb_begin;
         d->kb_stop = un.kb_stop, d->split = un.split ? 1 : 0, d->slot = un.slot, d->live = live;
       }
-      if (kForm == Form::kGrouped && p.tma_out && p.row_weights != nullptr) {
+      float row_w[4];  // (stored with the tile's first scales, which the promotion warps wait for as well)
+      float* row_w_at = &ctl->row_w[ds][0];
+      if (sorted_weights) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int32_t id = p.sorted_ids[(int64_t)m_tile * BM + 32 * k + lane];
-          ctl->row_w[ds][32 * k + lane] = id >= 0 && id < p.numel ? __ldg(p.row_weights + id) : 0.f;
-        }
+        for (int k = 0; k < 4; ++k)
+          row_w[k] = next_id[k] >= 0 && next_id[k] < p.numel ? ptx::ldg_here_f32(p.row_weights + next_id[k]) : 0.f;
       }
       ptx::mbar_arrive(bar_dfull0 + ds * 8);  // every lane: its own writes are released with its arrival
+      look_ahead(u + gridDim.x);
       if (++ds == 2u) {
         ds = 0;
         dph ^= 1u;
@@ -592,34 +645,38 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const float* b_row0 = p.b_s + ((int64_t)e * p.nb_total + nb_tile) * kb_total;
       const float* b_row1 = p.b_s + ((int64_t)e * p.nb_total + nb_next) * kb_total;
       for (int kb = un.kb_begin; kb < un.kb_stop; kb += kScSlabs) {
-        float b0[kScSlabs], b1[kScSlabs];
-#pragma unroll
-        for (int j = 0; j < kScSlabs; ++j) {
-          b0[j] = kb + j < kb_total ? __ldg(b_row0 + kb + j) : 0.f;
-          b1[j] = BN > kScaleBlockN && kb + j < kb_total ? __ldg(b_row1 + kb + j) : 0.f;
-        }
+        // (lanes 0-3: the scales of the tile's first weight block, lanes 4-7: of the second)
+        float bv = 0.f;
+        if (lane < (BN > kScaleBlockN ? 2 : 1) * kScSlabs && kb + (lane & 3) < kb_total)
+          bv = __ldg((lane < kScSlabs ? b_row0 : b_row1) + kb + (lane & 3));
         const uint32_t sc_addr = ptx::smem_u32(&ctl->sc[ss][0][lane][0]);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {  // (two rows at a time: registers)
-          float4 av[2];
+        for (int half = 0; half < 4 / kRowsAhead; ++half) {
+          float4 av[kRowsAhead];
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int row = m_tile * BM + lane + 32 * (2 * half + k);  // rows past M read a valid row; never stored
-            av[k] = load_a4_row(p.a_s + min(row, (int)rows - 1) * p.as_stride_m, kb);
+          for (int k = 0; k < kRowsAhead; ++k) {
+            const int row = m_tile * BM + lane + 32 * (kRowsAhead * half + k);  // rows past M read a valid row; never stored
+            av[k] = load_a4_row(kGrouped ? p.a_s + (uint64_t)(uint32_t)row * (uint32_t)kb_total
+                                         : p.a_s + min(row, (int)rows - 1) * p.as_stride_m, kb);
           }
           if (half == 0 && !SGLB_WAIT(bar_sempty0 + ss * 8, sph ^ 1u)) {
             *abort_flag = 1;
             alive = false;
             break;
           }
+          if (half == 0 && kb == 0 && sorted_weights) {
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const uint32_t at = sc_addr + (2 * half + k) * (32 * 16);
-            ptx::sts_128(at, make_uint4(__float_as_uint(av[k].x * b0[0]), __float_as_uint(av[k].y * b0[1]),
-                                        __float_as_uint(av[k].z * b0[2]), __float_as_uint(av[k].w * b0[3])));
-            if (BN > kScaleBlockN)
-              ptx::sts_128(at + BM * 16, make_uint4(__float_as_uint(av[k].x * b1[0]), __float_as_uint(av[k].y * b1[1]),
-                                                    __float_as_uint(av[k].z * b1[2]), __float_as_uint(av[k].w * b1[3])));
+            for (int k = 0; k < 4; ++k) row_w_at[32 * k + lane] = row_w[k];
+          }
+#pragma unroll
+          for (int w = 0; w < (BN > kScaleBlockN ? 2 : 1); ++w) {
+            const float b0 = __shfl_sync(0xffffffffu, bv, 4 * w), b1 = __shfl_sync(0xffffffffu, bv, 4 * w + 1),
+                        b2 = __shfl_sync(0xffffffffu, bv, 4 * w + 2), b3 = __shfl_sync(0xffffffffu, bv, 4 * w + 3);
+#pragma unroll
+            for (int k = 0; k < kRowsAhead; ++k)
+              ptx::sts_128(sc_addr + w * (BM * 16) + (kRowsAhead * half + k) * (32 * 16),
+                           make_uint4(__float_as_uint(av[k].x * b0), __float_as_uint(av[k].y * b1), __float_as_uint(av[k].z * b2),
+                                      __float_as_uint(av[k].w * b3)));
           }
         }
         if (!alive) break;
@@ -816,7 +873,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         un.split = __float_as_int(h1.y) != 0, un.slot = __float_as_int(h1.z);
       }
       if constexpr (kForm == Form::kGrouped) {
-        if (p.tma_out && p.row_weights != nullptr) {
+        if (e >= 0 && p.tma_out && p.row_weights != nullptr) {  // (rows of no expert stay zero, and have no weights there)
           const float w = ptx::lds_f32(ptx::smem_u32(&ctl->row_w[ds][row_in_tile]));
 #pragma unroll
           for (int j = 0; j < kEpiCols; ++j) acc[j] *= w;

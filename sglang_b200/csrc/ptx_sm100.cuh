@@ -136,6 +136,19 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
   return v;
 }
 
+// A load that stays where it is written: asked for early, its value is used much later.
+__device__ __forceinline__ int ldg_here_s32(const int32_t* at) {
+  int v;
+  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(at));
+  return v;
+}
+
+__device__ __forceinline__ float ldg_here_f32(const float* at) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(at));
+  return v;
+}
+
 __device__ __forceinline__ float4 lds_f32x4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
