@@ -1334,9 +1334,13 @@ static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
 }
 
 // Few activation rows take the kernel with the weights on the M side (gemm_rows.cu): up to 64 rows its tiles follow the
-// rows there are, beyond that this kernel's 128-row tiles are at least half full.
-static bool use_rows(int64_t M) {
-  return M <= 64;
+// rows there are, beyond that this kernel's 128-row tiles are at least half full.  Up to 256 rows it also takes problems of at most
+// 32 tiles of 64 rows x 128 columns, of which it puts two on an SM and splits K over up to sixteen CTAs each; the weights that
+// every 64 rows fetch anew come from L2.  Us of the layer, both ways: 128 rows, 512 x 7168 9.6 against 21.2, 1024 x 4096 9.5 / 14.3,
+// 2048 x 1024 7.7 / 8.0; 256 rows, 512 x 2048 7.9 / 9.5, 1024 x 7168 12.8 / 20.7.  Not beyond: 128 rows, 3072 x 2048 10.8 / 10.3.
+static bool use_rows(int64_t M, int64_t N, int64_t K) {
+  const int64_t tiles = ((M + 63) / 64) * ((N + 127) / 128);
+  return M <= 64 || (M <= 256 && tiles <= (K <= 8192 ? 32 : 8));
 }
 
 uint32_t g_gemm_wait_probes = ptx::kProbeLimit;
@@ -1537,7 +1541,7 @@ extern "C" int sglb200_gemm_status(void) {
 extern "C" void sglb200_gemm_set_wait_probes(uint32_t probes) { g_gemm_wait_probes = probes == 0 ? ptx::kProbeLimit : probes; }
 
 extern "C" int64_t sglb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0 || use_rows(M)) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || use_rows(M, N, K)) return 0;
   return plan_dense(M, N, K).scratch_bytes();
 }
 
@@ -1562,7 +1566,7 @@ int sglb200::scaled_mm(const void* A, const void* B, const float* a_s, const flo
   SGLB_REQUIRE(aligned16(A) && aligned16(B) && aligned16(C) && (bias == nullptr || aligned16(bias)),
                "fp8_blockwise_scaled_mm: A, B, C and bias must be 16-byte aligned");
   SGLB_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "fp8_blockwise_scaled_mm: dimension too large");
-  if (use_rows(M))
+  if (use_rows(M, N, K))
     return rows_dense_mm(A, B, a_s, b_s, C, bias, M, N, K, as_stride_m, as_stride_k, out_dtype, after_quantizer, st);
   const DensePlan dp = plan_dense(M, N, K);
   if (dp.bn == 128)

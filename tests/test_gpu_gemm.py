@@ -49,6 +49,14 @@ def test_dense_gemm_one_tile_a_cta(ops, M, N, K, dtype):
     assert_close_fp(got, ref)
 
 
+# up to 256 rows in tiles of 64: one row in the last, the most tiles that there are, one column block too many for it
+@pytest.mark.parametrize("M,N,K,dtype", [
+    (65, 512, 1024, torch.bfloat16), (256, 1024, 2048, torch.float16), (193, 1032, 1536, torch.bfloat16), (129, 1416, 640, torch.bfloat16)])
+def test_dense_gemm_few_tiles(ops, M, N, K, dtype):
+    got, ref = _dense_case(ops, M, N, K, seed=M + N + K, out_dtype=dtype)
+    assert_close_fp(got, ref)
+
+
 def test_dense_gemm_many_tiles_and_fp16(ops):
     got, ref = _dense_case(ops, 1000, 4096, 2048, seed=11)
     assert_close_fp(got, ref)
