@@ -88,4 +88,22 @@ inline int small_splits(int64_t tiles, int kb, int most_slabs, const ClusterFits
   return best;
 }
 
+// The same for the 128-row kernel, one CTA an SM, on `tiles` tiles of 128 x 128: 1, or two, three, four, six or eight CTAs (what
+// five and seven would have to exchange does not fit beside their operands).  Counted in slabs (0.25 us): the exchange is six and one
+// for every 32 rows of a tile, and one for every 48 CTAs of the grid, which share DRAM and L2.  Measured over all of them, us of the
+// layer: 128 x 4096 x 7168 one 20.6, two 16.1, three 15.4, four 14.2; 128 x 1536 x 16384 four 17.4, six 16.9, eight 15.0; 80 x 2048 x
+// 7168 four 12.0, six 11.5; 80 x 4096 x 2048 one 10.4, two 9.8, four 9.7; 128 x 4096 x 2048 one 10.6, two 10.5, four 10.9; 128 x 7168 x
+// 2048 one 10.9, two 11.1; 192 x 4096 x 1024 one 8.6, two 9.7; 128 x 9216 x 4096 one 15.1, two 15.1.
+inline int tile_splits(int64_t tiles, int kb, int64_t rows, const ClusterFits& fits) {
+  const int exchange = 6 + (int)((rows < 128 ? rows + 31 : 128) / 32);
+  int best = 1;
+  int64_t best_cost = kb;
+  for (int s = 2; s <= 8; ++s) {
+    if (s == 5 || s == 7 || s > kb || tiles > fits.alone[s]) continue;
+    const int64_t cost = (kb + s - 1) / s + exchange + tiles * s / 48;
+    if (cost < best_cost) best = s, best_cost = cost;
+  }
+  return best;
+}
+
 }  // namespace sglb200

@@ -96,14 +96,23 @@ __device__ long long g_trace[2][kTraceUnits][kTraceStamps];
 // brought the weights), so it is bytes in flight that count.  Us with the quantizer, ring of three stages -> four, both in turn
 // on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 256 x 7168 x 16384 55.4 -> 53.0, 100 x 4096 x 7168 23.1 -> 21.2, 512 x 7168 x
 // 16384 86.3 -> 82.1; below 32 slabs the ring is filled too few times: 7168 x 2048 with 65 to 512 rows 10.2-15.2 -> 0.1 more.
-enum class Form { kDense, kGrouped, kActivated, kOnce };
+// kSplit: a dense product of few 128-wide tiles and a long K, whose slabs are split over the CTAs of a cluster (`tile_splits`); their
+// partial sums meet in distributed shared memory (written once, added once) instead of in global memory and a second launch.
+// Beside the ring of five stages lies room for what the other CTAs send; sums fetched from the others' memory after a barrier,
+// and then a second one before anybody may leave: 0.7 us more.  What is left of the exchange is about 1.6 us (pushing 0.7 to 1.1,
+// barrier 0.6 to 1.0, sum 1.0 to 1.4, against 1.1 for a tile that leaves through TMA).  Us of the layer, before (split-K partial
+// sums in global memory, or one CTA a tile) and so: 128 x 4096 x 7168 20.6 -> 14.2, 128 x 2112 x 7168 20.8 -> 13.7, 80 x 3072 x
+// 4096 14.1 -> 10.5, 256 x 4096 x 7168 21.8 -> 16.5, 128 x 7168 x 16384 36.1 -> 31.5, 1024 x 1024 x 4096 16.2 -> 14.2.
+// 256-wide tiles lost up to 4 us on the exchange of twice the sums.
+enum class Form { kDense, kGrouped, kActivated, kOnce, kSplit };
 
 // Tile width BN: 256 columns with two TMEM accumulator buffers, or 128 columns with four (more tiles for the same
 // problem: where one wave of wide tiles would leave SMs idle).
 template <int BN_, Form kForm = Form::kDense>
 struct TileCfg {
   static constexpr int BN = BN_;
-  static constexpr int kStages = (BN_ >= 256 ? 3 : 5) + (kForm == Form::kOnce ? 1 : 0);
+  static constexpr bool kInRing = kForm == Form::kOnce;  // the staging area
+  static constexpr int kStages = (BN_ >= 256 ? 3 : 5) + (kInRing ? 1 : 0);
   // registers per thread after the split: promotion warps / the others.  The block is launched with 168 x 384 threads:
   // 256 * kPromoRegs + 128 * kOtherRegs <= 64512.
   static constexpr int kPromoRegs = BN_ >= 256 ? 224 : 200;
@@ -116,9 +125,12 @@ struct TileCfg {
   // output staging for the TMA store: per 64 columns a [128 rows][64 columns] 2-byte tile in the 128-byte swizzle
   static constexpr int kOutGroups = BN_ / 64;
   static constexpr uint32_t kOutGroupBytes = BM * 64 * 2;
-  static constexpr uint32_t kOutBytes = kForm == Form::kActivated ? BM * 128 : kOutGroups * kOutGroupBytes;
-  static constexpr uint32_t kOutOffset = kForm == Form::kOnce ? 0 : kStages * kStageBytes;  // of the staging area, from the ring
-  static constexpr uint32_t kTileArea = kForm == Form::kOnce ? kStages * kStageBytes : kOutOffset + kOutBytes;
+  static constexpr uint32_t kOutBytes = kForm == Form::kActivated ? BM * 128
+                                        : kForm == Form::kSplit   ? 60 * 1024
+                                                                  : kOutGroups * kOutGroupBytes;
+  static constexpr uint32_t kOutOffset = kInRing ? 0 : kStages * kStageBytes;  // of the staging area, from the ring
+  static constexpr uint32_t kTileArea = kInRing ? kStages * kStageBytes : kOutOffset + kOutBytes;
+  static constexpr int kScBlocks = BN_ > kScaleBlockN ? 2 : 1;
   static constexpr int kWeightRows = kForm == Form::kGrouped ? BM : 1;
   static constexpr int kHalfRows = kForm == Form::kActivated ? BM : 1;
   static_assert(kEpiWarps % 4 == 0 && BN_ % kColGroups == 0 && kEpiCols % 32 == 0 && BN_ % 64 == 0 &&
@@ -180,7 +192,7 @@ constexpr int kScSlabs = 4;  // slabs per slot of the scale ring: one 16-byte re
 
 template <class Cfg>
 struct SharedCtl {
-  alignas(16) float sc[2][2][BM][kScSlabs];  // a_s * b_s: slot, weight block of the tile (at most two), tile row, slab
+  alignas(16) float sc[2][Cfg::kScBlocks][BM][kScSlabs];  // a_s * b_s: slot, weight block of the tile, tile row, slab
   UnitDesc desc[2];
   float row_w[2][Cfg::kWeightRows];  // grouped, rows stored in sorted order: their routing weights, a slot as the descriptor's
   uint64_t sc_full[2];     // the slot is written (every scout lane arrives)
@@ -239,10 +251,17 @@ struct Unit {
   int slot;  // split units: which [BM][BN] float32 block of the partial-sum scratch
   bool split;
 };
-template <bool kGrouped>
+template <Form kForm>
 __device__ __forceinline__ Unit decode_unit(const GemmParams& p, int u) {
+  constexpr bool kGrouped = kForm == Form::kGrouped || kForm == Form::kActivated;
   Unit x;
   x.slot = 0;
+  if constexpr (kForm == Form::kSplit) {  // CTA `rank` of a cluster of p.splits: that part of the tile's slabs
+    x.tile = u / p.splits, x.split = true;
+    const int rank = u - x.tile * p.splits;
+    x.kb_begin = rank * p.kb_total / p.splits, x.kb_stop = (rank + 1) * p.kb_total / p.splits;
+    return x;
+  }
   if (!kGrouped && p.sk_share > 0) {
     // unit u = piece u / sk_ctas of the run of CTA u % sk_ctas
     const int piece = u / p.sk_ctas, c = u - piece * p.sk_ctas;
@@ -336,6 +355,65 @@ __device__ __forceinline__ bool activate_row(const GemmParams& p, const float (&
   return true;
 }
 
+// A tile whose K range the CTAs of a cluster have split.  CTA r owns `cluster_groups` groups of eight columns from the
+// r-th on; every CTA writes the partial sums of the others' columns straight into their shared memory (of its own into the
+// ring, which has been consumed), and after one barrier of the cluster each adds what it owns.  A source's sums lie as
+// [owned group of eight][columns 0-3, 4-7][row][4] of float32.
+template <int BN>
+__host__ __device__ constexpr int cluster_groups(int splits) { return (BN / 8 + splits - 1) / splits; }
+constexpr uint32_t kClusterGroupBytes = 2 * BM * 16;
+
+// The owned columns: the sources' sums in ascending K order, bias, one rounding.  A warp takes 2 x 8 rows of 32 columns at a time.
+template <int BN>
+__device__ __forceinline__ void cluster_sum(const GemmParams& p, int rank, int m_tile, int n_tile, uint32_t own, uint32_t recv,
+                                            int warp, int lane) {
+  const int rows = (int)min((int64_t)BM, p.M - (int64_t)m_tile * BM), groups = cluster_groups<BN>(p.splits);
+  const int first = rank * groups, stop = min(first + groups, BN / 8), splits = p.splits;
+  const int row = warp * 8 + (lane & 7);  // and 64 further on
+  const uint32_t bytes = groups * kClusterGroupBytes;
+  int c8 = first + (lane >> 3), col = n_tile * BN + c8 * 8;
+  uint32_t at = (uint32_t)(lane >> 3) * kClusterGroupBytes + row * 16;
+  uint16_t* out = static_cast<uint16_t*>(p.C) + ((int64_t)m_tile * BM + row) * p.N + col;
+  const uint16_t* bias = static_cast<const uint16_t*>(p.bias);
+  for (; c8 < stop && col < p.N && row < rows; c8 += 4, col += 32, at += 4 * kClusterGroupBytes, out += 32) {  // (N: a multiple of 8)
+    float a[2][8];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[k][j] = 0.f;
+    uint32_t from = recv + at;
+    for (int s = 0; s < splits; ++s) {
+      const uint32_t src = s == rank ? own + at : from;
+      if (s != rank) from += bytes;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float4 v = ptx::lds_f32x4(src + k * (64 * 16)), w = ptx::lds_f32x4(src + k * (64 * 16) + BM * 16);
+        a[k][0] += v.x, a[k][1] += v.y, a[k][2] += v.z, a[k][3] += v.w;
+        a[k][4] += w.x, a[k][5] += w.y, a[k][6] += w.z, a[k][7] += w.w;
+      }
+    }
+    if (bias != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint16_t raw16 = __ldg(bias + col + j);
+        const float b = p.out_fp16 ? __half2float(__ushort_as_half(raw16)) : __bfloat162float(__ushort_as_bfloat16(raw16));
+        a[0][j] += b, a[1][j] += b;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      uint32_t word[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __half2 h = __floats2half2_rn(a[k][2 * j], a[k][2 * j + 1]);
+        const __nv_bfloat162 b = __floats2bfloat162_rn(a[k][2 * j], a[k][2 * j + 1]);
+        word[j] = p.out_fp16 ? *reinterpret_cast<const uint32_t*>(&h) : *reinterpret_cast<const uint32_t*>(&b);
+      }
+      if (row + 64 * k < rows) *reinterpret_cast<uint4*>(out + (int64_t)(64 * k) * p.N) = make_uint4(word[0], word[1], word[2], word[3]);
+    }
+  }
+}
+
 template <Form kForm, int BN_>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     fp8_blockscale_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -343,6 +421,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                                const GemmParams p) {
   constexpr bool kGrouped = kForm == Form::kGrouped || kForm == Form::kActivated, kAct = kForm == Form::kActivated;
   static_assert(!kAct || BN_ == 256, "a tile of 128 gate and 128 up columns");
+  static_assert(kForm != Form::kSplit || BN_ == 128, "partial sums beside the ring");
   using Cfg = TileCfg<BN_, kForm>;
   constexpr int BN = Cfg::BN, kStages = Cfg::kStages, kAccBufs = Cfg::kAccBufs, kAccStride = Cfg::kAccStride,
                 kEpiCols = Cfg::kEpiCols, kOutGroups = Cfg::kOutGroups;
@@ -355,6 +434,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &ctl->abort_flag;
 
+  if constexpr (kForm == Form::kSplit) ptx::cluster_arrive();  // (a CTA's memory may be written once it runs)
   // (the reduction kernel that follows a split launch is launched programmatically: letting it be scheduled now
   // hides its launch latency; it waits for this grid to complete before it reads a partial sum)
   ptx::launch_dependents();
@@ -397,12 +477,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int tiles_n = p.tiles_n;
   const int num_tiles = tiles_m * tiles_n;
   const int kb_total = p.kb_total;
-  const int num_units = kGrouped         ? num_tiles
+  const int num_units = kForm == Form::kSplit ? num_tiles * p.splits
+                        : kGrouped       ? num_tiles
                         : p.sk_share > 0 ? p.sk_pieces * p.sk_ctas
                                          : p.full_units + (num_tiles - p.full_units) * p.splits;
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
+  if constexpr (kForm == Form::kSplit) ptx::cluster_wait();
   const uint32_t tmem_base = ctl->tmem_base;
   const int64_t as_stride_k = kGrouped ? 1 : p.as_stride_k;  // (experts: dense rows)
   const bool vec_scales = as_stride_k == 1 && ((kGrouped ? kb_total : p.as_stride_m) & 3) == 0 &&
@@ -437,7 +519,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       };
       look_ahead(blockIdx.x);
       for (int u = blockIdx.x; u < num_units && alive; u += gridDim.x) {
-        const Unit un = decode_unit<kGrouped>(p, u);
+        const Unit un = decode_unit<kForm>(p, u);
         const int kb_begin = un.kb_begin, kb_stop = un.kb_stop;
         if (kb_begin >= kb_stop) continue;  // (an empty piece of a stream-K run)
         const TileInfo at = kGrouped ? next : tile_info<kGrouped>(p, un.tile, tiles_m, tiles_n);
@@ -495,7 +577,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       };
       int e_next = expert_of(blockIdx.x);
       for (int u = blockIdx.x; u < num_units && alive; u += gridDim.x) {
-        const Unit un = decode_unit<kGrouped>(p, u);
+        const Unit un = decode_unit<kForm>(p, u);
         const int kb_begin = un.kb_begin, kb_stop = un.kb_stop, e = e_next;
         e_next = expert_of(u + gridDim.x);
         if (kb_begin >= kb_stop || e < 0) continue;
@@ -536,7 +618,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const uint32_t bar_out_full = ptx::smem_u32(&ctl->out_full), bar_out_free = ptx::smem_u32(&ctl->out_free);
       uint32_t oph = 0;
       for (int u = blockIdx.x; u < num_units; u += gridDim.x) {
-        const Unit un = decode_unit<kGrouped>(p, u);
+        const Unit un = decode_unit<kForm>(p, u);
         if (un.kb_begin >= un.kb_stop || un.split) continue;
         if (!SGLB_WAIT(bar_out_full, oph)) {
           *abort_flag = 1;
@@ -612,7 +694,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         *abort_flag = 1;
         break;
       }
-      const Unit un = decode_unit<kGrouped>(p, u);
+      const Unit un = decode_unit<kForm>(p, u);
       UnitDesc* d = &ctl->desc[ds];
       int m_tile = 0, n_tile = 0, e = 0, live = 4;
       const bool work = un.kb_begin < un.kb_stop;
@@ -783,12 +865,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // block; columns wholly past N take the last block's.
         static_assert(kScaleBlockN % kEpiCols == 0 && kAccBufs <= 4 && 4 % kAccBufs == 0, "one weight block per warp");
         const bool second = !kAct && BN > kScaleBlockN && n0 / kScaleBlockN != n_tile * BN / kScaleBlockN && n0 / kScaleBlockN < p.nb_total;
-        const uint32_t sc_addr0 = ptx::smem_u32(&ctl->sc[0][second ? 1 : 0][row_in_tile][0]);
+        const uint32_t sc_addr0 = ptx::smem_u32(&ctl->sc[0][0][row_in_tile][0]) + (second ? BM * 16 : 0);
         float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f), s4_up = s4;
         auto fetch_scales = [&]() -> bool {
           if (!SGLB_WAIT(bar_sfull0 + ss * 8, sph)) return false;
-          s4 = ptx::lds_f32x4(sc_addr0 + ss * (2 * BM * 16));
-          if (kAct) s4_up = ptx::lds_f32x4(sc_addr0 + ss * (2 * BM * 16) + BM * 16);
+          s4 = ptx::lds_f32x4(sc_addr0 + ss * (Cfg::kScBlocks * BM * 16));
+          if (kAct) s4_up = ptx::lds_f32x4(sc_addr0 + ss * (Cfg::kScBlocks * BM * 16) + BM * 16);
           return true;
         };
         int left = kb_stop - kb_begin;  // slabs from the current group of four on
@@ -885,7 +967,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (un.split) {
         // this unit's float32 partial sums, tile-local layout; a second kernel adds the units of a tile in a
         // fixed order, adds the bias and rounds once
-        if (row < rows) {  // (rows past M are never read back)
+        if (kForm == Form::kSplit) {
+          if (row < rows) {
+            const int rank = (int)blockIdx.x % p.splits, groups = cluster_groups<BN>(p.splits), c0 = cgrp * (kEpiCols / 8);
+            int owner = c0 / groups, idx = c0 - owner * groups;
+            const uint32_t own = ptx::smem_u32(tiles) + row_in_tile * 16, bytes = groups * kClusterGroupBytes;
+            const uint32_t before = ptx::smem_u32(out_stage) + row_in_tile * 16 + (rank - 1) * bytes, after = before + bytes;
+#pragma unroll
+            for (int j = 0; j < kEpiCols / 8; ++j) {
+              const float* a = acc + 8 * j;
+              // (to CTAs of lower rank this one is source rank - 1 of the others')
+              const uint32_t to = ptx::cluster_map((owner == rank ? own : owner < rank ? before : after) + idx * kClusterGroupBytes, owner);
+              ptx::sts_cluster_f32x4(to, a[0], a[1], a[2], a[3]);
+              ptx::sts_cluster_f32x4(to + BM * 16, a[4], a[5], a[6], a[7]);
+              if (++idx == groups) idx = 0, ++owner;
+            }
+          }
+        } else if (row < rows) {  // (rows past M are never read back)
           // [column / 4][row][4]: the 32 lanes of a warp (32 consecutive rows) write 512 contiguous bytes per store.
           float* dst = p.partial + (int64_t)un.slot * (BM * BN) + ((int64_t)(cgrp * kEpiCols / 4) * BM + row_in_tile) * 4;
 #pragma unroll
@@ -1017,6 +1115,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
         }
       }
+    }
+  }
+
+  // ------------------------------ sum over the CTAs of the cluster ------------------------------
+  if constexpr (kForm == Form::kSplit) {
+    __syncwarp();
+    ptx::cluster_sync();  // (nobody touches another CTA's memory after it)
+    if (warp >= kEpiWarp0 && ctl->abort_flag == 0) {
+      const int tile = blockIdx.x / p.splits;
+      int m_tile, n_tile;
+      tile_coord(tile, tiles_m, tiles_n, p.group_m, m_tile, n_tile);
+      cluster_sum<BN>(p, (int)blockIdx.x - tile * p.splits, m_tile, n_tile, ptx::smem_u32(tiles), ptx::smem_u32(out_stage),
+                      warp - kEpiWarp0, lane);
     }
   }
 
@@ -1323,12 +1434,14 @@ static int choose_bn_grouped(int64_t numel) {
 // How a dense problem runs: tile width and the cut into units.
 struct DensePlan {
   int bn;
+  int cluster;  // CTAs of a cluster over which every tile's slabs are split (`units` then does not count), or 1
   UnitPlan units;
-  int64_t scratch_bytes() const { return units.scratch_blocks() * (int64_t)BM * bn * (int64_t)sizeof(float); }
+  int64_t scratch_bytes() const { return cluster > 1 ? 0 : units.scratch_blocks() * (int64_t)BM * bn * (int64_t)sizeof(float); }
 };
 static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
   DensePlan d;
-  d.bn = choose_bn(M, N, K);
+  d.cluster = tile_splits(((M + BM - 1) / BM) * ((N + 127) / 128), (int)((K + BK - 1) / BK), M, cluster_fits());
+  d.bn = d.cluster > 1 ? 128 : choose_bn(M, N, K);
   d.units = plan_units(M, N, K, d.bn, sm_count());
   return d;
 }
@@ -1336,8 +1449,10 @@ static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
 // Few activation rows take the kernel with the weights on the M side (gemm_rows.cu): up to 64 rows its tiles follow the
 // rows there are, beyond that this kernel's 128-row tiles are at least half full.  Up to 256 rows it also takes problems of at most
 // 32 tiles of 64 rows x 128 columns, of which it puts two on an SM and splits K over up to sixteen CTAs each; the weights that
-// every 64 rows fetch anew come from L2.  Us of the layer, both ways: 128 rows, 512 x 7168 9.6 against 21.2, 1024 x 4096 9.5 / 14.3,
-// 2048 x 1024 7.7 / 8.0; 256 rows, 512 x 2048 7.9 / 9.5, 1024 x 7168 12.8 / 20.7.  Not beyond: 128 rows, 3072 x 2048 10.8 / 10.3.
+// every 64 rows fetch anew come from L2.  Us of the layer, both ways: 128 rows, 512 x 7168 9.6 against 21.2 (11.3 with the K of
+// 128-row tiles split over clusters), 1024 x 4096 9.5 / 14.3 (10.5), 2048 x 1024 7.7 / 8.0 (9.1); 256 rows, 512 x 2048 7.9 / 9.5
+// (9.3), 1024 x 7168 12.8 / 20.7 (12.7).  Not beyond: 128 rows, 3072 x 2048 10.8 / 10.3; 192 rows, 2048 x 7168 15.2 (13.8).  With
+// a long K the clusters of 128-row tiles fetch less: 128 rows, 1024 x 16384 15.8 (14.7), 512 x 16384 12.8 (13.5).
 static bool use_rows(int64_t M, int64_t N, int64_t K) {
   const int64_t tiles = ((M + 63) / 64) * ((N + 127) / 128);
   return M <= 64 || (M <= 256 && tiles <= (K <= 8192 ? 32 : 8));
@@ -1367,10 +1482,17 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   const unsigned grid = (unsigned)(max_units < sms ? max_units : sms);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1), cfg.blockDim = dim3(kGemmThreads, 1, 1), cfg.dynamicSmemBytes = smem, cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
+  if constexpr (kForm == Form::kSplit) {  // (max_units: CTAs, as many as clusters have room at once)
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.splits, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.gridDim.x = (unsigned)max_units, cfg.numAttrs = 2;
+    SGLB_CUDA(cudaLaunchKernelEx(&cfg, fp8_blockscale_gemm_kernel<kForm, BN>, ma, mb, mc, ma32, p));
+    return SGLB200_OK;
+  }
   // A single wave is launched programmatically.  With their quantizer, both ways in turn on one GPU: 100 x 4096 x 4096 15.1 ->
   // 14.4 us, 512 x 4096 x 4096 16.9 -> 16.1, 200 x 8192 x 1024 9.7 -> 9.0; 257 x 10240 x 8192 40.4 -> 39.6, which is less than
   // GPUs and runs differ by.  With several waves the CTAs, which then start wherever an SM falls free, no longer share L2 as
@@ -1399,8 +1521,14 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
   p.group_m = choose_group_m(M, K, BM);
   p.out_fp16 = out_dtype;
   p.wait_probes = g_gemm_wait_probes;
-  UnitPlan pl = dp.units;
   const int64_t tiles = ((M + BM - 1) / BM) * p.tiles_n;
+  if constexpr (BN == 128) {
+    if (dp.cluster > 1) {
+      p.splits = dp.cluster;
+      return launch_gemm<Form::kSplit, BN>(ma, mb, ma, ma, p, tiles * dp.cluster, st);
+    }
+  }
+  UnitPlan pl = dp.units;
   if (pl.scratch_blocks() > 0 &&
       (workspace == nullptr || !aligned16(workspace) || workspace_bytes < dp.scratch_bytes()))
     pl = UnitPlan{(int)tiles, 1, p.kb_total, 0, 0, 0, 2};  // no scratch offered: one unit per tile

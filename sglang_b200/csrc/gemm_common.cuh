@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda.h>
 
+#include "cluster_rule.h"
 #include "common.cuh"
 
 namespace sglb200 {
@@ -62,6 +63,9 @@ bool align_quant_fits(const void* x, int64_t numel, int buckets);
 int align_quant(const int32_t* ids, int64_t numel, int buckets, int block_size, int32_t* sorted, int32_t* expert_ids,
                 int32_t* post_pad, int32_t* cumsum, const void* x, int dtype, void* out_q, float* out_s, int64_t tokens,
                 int64_t hidden, float eps, float fp8_max, int32_t* inverse, int32_t* zeros, cudaStream_t st);
+
+// What the current GPU holds of clusters (the driver is asked once per device).
+const ClusterFits& cluster_fits();
 
 // gemm.cu: the dense product (arguments as sglb200_fp8_blockwise_scaled_mm).  `after_quantizer`: the kernel before it in
 // the stream is this library's quantizer, launched by the same call, so that the weights may be fetched while that runs.

@@ -27,9 +27,6 @@ __device__ __forceinline__ int frag_column(int j) { return (j & ~15) + ((j & 7) 
 // with 256 columns there is room for one other of either kind, without one for three of 128.  The 128-row kernel, which takes
 // all columns, leaves no registers for another CTA.
 
-// What the current GPU holds of clusters (the driver is asked once per device).
-const ClusterFits& cluster_fits();
-
 struct RowsParams {
   const float* a_s;
   const float* b_s;

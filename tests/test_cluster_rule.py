@@ -14,6 +14,7 @@ extern "C" void fits(const int64_t* one, const int64_t* two, int64_t sms, Cluste
 }
 extern "C" int rows(int64_t tiles, int kb, int m, const ClusterFits* f) { return rows_splits(tiles, kb, m, *f); }
 extern "C" int one_launch(int64_t tiles, int kb, int most, const ClusterFits* f) { return small_splits(tiles, kb, most, *f); }
+extern "C" int tile(int64_t tiles, int kb, int m, const ClusterFits* f) { return tile_splits(tiles, kb, m, *f); }
 """
 ROW = ctypes.c_int64 * 17
 # clusters of 0, 1, .. 16 CTAs that a B200 holds, as its driver says: one CTA on an SM, two on an SM
@@ -34,7 +35,7 @@ def rule(tmp_path_factory):
     (d / "shim.cpp").write_text(SHIM)
     subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", CSRC, "-o", str(d / "shim.so"), str(d / "shim.cpp")])
     lib = ctypes.CDLL(str(d / "shim.so"))
-    lib.rows.argtypes = lib.one_launch.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.POINTER(Fits)]
+    lib.rows.argtypes = lib.one_launch.argtypes = lib.tile.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.POINTER(Fits)]
 
     def fits(gpu):
         f = Fits()
@@ -80,3 +81,18 @@ def test_a_size_that_the_driver_refuses_is_never_taken(rule, gpu):
                                              (25, 78, 20, 5), (30, 64, 30, 8), (12, 127, 17, 8)])
 def test_large_clusters_that_share_sms_have_to_gain_too(rule, tiles, kb, m, want):
     assert rule.rows(tiles, kb, m, rule.of(B200)) == want
+
+
+def test_tiles_of_128_rows_are_split_where_that_was_faster(rule):
+    """Clusters that run at once, of sizes whose exchange fits beside the operands; short K and many tiles stay whole."""
+    for gpu in (B200, PORTABLE, SILENT):
+        f = rule.of(gpu)
+        for tiles in TILES:
+            for kb in SLABS:
+                s = rule.tile(tiles, kb, 128, f)
+                assert s in (1, 2, 3, 4, 6, 8) and s <= kb and (s == 1 or tiles <= f.alone[s]), (tiles, kb, s)
+                if kb <= 12 or tiles > 74:
+                    assert s == 1
+    f = rule.of(B200)
+    measured = {(32, 56, 128): 4, (12, 128, 128): 8, (16, 56, 80): 6, (32, 16, 80): 4, (32, 16, 128): 1, (56, 16, 128): 1, (64, 56, 256): 2}
+    assert {k: rule.tile(*k, f) for k in measured} == measured

@@ -49,8 +49,11 @@ def test_dense_gemm_one_tile_a_cta(ops, M, N, K, dtype):
     assert_close_fp(got, ref)
 
 
-# up to 256 rows in tiles of 64: one row in the last, the most tiles that there are, one column block too many for it
+# slabs of 128-row tiles split over clusters of six, three, four, eight and two CTAs (uneven shares, part of a tile's rows and
+# columns), and up to 256 rows in tiles of 64 (one row in the last, most tiles that there are, one column block too many for it)
 @pytest.mark.parametrize("M,N,K,dtype", [
+    (65, 2056, 4096, torch.bfloat16), (129, 2568, 2944, torch.float16), (300, 1032, 8192, torch.bfloat16),
+    (128, 1536, 16384, torch.bfloat16), (511, 2048, 4992, torch.float16),
     (65, 512, 1024, torch.bfloat16), (256, 1024, 2048, torch.float16), (193, 1032, 1536, torch.bfloat16), (129, 1416, 640, torch.bfloat16)])
 def test_dense_gemm_few_tiles(ops, M, N, K, dtype):
     got, ref = _dense_case(ops, M, N, K, seed=M + N + K, out_dtype=dtype)
