@@ -95,7 +95,8 @@ __device__ long long g_trace[2][kTraceUnits][kTraceStamps];
 // wave takes 1 100 clocks, most of them the way from DRAM and L2 to shared memory (of many waves 850: other rows' CTAs have
 // brought the weights), so it is bytes in flight that count.  Us with the quantizer, ring of three stages -> four, both in turn
 // on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 256 x 7168 x 16384 55.4 -> 53.0, 100 x 4096 x 7168 23.1 -> 21.2, 512 x 7168 x
-// 16384 86.3 -> 82.1; below 32 slabs the ring is filled too few times: 7168 x 2048 with 65 to 512 rows 10.2-15.2 -> 0.1 more.
+// 16384 86.3 -> 82.1.  Shorter K pays with the early weights below, from 12 slabs and 32 CTAs on: 128 x 24576 x 1536 14.5 -> 14.1,
+// 128 x 9216 x 2048 11.4 -> 11.1; 128 x 3072 x 2048 (24 CTAs) 10.3 -> 10.5, 128 x 4096 x 512 7.1 -> 7.3.
 // kSplit: a dense product of few 128-wide tiles and a long K, whose slabs are split over the CTAs of a cluster (`tile_splits`); their
 // partial sums meet in distributed shared memory (written once, added once) instead of in global memory and a second launch.
 // Beside the ring of five stages lies room for what the other CTAs send; sums fetched from the others' memory after a barrier,
@@ -176,6 +177,7 @@ struct GemmParams {
   int sk_ctas;
   int sk_pieces;                 // 2 or 3
   int sk_total;                  // tiles * kb_total
+  int early_weights;             // the weights may be read before the predecessor in the stream has finished (kOnce, kSplit)
   uint32_t wait_probes;          // probes after which a pipeline wait gives up
   int skip_padding;              // grouped: nobody reads the rows of a 32-row quadrant that is all padding (sorted_ids >= numel)
   float* act_s;                  // activated form: C holds codes [row][N / 2], this their scales [row][N / 256]
@@ -420,6 +422,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_a32,
                                const GemmParams p) {
   constexpr bool kGrouped = kForm == Form::kGrouped || kForm == Form::kActivated, kAct = kForm == Form::kActivated;
+  constexpr bool kEarly = kForm == Form::kOnce || kForm == Form::kSplit;  // (a CTA's first unit is known before the wait)
   static_assert(!kAct || BN_ == 256, "a tile of 128 gate and 128 up columns");
   static_assert(kForm != Form::kSplit || BN_ == 128, "partial sums beside the ring");
   using Cfg = TileCfg<BN_, kForm>;
@@ -460,6 +463,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     ptx::mbar_fence_init();
     ptx::tma_prefetch_desc(&map_a);
     ptx::tma_prefetch_desc(&map_b);
+    if constexpr (kEarly) {
+      // The weights of the first slabs, while the quantizer before this kernel (which triggers behind its own wait, so that all
+      // before it is complete) still makes the activations: 100 to 300 ns, 256 x 7168 x 2048 with it 11.16 -> 10.80 us.
+      if (p.early_weights) {
+        const Unit un = decode_unit<kForm>(p, blockIdx.x);
+        int m_tile, n_tile;
+        tile_coord(un.tile, (int)((p.M + BM - 1) / BM), p.tiles_n, p.group_m, m_tile, n_tile);
+        for (int s = 0; s < min(kStages, un.kb_stop - un.kb_begin); ++s) {
+          const uint32_t bar = ptx::smem_u32(&ctl->full[s]);
+          ptx::mbar_arrive_expect_tx(bar, kStageBytes);
+          ptx::tma_load_3d(ptx::smem_u32(tiles) + s * kStageBytes + kTileBytesA, &map_b, bar, (un.kb_begin + s) * BK, n_tile * BN, 0);
+        }
+      }
+    }
   }
   if (warp == 1) {
     ptx::tmem_alloc(ptx::smem_u32(&ctl->tmem_base), kTmemCols);
@@ -510,6 +527,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const uint32_t bar_empty0 = ptx::smem_u32(&ctl->empty[0]), bar_full0 = ptx::smem_u32(&ctl->full[0]);
       const uint32_t tiles0 = ptx::smem_u32(tiles);
       uint32_t s = 0, ph = 0;
+      int ahead = kEarly && p.early_weights ? kStages : 0;  // slabs of the first unit whose weights are on their way
       bool alive = true;
       // With experts the next tile is looked up behind the first loads of this one: between two tiles the ring would otherwise
       // run dry for a round trip to L2.  (Dense tiles, whose coordinates are two divisions: 4096 x 32768 x 512 113.6 -> 115.9.)
@@ -536,7 +554,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         for (int k0 = kb_begin * BK; k0 < kb_stop * BK; k0 += BK) {
           if (!SGLB_WAIT(bar_empty0 + s * 8, ph ^ 1u)) { *abort_flag = 1; alive = false; break; }
           const uint32_t bar = bar_full0 + s * 8;
-          ptx::mbar_arrive_expect_tx(bar, kStageBytes);
+          const bool fetched = kEarly && ahead > 0;
+          if (!fetched) ptx::mbar_arrive_expect_tx(bar, kStageBytes);
           const uint32_t dst_a = tiles0 + s * kStageBytes;
           if (!kGrouped || live == 4) {
             ptx::tma_load_2d(dst_a, &map_a, bar, k0, row_a);
@@ -545,7 +564,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             for (int i = 0; i < 4; ++i)
               ptx::tma_load_2d(dst_a + i * (kTileBytesA / 4), &map_a32, bar, k0, i < live ? row_a + 32 * i : (int)p.M);
           }
-          ptx::tma_load_3d(dst_a + kTileBytesA, &map_b, bar, k0, row_b, e);
+          if (!fetched) ptx::tma_load_3d(dst_a + kTileBytesA, &map_b, bar, k0, row_b, e);
+          if (kEarly) --ahead;
           if (kAct) ptx::tma_load_3d(dst_a + kTileBytesA + Cfg::kTileBytesB / 2, &map_b, bar, k0, row_up, e);
           if (kGrouped && k0 == 0) look_ahead(u + gridDim.x);
           if (++s == (uint32_t)kStages) {
@@ -553,6 +573,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             ph ^= 1u;
           }
         }
+        ahead = 0;
       }
     }
   } else if (warp == 1) {
@@ -1505,7 +1526,7 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
 template <int BN>
 static int dense_mm(const DensePlan& dp, const void* A, const void* B, const float* a_s, const float* b_s, void* C,
                     const void* bias, int64_t M, int64_t N, int64_t K, int64_t as_stride_m, int64_t as_stride_k,
-                    int out_dtype, void* workspace, int64_t workspace_bytes, cudaStream_t st) {
+                    int out_dtype, void* workspace, int64_t workspace_bytes, bool after_quantizer, cudaStream_t st) {
   CUtensorMap ma, mb;
   int rc = get_tensor_map(A, (uint64_t)K, (uint64_t)M, 1, BM, 2, &ma);
   if (rc) return rc;
@@ -1521,6 +1542,7 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
   p.group_m = choose_group_m(M, K, BM);
   p.out_fp16 = out_dtype;
   p.wait_probes = g_gemm_wait_probes;
+  p.early_weights = after_quantizer ? 1 : 0;
   const int64_t tiles = ((M + BM - 1) / BM) * p.tiles_n;
   if constexpr (BN == 128) {
     if (dp.cluster > 1) {
@@ -1542,7 +1564,7 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
     if (rc) return rc;
   }
   const int64_t units = pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits;
-  const bool once = p.kb_total >= 32 && (!p.tma_out || units <= sm_count());
+  const bool once = p.kb_total >= (units >= 32 ? 12 : 32) && (!p.tma_out || units <= sm_count());
   rc = once ? launch_gemm<Form::kOnce, BN>(ma, mb, mc, ma, p, units, st) : launch_gemm<Form::kDense, BN>(ma, mb, mc, ma, p, units, st);
   if (rc != SGLB200_OK || pl.scratch_blocks() == 0) return rc;
   const int tiles_m = (int)((M + BM - 1) / BM);
@@ -1699,9 +1721,9 @@ int sglb200::scaled_mm(const void* A, const void* B, const float* a_s, const flo
   const DensePlan dp = plan_dense(M, N, K);
   if (dp.bn == 128)
     return dense_mm<128>(dp, A, B, a_s, b_s, C, bias, M, N, K, as_stride_m, as_stride_k, out_dtype, workspace,
-                         workspace_bytes, st);
+                         workspace_bytes, after_quantizer, st);
   return dense_mm<256>(dp, A, B, a_s, b_s, C, bias, M, N, K, as_stride_m, as_stride_k, out_dtype, workspace,
-                       workspace_bytes, st);
+                       workspace_bytes, after_quantizer, st);
 }
 
 extern "C" int sglb200_fp8_blockwise_grouped_mm(const void* A, const float* a_s, const void* B, const float* b_s,

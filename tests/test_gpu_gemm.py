@@ -60,6 +60,27 @@ def test_dense_gemm_few_tiles(ops, M, N, K, dtype):
     assert_close_fp(got, ref)
 
 
+# as a layer calls them, behind the quantizer and with a bias: the same bits as the two steps one by one (the weights of the first
+# slabs are fetched while the quantizer runs)
+@pytest.mark.parametrize("M,N,K,dtype", [
+    (300, 1032, 8192, torch.bfloat16), (65, 4104, 2048, torch.float16), (80, 512, 2048, torch.bfloat16), (257, 10240, 1536, torch.float16),
+    (200, 16384, 4096, torch.bfloat16), (620, 3832, 12800, torch.bfloat16), (300, 520, 512, torch.bfloat16)])
+def test_linear_equals_its_steps(ops, M, N, K, dtype):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+    w = (torch.randn(N, K, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    ws = torch.rand(-(-N // 128), K // 128, device="cuda", generator=g) * 1e-3
+    bias = torch.randn(N, device="cuda", generator=g).to(dtype)
+    xq, xs = ops.per_token_group_quant_fp8(x, 128)
+    want = ops.w8a8_block_fp8_matmul(xq, w, xs, ws, [128, 128], dtype, bias=bias)
+    got = [ops.host.linear(x, w, ws, bias) for _ in range(3)]
+    assert ops.gemm_status() == 0 and all(torch.equal(out, want) for out in got)
+    exact = (xq.double() * xs.double().repeat_interleave(128, 1)) @ (w.double() * ws.double().repeat_interleave(128, 0)[:N]
+                                                                     .repeat_interleave(128, 1)).T + bias.double()
+    eps = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11  # one rounding; float32 sums are far below it
+    assert ((want.double() - exact).norm() / exact.norm()).item() < eps
+
+
 def test_dense_gemm_many_tiles_and_fp16(ops):
     got, ref = _dense_case(ops, 1000, 4096, 2048, seed=11)
     assert_close_fp(got, ref)
