@@ -37,6 +37,7 @@ struct RowsParams {
   int kb_total, nb_total, tiles_n;
   int tiles_m;                     // dense
   int splits;                      // CTAs of a cluster, each with its part of K (1 = no cluster)
+  uint32_t per_row;                // one-launch linear: g / M = g * per_row >> 16 for the groups of a CTA (g < 128, M <= 16)
   int early_weights;               // the weights may be read before the predecessor in the stream has finished
   int out_fp16;
   int group_m;                     // token tiles of a group sweep over the weight tiles together

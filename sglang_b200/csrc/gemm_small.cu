@@ -4,8 +4,7 @@
 //   C[m,n] = out_t( sum_kb a_s[m,kb] * b_s[n/128,kb] * sum_{k in kb} q(x)[m,k] * B[n,k] ) (+ bias)
 //
 // A decoded token through a 2112 x 7168 layer is 2.3 us of HBM time.  As quantizer + GEMM it took 8.5 us: two launches, a
-// round trip of the codes through L2, a ring with per-slab hand-offs; in one launch 6.7 us, called or from a graph (6.2 with
-// the weights in L2, 7.1 with 15 MB of others per call), so the GPU and not the host is what it waits for.  The CTAs of a
+// round trip of the codes through L2, a ring with per-slab hand-offs; in one launch 5.7 us.  The CTAs of a
 // cluster share K and each holds its few slabs whole: one thread requests all of its weight tiles as soon as the kernel
 // before is complete (0.1 to 0.5 us later than at the start of the launch, which is not safe: that kernel may have
 // written them; asking for them towards L2 at the start gained nothing), meanwhile the other warps quantise the CTA's part
@@ -104,17 +103,20 @@ __global__ void __launch_bounds__(kSmallThreads, 2)
   } else {
     // ------------------------------ quantise this CTA's activations ------------------------------
     // Four lanes per (row, slab) group, eight groups per warp and step, rows fastest (their swizzled places differ in
-    // banks).
-    const int l = lane & 3, total = kSmallRows * slabs;
+    // banks).  Rows past M are neither read nor written: what lies there is multiplied into columns that nobody reads.  With all
+    // sixteen quantised, one row and more than four slabs took two steps, one round trip to memory after the other: 1 x 2112 x
+    // 7168 6.70 us, so 5.66; 8 x 2112 x 7168 7.27 -> 6.48; up to four slabs and sixteen rows alike.  (Asking for the second step's
+    // activations before the first is quantised: 16 x 2112 x 7168 7.8 -> 8.2.)
+    const int l = lane & 3, total = (int)p.M * slabs;
     const float* b_row = p.b_s + (int64_t)n_tile * p.kb_total + kb_begin;
     ptx::grid_dependency_wait();
-    for (int g0 = warp * 8; g0 < total; g0 += kSmallWarps * 8) {  // (uniform over the warp: total is a multiple of 8)
-      const int g = g0 + (lane >> 2), slab = g / kSmallRows, row = g % kSmallRows;
-      const bool on = row < p.M;
-      const T* src = x + (int64_t)(on ? row : 0) * K + (kb_begin + slab) * kRowsBK + l * 8;
+    for (int g0 = warp * 8; g0 < total; g0 += kSmallWarps * 8) {  // (uniform over the warp)
+      const int g = min(g0 + (lane >> 2), total - 1);  // (lanes past the last group do as the last)
+      const int slab = (int)((uint32_t)g * p.per_row >> 16), row = g - slab * (int)p.M;
+      const T* src = x + (int64_t)row * K + (kb_begin + slab) * kRowsBK + l * 8;
       uint4 raw[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) raw[j] = on ? ld_nc_16(src + j * 32) : make_uint4(0, 0, 0, 0);
+      for (int j = 0; j < 4; ++j) raw[j] = ld_nc_16(src + j * 32);
       const float bs = __ldg(b_row + slab);
       float v[32];
 #pragma unroll
@@ -242,6 +244,7 @@ int small_linear(const void* x, int dtype, const void* B, const float* b_s, void
   p.b_s = b_s, p.C = C, p.bias = bias, p.M = M, p.N = N;
   p.kb_total = (int)(K / kRowsBK), p.nb_total = (int)((N + 127) / 128), p.tiles_n = p.nb_total;
   p.splits = pl.splits, p.out_fp16 = dtype;
+  p.per_row = (uint32_t)((65536 + M - 1) / M);
   p.wait_probes = g_gemm_wait_probes;
   return dtype == 0 ? launch_small<__nv_bfloat16>(mw, x, K, pl, p, st) : launch_small<__half>(mw, x, K, pl, p, st);
 }
