@@ -5,7 +5,10 @@
 // each took three times as long), after which only the winner's lane looks for its next best.  The softmax gate keeps
 // expert e in lane e % 32 (coalesced loads, sums in a fixed order); the fused gate gives every lane consecutive experts,
 // so that a group's two largest scores come from the lanes' registers and a few shuffles instead of a serial walk
-// through shared memory (64 x 256 scores: 12.7 us with the walk).
+// through shared memory (64 x 256 scores: 12.7 us with the walk).  The picks stay in registers, their weights in shared memory,
+// and both leave in one store each: written pick by pick and read back for the normalisation, with the scores loaded four bytes
+// at a time and a division an expert for its group, the fused gate took 5.3 us for one row of 256 experts (4.0 so), 6.0 for 64
+// (4.6), 15.1 for 4096 (12.0); the softmax gate, which is short of issue slots (16384 x 128 14.1 us), hardly changed.
 #include <cfloat>
 
 #include "common.cuh"
@@ -34,49 +37,53 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Picks the k best of sel[] (kPerLane registers per lane, the expert of register j being index(j), ascending in j);
-// reports the matching entries of wgt[] in pick order through lane 0.  `out_w` / `out_i` are this row's k output slots.
-template <int kPerLane, class Index>
-__device__ __forceinline__ float pick_topk(float (&sel)[kPerLane], const float (&wgt)[kPerLane], Index index, int lane, int k,
-                                           float* out_w, int32_t* out_i) {
-  float sum = 0.f;
-  // this lane's best entry: value (never a NaN), expert (INT_MAX: nothing above -inf left), weight, register
-  float best, best_w;
-  int best_e, best_j;
+// Picks the k best of sel[] (kPerLane registers per lane, the expert of register j being index(j), ascending in j) and writes their
+// ids to out_i and what finish(weight(expert), sum of the k weights) gives to out_w, lane p the p-th pick of every 32; `weight` is
+// asked by that lane alone.  A pick keeps the winner's expert in a register of lane p; weights and ids leave once, together.
+template <int kPerLane, class Index, class Weight, class Finish>
+__device__ __forceinline__ float pick_topk(float (&sel)[kPerLane], Index index, Weight weight, int lane, int k, float* out_w,
+                                           int32_t* out_i, Finish finish) {
+  float best;  // this lane's best entry: value (never a NaN) and register (-1: nothing above -inf left)
+  int best_j;
   auto look = [&]() {
-    best = kNegInf, best_w = 0.f, best_e = INT_MAX, best_j = -1;
+    best = kNegInf, best_j = -1;
 #pragma unroll
-    for (int j = 0; j < kPerLane; ++j) {
-      if (sel[j] > best) {  // ascending j = ascending expert within the lane: the first hit keeps the lower index
-        best = sel[j];
-        best_w = wgt[j];
-        best_e = index(j);
-        best_j = j;
-      }
-    }
+    for (int j = 0; j < kPerLane; ++j)
+      if (sel[j] > best) best = sel[j], best_j = j;  // ascending j = ascending expert within the lane: the first hit keeps the lower index
   };
   look();
-  // fewer candidates than k: every remaining value is -inf, and expert 0 with its weight is reported again
-  const float w_of_0 = __shfl_sync(0xffffffffu, wgt[0], 0);
-  for (int pick = 0; pick < k; ++pick) {
-    const uint32_t key = ordered_bits(best), top = __reduce_max_sync(0xffffffffu, key);
-    const int e = __reduce_min_sync(0xffffffffu, key == top ? best_e : INT_MAX);
-    float w = w_of_0;
-    if (e != INT_MAX) {
-      const bool mine = best_e == e;
-      w = __shfl_sync(0xffffffffu, best_w, __ffs(__ballot_sync(0xffffffffu, mine)) - 1);
-      if (mine) {
+  float sum = 0.f, mine_w = 0.f;
+  int mine_e = 0;
+  for (int first = 0; first < k; first += 32) {
+    const int count = min(k - first, 32);
+    for (int pick = 0; pick < count; ++pick) {
+      const uint32_t key = ordered_bits(best), top = __reduce_max_sync(0xffffffffu, key);
+      const bool wins = key == top && best_j >= 0;
+      const uint32_t who = __ballot_sync(0xffffffffu, wins);
+      // fewer candidates than k: every remaining value is -inf, and expert 0 with its weight is reported again
+      int e = 0;
+      if (who != 0) {
+        const int e_lane = index(best_j);
+        // (equal values in several lanes: the lowest expert)
+        e = (who & (who - 1)) == 0 ? __shfl_sync(0xffffffffu, e_lane, __ffs(who) - 1)
+                                   : __reduce_min_sync(0xffffffffu, wins ? e_lane : INT_MAX);
+        if (wins && e_lane == e) {
 #pragma unroll
-        for (int j = 0; j < kPerLane; ++j)
-          if (j == best_j) sel[j] = kNegInf;
-        look();
+          for (int j = 0; j < kPerLane; ++j)
+            if (j == best_j) sel[j] = kNegInf;
+          look();
+        }
       }
+      if (lane == pick) mine_e = e;
     }
-    if (lane == 0) {
-      out_w[pick] = w;
-      out_i[pick] = e == INT_MAX ? 0 : e;
-    }
-    sum += w;  // same order and values in every lane
+    if (lane < count) mine_w = weight(mine_e);
+    for (int p = 0; p < count; ++p) sum += __shfl_sync(0xffffffffu, mine_w, p);  // in the order of the picks, the same in every lane
+    if (k > 32 && lane < count) out_w[first + lane] = mine_w, out_i[first + lane] = mine_e;
+  }
+  if (k <= 32) {
+    if (lane < k) out_w[lane] = finish(mine_w, sum), out_i[lane] = mine_e;
+  } else {  // (the sum is known only now)
+    for (int p = lane; p < k; p += 32) out_w[p] = finish(out_w[p], sum);
   }
   return sum;
 }
@@ -93,7 +100,7 @@ __global__ void __launch_bounds__(kGateWarps * 32)
   ptx::grid_dependency_wait();
   if (row >= rows) return;
   const T* x = gating + row * E;
-  float sel[kPerLane], wgt[kPerLane];
+  float sel[kPerLane];
 #pragma unroll
   for (int j = 0; j < kPerLane; ++j) {
     const int e = j * 32 + lane;
@@ -123,24 +130,36 @@ __global__ void __launch_bounds__(kGateWarps * 32)
     }
     const float inv = 1.f / warp_sum(s);
 #pragma unroll
-    for (int j = 0; j < kPerLane; ++j) {
-      wgt[j] = sel[j] * inv;
-      sel[j] = (j * 32 + lane < E) ? wgt[j] : kNegInf;
-    }
+    for (int j = 0; j < kPerLane; ++j) sel[j] = (j * 32 + lane < E) ? sel[j] * inv : kNegInf;
+  }
+  // the row's values once more, for the weights of the picks
+  extern __shared__ float gate_smem[];  // per warp: E values
+  float* kept = gate_smem + (threadIdx.x >> 5) * E;
+#pragma unroll
+  for (int j = 0; j < kPerLane; ++j)
+    if (j * 32 + lane < E) kept[j * 32 + lane] = sel[j];
+  __syncwarp();
+  pick_topk<kPerLane>(
+      sel, [&](int j) { return j * 32 + lane; },
+      [&](int e) { return kMode == 1 && bias != nullptr ? kept[e] - bias[e] : kept[e]; }, lane, k, out_w + row * k, out_i + row * k,
+      [&](float w, float sum) { return renormalize ? w * (1.f / sum) : w; });
+}
+
+// Lane `lane`'s N consecutive values of the E at `p` (0 past the end), 16 bytes at a time where they lie so.
+template <typename T, int N>
+__device__ __forceinline__ void load_run(const T* p, int E, int lane, float (&v)[N]) {
+  constexpr int kVec = 16 / (int)sizeof(T);
+  p += lane * N;
+  if (N % kVec == 0 && E % N == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+    uint4 raw[N % kVec == 0 ? N / kVec : 1];
+    const bool on = lane * N < E;
+#pragma unroll
+    for (int c = 0; c < N / kVec; ++c) raw[c] = on ? __ldg(reinterpret_cast<const uint4*>(p) + c) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = ElemTraits<T>::to_f32(reinterpret_cast<const T*>(raw)[j]);
   } else {
 #pragma unroll
-    for (int j = 0; j < kPerLane; ++j) {
-      const int e = j * 32 + lane;
-      wgt[j] = (bias != nullptr && e < E) ? sel[j] - bias[e] : sel[j];
-    }
-  }
-  float* ow = out_w + row * k;
-  int32_t* oi = out_i + row * k;
-  const float sum = pick_topk<kPerLane>(sel, wgt, [&](int j) { return j * 32 + lane; }, lane, k, ow, oi);
-  if (renormalize) {
-    __syncwarp();
-    const float inv = 1.f / sum;
-    for (int p = lane; p < k; p += 32) ow[p] = ow[p] * inv;
+    for (int j = 0; j < N; ++j) v[j] = lane * N + j < E ? ElemTraits<T>::to_f32(p[j]) : 0.f;
   }
 }
 
@@ -155,25 +174,26 @@ __global__ void __launch_bounds__(kGateWarps * 32)
     fused_gate_kernel(const T* __restrict__ input, const T* __restrict__ bias, int64_t rows, int E, int G, int topk_group,
                       int topk, int n_shared, float factor, int scale_output, float* __restrict__ out_w,
                       int32_t* __restrict__ out_i) {
-  extern __shared__ float gate_smem[];  // per warp: E biased scores (group sizes that lanes do not divide)
+  extern __shared__ float gate_smem[];  // per warp: E scores
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* score = gate_smem + warp * E;
   const int64_t row = (int64_t)blockIdx.x * kGateWarps + warp;
   ptx::launch_dependents();
   ptx::grid_dependency_wait();
   if (row >= rows) return;
   const T* x = input + row * E;
-  float sel[kPerLane], wgt[kPerLane];
+  auto biased = [](float s, float b) { return ElemTraits<T>::to_f32(ElemTraits<T>::from_f32(s + b)); };
+  float sel[kPerLane], in[kPerLane], add[kPerLane];
+  load_run<T, kPerLane>(x, E, lane, in);
+  load_run<T, kPerLane>(bias, E, lane, add);
 #pragma unroll
   for (int j = 0; j < kPerLane; ++j) {
     const int e = lane * kPerLane + j;
     sel[j] = kNegInf;
-    wgt[j] = 0.f;
     if (e < E) {
-      const float xv = ElemTraits<T>::to_f32(x[e]);
-      const T s = ElemTraits<T>::from_f32(1.0f / (1.0f + expf(-xv)));
-      const T b = ElemTraits<T>::from_f32(ElemTraits<T>::to_f32(s) + ElemTraits<T>::to_f32(bias[e]));
-      wgt[j] = ElemTraits<T>::to_f32(s);
-      sel[j] = ElemTraits<T>::to_f32(b);
+      const float s = ElemTraits<T>::to_f32(ElemTraits<T>::from_f32(1.0f / (1.0f + expf(-in[j]))));
+      score[e] = s;
+      sel[j] = biased(s, add[j]);
     }
   }
   // The two largest scores of every group, of which lane g keeps group g's sum.
@@ -187,7 +207,8 @@ __global__ void __launch_bounds__(kGateWarps * 32)
       m2 = v;
     }
   };
-  if (gs % kPerLane == 0 && (lanes_per_group & (lanes_per_group - 1)) == 0) {
+  const bool runs = gs % kPerLane == 0 && (lanes_per_group & (lanes_per_group - 1)) == 0;
+  if (runs) {
     // a group is a run of 2^n lanes: best two of the lane's registers, merged over the run
     float m1 = -FLT_MAX, m2 = -FLT_MAX;
 #pragma unroll
@@ -201,14 +222,10 @@ __global__ void __launch_bounds__(kGateWarps * 32)
     gscore = __shfl_sync(0xffffffffu, sc, (lane * lanes_per_group) & 31);
     if (lane >= G) gscore = kNegInf;
   } else {
-    float* b_sh = gate_smem + warp * E;
-#pragma unroll
-    for (int j = 0; j < kPerLane; ++j)
-      if (lane * kPerLane + j < E) b_sh[lane * kPerLane + j] = sel[j];
     __syncwarp();
     if (lane < G) {
       float m1 = -FLT_MAX, m2 = -FLT_MAX;
-      for (int i = 0; i < gs; ++i) push(b_sh[lane * gs + i], m1, m2);
+      for (int i = lane * gs; i < lane * gs + gs; ++i) push(biased(score[i], ElemTraits<T>::to_f32(bias[i])), m1, m2);
       gscore = ElemTraits<T>::to_f32(ElemTraits<T>::from_f32(m1 + m2));
     }
   }
@@ -219,25 +236,27 @@ __global__ void __launch_bounds__(kGateWarps * 32)
     if (og > gscore || (og == gscore && g < lane)) ++beaten_by;
   }
   const uint32_t keep_mask = __ballot_sync(0xffffffffu, lane < G && beaten_by < topk_group);
+  if (runs) {  // (a lane's experts are of one group)
+    if (!((keep_mask >> (lane >> (__ffs(lanes_per_group) - 1))) & 1u))
 #pragma unroll
-  for (int j = 0; j < kPerLane; ++j) {
-    const int e = lane * kPerLane + j;
-    if (e < E && !((keep_mask >> (e / gs)) & 1u)) sel[j] = kNegInf;
+      for (int j = 0; j < kPerLane; ++j) sel[j] = kNegInf;
+  } else {
+#pragma unroll
+    for (int j = 0; j < kPerLane; ++j) {
+      const int e = lane * kPerLane + j;
+      if (e < E && !((keep_mask >> (e / gs)) & 1u)) sel[j] = kNegInf;
+    }
   }
   const int k_routed = topk - n_shared;
   float* ow = out_w + row * topk;
   int32_t* oi = out_i + row * topk;
-  const float sum = pick_topk<kPerLane>(sel, wgt, [&](int j) { return lane * kPerLane + j; }, lane, k_routed, ow, oi);
   __syncwarp();
+  auto finish = [&](float w, float sum) { return scale_output ? w / sum * factor : w / sum; };
+  const float sum = pick_topk<kPerLane>(sel, [&](int j) { return lane * kPerLane + j; }, [&](int e) { return score[e]; }, lane,
+                                        k_routed, ow, oi, finish);
   for (int i = lane; i < n_shared; i += 32) {
     oi[k_routed + i] = E + i;
-    ow[k_routed + i] = sum / factor;
-  }
-  __syncwarp();
-  for (int p = lane; p < topk; p += 32) {
-    float w = ow[p] / sum;
-    if (scale_output) w *= factor;
-    ow[p] = w;
+    ow[k_routed + i] = finish(sum / factor, sum);
   }
 }
 
@@ -248,7 +267,7 @@ static int launch_topk(const void* gating, const float* bias, int64_t rows, int 
   const T* g = static_cast<const T*>(gating);
 #define SGLB_GATE_CASE(P)                                                                                        \
   if (E <= 32 * P) {                                                                                             \
-    SGLB_CUDA(launch_pdl(topk_gate_kernel<T, P, kMode>, grid, kGateWarps * 32, 0, st, g, bias, rows, E, k, renorm, softcap, \
+    SGLB_CUDA(launch_pdl(topk_gate_kernel<T, P, kMode>, grid, kGateWarps * 32, (size_t)kGateWarps * E * sizeof(float), st, g, bias, rows, E, k, renorm, softcap, \
                          out_w, out_i));                                                                         \
     return SGLB200_OK;                                                                                           \
   }

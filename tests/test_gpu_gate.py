@@ -111,6 +111,30 @@ def test_topk_softmax(ops, rows, E, k, renorm, softcap, with_bias, dtype):
     _compare(w, ids, rw, rids, rtol=3e-5)
 
 
+# picks beyond the 32 that a warp keeps in registers, all experts, and logits many of which are equal
+@pytest.mark.parametrize("rows,E,k", [(5, 64, 33), (3, 40, 40), (70, 256, 65), (64, 128, 32)])
+@pytest.mark.parametrize("coarse", [False, True])
+def test_topk_softmax_many_picks(ops, rows, E, k, coarse):
+    x = torch.randn(rows, E, generator=torch.Generator().manual_seed(rows + E + k)) * 3
+    if coarse:
+        x = x.round()
+    w = torch.empty(rows, k, device="cuda")
+    ids = torch.empty(rows, k, dtype=torch.int32, device="cuda")
+    ops.topk_softmax_out(w, ids, x.cuda(), True)
+    rw, rids = O.topk_softmax(x.numpy(), k, True)
+    _compare(w, ids, rw, rids, rtol=3e-5)
+
+
+# the same behind groups of experts: of 32 experts (runs of lanes), and of three (no runs)
+@pytest.mark.parametrize("E,G,tg,k", [(1024, 32, 8, 40), (96, 32, 16, 36)])
+def test_fused_gate_many_picks(ops, E, G, tg, k):
+    g = torch.Generator().manual_seed(E)
+    x, bias = torch.randn(33, E, generator=g), torch.rand(E, generator=g)
+    w, ids = ops.moe_fused_gate(x.cuda(), bias.cuda(), G, tg, k, 0, 2.5, True)
+    rw, rids = O.moe_fused_gate(x.numpy(), bias.numpy(), G, tg, k, 0, 2.5, True)
+    _compare(w, ids, rw, rids, rtol=3e-5)
+
+
 @pytest.mark.parametrize("rows,E,k", [(2, 16, 3), (300, 64, 6), (4096, 256, 8)])
 @pytest.mark.parametrize("renorm", [False, True])
 @pytest.mark.parametrize("with_bias", [False, True])
