@@ -1251,11 +1251,9 @@ __global__ void __launch_bounds__(256)
   *reinterpret_cast<uint4*>(C + row * N + col) = raw;
 }
 
-// How a dense problem is cut into units.
-//  * Few tiles, long K, M of 65 to 128 (weight streaming): stream-K over all SMs while the partial sums cost less than a
-//    quarter of the weight bytes.
-//  * Fewer than two waves of tiles with a long K otherwise (M = 256 or so): stream-K when its run of slabs plus
-//    the cost of the partial sums is shorter than the whole waves it replaces.
+// How a dense problem whose 128-wide tiles are more than one wave is cut into units.
+//  * Fewer than two waves of tiles with a long K (256 to 512 rows or so): stream-K when its run of slabs plus the cost of the
+//    partial sums is shorter than the whole waves it replaces.
 //  * More tiles than SMs with a last wave that fills at most half of them: the tiles of that wave are split so
 //    that the tail takes 1/splits of a tile time instead of a whole one (the other tiles are untouched).
 #ifndef SGLB_TAIL_SPLIT
@@ -1284,14 +1282,9 @@ static UnitPlan plan_units(int64_t M, int64_t N, int64_t K, int BN, int sms) {
     int64_t share = (total + sms - 1) / sms;
     share = (share + 3) / 4 * 4;  // runs start on multiples of four slabs: aligned 128-bit loads of the activation scales
     const int64_t ctas = (total + share - 1) / share;
-    const int64_t rows = M < BM ? M : BM;
     const int pieces = share <= kb_total ? 2 : 3;
     bool take = false;
-    if (tiles * 2 <= sms && pieces == 2) {
-      // weight streaming: the partial sums (two pieces per CTA, M rows each, written and read back) stay below a
-      // quarter of the weight bytes
-      take = 2 * ctas * rows * BN * 4 * 2 * 4 <= N * K;
-    } else if (share <= 2 * (int64_t)kb_total) {
+    if (share <= 2 * (int64_t)kb_total) {
       // Compared in slab times (about 0.45 us each): the run plus the partial sums (one piece per run and per
       // tile boundary, written and read back at about 4 TB/s, plus the second launch) against the whole waves.
       const int64_t waves = (tiles + sms - 1) / sms;
@@ -1304,16 +1297,7 @@ static UnitPlan plan_units(int64_t M, int64_t N, int64_t K, int BN, int sms) {
       return pl;
     }
   }
-  if (tiles * 2 <= sms && kb_total >= 8) {
-    // (measured: splitting further, to several units per SM, costs more in partial-sum traffic and per-unit
-    // start-up than it gains in balance)
-    s = sms / tiles;
-    const int64_t by_traffic = K / (32 * M);
-    if (s > by_traffic) s = by_traffic;
-    if (s > kb_total / 4) s = kb_total / 4;
-    if (s > 16) s = 16;
-    split_tiles = tiles;
-  } else if (kTailSplit && tiles > sms && kb_total >= 32) {
+  if (kTailSplit && tiles > sms && kb_total >= 32) {
     const int64_t tail = tiles % sms;
     if (tail > 0 && tail * 2 <= sms) {
       s = sms / tail;
@@ -1435,10 +1419,13 @@ int choose_group_m(int64_t rows, int64_t K, int tile_rows) {
   return (int)((tiles_m + groups - 1) / groups);
 }
 
-// Tile width of a dense problem (TileCfg).  Where the 256-wide tiling splits K (stream-K, split tiles) or makes several
-// waves, it wins; where one wave of it leaves SMs idle and K is not split, the 128-wide tile's extra tiles fill them.
-// Compared as waves x tile width, the 128-wide tile charged 156 instead of 128 (it takes 0.61 of a wide tile's time).
+// Tile width of a dense problem (TileCfg): 128 columns where one wave of such tiles holds it.  Against 256-wide tiles that are
+// split or run stream-K over all SMs, with the quantizer: 128 x 10240 x 8192 29.3 -> 24.4 us, 80 x 18432 x 7168 35.1 -> 28.9, 128 x
+// 16384 x 8192 37.7 -> 32.0, 256 x 7168 x 16384 46.0 -> 44.0.  Else 256 columns where that splits K (stream-K, split tiles); else
+// compared as waves x tile width, the 128-wide tile charged 156 instead of 128 (it takes 0.61 of a wide tile's time).
+static bool one_narrow_wave(int64_t M, int64_t N) { return ((M + BM - 1) / BM) * ((N + 127) / 128) <= sm_count(); }
 static int choose_bn(int64_t M, int64_t N, int64_t K) {
+  if (one_narrow_wave(M, N)) return 128;
   const int sms = sm_count();
   if (plan_units(M, N, K, 256, sms).scratch_blocks() > 0) return 256;
   const int64_t tiles_m = (M + BM - 1) / BM;
@@ -1463,7 +1450,9 @@ static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
   DensePlan d;
   d.cluster = tile_splits(((M + BM - 1) / BM) * ((N + 127) / 128), (int)((K + BK - 1) / BK), M, cluster_fits());
   d.bn = d.cluster > 1 ? 128 : choose_bn(M, N, K);
-  d.units = plan_units(M, N, K, d.bn, sm_count());
+  // (one wave of 128-wide tiles is not cut in units of its own)
+  if (one_narrow_wave(M, N)) d.units = UnitPlan{(int)(((M + BM - 1) / BM) * ((N + 127) / 128)), 1, (int)((K + BK - 1) / BK), 0, 0, 0, 2};
+  else d.units = plan_units(M, N, K, d.bn, sm_count());
   return d;
 }
 

@@ -39,11 +39,11 @@ def test_dense_gemm_matches_oracle(ops, M, N, K):
     assert_close_fp(got, ref)
 
 
-# the staging area inside the operand ring (from 32 slabs on): one slab fewer, the first size, part of a tile's rows and columns, a
-# single wave of 128-wide tiles and of 256-wide ones, split tiles (partial sums only), equal runs of slabs over all SMs
+# the staging area inside the operand ring: one wave of 128-wide tiles (one slab fewer than it takes, the fewest, many), of 256-wide
+# ones, equal runs of slabs over all SMs
 @pytest.mark.parametrize("M,N,K,dtype", [
-    (65, 512, 3968, torch.bfloat16), (65, 512, 4096, torch.bfloat16), (300, 520, 4096, torch.float16), (129, 1032, 4224, torch.bfloat16),
-    (200, 12288, 4096, torch.bfloat16), (65, 512, 8192, torch.float16), (620, 3832, 12800, torch.bfloat16)])
+    (200, 5128, 1408, torch.bfloat16), (200, 5128, 1536, torch.float16), (129, 9480, 4096, torch.bfloat16),
+    (200, 12288, 4096, torch.bfloat16), (620, 3832, 12800, torch.bfloat16)])
 def test_dense_gemm_one_tile_a_cta(ops, M, N, K, dtype):
     got, ref = _dense_case(ops, M, N, K, seed=M + N + K, out_dtype=dtype)
     assert_close_fp(got, ref)

@@ -52,8 +52,9 @@ def test_gemm_wait_runs_out_and_recovers(M, N, K):
     assert ops.gemm_status() == 0 and torch.equal(again, good)
 
 
-# the staging area inside the operand ring (256-wide tiles, partial sums only), slabs split over a cluster, two tiles of 64 rows
-@pytest.mark.parametrize("M,N,K", [(256, 16384, 4096), (620, 3832, 12800), (300, 512, 4096), (100, 512, 8192)])
+# the staging area inside the operand ring (256-wide tiles, 128-wide ones, partial sums only), slabs split over a cluster, two
+# tiles of 64 rows
+@pytest.mark.parametrize("M,N,K", [(256, 16384, 4096), (256, 9216, 2048), (620, 3832, 12800), (300, 512, 4096), (100, 512, 8192)])
 def test_one_tile_a_cta_wait_runs_out_and_recovers(M, N, K):
     test_gemm_wait_runs_out_and_recovers(M, N, K)
 
