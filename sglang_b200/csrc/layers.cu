@@ -42,6 +42,7 @@ struct ExpertsPlan {
   int tile, block;
   int64_t cap, rows;  // entries of the sort's output; rows that can be in use
   int64_t q, s, sorted, inv, eid, post, next, cum, sort, sort_bytes, a1, a1s, ic1, a2, a2s, ic3, total;
+  bool apart;         // the activation is a launch of its own between the products (128-row tiles)
   bool direct;        // one expert per token and no factor: the second GEMM writes the result itself
 };
 
@@ -62,6 +63,16 @@ static int experts_row_tile(int64_t numel, int64_t E) {
   return 0;
 }
 
+// Whether the activation runs between the products instead of in the first one's epilogue: with a little more than one wave of
+// tiles, up to two and a half.  A tile's epilogue is a microsecond longer for it, which few tiles a CTA do not hide, and what the
+// launch reads back lies in L2 then.  Us of the layer, in the epilogue / apart (tiles as estimated here, of 148 SMs): 176 tiles 92.2 /
+// 88.3 (600 tokens, two of 8 experts of 4096 x 1408), 208 54.5 / 52.8, 256 88.5 / 86.2, 320 181.9 / 180.1, 312 66.4 / 65.7; but 64
+// 36.5 / 38.7, 80 43.3 / 44.6, 1024 145.9 / 154.2, 1248 221.3 / 232.1, 8448 1337 / 1409.
+static bool activation_apart(int64_t numel, int64_t E, int64_t I) {
+  const int64_t experts = std::min(numel, E), tiles = experts * ((numel / experts + 127) / 128) * (I / 128), sms = sm_count();
+  return tiles > sms && 2 * tiles <= 5 * sms;
+}
+
 static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int64_t I, int64_t Ho, float factor) {
   ExpertsPlan p{};
   const int64_t numel = T * k;
@@ -76,7 +87,8 @@ static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int6
   p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4), p.next = c.take(8);
   p.cum = c.take((E + 2) * 4), p.sort = c.take(p.sort_bytes);
   if (p.tile == 0) p.inv = c.take(numel * 4), p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
-  else p.ic1 = c.take(p.rows * 2 * I * 2);
+  p.apart = p.tile == 0 && activation_apart(numel, E, I);
+  if (p.tile > 0 || p.apart) p.ic1 = c.take(p.rows * 2 * I * 2);
   p.a2 = c.take(p.rows * I), p.a2s = c.take(p.rows * (I / 128) * 4);
   if (!p.direct) p.ic3 = c.take((p.tile == 0 ? p.rows : numel) * Ho * 2);
   p.total = c.bytes;
@@ -183,8 +195,15 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
                                    stream);
       if (rc) return rc;
     }
-    rc = grouped_act_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.a2, f(p.a2s), i(p.sorted), i(p.eid), i(p.post),
-                        p.rows, numel, (int)E, I, H, dtype, st);
+    if (p.apart) {
+      rc = grouped_mm_any(base + p.a1, f(p.a1s), w13, w13_s, base + p.ic1, i(p.sorted), i(p.eid), i(p.post), nullptr, p.rows, numel,
+                          (int)E, 2 * I, H, 0, dtype, true, st);
+      if (rc) return rc;
+      rc = silu_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), true, st);
+    } else {
+      rc = grouped_act_mm(base + p.a1, f(p.a1s), w13, w13_s, base + p.a2, f(p.a2s), i(p.sorted), i(p.eid), i(p.post),
+                          p.rows, numel, (int)E, I, H, dtype, st);
+    }
     if (rc) return rc;
     rc = grouped_mm_any(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights, p.rows, numel, (int)E,
                         Ho, I, p.direct, dtype, true, st);

@@ -141,6 +141,13 @@ def test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd):
         assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.nan_to_num(**kept), want.nan_to_num(**kept))
 
 
+# the activation in a launch of its own: one to two and a half waves of tiles, behind the sort of up to 2048 ids and of more
+@pytest.mark.parametrize("T,E,topk,H,I,dtype,odd", [
+    (600, 8, 2, 1152, 1408, torch.bfloat16, False), (500, 8, 2, 256, 1664, torch.float16, True), (1100, 8, 2, 1152, 1664, torch.bfloat16, True)])
+def test_experts_with_the_activation_apart_equal_their_steps(T, E, topk, H, I, dtype, odd):
+    test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd)
+
+
 # more tiles of the first product than CTAs, behind the sort of up to 2048 ids and of more; experts without rows among them
 @pytest.mark.parametrize("T,E,topk", [(40, 64, 2), (700, 96, 3)])
 def test_experts_many_tiles(T, E, topk):
