@@ -27,15 +27,15 @@
 // scout's ring, relaxed hand-backs of tensor memory and the two-step question; 1056 to 1077 (the spread over boxes) with
 // the promotion loop unrolled by four, so that buffers, barriers and scales are compile-time (its bookkeeping was a chain
 // of dependent instructions as long as the FMAs).  Keeping one TMEM load in flight across the FMAs, chunk by chunk, was
-// slower (1250): every extra wait for a load costs more than the overlap gives.  ptxas spills at 168 registers a thread: 12
-// to 16 bytes of stores in every instance, 40 to 44 bytes of loads in the 256-wide ones, 248 to 264 in the 128-wide ones.
+// slower (1250): every extra wait for a load costs more than the overlap gives.  ptxas spills at 168 registers a thread: 4
+// to 16 bytes of stores in the dense instances, 56 with experts, 248 where the epilogue activates.
 // The epilogue rounds to bf16/fp16, parks the tile in swizzled shared memory, from where TMA stores drain it
 // during the next tile; in grouped "scatter" mode it multiplies by the routing weight, parks likewise and writes 128
 // contiguous bytes at a time to the token-major row named by sorted_token_ids.
-// Scheduling: with fewer than two waves of tiles and a long K the tiles x slabs space is cut into one equal run
-// of slabs per SM (stream-K; a run covers the end of one tile, possibly a whole tile, and the start of the next);
-// otherwise the tiles of a short last wave are split along K.  Split work writes float32 partial sums that a
-// second kernel adds in ascending K order.  In push mode (row-parallel layers under tensor parallelism) a tile is
+// Scheduling: one wave of 128-wide tiles is taken as it is, or, with few tiles and a long K, split over clusters.  With more, but
+// fewer than two waves of 256-wide tiles and a long K, the tiles x slabs space is cut into one equal run of slabs per SM
+// (stream-K; a run covers the end of one tile, possibly a whole tile, and the start of the next); otherwise the tiles of a short
+// last wave are split along K.  Both write float32 partial sums that a second kernel adds in ascending K order.  In push mode (row-parallel layers under tensor parallelism) a tile is
 // stored through the tensor map of the staging buffer of the GPU that owns its rows, which folds the
 // reduce-scatter of the all-reduce into the epilogue.
 //
@@ -94,8 +94,7 @@ __device__ long long g_trace[2][kTraceUnits][kTraceStamps];
 // (partial sums only): the staging area then lies in the operand ring, which has room for one stage more.  A slab of a single
 // wave takes 1 100 clocks, most of them the way from DRAM and L2 to shared memory (of many waves 850: other rows' CTAs have
 // brought the weights), so it is bytes in flight that count.  Us with the quantizer, ring of three stages -> four, both in turn
-// on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 256 x 7168 x 16384 55.4 -> 53.0, 100 x 4096 x 7168 23.1 -> 21.2, 512 x 7168 x
-// 16384 86.3 -> 82.1.  Shorter K pays with the early weights below, from 12 slabs and 32 CTAs on: 128 x 24576 x 1536 14.5 -> 14.1,
+// on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 512 x 7168 x 16384 86.3 -> 82.1, 192 x 10240 x 8192 40.8 -> 38.2.  Shorter K pays with the early weights below, from 12 slabs and 32 CTAs on: 128 x 24576 x 1536 14.5 -> 14.1,
 // 128 x 9216 x 2048 11.4 -> 11.1; 128 x 3072 x 2048 (24 CTAs) 10.3 -> 10.5, 128 x 4096 x 512 7.1 -> 7.3.
 // kSplit: a dense product of few 128-wide tiles and a long K, whose slabs are split over the CTAs of a cluster (`tile_splits`); their
 // partial sums meet in distributed shared memory (written once, added once) instead of in global memory and a second launch.
