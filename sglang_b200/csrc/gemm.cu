@@ -94,8 +94,9 @@ __device__ long long g_trace[2][kTraceUnits][kTraceStamps];
 // (partial sums only): the staging area then lies in the operand ring, which has room for one stage more.  A slab of a single
 // wave takes 1 100 clocks, most of them the way from DRAM and L2 to shared memory (of many waves 850: other rows' CTAs have
 // brought the weights), so it is bytes in flight that count.  Us with the quantizer, ring of three stages -> four, both in turn
-// on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 512 x 7168 x 16384 86.3 -> 82.1, 192 x 10240 x 8192 40.8 -> 38.2.  Shorter K pays with the early weights below, from 12 slabs and 32 CTAs on: 128 x 24576 x 1536 14.5 -> 14.1,
-// 128 x 9216 x 2048 11.4 -> 11.1; 128 x 3072 x 2048 (24 CTAs) 10.3 -> 10.5, 128 x 4096 x 512 7.1 -> 7.3.
+// on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 512 x 7168 x 16384 86.3 -> 82.1, 192 x 10240 x 8192 40.8 -> 38.2.
+// Shorter K pays with the early weights below, from 12 slabs and 32 CTAs on: 128 x 24576 x 1536 14.5 -> 14.1, 128 x 9216 x 2048
+// 11.4 -> 11.1; 128 x 3072 x 2048 (24 CTAs) 10.3 -> 10.5, 128 x 4096 x 512 7.1 -> 7.3.
 // kSplit: a dense product of few 128-wide tiles and a long K, whose slabs are split over the CTAs of a cluster (`tile_splits`); their
 // partial sums meet in distributed shared memory (written once, added once) instead of in global memory and a second launch.
 // Beside the ring of five stages lies room for what the other CTAs send; sums fetched from the others' memory after a barrier,
