@@ -286,7 +286,8 @@ int sglb200_fp8_blockwise_scaled_mm(const void* A, const void* B, const float* a
  * e = expert_ids[b]:  acc[r, n] = blockscaled( A[r, :], B[e, n, :] ) for the block's rows r.
  *   e == -1  -> the block contributes zeros.
  * Output modes:
- *   scatter == 0: C[r, n] = bf16(acc)                       (C is [max_rows, N], expert-sorted order)
+ *   scatter == 0: C[r, n] = bf16(acc)                       (C is [max_rows, N], expert-sorted order; row_weights and
+ *                 sorted_token_ids are not read and may be NULL)
  *   scatter == 1: id = sorted_token_ids[r]; if id < numel:
  *                 C[id, n] = bf16( acc * (row_weights ? row_weights[id] : 1) )   (C is [numel, N], token-major)
  * Replaces: fused_moe_kernel via invoke_fused_moe_kernel

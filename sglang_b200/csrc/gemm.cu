@@ -149,7 +149,7 @@ struct GemmParams {
   const int32_t* sorted_ids;   // grouped
   const int32_t* expert_ids;   // grouped
   const int32_t* num_rows_dev; // grouped: rows in use (multiple of 128)
-  const float* row_weights;    // grouped scatter, optional
+  const float* row_weights;    // grouped, optional: of the rows that are scattered, or stored in sorted order with padding to skip
   int64_t M;                   // dense: rows of A; grouped: max rows
   int64_t N, K;
   int64_t as_stride_m, as_stride_k;
@@ -1618,7 +1618,7 @@ static int grouped_mm(const void* A, const float* a_s, const void* B, const floa
   GemmParams p{};
   p.a_s = a_s, p.b_s = b_s, p.C = C, p.bias = nullptr;
   p.sorted_ids = sorted_token_ids, p.expert_ids = expert_ids, p.num_rows_dev = num_rows_dev;
-  p.row_weights = row_weights;
+  p.row_weights = scatter || skip_padding ? row_weights : nullptr;  // (elsewhere the sorted rows are the bare product, and may have no ids)
   p.M = max_rows, p.N = N, p.K = K;
   p.kb_total = (int)((K + BK - 1) / BK), p.nb_total = (int)((N + kScaleBlockN - 1) / kScaleBlockN);
   p.tiles_n = (int)((N + BN - 1) / BN);
@@ -1744,7 +1744,7 @@ int sglb200::grouped_mm_any(const void* A, const float* a_s, const void* B, cons
   SGLB_REQUIRE(out_dtype == 0 || out_dtype == 1, "grouped_mm: out_dtype %d (0 bf16, 1 fp16)", out_dtype);
   if (max_rows == 0) return SGLB200_OK;
   SGLB_REQUIRE(A && a_s && B && b_s && C && expert_ids && num_rows_dev, "grouped_mm: null pointer");
-  SGLB_REQUIRE(!scatter || sorted_token_ids, "grouped_mm: scatter mode needs sorted_token_ids");
+  SGLB_REQUIRE((!scatter && !skip_padding) || sorted_token_ids, "grouped_mm: scatter mode needs sorted_token_ids");
   SGLB_REQUIRE(aligned16(A) && aligned16(B) && aligned16(C), "grouped_mm: A, B and C must be 16-byte aligned");
   if (choose_bn_grouped(numel) == 128)
     return grouped_mm<128>(A, a_s, B, b_s, C, sorted_token_ids, expert_ids, num_rows_dev, row_weights, max_rows, numel,

@@ -173,6 +173,32 @@ def test_fused_experts_matches_oracle(ops, T, E, H, I, topk, filtered):
     assert torch.equal(out, out2)
 
 
+# 40 and 600 routed rows: tiles of 128 and of 256 columns
+@pytest.mark.parametrize("T", [20, 300])
+def test_grouped_gemm_in_sorted_order_takes_no_weights(ops, T, E=4, H=384, N=264, topk=2):
+    """Without scatter the rows are the bare product: weights change nothing, and no ids are needed."""
+    from sglang_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(E, N, H, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    ws = torch.rand(E, (N + 127) // 128, H // 128, device="cuda", generator=g) * 1e-3
+    ids = torch.randint(-1, E, (T, topk), device="cuda", generator=g).int()
+    wt = torch.rand(T, topk, device="cuda", generator=g) + 2.0
+    xq, xs = ops.per_token_group_quant_fp8(x, 128)
+    order, eid, post = ops.moe_align_block_size(ids, 128, E)
+    rows, numel = order.numel() // 128 * 128, T * topk
+    a, a_s = ops.gather_rows_fp8(xq, xs, order, post, numel, topk, rows)
+    want = ops.grouped_block_fp8_matmul(a, a_s, w, ws, order, eid, post, numel=numel, scatter=False)
+    got = ops.grouped_block_fp8_matmul(a, a_s, w, ws, order, eid, post, numel=numel, scatter=False, row_weights=wt)
+    bare = torch.empty_like(want)
+    check(lib.sglb200_fp8_blockwise_grouped_mm(a.data_ptr(), a_s.data_ptr(), w.data_ptr(), ws.data_ptr(), bare.data_ptr(), None,
+                                               eid.data_ptr(), post.data_ptr(), wt.data_ptr(), rows, numel, E, N, H, 0, 0,
+                                               torch.cuda.current_stream().cuda_stream))
+    n = int(post)
+    assert ops.gemm_status() == 0
+    assert want[:n].any() and torch.equal(got[:n], want[:n]) and torch.equal(bare[:n], want[:n])
+
+
 def test_fused_experts_all_ids_filtered(ops):
     from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
     x, w13q, w13s, w2q, w2s, w, ids = _moe_inputs(40, 8, 512, 256, 4, seed=5)
