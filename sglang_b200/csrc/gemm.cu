@@ -767,9 +767,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           float4 av[kRowsAhead];
 #pragma unroll
           for (int k = 0; k < kRowsAhead; ++k) {
-            const int row = m_tile * BM + lane + 32 * (kRowsAhead * half + k);  // rows past M read a valid row; never stored
-            av[k] = load_a4_row(kGrouped ? p.a_s + (uint64_t)(uint32_t)row * (uint32_t)kb_total
-                                         : p.a_s + min(row, (int)rows - 1) * p.as_stride_m, kb);
+            // (the last tile's rows past M, of which a_s has none, read the last row's scales and are never stored)
+            const int row = min(m_tile * BM + lane + 32 * (kRowsAhead * half + k), (int)p.M - 1);
+            av[k] = load_a4_row(p.a_s + (kGrouped ? (int64_t)((uint64_t)(uint32_t)row * (uint32_t)kb_total) : row * p.as_stride_m), kb);
           }
           if (half == 0 && !SGLB_WAIT(bar_sempty0 + ss * 8, sph ^ 1u)) {
             *abort_flag = 1;

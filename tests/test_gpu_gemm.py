@@ -199,6 +199,33 @@ def test_grouped_gemm_in_sorted_order_takes_no_weights(ops, T, E=4, H=384, N=264
     assert want[:n].any() and torch.equal(got[:n], want[:n]) and torch.equal(bare[:n], want[:n])
 
 
+@pytest.mark.parametrize("scatter", [False, True])
+def test_grouped_gemm_with_rows_that_do_not_fill_the_last_tile(ops, scatter, E=3, H=640, N=264):
+    """Room for 300 rows where the order has 384: the last tile's other rows are neither read nor stored.  What lies behind the 300
+    is memory of the same tensors (NaN scales)."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    T, rows = 220, 300
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(E, N, H, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    ws = torch.rand(E, (N + 127) // 128, H // 128, device="cuda", generator=g) * 1e-3
+    ids = (torch.arange(T, device="cuda") * E // T).int().view(T, 1)
+    xq, xs = ops.per_token_group_quant_fp8(x, 128)
+    order, eid, post = ops.moe_align_block_size(ids, 128, E)
+    assert int(post) == 384
+    a, a_s = ops.gather_rows_fp8(xq, xs, order, post, T, 1, 384)
+    a_s[rows:] = float("nan")
+    out = torch.full((384, N), 5.0, device="cuda", dtype=torch.bfloat16)
+    ops.grouped_block_fp8_matmul(a[:rows], a_s[:rows], w, ws, order, eid, post, numel=T, scatter=scatter, out=out)
+    order, ref = order[:rows].long(), torch.full((384, N), 5.0)
+    for r in range(rows):
+        t, e = int(order[r]), int(eid[r // 128])
+        if t < T or not scatter:
+            s = torch.repeat_interleave(ws[e], 128, 0)[:N] * a_s[r]  # [N][K / 128]
+            ref[t if scatter else r] = ((a[r].float() * w[e].float()).view(N, H // 128, 128).sum(-1) * s).sum(-1).cpu()
+    assert ops.gemm_status() == 0
+    assert_close_fp(to_f32_np(out), ref.numpy())
+
+
 def test_fused_experts_all_ids_filtered(ops):
     from sglang_b200.srt.layers.moe.fused_moe_triton.fused_moe import fused_experts_impl
     x, w13q, w13s, w2q, w2s, w, ids = _moe_inputs(40, 8, 512, 256, 4, seed=5)

@@ -1,5 +1,5 @@
-"""Orderings between threads that a run cannot show, because a wrong order almost always gives the right result: checked in
-the kernels' sources."""
+"""Orderings between threads, and bounds of reads, that a run cannot show, because a wrong one almost always gives the right
+result: checked in the kernels' sources."""
 import os
 import re
 
@@ -61,3 +61,13 @@ def test_every_sort_zeroes_the_tile_counters():
     layer = _code("layers.cu")
     layer = layer[layer.index("int sglb200_fused_experts("):]
     assert re.search(r"int32_t\* next = i\(p\.next\);", layer) and not re.search(r"\bnext = (?!i\(p\.next\);)|\bnext \?", layer)
+
+
+def test_activation_scales_are_read_of_rows_that_exist():
+    """A tile's rows past the last one have no scales, also with experts, where neither the rows that a call has room for nor those
+    that are in use need fill their last tile; what is read for them is never stored."""
+    gemm = _code("gemm.cu")
+    reads = re.findall(r"load_a4_row\((p\.a_s.*)\);", gemm)
+    assert len(reads) == 1 and gemm.count("load_a4_row(") == 1 and set(re.findall(r"\brow\w*", reads[0])) == {"row"}
+    rows = re.findall(r"const int row = (.*);\s+av\[k\] = load_a4_row", gemm)
+    assert len(rows) == 1 and re.fullmatch(r"min\(.*, \(int\)p\.M - 1\)", rows[0])
