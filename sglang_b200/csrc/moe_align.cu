@@ -457,7 +457,9 @@ constexpr int kTsItems = 8;
 constexpr int kTsTile = kTsThreads * kTsItems;  // 4096 ids
 constexpr int64_t kLargeMin = 1 << 20;          // inputs above this take the tile-sorted path
 
-template <int NBITS>
+// kInverse: a layer of experts, which also wants the inverse order.  (Asked at run time, the sort alone took 536 us of 64 Mi ids
+// for 471: the kernel is bound by instruction issue.)
+template <int NBITS, bool kInverse>
 __global__ void __launch_bounds__(kTsThreads, 2)
     moe_align_tile_scatter_kernel(const int32_t* __restrict__ ids, int64_t numel, int64_t chunk_len, int B,
                                   int block_size, const int* __restrict__ chunk_hist, const int* __restrict__ totals,
@@ -495,7 +497,7 @@ __global__ void __launch_bounds__(kTsThreads, 2)
       int b = i < end ? ids[i] + 1 : -1;
       if (b >= B) b = -1;
       key[j] = b;
-      if (inverse != nullptr && b < 0 && i < end) inverse[i] = -1;
+      if (kInverse && b < 0 && i < end) inverse[i] = -1;
     }
     __syncwarp();
 #pragma unroll
@@ -542,7 +544,7 @@ __global__ void __launch_bounds__(kTsThreads, 2)
     for (int p = tid; p < n; p += kTsThreads) {
       const int e = val[p], place = ttot[e >> 12] + p, id = t_lo + (e & (kTsTile - 1));
       sorted[place] = id;
-      if (inverse != nullptr) inverse[id] = place;
+      if (kInverse) inverse[id] = place;
     }
     __syncthreads();
   }
@@ -667,14 +669,14 @@ int sglb200::align_block_size(const int32_t* topk_ids, int64_t numel, int num_ex
     moe_align_scan_kernel<<<(unsigned)((B + kAlignWarps - 1) / kAlignWarps), kAlignThreads, 0, st>>>(hist, tot,
                                                                                                      (int)lchunks, B);
 #define SGLB_TILE_SCATTER(NB)                                                                                       \
-  case NB:                                                                                                          \
+  case NB: {                                                                                                        \
+    const auto kernel = inverse ? moe_align_tile_scatter_kernel<NB, true> : moe_align_tile_scatter_kernel<NB, false>; \
     if (ts_smem > kSmemDefault)                                                                                     \
-      SGLB_CUDA(cudaFuncSetAttribute(moe_align_tile_scatter_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                     (int)kAlignSmemMax));                                                          \
-    moe_align_tile_scatter_kernel<NB><<<(unsigned)lchunks, kTsThreads, ts_smem, st>>>(                              \
+      SGLB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlignSmemMax));     \
+    kernel<<<(unsigned)lchunks, kTsThreads, ts_smem, st>>>(                                                         \
         topk_ids, numel, chunk_len, B, block_size, hist, tot, sorted_token_ids, expert_ids, num_tokens_post_pad,    \
         cumsum_buffer, pad_sorted_token_ids != 0, inverse, zeros);                                                  \
-    break
+  } break
     switch (nbits) {
       SGLB_TILE_SCATTER(6);
       SGLB_TILE_SCATTER(7);
