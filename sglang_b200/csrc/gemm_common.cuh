@@ -46,10 +46,9 @@ int sum_sorted(const void* src, const int32_t* inverse, void* out, int dtype, in
 
 // quant.cu: the quantizer (groups of 128) of a layer's activations with every row's codes and scales written to its `topk`
 // places in the sorted order (`inverse` of the sort, -1 = nowhere), and zeros to the padding rows of 32-row quadrants that
-// hold rows; other padding is not written.
+// hold rows; other padding is not written.  `starts`: the padded starts of the `buckets` of the sort, in blocks of 128, and the end.
 int quant_sorted(const void* x, int dtype, void* out_q, float* out_s, const int32_t* inverse, const int32_t* sorted_ids,
-                 const int32_t* num_rows_dev, int64_t max_rows, int64_t tokens, int topk, int64_t hidden, float eps,
-                 cudaStream_t st);
+                 const int32_t* starts, int buckets, int64_t tokens, int topk, int64_t hidden, float eps, cudaStream_t st);
 
 // moe_align.cu: the sort (arguments as sglb200_moe_align_block_size).  `inverse` (or nullptr): the place of every flat index in
 // the order, -1 for an id that is no bucket's.  `zeros` (or nullptr): zeros[0] and zeros[1] are set to 0.

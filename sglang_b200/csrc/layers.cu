@@ -169,7 +169,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     rc = align_block_size(topk_ids, numel, (int)E + 1, p.block, i(p.sorted), i(p.eid), i(p.post), i(p.cum), 1,
                           p.sort_bytes ? base + p.sort : nullptr, p.sort_bytes, i(p.inv), next, st);
     if (rc) return rc;
-    rc = quant_sorted(x, dtype, base + p.a1, f(p.a1s), i(p.inv), i(p.sorted), i(p.post), p.rows, T, (int)k, H, kQuantEps, st);
+    rc = quant_sorted(x, dtype, base + p.a1, f(p.a1s), i(p.inv), i(p.sorted), i(p.cum), (int)E + 1, T, (int)k, H, kQuantEps, st);
   } else {
     rc = quant_fp8(x, dtype, base + p.q, f(p.s), T, H, 128, kQuantEps, -kFp8Max, kFp8Max, hb, 1, true, st);
     if (rc) return rc;

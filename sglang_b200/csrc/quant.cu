@@ -344,35 +344,36 @@ __global__ void __launch_bounds__(kQuantThreads)
 }
 
 // The quantizer of a MoE layer's activations, which go to expert-sorted rows: a warp quantises four groups of a token's row
-// and writes their codes to every place the token has (512 bytes of each), so that no other launch copies rows.  The warps of
-// the first `pad_ctas` CTAs take the 32-row quadrants of the order and zero the padding rows of those that also hold rows
-// (first, as a quadrant can have 31 of them: behind the rows they were the tail of the launch).  Bound by HBM writes: 16384
+// and writes their codes to every place the token has (512 bytes of each), so that no other launch copies rows.  The first
+// `buckets` CTAs take a bucket of the sort each and zero its padding rows in the 32-row quadrant of its last block that also
+// holds rows, the eight warps in turn.  (One warp a quadrant, of up to 31 rows, was as long as a small layer's whole launch:
+// 2000 tokens of 1024 to two places 8.2 us of kernel, so 2.9; 1100 of 1152 8.1, so 3.1.)  Bound by HBM writes: 16384
 // tokens of 2048 to eight places 58.6 us (5.7 TB/s), quantizer and gather 89.1; 4096 tokens of 7168 64.1 us, before 137.  With
 // eight and sixteen groups a warp 58.6 and 60.9, 62.5 and 67.1.
 template <typename T>
 __global__ void __launch_bounds__(kQuantThreads)
     quant_sorted_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q, float* __restrict__ out_s,
                         const int32_t* __restrict__ inverse, const int32_t* __restrict__ sorted_ids,
-                        const int32_t* __restrict__ num_rows_dev, int64_t items, int pad_ctas, int pieces, int groups, int topk,
+                        const int32_t* __restrict__ starts, int64_t items, int buckets, int pieces, int groups, int topk,
                         int64_t numel, float eps, bool wide_in) {
-  constexpr int LPG = 8, CE = 8, NCH = 2, G = 128;
+  constexpr int LPG = 8, CE = 8, NCH = 2, G = 128, kBlock = 128;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   ptx::grid_dependency_wait();
   ptx::launch_dependents();
   const int64_t hidden = (int64_t)groups * G;
-  if ((int)blockIdx.x < pad_ctas) {
-    const int64_t r0 = ((int64_t)blockIdx.x * (kQuantThreads / 32) + warp) * 32;
-    if (r0 >= *num_rows_dev) return;
-    unsigned padding = __ballot_sync(0xffffffffu, sorted_ids[r0 + lane] >= numel);
-    if (padding & 1u) return;  // an expert's rows come first: nothing but padding
-    for (; padding != 0; padding &= padding - 1) {
-      const int64_t r = r0 + __ffs(padding) - 1;
-      for (int64_t c = lane * 16; c < hidden; c += 512) *reinterpret_cast<uint4*>(out_q + r * hidden + c) = make_uint4(0, 0, 0, 0);
-      for (int g = lane; g < groups; g += 32) out_s[r * groups + g] = 0.f;
+  if ((int)blockIdx.x < buckets) {
+    const int stop = starts[blockIdx.x + 1];
+    if (starts[blockIdx.x] == stop) return;
+    // (a bucket's rows come first, and only its last block has padding)
+    const int held = __syncthreads_count(threadIdx.x < kBlock && sorted_ids[stop - kBlock + (int)threadIdx.x] < numel);
+    for (int r = stop - kBlock + held + warp; r < stop - kBlock + (held + 31) / 32 * 32; r += kQuantThreads / 32) {
+      uint8_t* q = out_q + r * hidden;
+      for (int c = lane * 16; c < (int)hidden; c += 512) *reinterpret_cast<uint4*>(q + c) = make_uint4(0, 0, 0, 0);
+      for (int g = lane; g < groups; g += 32) out_s[(int64_t)r * groups + g] = 0.f;
     }
     return;
   }
-  const int64_t it = (int64_t)(blockIdx.x - pad_ctas) * (kQuantThreads / 32) + warp;
+  const int64_t it = (int64_t)(blockIdx.x - buckets) * (kQuantThreads / 32) + warp;
   if (it >= items) return;
   const int64_t t = it / pieces;
   const int g = (int)(it - t * pieces) * (32 / LPG) + lane / LPG, l = lane % LPG;
@@ -604,14 +605,14 @@ static int launch_quant_inst(const void* input, void* output_q, float* output_s,
 
 template <typename T>
 static int launch_quant_sorted(const void* x, void* out_q, float* out_s, const int32_t* inverse, const int32_t* sorted_ids,
-                               const int32_t* num_rows_dev, int64_t max_rows, int64_t tokens, int topk, int64_t hidden, float eps,
+                               const int32_t* starts, int buckets, int64_t tokens, int topk, int64_t hidden, float eps,
                                cudaStream_t st) {
   constexpr int kWarps = kQuantThreads / 32;
   const int groups = (int)(hidden / 128), pieces = (groups + 3) / 4;
-  const int64_t items = tokens * pieces, row_ctas = (items + kWarps - 1) / kWarps, pad_ctas = (max_rows / 32 + kWarps - 1) / kWarps;
-  SGLB_REQUIRE(row_ctas + pad_ctas < (1ll << 31), "quantizer: input too large");
-  SGLB_CUDA(launch_pdl(quant_sorted_kernel<T>, (unsigned)(row_ctas + pad_ctas), kQuantThreads, 0, st, static_cast<const T*>(x),
-                       static_cast<uint8_t*>(out_q), out_s, inverse, sorted_ids, num_rows_dev, items, (int)pad_ctas, pieces,
+  const int64_t items = tokens * pieces, row_ctas = (items + kWarps - 1) / kWarps;
+  SGLB_REQUIRE(row_ctas + buckets < (1ll << 31), "quantizer: input too large");
+  SGLB_CUDA(launch_pdl(quant_sorted_kernel<T>, (unsigned)(row_ctas + buckets), kQuantThreads, 0, st, static_cast<const T*>(x),
+                       static_cast<uint8_t*>(out_q), out_s, inverse, sorted_ids, starts, items, buckets, pieces,
                        groups, topk, tokens * topk, eps, aligned_to(x, 32)));
   return SGLB200_OK;
 }
@@ -760,12 +761,12 @@ int sglb200::quant_fp8(const void* input, int in_dtype, void* output_q, float* o
 }
 
 int sglb200::quant_sorted(const void* x, int dtype, void* out_q, float* out_s, const int32_t* inverse, const int32_t* sorted_ids,
-                          const int32_t* num_rows_dev, int64_t max_rows, int64_t tokens, int topk, int64_t hidden, float eps,
+                          const int32_t* starts, int buckets, int64_t tokens, int topk, int64_t hidden, float eps,
                           cudaStream_t st) {
   SGLB_REQUIRE(aligned16(x), "quantizer: input must be 16-byte aligned");
-  return dtype == 0 ? launch_quant_sorted<__nv_bfloat16>(x, out_q, out_s, inverse, sorted_ids, num_rows_dev, max_rows, tokens, topk,
+  return dtype == 0 ? launch_quant_sorted<__nv_bfloat16>(x, out_q, out_s, inverse, sorted_ids, starts, buckets, tokens, topk,
                                                          hidden, eps, st)
-                    : launch_quant_sorted<__half>(x, out_q, out_s, inverse, sorted_ids, num_rows_dev, max_rows, tokens, topk, hidden,
+                    : launch_quant_sorted<__half>(x, out_q, out_s, inverse, sorted_ids, starts, buckets, tokens, topk, hidden,
                                                   eps, st);
 }
 
