@@ -82,15 +82,32 @@ static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int6
   p.rows = (numel + std::min(numel, E + 1) * (p.block - 1) + p.block - 1) / p.block * p.block;
   p.direct = k == 1 && factor == 1.0f;
   p.sort_bytes = sglb200_moe_align_workspace_bytes(numel, (int)E + 1);
+  p.apart = p.tile == 0 && activation_apart(numel, E, I);
   Carver c;
-  p.q = c.take(T * H), p.s = c.take(T * (H / 128) * 4);
   p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4), p.next = c.take(8);
   p.cum = c.take((E + 2) * 4), p.sort = c.take(p.sort_bytes);
-  if (p.tile == 0) p.inv = c.take(numel * 4), p.a1 = c.take(p.rows * H), p.a1s = c.take(p.rows * (H / 128) * 4);
-  p.apart = p.tile == 0 && activation_apart(numel, E, I);
-  if (p.tile > 0 || p.apart) p.ic1 = c.take(p.rows * 2 * I * 2);
-  p.a2 = c.take(p.rows * I), p.a2s = c.take(p.rows * (I / 128) * 4);
-  if (!p.direct) p.ic3 = c.take((p.tile == 0 ? p.rows : numel) * Ho * 2);
+  const int64_t q = T * H, s = T * (H / 128) * 4, a2 = p.rows * I, a2s = p.rows * (I / 128) * 4;
+  if (p.tile > 0) {
+    p.q = c.take(q), p.s = c.take(s);
+    p.ic1 = c.take(p.rows * 2 * I * 2);
+    p.a2 = c.take(a2), p.a2s = c.take(a2s);
+    if (!p.direct) p.ic3 = c.take(numel * Ho * 2);
+  } else {
+    // Sorted rows are more than the ids by the padding of every expert, several times as many where experts average 49 rows, so
+    // what is dead makes room: the codes in token order (read by the gather alone, where there is one) for the second product's
+    // rows, the first product's rows and what it stores for what the second one stores.  1600 tokens of 7168 to eight of 256
+    // experts: I = 2048 1.10 GB side by side, 0.75 so; I = 256 1.01 GB, 0.66.
+    p.inv = c.take(numel * 4);
+    Carver first = c, second = c;
+    p.q = first.take(q), p.s = first.take(s);
+    p.a2 = second.take(a2), p.a2s = second.take(a2s);
+    c.bytes = std::max(first.bytes, second.bytes);
+    first = second = c;
+    p.a1 = first.take(p.rows * H), p.a1s = first.take(p.rows * (H / 128) * 4);
+    if (p.apart) p.ic1 = first.take(p.rows * 2 * I * 2);
+    if (!p.direct) p.ic3 = second.take(p.rows * Ho * 2);
+    c.bytes = std::max(first.bytes, second.bytes);
+  }
   p.total = c.bytes;
   return p;
 }
