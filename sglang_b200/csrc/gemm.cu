@@ -1607,7 +1607,7 @@ template <int BN>
 static int grouped_mm(const void* A, const float* a_s, const void* B, const float* b_s, void* C,
                       const int32_t* sorted_token_ids, const int32_t* expert_ids, const int32_t* num_rows_dev,
                       const float* row_weights, int64_t max_rows, int64_t numel, int num_experts, int64_t N, int64_t K,
-                      int scatter, int out_dtype, bool skip_padding, cudaStream_t st) {
+                      int scatter, int out_dtype, Padding padding, cudaStream_t st) {
   CUtensorMap ma, mb, ma32;
   int rc = get_tensor_map(A, (uint64_t)K, (uint64_t)max_rows, 1, BM, 2, &ma);
   if (rc) return rc;
@@ -1618,20 +1618,20 @@ static int grouped_mm(const void* A, const float* a_s, const void* B, const floa
   GemmParams p{};
   p.a_s = a_s, p.b_s = b_s, p.C = C, p.bias = nullptr;
   p.sorted_ids = sorted_token_ids, p.expert_ids = expert_ids, p.num_rows_dev = num_rows_dev;
-  p.row_weights = scatter || skip_padding ? row_weights : nullptr;  // (elsewhere the sorted rows are the bare product, and may have no ids)
+  p.row_weights = scatter || padding != Padding::kKept ? row_weights : nullptr;  // (elsewhere the sorted rows are the bare product, and may have no ids)
   p.M = max_rows, p.N = N, p.K = K;
   p.kb_total = (int)((K + BK - 1) / BK), p.nb_total = (int)((N + kScaleBlockN - 1) / kScaleBlockN);
   p.tiles_n = (int)((N + BN - 1) / BN);
   p.group_m = choose_group_m(max_rows, K, BM);
   p.as_stride_m = p.kb_total, p.as_stride_k = 1;
-  p.numel = numel, p.scatter = scatter, p.out_fp16 = out_dtype, p.skip_padding = skip_padding;
+  p.numel = numel, p.scatter = scatter, p.out_fp16 = out_dtype, p.skip_padding = padding == Padding::kSkipped;
   p.wait_probes = g_gemm_wait_probes;
   p.full_units = 0, p.splits = 1, p.kb_per_split = p.kb_total, p.partial = nullptr;  // grouped: one unit per tile
   p.sk_pieces = 2;
   CUtensorMap mc{};
   p.tma_out = !scatter;  // sorted-row output is contiguous; the scatter form writes token-major rows one by one
   if (p.tma_out) {
-    rc = get_out_map(C, (uint64_t)N, (uint64_t)max_rows, out_dtype, skip_padding ? 32 : BM, &mc);
+    rc = get_out_map(C, (uint64_t)N, (uint64_t)max_rows, out_dtype, p.skip_padding ? 32 : BM, &mc);
     if (rc) return rc;
   }
   const int64_t tiles = ((max_rows + BM - 1) / BM) * p.tiles_n;
@@ -1731,26 +1731,26 @@ extern "C" int sglb200_fp8_blockwise_grouped_mm(const void* A, const float* a_s,
                                                 int64_t max_rows, int64_t numel, int num_experts, int64_t N, int64_t K,
                                                 int scatter, int out_dtype, void* stream) {
   return sglb200::grouped_mm_any(A, a_s, B, b_s, C, sorted_token_ids, expert_ids, num_rows_dev, row_weights, max_rows, numel,
-                                 num_experts, N, K, scatter, out_dtype, false, static_cast<cudaStream_t>(stream));
+                                 num_experts, N, K, scatter, out_dtype, Padding::kKept, static_cast<cudaStream_t>(stream));
 }
 
 int sglb200::grouped_mm_any(const void* A, const float* a_s, const void* B, const float* b_s, void* C,
                             const int32_t* sorted_token_ids, const int32_t* expert_ids, const int32_t* num_rows_dev,
                             const float* row_weights, int64_t max_rows, int64_t numel, int num_experts, int64_t N, int64_t K,
-                            int scatter, int out_dtype, bool skip_padding, cudaStream_t st) {
+                            int scatter, int out_dtype, Padding padding, cudaStream_t st) {
   SGLB_REQUIRE(max_rows >= 0 && N > 0 && K > 0 && num_experts >= 1, "grouped_mm: bad shape rows=%lld N=%lld K=%lld E=%d",
                (long long)max_rows, (long long)N, (long long)K, num_experts);
   SGLB_REQUIRE(K % 16 == 0 && N % 8 == 0, "grouped_mm: K must be a multiple of 16 and N of 8");
   SGLB_REQUIRE(out_dtype == 0 || out_dtype == 1, "grouped_mm: out_dtype %d (0 bf16, 1 fp16)", out_dtype);
   if (max_rows == 0) return SGLB200_OK;
   SGLB_REQUIRE(A && a_s && B && b_s && C && expert_ids && num_rows_dev, "grouped_mm: null pointer");
-  SGLB_REQUIRE((!scatter && !skip_padding) || sorted_token_ids, "grouped_mm: scatter mode needs sorted_token_ids");
+  SGLB_REQUIRE((!scatter && padding == Padding::kKept) || sorted_token_ids, "grouped_mm: scatter mode needs sorted_token_ids");
   SGLB_REQUIRE(aligned16(A) && aligned16(B) && aligned16(C), "grouped_mm: A, B and C must be 16-byte aligned");
   if (choose_bn_grouped(numel) == 128)
     return grouped_mm<128>(A, a_s, B, b_s, C, sorted_token_ids, expert_ids, num_rows_dev, row_weights, max_rows, numel,
-                           num_experts, N, K, scatter, out_dtype, skip_padding, st);
+                           num_experts, N, K, scatter, out_dtype, padding, st);
   return grouped_mm<256>(A, a_s, B, b_s, C, sorted_token_ids, expert_ids, num_rows_dev, row_weights, max_rows, numel,
-                         num_experts, N, K, scatter, out_dtype, skip_padding, st);
+                         num_experts, N, K, scatter, out_dtype, padding, st);
 }
 
 

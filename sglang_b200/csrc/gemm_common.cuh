@@ -72,12 +72,14 @@ int scaled_mm(const void* A, const void* B, const float* a_s, const float* b_s, 
               int64_t K, int64_t as_stride_m, int64_t as_stride_k, int out_dtype, void* workspace, int64_t workspace_bytes,
               bool after_quantizer, cudaStream_t st);
 
-// gemm.cu: the product of sorted rows with their experts (arguments as sglb200_fp8_blockwise_grouped_mm).  `skip_padding`: the
-// rows are as the sort leaves them, every expert's padding after its rows, and nobody reads what belongs to a padding row;
-// without `scatter`, `row_weights` then apply to the sorted rows.
+// gemm.cu: the product of sorted rows with their experts (arguments as sglb200_fp8_blockwise_grouped_mm).  Padding other than
+// kKept: the rows are as the sort leaves them, every expert's padding after its rows, and nobody reads what belongs to a padding
+// row; without `scatter`, `row_weights` then apply to the sorted rows.  kSkipped: 32-row quadrants of padding may hold anything
+// and are not stored.
+enum class Padding { kKept, kUnread, kSkipped };
 int grouped_mm_any(const void* A, const float* a_s, const void* B, const float* b_s, void* C, const int32_t* sorted_token_ids,
                    const int32_t* expert_ids, const int32_t* num_rows_dev, const float* row_weights, int64_t max_rows,
-                   int64_t numel, int num_experts, int64_t N, int64_t K, int scatter, int out_dtype, bool skip_padding,
+                   int64_t numel, int num_experts, int64_t N, int64_t K, int scatter, int out_dtype, Padding padding,
                    cudaStream_t st);
 // The experts' first product with activation and re-quantisation in its epilogue (see there).
 int grouped_act_mm(const void* A, const float* a_s, const void* w13, const float* b_s, void* out_q, float* out_s,

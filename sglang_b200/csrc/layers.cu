@@ -63,14 +63,22 @@ static int experts_row_tile(int64_t numel, int64_t E) {
   return 0;
 }
 
-// Whether the activation runs between the products instead of in the first one's epilogue: with a little more than one wave of
-// tiles, up to two and a half.  A tile's epilogue is a microsecond longer for it, which few tiles a CTA do not hide, and what the
-// launch reads back lies in L2 then.  Us of the layer, in the epilogue / apart (tiles as estimated here, of 148 SMs): 176 tiles 92.2 /
-// 88.3 (600 tokens, two of 8 experts of 4096 x 1408), 208 54.5 / 52.8, 256 88.5 / 86.2, 320 181.9 / 180.1, 312 66.4 / 65.7; but 64
-// 36.5 / 38.7, 80 43.3 / 44.6, 1024 145.9 / 154.2, 1248 221.3 / 232.1, 8448 1337 / 1409.
+// Tiles of a product with `tiles_n` of them beside one another, if the experts have equally many rows.
+static int64_t expert_tiles(int64_t numel, int64_t E, int64_t tiles_n) {
+  const int64_t experts = std::min(numel, E);
+  return experts * ((numel / experts + 127) / 128) * tiles_n;
+}
+
+// Whether the activation runs between the products instead of in the first one's epilogue.  A tile's epilogue is one to two
+// microseconds longer for it, which only many tiles a CTA hide; a launch of its own takes 2 us and what it writes and reads back
+// of L2, so that of one wave only the middle goes to the epilogue: fewer tiles leave SMs without a part of the work, and of more
+// some are a second round, as experts are not equal.  Us of the layer, in the epilogue / apart (tiles as estimated here, of 148
+// SMs, weights from HBM): 8 tiles 25.6 / 23.2, 16 32.9 / 29.9, 32 44.0 / 42.2, 48 35.6 / 35.9, 72 42.2 / 43.6, 88 35.1 / 36.0, 96
+// 47.2 / 45.6, 104 46.0 / 44.0, 128 116.6 / 111.2 and 36.1 / 37.7, 176 84.4 / 79.6, 256 97.3 / 93.4, 512 92.0 / 89.1 and 92.8 /
+// 87.8, 640 117.7 / 114.2, 704 124.3 / 123.4, 768 89.6 / 89.8, 1152 155.9 / 158.0, 8448 1337 / 1409.
 static bool activation_apart(int64_t numel, int64_t E, int64_t I) {
-  const int64_t experts = std::min(numel, E), tiles = experts * ((numel / experts + 127) / 128) * (I / 128), sms = sm_count();
-  return tiles > sms && 2 * tiles <= 5 * sms;
+  const int64_t tiles = expert_tiles(numel, E, I / 128), sms = sm_count();
+  return tiles <= 5 * sms && !(10 * tiles >= 3 * sms && 8 * tiles <= 5 * sms);
 }
 
 static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int64_t I, int64_t Ho, float factor) {
@@ -212,9 +220,12 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
                                    stream);
       if (rc) return rc;
     }
+    // Gathered rows have zeros for padding.  With a tile a CTA at most, tiles that are fetched and stored whole take fewer and larger
+    // copies than their quadrants: 1024 tokens to one of 8 experts of 2048 x 1024 39.4 -> 38.6 us, of 512 x 128 23.2 -> 22.8.
+    auto padding = [&](int64_t n) { return beside && expert_tiles(numel, E, (n + 255) / 256) <= sm_count() ? Padding::kUnread : Padding::kSkipped; };
     if (p.apart) {
       rc = grouped_mm_any(base + p.a1, f(p.a1s), w13, w13_s, base + p.ic1, i(p.sorted), i(p.eid), i(p.post), nullptr, p.rows, numel,
-                          (int)E, 2 * I, H, 0, dtype, true, st);
+                          (int)E, 2 * I, H, 0, dtype, padding(2 * I), st);
       if (rc) return rc;
       rc = silu_mul_quant_fp8(base + p.ic1, dtype, base + p.a2, f(p.a2s), p.rows, I, 128, kQuantEps, i(p.post), true, st);
     } else {
@@ -223,7 +234,7 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     }
     if (rc) return rc;
     rc = grouped_mm_any(base + p.a2, f(p.a2s), w2, w2_s, ic3, i(p.sorted), i(p.eid), i(p.post), topk_weights, p.rows, numel, (int)E,
-                        Ho, I, p.direct, dtype, true, st);
+                        Ho, I, p.direct, dtype, padding(Ho), st);
   }
   if (rc || p.direct) return rc;
   // (the rows kernel leaves the slots of negative ids unwritten)

@@ -148,6 +148,16 @@ def test_experts_with_the_activation_apart_equal_their_steps(T, E, topk, H, I, d
     test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd)
 
 
+# the activation in the epilogue behind the sort of up to 2048 ids, whose codes are gathered, of tiles in the middle of one wave and
+# of more than five; apart with fewer tiles and with almost one wave, behind both sorts; one slot a token among them
+@pytest.mark.parametrize("T,E,topk,H,I,dtype,odd", [
+    (250, 8, 2, 384, 768, torch.bfloat16, False), (400, 8, 2, 256, 1024, torch.float16, True), (1000, 2, 2, 128, 6400, torch.bfloat16, True),
+    (500, 8, 1, 640, 256, torch.float16, True), (1024, 4, 1, 384, 2048, torch.bfloat16, False), (2100, 8, 1, 256, 128, torch.bfloat16, True),
+    (900, 16, 2, 256, 896, torch.bfloat16, False), (1100, 4, 2, 128, 896, torch.float16, False)])
+def test_experts_where_the_activation_moves_equal_their_steps(T, E, topk, H, I, dtype, odd):
+    test_experts_equal_their_steps(T, E, topk, H, I, dtype, odd)
+
+
 # more tiles of the first product than CTAs, behind the sort of up to 2048 ids and of more; experts without rows among them
 @pytest.mark.parametrize("T,E,topk", [(40, 64, 2), (700, 96, 3)])
 def test_experts_many_tiles(T, E, topk):
