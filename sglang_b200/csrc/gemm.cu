@@ -1433,10 +1433,10 @@ int choose_group_m(int64_t rows, int64_t K, int tile_rows) {
 // split or run stream-K over all SMs, with the quantizer: 128 x 10240 x 8192 29.3 -> 24.4 us, 80 x 18432 x 7168 35.1 -> 28.9, 128 x
 // 16384 x 8192 37.7 -> 32.0, 256 x 7168 x 16384 46.0 -> 44.0.  Else 256 columns where that splits K (stream-K, split tiles); else
 // compared as waves x tile width, the 128-wide tile charged 156 instead of 128 (it takes 0.61 of a wide tile's time).
-static bool one_narrow_wave(int64_t M, int64_t N) { return ((M + BM - 1) / BM) * ((N + 127) / 128) <= sm_count(); }
-static int choose_bn(int64_t M, int64_t N, int64_t K) {
-  if (one_narrow_wave(M, N)) return 128;
-  const int sms = sm_count();
+// `sms`: those that the launch may use.
+static bool one_narrow_wave(int64_t M, int64_t N, int sms) { return ((M + BM - 1) / BM) * ((N + 127) / 128) <= sms; }
+static int choose_bn(int64_t M, int64_t N, int64_t K, int sms) {
+  if (one_narrow_wave(M, N, sms)) return 128;
   if (plan_units(M, N, K, 256, sms).scratch_blocks() > 0) return 256;
   const int64_t tiles_m = (M + BM - 1) / BM;
   const int64_t waves256 = (tiles_m * ((N + 255) / 256) + sms - 1) / sms;
@@ -1458,11 +1458,12 @@ struct DensePlan {
 };
 static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
   DensePlan d;
+  const int sms = sm_count();
   d.cluster = tile_splits(((M + BM - 1) / BM) * ((N + 127) / 128), (int)((K + BK - 1) / BK), M, cluster_fits());
-  d.bn = d.cluster > 1 ? 128 : choose_bn(M, N, K);
+  d.bn = d.cluster > 1 ? 128 : choose_bn(M, N, K, sms);
   // (one wave of 128-wide tiles is not cut in units of its own)
-  if (one_narrow_wave(M, N)) d.units = UnitPlan{(int)(((M + BM - 1) / BM) * ((N + 127) / 128)), 1, (int)((K + BK - 1) / BK), 0, 0, 0, 2};
-  else d.units = plan_units(M, N, K, d.bn, sm_count());
+  if (one_narrow_wave(M, N, sms)) d.units = UnitPlan{(int)(((M + BM - 1) / BM) * ((N + 127) / 128)), 1, (int)((K + BK - 1) / BK), 0, 0, 0, 2};
+  else d.units = plan_units(M, N, K, d.bn, sms);
   return d;
 }
 
@@ -1871,7 +1872,7 @@ extern "C" int sglb200_fp8_blockwise_scaled_mm_push(const void* A, const void* B
   SGLB_REQUIRE(aligned16(A) && aligned16(B), "mm_push: A and B must be 16-byte aligned");
   SGLB_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "mm_push: dimension too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (choose_bn(M, N, K) == 128)
+  if (choose_bn(M, N, K, sm_count() - sm_margin) == 128)
     return push_mm<128>(A, B, a_s, b_s, stage_ptrs, world, rank, M, N, K, as_stride_m, as_stride_k, out_dtype, sm_margin, st);
   return push_mm<256>(A, B, a_s, b_s, stage_ptrs, world, rank, M, N, K, as_stride_m, as_stride_k, out_dtype, sm_margin, st);
 }

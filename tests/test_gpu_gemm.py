@@ -2,6 +2,7 @@
 
 Tolerance (from the path's specification): rtol 1e-2, atol 1e-2 and cosine >= 0.9999 against the
 dequantised float32 reference computed by the oracle."""
+import ctypes
 import os
 
 import numpy as np
@@ -224,6 +225,28 @@ def test_grouped_gemm_with_rows_that_do_not_fill_the_last_tile(ops, scatter, E=3
             ref[t if scatter else r] = ((a[r].float() * w[e].float()).view(N, H // 128, 128).sum(-1) * s).sum(-1).cpu()
     assert ops.gemm_status() == 0
     assert_close_fp(to_f32_np(out), ref.numpy())
+
+
+# 140 tiles of 128 columns: one wave of all SMs, but not of those that a margin of 20 leaves
+def test_push_with_sms_left_free(ops, M=200, N=8960, K=640):
+    """The product in push mode, to two owners that are both on this GPU: with the narrow and with the wide tiles the same bits."""
+    from sglang_b200._lib import check, lib
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, a_s = ops.per_token_group_quant_fp8(torch.randn(M, K, device="cuda", generator=g).bfloat16(), 128)
+    w = (torch.randn(N, K, device="cuda", generator=g) * 50).clamp(-448, 448).to(torch.float8_e4m3fn)
+    ws = torch.rand(N // 128, K // 128, device="cuda", generator=g) * 1e-3
+    outs = []
+    for margin in (0, 20):
+        stage = torch.zeros(2, 2, 128, N, device="cuda", dtype=torch.bfloat16)  # owner, rank, row
+        ptrs = (ctypes.c_void_p * 2)(stage[0].data_ptr(), stage[1].data_ptr())
+        check(lib.sglb200_fp8_blockwise_scaled_mm_push(a.data_ptr(), w.data_ptr(), a_s.data_ptr(), ws.data_ptr(), ptrs, 2, 1, M, N, K,
+                                                       a_s.stride(0), a_s.stride(1), 0, margin, torch.cuda.current_stream().cuda_stream))
+        assert not stage[:, 0].any()
+        outs.append(torch.cat([stage[0, 1], stage[1, 1, :M - 128]]))
+    wide = torch.repeat_interleave(torch.repeat_interleave(ws, 128, 0), 128, 1) * w.float()
+    ref = (torch.repeat_interleave(a_s, 128, 1) * a.float()).double() @ wide.double().T
+    assert ops.gemm_status() == 0 and torch.equal(outs[0], outs[1])
+    assert_close_fp(to_f32_np(outs[0]), ref.float().cpu().numpy())
 
 
 def test_fused_experts_all_ids_filtered(ops):

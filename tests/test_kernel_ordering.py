@@ -71,3 +71,12 @@ def test_activation_scales_are_read_of_rows_that_exist():
     assert len(reads) == 1 and gemm.count("load_a4_row(") == 1 and set(re.findall(r"\brow\w*", reads[0])) == {"row"}
     rows = re.findall(r"const int row = (.*);\s+av\[k\] = load_a4_row", gemm)
     assert len(rows) == 1 and re.fullmatch(r"min\(.*, \(int\)p\.M - 1\)", rows[0])
+
+
+def test_the_tile_width_is_chosen_for_the_sms_of_the_launch():
+    """One wave of narrow tiles is one of the SMs that the launch may use; a product in push mode leaves some to other kernels."""
+    gemm = _code("gemm.cu")
+    push = gemm[gemm.index("int sglb200_fp8_blockwise_scaled_mm_push("):]
+    assert re.findall(r"choose_bn\((.*?)\) ==", push) == ["M, N, K, sm_count() - sm_margin"]
+    rule = gemm[gemm.index("static bool one_narrow_wave("):gemm.index("static int choose_bn_grouped(")]
+    assert "int sms)" in rule and "sm_count()" not in rule
