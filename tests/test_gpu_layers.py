@@ -74,6 +74,13 @@ def test_linear_after_its_weights_were_written(M, N, K):
         assert torch.equal(out, want[i % 2])
 
 
+# more than 64 rows: split over a cluster, a single wave of 128- and of 256-wide tiles, equal runs of slabs, and the kernel with
+# the weights on the M side, all of which ask for their first weights while the quantizer runs
+@pytest.mark.parametrize("M,N,K", [(128, 4096, 7168), (200, 8192, 4096), (257, 10240, 8192), (620, 3832, 16384), (128, 512, 7168)])
+def test_linear_of_many_rows_after_its_weights_were_written(M, N, K):
+    test_linear_after_its_weights_were_written(M, N, K)
+
+
 # (tokens, experts, topk): on average 1 to some hundred rows per expert, so that every tile height of the dispatch is taken;
 # the ids are skewed towards expert 0 and leave some experts without rows
 @pytest.mark.parametrize("T,E,topk", [(1, 8, 8), (5, 32, 2), (16, 8, 1), (40, 16, 4), (70, 6, 3), (160, 8, 2), (333, 4, 2)])
