@@ -1,5 +1,5 @@
-// Over how many CTAs of a thread-block cluster the kernels with the weights on the M side split K (gemm_rows.cu,
-// gemm_small.cu).  Plain C++ without CUDA: what a GPU holds comes in as counts, so that the rules can be tested for any.
+// Over how many CTAs of a thread-block cluster K is split: by the kernels with the weights on the M side (gemm_rows.cu,
+// gemm_small.cu) and by the 128-row kernel (gemm.cu).  Plain C++ without CUDA: what a GPU holds comes in as counts, so that the rules can be tested for any.
 #pragma once
 #include <stdint.h>
 

@@ -35,9 +35,9 @@
 // Scheduling: one wave of 128-wide tiles is taken as it is, or, with few tiles and a long K, split over clusters.  With more, but
 // fewer than two waves of 256-wide tiles and a long K, the tiles x slabs space is cut into one equal run of slabs per SM
 // (stream-K; a run covers the end of one tile, possibly a whole tile, and the start of the next); otherwise the tiles of a short
-// last wave are split along K.  Both write float32 partial sums that a second kernel adds in ascending K order.  In push mode (row-parallel layers under tensor parallelism) a tile is
-// stored through the tensor map of the staging buffer of the GPU that owns its rows, which folds the
-// reduce-scatter of the all-reduce into the epilogue.
+// last wave are split along K.  Both write float32 partial sums that a second kernel adds in ascending K order.  In push mode
+// (row-parallel layers under tensor parallelism) a tile is stored through the tensor map of the staging buffer of the GPU that
+// owns its rows, which folds the reduce-scatter of the all-reduce into the epilogue.
 //
 // Every mbarrier wait is bounded; on expiry the role raises a flag in shared memory and leaves its loops, the other
 // roles sit out their own limits, the CTA sets a status word, drains, frees its TMEM and returns
@@ -218,19 +218,21 @@ struct TileCoord {
   int m_tile, n_tile, expert;
 };
 
-// Leading 32-row quadrants of a tile that hold rows.  An expert's rows come first and its padding last, and a tile has a row.
+// Leading 32-row quadrants of a tile that hold rows, by the first ids of the second to the fourth.  An expert's rows come first and
+// its padding last, and a tile has a row.
+__device__ __forceinline__ int live_quadrants(const GemmParams& p, int id1, int id2, int id3) {
+  return 1 + (id1 < p.numel) + (id2 < p.numel) + (id3 < p.numel);
+}
 __device__ __forceinline__ int live_quadrants(const GemmParams& p, int m_tile) {
   const int32_t* id = p.sorted_ids + (int64_t)m_tile * BM;
-  const int a = id[32], b = id[64], c = id[96];
-  return 1 + (a < p.numel) + (b < p.numel) + (c < p.numel);
+  return live_quadrants(p, id[32], id[64], id[96]);
 }
 
 // Where a unit lies, and what its tile's rows are: looked up a unit ahead by the roles that must not stall between two tiles.
 // The ids stay as they came from memory until the tile is begun, so that nothing waits for them before.
 struct TileInfo {
   int m_tile, n_tile, expert, id1, id2, id3;
-  // Leading 32-row quadrants that hold rows.  An expert's rows come first and its padding last, and a tile has a row.
-  __device__ __forceinline__ int live(const GemmParams& p) const { return 1 + (id1 < p.numel) + (id2 < p.numel) + (id3 < p.numel); }
+  __device__ __forceinline__ int live(const GemmParams& p) const { return live_quadrants(p, id1, id2, id3); }
 };
 template <bool kGrouped>
 __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int tile, int tiles_m, int tiles_n) {

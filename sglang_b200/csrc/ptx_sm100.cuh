@@ -228,12 +228,6 @@ __device__ __forceinline__ float2 lds_f32x2(uint32_t addr) {
   asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
   return v;
 }
-// 32 bytes to global memory (a whole sector; 32-byte aligned).
-__device__ __forceinline__ void stg_256(void* p, const uint32_t (&v)[4][2]) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0][0]), "r"(v[0][1]), "r"(v[1][0]),
-               "r"(v[1][1]), "r"(v[2][0]), "r"(v[2][1]), "r"(v[3][0]), "r"(v[3][1])
-               : "memory");
-}
 
 // ---- thread-block clusters (partial sums of a split K, exchanged through distributed shared memory) --------------
 __device__ __forceinline__ void cluster_sync() {

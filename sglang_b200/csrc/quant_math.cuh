@@ -151,7 +151,7 @@ __device__ __forceinline__ void quant_chunk_fast(const uint4& raw, const float* 
 //
 // The contract is code = e4m3(min(max(RN(x / scale), qmin), qmax)) with an IEEE float32 division.  A
 // div.rn.f32 costs about ten instructions per element, which makes the kernel issue-bound, so the quotient
-// is formed without dividing: with r = RN(1/scale) computed once per group,
+// is formed without dividing (one step of Markstein's correction by the exact residual): with r = RN(1/scale) once per group,
 //     q0 = RN(x*r);  e = fma(-q0, scale, x) (exact residual);  q = fma(e, r, q0);  q = copysign(q, x)
 // equals RN(x / scale) bit for bit whenever |q| >= 2^-20 (checked exhaustively for every bf16 / fp16 input
 // pair and on ~1e8 random float32 pairs by tests/exact_div_check.c); smaller quotients may differ in float32
