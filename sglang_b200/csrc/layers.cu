@@ -92,11 +92,12 @@ static ExpertsPlan experts_plan(int64_t T, int64_t k, int64_t E, int64_t H, int6
   p.sort_bytes = sglb200_moe_align_workspace_bytes(numel, (int)E + 1);
   p.apart = p.tile == 0 && activation_apart(numel, E, I);
   Carver c;
+  const int64_t q = T * H, s = T * (H / 128) * 4, a2 = p.rows * I, a2s = p.rows * (I / 128) * 4;
+  // (codes and scales first: behind the small parts, four tokens to eight of 128 experts of 2048 x 768 46.7 -> 47.8 us)
+  if (p.tile > 0) p.q = c.take(q), p.s = c.take(s);
   p.sorted = c.take(p.cap * 4), p.eid = c.take((p.cap + p.block - 1) / p.block * 4), p.post = c.take(4), p.next = c.take(8);
   p.cum = c.take((E + 2) * 4), p.sort = c.take(p.sort_bytes);
-  const int64_t q = T * H, s = T * (H / 128) * 4, a2 = p.rows * I, a2s = p.rows * (I / 128) * 4;
   if (p.tile > 0) {
-    p.q = c.take(q), p.s = c.take(s);
     p.ic1 = c.take(p.rows * 2 * I * 2);
     p.a2 = c.take(a2), p.a2s = c.take(a2s);
     if (!p.direct) p.ic3 = c.take(numel * Ho * 2);
