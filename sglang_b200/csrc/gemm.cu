@@ -1476,9 +1476,11 @@ static DensePlan plan_dense(int64_t M, int64_t N, int64_t K) {
 // 128-row tiles split over clusters), 1024 x 4096 9.5 / 14.3 (10.5), 2048 x 1024 7.7 / 8.0 (9.1); 256 rows, 512 x 2048 7.9 / 9.5
 // (9.3), 1024 x 7168 12.8 / 20.7 (12.7).  Not beyond: 128 rows, 3072 x 2048 10.8 / 10.3; 192 rows, 2048 x 7168 15.2 (13.8).  With
 // a long K the clusters of 128-row tiles fetch less: 128 rows, 1024 x 16384 15.8 (14.7), 512 x 16384 12.8 (13.5).
-static bool use_rows(int64_t M, int64_t N, int64_t K) {
+// A product whose activations are codes already, which has no quantizer to fetch the first weights under, gains from a K above 1024
+// only: 128 rows, 512 x 512 5.6 / 5.0, 1024 x 1024 6.4 / 6.0, 512 x 2048 6.3 / 7.8.
+static bool use_rows(int64_t M, int64_t N, int64_t K, bool after_quantizer) {
   const int64_t tiles = ((M + 63) / 64) * ((N + 127) / 128);
-  return M <= 64 || (M <= 256 && tiles <= (K <= 8192 ? 32 : 8));
+  return M <= 64 || (M <= 256 && tiles <= (K <= 8192 ? 32 : 8) && (after_quantizer || K > 1024));
 }
 
 uint32_t g_gemm_wait_probes = ptx::kProbeLimit;
@@ -1693,7 +1695,7 @@ extern "C" int sglb200_gemm_status(void) {
 extern "C" void sglb200_gemm_set_wait_probes(uint32_t probes) { g_gemm_wait_probes = probes == 0 ? ptx::kProbeLimit : probes; }
 
 extern "C" int64_t sglb200_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0 || use_rows(M, N, K)) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || use_rows(M, N, K, true)) return 0;  // (what a plain product of such a size takes needs none)
   return plan_dense(M, N, K).scratch_bytes();
 }
 
@@ -1718,7 +1720,7 @@ int sglb200::scaled_mm(const void* A, const void* B, const float* a_s, const flo
   SGLB_REQUIRE(aligned16(A) && aligned16(B) && aligned16(C) && (bias == nullptr || aligned16(bias)),
                "fp8_blockwise_scaled_mm: A, B, C and bias must be 16-byte aligned");
   SGLB_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "fp8_blockwise_scaled_mm: dimension too large");
-  if (use_rows(M, N, K))
+  if (use_rows(M, N, K, after_quantizer))
     return rows_dense_mm(A, B, a_s, b_s, C, bias, M, N, K, as_stride_m, as_stride_k, out_dtype, after_quantizer, st);
   const DensePlan dp = plan_dense(M, N, K);
   if (dp.bn == 128)
