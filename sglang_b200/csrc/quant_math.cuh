@@ -124,14 +124,22 @@ __device__ __forceinline__ void quotient2(float x0, float x1, float scale, float
 // division-free quotient is exact (see quant_chunk_careful).  With the standard range no clamp is needed: a quotient can
 // exceed 448 only by rounding and the conversion saturates; the sign of a zero quotient is taken from the
 // input bits (it is the only case in which the computed sign can differ from the numerator's).
-template <typename T, bool kStdRange>
+template <typename T, bool kStdRange, bool kPairs = true>
 __device__ __forceinline__ void quant_chunk_fast(const uint4& raw, const float* v, float scale, float r, float qmin,
                                                  float qmax, uint32_t* codes) {
   constexpr int CE = Chunk<T>::kElems;
   float q[CE];
 #pragma unroll
   for (int i = 0; i < CE; i += 2) {
-    quotient2(v[i], v[i + 1], scale, r, q[i], q[i + 1]);
+    if (kPairs) {
+      quotient2(v[i], v[i + 1], scale, r, q[i], q[i + 1]);
+    } else {
+#pragma unroll
+      for (int j = i; j < i + 2; ++j) {
+        const float q0 = __fmul_rn(v[j], r);
+        q[j] = __fmaf_rn(__fmaf_rn(-q0, scale, v[j]), r, q0);
+      }
+    }
     if (!kStdRange) {
       q[i] = fminf(fmaxf(copysignf(q[i], v[i]), qmin), qmax);
       q[i + 1] = fminf(fmaxf(copysignf(q[i + 1], v[i + 1]), qmin), qmax);
@@ -196,7 +204,7 @@ __device__ __forceinline__ float quant_group(const uint4* raw, const float* v, f
   if (m < __int_as_float(0x7f800000) && scale >= 1e-30f && scale <= 1e36f) {
     const float r = __frcp_rn(scale);
 #pragma unroll
-    for (int j = 0; j < NCH; ++j) quant_chunk_fast<T, kStdRange>(raw[j], v + j * CE, scale, r, qmin, qmax, codes[j]);
+    for (int j = 0; j < NCH; ++j) quant_chunk_fast<T, kStdRange, (LPG >= 4)>(raw[j], v + j * CE, scale, r, qmin, qmax, codes[j]);
   } else {
     // a NaN or an infinity in the group, or an extreme scale: the reference's maximum ignores NaNs
     const unsigned lane = threadIdx.x & 31u;
