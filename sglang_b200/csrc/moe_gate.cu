@@ -7,8 +7,9 @@
 // so that a group's two largest scores come from the lanes' registers and a few shuffles instead of a serial walk
 // through shared memory (64 x 256 scores: 12.7 us with the walk).  The picks stay in registers, their weights in shared memory,
 // and both leave in one store each: written pick by pick and read back for the normalisation, with the scores loaded four bytes
-// at a time and a division an expert for its group, the fused gate took 5.3 us for one row of 256 experts (4.0 so), 6.0 for 64
-// (4.6), 15.1 for 4096 (12.0); the softmax gate, which is short of issue slots (16384 x 128 14.1 us), hardly changed.
+// at a time and a division an expert for its group, the fused gate took 5.4 us for one row of 256 experts (3.8 so), 6.1 for 64
+// (4.4), 30.5 for 16384 (24.5); the softmax gate 2.8 for one row of 128 experts, best eight (2.6), 14.6 for 16384 (14.0), which is
+// short of issue slots; best 40 of 256 of 16384 rows 72.7 (75.3).
 #include <cfloat>
 
 #include "common.cuh"
@@ -38,18 +39,21 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // Picks the k best of sel[] (kPerLane registers per lane, the expert of register j being index(j), ascending in j) and writes their
-// ids to out_i and what finish(weight(expert), sum of the k weights) gives to out_w, lane p the p-th pick of every 32; `weight` is
-// asked by that lane alone.  A pick keeps the winner's expert in a register of lane p; weights and ids leave once, together.
+// ids to out_i and what finish(weight(expert), sum of the k weights) gives to out_w, lane p the p-th pick of every 32.  Every lane asks
+// for every weight, beside the next pick, which does not wait for it.  (Asked by lane p alone and added up behind the last pick, with
+// the winner found by a vote and a shuffle: one row of 64, best 40 7.3 us for 5.5, 16384 rows 40.6 for 37.9.)  Pick p stays in
+// registers of lane p; weights and ids leave once, together.
 template <int kPerLane, class Index, class Weight, class Finish>
 __device__ __forceinline__ float pick_topk(float (&sel)[kPerLane], Index index, Weight weight, int lane, int k, float* out_w,
                                            int32_t* out_i, Finish finish) {
-  float best;  // this lane's best entry: value (never a NaN) and register (-1: nothing above -inf left)
-  int best_j;
+  float best;  // this lane's best entry: value (never a NaN), expert (INT_MAX: nothing above -inf left) and register
+  int best_e, best_j;
   auto look = [&]() {
     best = kNegInf, best_j = -1;
 #pragma unroll
     for (int j = 0; j < kPerLane; ++j)
       if (sel[j] > best) best = sel[j], best_j = j;  // ascending j = ascending expert within the lane: the first hit keeps the lower index
+    best_e = best_j < 0 ? INT_MAX : index(best_j);
   };
   look();
   float sum = 0.f, mine_w = 0.f;
@@ -58,26 +62,20 @@ __device__ __forceinline__ float pick_topk(float (&sel)[kPerLane], Index index, 
     const int count = min(k - first, 32);
     for (int pick = 0; pick < count; ++pick) {
       const uint32_t key = ordered_bits(best), top = __reduce_max_sync(0xffffffffu, key);
-      const bool wins = key == top && best_j >= 0;
-      const uint32_t who = __ballot_sync(0xffffffffu, wins);
-      // fewer candidates than k: every remaining value is -inf, and expert 0 with its weight is reported again
-      int e = 0;
-      if (who != 0) {
-        const int e_lane = index(best_j);
-        // (equal values in several lanes: the lowest expert)
-        e = (who & (who - 1)) == 0 ? __shfl_sync(0xffffffffu, e_lane, __ffs(who) - 1)
-                                   : __reduce_min_sync(0xffffffffu, wins ? e_lane : INT_MAX);
-        if (wins && e_lane == e) {
+      // (equal values in several lanes: the lowest expert)
+      int e = __reduce_min_sync(0xffffffffu, key == top ? best_e : INT_MAX);
+      if (e == INT_MAX) {
+        e = 0;  // fewer candidates than k: every remaining value is -inf, and expert 0 with its weight is reported again
+      } else if (best_e == e) {
 #pragma unroll
-          for (int j = 0; j < kPerLane; ++j)
-            if (j == best_j) sel[j] = kNegInf;
-          look();
-        }
+        for (int j = 0; j < kPerLane; ++j)
+          if (j == best_j) sel[j] = kNegInf;
+        look();
       }
-      if (lane == pick) mine_e = e;
+      const float w = weight(e);
+      sum += w;  // in the order of the picks, the same in every lane
+      if (lane == pick) mine_e = e, mine_w = w;
     }
-    if (lane < count) mine_w = weight(mine_e);
-    for (int p = 0; p < count; ++p) sum += __shfl_sync(0xffffffffu, mine_w, p);  // in the order of the picks, the same in every lane
     if (k > 32 && lane < count) out_w[first + lane] = mine_w, out_i[first + lane] = mine_e;
   }
   if (k <= 32) {
@@ -100,6 +98,8 @@ __global__ void __launch_bounds__(kGateWarps * 32)
   ptx::grid_dependency_wait();
   if (row >= rows) return;
   const T* x = gating + row * E;
+  extern __shared__ float gate_smem[];  // per warp: E values
+  float* kept = gate_smem + (threadIdx.x >> 5) * E;  // the row's weights, for the picks
   float sel[kPerLane];
 #pragma unroll
   for (int j = 0; j < kPerLane; ++j) {
@@ -112,7 +112,9 @@ __global__ void __launch_bounds__(kGateWarps * 32)
         if (bias != nullptr) v += bias[e];
       } else {
         v = 1.0f / (1.0f + expf(-v));
-        if (bias != nullptr) v += bias[e];
+        const float b = bias != nullptr ? bias[e] : 0.f;
+        v += b;
+        kept[e] = v - b;
       }
     }
     sel[j] = v;
@@ -130,18 +132,15 @@ __global__ void __launch_bounds__(kGateWarps * 32)
     }
     const float inv = 1.f / warp_sum(s);
 #pragma unroll
-    for (int j = 0; j < kPerLane; ++j) sel[j] = (j * 32 + lane < E) ? sel[j] * inv : kNegInf;
+    for (int j = 0; j < kPerLane; ++j) {
+      const int e = j * 32 + lane;
+      sel[j] = e < E ? sel[j] * inv : kNegInf;
+      if (e < E) kept[e] = sel[j];
+    }
   }
-  // the row's values once more, for the weights of the picks
-  extern __shared__ float gate_smem[];  // per warp: E values
-  float* kept = gate_smem + (threadIdx.x >> 5) * E;
-#pragma unroll
-  for (int j = 0; j < kPerLane; ++j)
-    if (j * 32 + lane < E) kept[j * 32 + lane] = sel[j];
   __syncwarp();
   pick_topk<kPerLane>(
-      sel, [&](int j) { return j * 32 + lane; },
-      [&](int e) { return kMode == 1 && bias != nullptr ? kept[e] - bias[e] : kept[e]; }, lane, k, out_w + row * k, out_i + row * k,
+      sel, [&](int j) { return j * 32 + lane; }, [&](int e) { return kept[e]; }, lane, k, out_w + row * k, out_i + row * k,
       [&](float w, float sum) { return renormalize ? w * (1.f / sum) : w; });
 }
 
