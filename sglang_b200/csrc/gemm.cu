@@ -95,8 +95,10 @@ __device__ long long g_trace[2][kTraceUnits][kTraceStamps];
 // wave takes 1 100 clocks, most of them the way from DRAM and L2 to shared memory (of many waves 850: other rows' CTAs have
 // brought the weights), so it is bytes in flight that count.  Us with the quantizer, ring of three stages -> four, both in turn
 // on one GPU: 257 x 10240 x 8192 47.6 -> 44.9, 512 x 7168 x 16384 86.3 -> 82.1, 192 x 10240 x 8192 40.8 -> 38.2.
-// Shorter K pays with the early weights below, from 12 slabs and 32 CTAs on: 128 x 24576 x 1536 14.5 -> 14.1, 128 x 9216 x 2048
-// 11.4 -> 11.1; 128 x 3072 x 2048 (24 CTAs) 10.3 -> 10.5, 128 x 4096 x 512 7.1 -> 7.3.
+// Shorter K pays with the early weights below, from 12 slabs and 32 CTAs on, 96 where there are more than 128 rows and the CTAs of
+// one column ask for the same weights: 128 x 24576 x 1536 14.5 -> 14.1, 128 x 9216 x 2048 11.0 -> 10.6, 128 x 6144 x 2048 10.1 -> 9.9,
+// 256 x 7168 x 2048 (112 CTAs) 11.3 -> 11.0, 900 x 2048 x 2048 (128) 11.6 -> 11.3; not 128 x 3072 x 2048 (24) 10.3 -> 10.5, 128 x 4096 x
+// 512 7.1 -> 7.3, 160 x 3072 x 1536 (48) 8.7 -> 8.8, 192 x 4096 x 2048 (64) 9.8 -> 10.1, 384 x 3072 x 1536 (72) 9.1 -> 9.5.
 // kSplit: a dense product of few 128-wide tiles and a long K, whose slabs are split over the CTAs of a cluster (`tile_splits`); their
 // partial sums meet in distributed shared memory (written once, added once) instead of in global memory and a second launch.
 // Beside the ring of five stages lies room for what the other CTAs send; sums fetched from the others' memory after a barrier,
@@ -1568,7 +1570,7 @@ static int dense_mm(const DensePlan& dp, const void* A, const void* B, const flo
     if (rc) return rc;
   }
   const int64_t units = pl.sk_share > 0 ? pl.sk_ctas : pl.full_units + pl.split_tiles * pl.splits;
-  const bool once = p.kb_total >= (units >= 32 ? 12 : 32) && (!p.tma_out || units <= sm_count());
+  const bool once = p.kb_total >= (units >= (M <= BM ? 32 : 96) ? 12 : 32) && (!p.tma_out || units <= sm_count());
   rc = once ? launch_gemm<Form::kOnce, BN>(ma, mb, mc, ma, p, units, st) : launch_gemm<Form::kDense, BN>(ma, mb, mc, ma, p, units, st);
   if (rc != SGLB200_OK || pl.scratch_blocks() == 0) return rc;
   const int tiles_m = (int)((M + BM - 1) / BM);
