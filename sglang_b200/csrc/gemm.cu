@@ -28,7 +28,7 @@
 // the promotion loop unrolled by four, so that buffers, barriers and scales are compile-time (its bookkeeping was a chain
 // of dependent instructions as long as the FMAs).  Keeping one TMEM load in flight across the FMAs, chunk by chunk, was
 // slower (1250): every extra wait for a load costs more than the overlap gives.  ptxas spills at 168 registers a thread: 4
-// to 16 bytes of stores in the dense instances, 56 with experts, 248 where the epilogue activates.
+// to 16 bytes of stores in the dense instances, 60 with experts, 248 where the epilogue activates.
 // The epilogue rounds to bf16/fp16, parks the tile in swizzled shared memory, from where TMA stores drain it
 // during the next tile; in grouped "scatter" mode it multiplies by the routing weight, parks likewise and writes 128
 // contiguous bytes at a time to the token-major row named by sorted_token_ids.
