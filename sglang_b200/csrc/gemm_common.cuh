@@ -46,8 +46,8 @@ int sum_sorted(const void* src, const int32_t* inverse, void* out, int dtype, in
 
 // quant.cu: the quantizer (groups of 128) of a layer's activations with every row's codes and scales written to its `topk`
 // places in the sorted order (`inverse` of the sort, -1 = nowhere), and zeros to the padding rows of 32-row quadrants that
-// hold rows; other padding is not written.  `starts`: the first row of each of the
-// sort's `buckets`, which take whole blocks of 128 rows, and the end.
+// hold rows; other padding is not written.  `starts`: the first row of each of the sort's `buckets`, which take whole blocks of
+// 128 rows, and the end.
 int quant_sorted(const void* x, int dtype, void* out_q, float* out_s, const int32_t* inverse, const int32_t* sorted_ids,
                  const int32_t* starts, int buckets, int64_t tokens, int topk, int64_t hidden, float eps, cudaStream_t st);
 

@@ -72,7 +72,7 @@ static int64_t expert_tiles(int64_t numel, int64_t E, int64_t tiles_n) {
 // Whether the activation runs between the products instead of in the first one's epilogue.  A tile's epilogue is one to two
 // microseconds longer for it, which only many tiles a CTA hide; a launch of its own takes 2 us and what it writes and reads back
 // of L2, so that of one wave only the middle goes to the epilogue: fewer tiles leave SMs without a part of the work, and of more
-// some are a second round, as experts are not equal.  Us of the layer, in the epilogue / apart (tiles as estimated here, of 148
+// some are a second wave, as experts are not equal.  Us of the layer, in the epilogue / apart (tiles as estimated here, of 148
 // SMs, weights from HBM): 8 tiles 25.6 / 23.2, 16 32.9 / 29.9, 32 44.0 / 42.2, 48 35.6 / 35.9, 72 42.2 / 43.6, 88 35.1 / 36.0, 96
 // 47.2 / 45.6, 104 46.0 / 44.0, 128 116.6 / 111.2 and 36.1 / 37.7, 176 84.4 / 79.6, 256 97.3 / 93.4, 512 92.0 / 89.1 and 92.8 /
 // 87.8, 640 117.7 / 114.2, 704 124.3 / 123.4, 768 89.6 / 89.8, 1152 155.9 / 158.0, 8448 1337 / 1409.
@@ -223,7 +223,9 @@ extern "C" int sglb200_fused_experts(const void* x, int dtype, const void* w13, 
     }
     // Gathered rows have zeros for padding.  With a tile a CTA at most, tiles that are fetched and stored whole take fewer and larger
     // copies than their quadrants: 1024 tokens to one of 8 experts of 2048 x 1024 39.4 -> 38.6 us, of 512 x 128 23.2 -> 22.8.
-    auto padding = [&](int64_t n) { return beside && expert_tiles(numel, E, (n + 255) / 256) <= sm_count() ? Padding::kUnread : Padding::kSkipped; };
+    auto padding = [&](int64_t n) {
+      return beside && expert_tiles(numel, E, (n + 255) / 256) <= sm_count() ? Padding::kUnread : Padding::kSkipped;
+    };
     if (p.apart) {
       rc = grouped_mm_any(base + p.a1, f(p.a1s), w13, w13_s, base + p.ic1, i(p.sorted), i(p.eid), i(p.post), nullptr, p.rows, numel,
                           (int)E, 2 * I, H, 0, dtype, padding(2 * I), st);
